@@ -36,21 +36,36 @@ struct Workspace {
   int nms_strips = 0;
 };
 
+// Device tables of a launch over several frames: frame records, tile prefixes
+// and, for batches, the matching jobs, in one allocation filled by one copy.
 struct BatchSlot {
-  Frame* d_frames = nullptr;
-  int* d_bases = nullptr;  // 3 * (cap + 1)
-  unsigned int* d_ticket = nullptr;
+  uint8_t* d_tables = nullptr;
   uint8_t* h_stage = nullptr;  // pinned staging for the upload
-  int cap = 0;
+  size_t cap = 0;              // bytes of both
+  unsigned int* d_ticket = nullptr;
   cudaEvent_t uploaded = nullptr;
-  std::vector<uint8_t> last;
+  std::vector<uint8_t> last;   // content of the last upload
 };
 
+// A launch sequence with the parameters baked into it as `key`.  Capturing and
+// instantiating a graph costs the host 60 to 100 us, more than issuing its
+// launches (about 3 us each), and pays only when the same buffers come again:
+// a call whose key is not the previous call's is issued launch by launch, the
+// next call with the same key captures the graph, and later ones replay it.
 struct PairGraph {
-  bool valid = false;
-  std::vector<uint8_t> key;
+  std::vector<uint8_t> key;  // of the last call
+  cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  cudaGraphNode_t copy_node[2] = {nullptr, nullptr};  // orbx_pair_host: the image copies and their sources
+  const void* copy_src[2] = {nullptr, nullptr};
   MatchWork mw{};
+  void drop() {
+    if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
+    exec = nullptr;
+    graph = nullptr;
+    key.clear();
+  }
 };
 
 // Device tables of one persistent launch (orbx_persist.cu), reused while
@@ -61,9 +76,14 @@ struct PersistBufs {
   int* done = nullptr;       // [4 * frames + 1 + frames]: stage counters, item counter, upload flags
   MatchJob* jobs = nullptr;
   PersistRows* rows = nullptr;  // [frames] row-counter offsets (row-level dependencies)
+  MatchJob* h_jobs = nullptr;   // pinned staging of jobs
+  cudaEvent_t jobs_sent = nullptr;
   size_t items_cap = 0, frames_cap = 0, jobs_cap = 0, done_cap = 0;
-  size_t done_ints = 0;       // counters to clear before each launch
-  std::vector<uint8_t> last;  // content of the last upload
+  size_t n_items = 0;
+  int n_rows = 0;
+  size_t done_ints = 0;          // counters to clear before each launch
+  std::vector<int> layout;       // frame sizes and launch shapes the item tables were built for
+  std::vector<MatchJob> last_jobs;  // content of the last upload of jobs
 };
 
 static void persist_free(PersistBufs& pb) {
@@ -72,6 +92,8 @@ static void persist_free(PersistBufs& pb) {
   cudaFree(pb.done);
   cudaFree(pb.jobs);
   cudaFree(pb.rows);
+  cudaFreeHost(pb.h_jobs);
+  if (pb.jobs_sent) cudaEventDestroy(pb.jobs_sent);
   pb = PersistBufs();
 }
 
@@ -132,13 +154,10 @@ struct orbx_ctx {
   // batched pairs
   std::vector<Workspace> bws;
   BatchSlot batch;
-  MatchJob* d_jobs = nullptr;
-  int jobs_cap = 0;
   uint32_t* batch_part = nullptr;
   unsigned int* batch_tile_done = nullptr;
   size_t batch_part_words = 0, batch_tile_words = 0;
-  std::vector<uint8_t> batch_key;
-  cudaGraphExec_t batch_exec = nullptr;
+  PairGraph bg;  // orbx_batch_pairs, either form
   // persistent batch form: run table, describe slices, completion counters
   int batch_form = 0;
   int persist_group = 0;
@@ -426,7 +445,12 @@ struct LaunchPlan {
   int pyr_tiles = 0, det_tiles = 0, nms_strips = 0, total_max_pts = 0;
 };
 
-static int upload_batch(orbx_ctx* c, BatchSlot& bs, const std::vector<Frame>& frames, LaunchPlan* plan) {
+// Fills the launch plan of `frames`.  Their device tables (and the batch's
+// matching jobs behind them) are uploaded when their content changed; frames
+// that travel in the launch parameters need none unless `tables` is set.
+static int upload_batch(orbx_ctx* c, BatchSlot& bs, const std::vector<Frame>& frames, LaunchPlan* plan,
+                        bool tables = false, const std::vector<MatchJob>* jobs = nullptr,
+                        const MatchJob** d_jobs = nullptr) {
   const int nf = (int)frames.size();
   if (nf <= 0 || nf > kMaxFramesPerLaunch) return ORBX_ERR_SIZE;
   std::vector<int> bases(3 * (nf + 1));
@@ -442,42 +466,47 @@ static int upload_batch(orbx_ctx* c, BatchSlot& bs, const std::vector<Frame>& fr
     nb[f + 1] = nb[f] + F.nms_strips;
     tmp += F.max_pts;
   }
+  if (!bs.d_ticket) ORBX_CUDA(cudaMalloc(&bs.d_ticket, sizeof(unsigned int)));
   const size_t fbytes = sizeof(Frame) * nf;
-  const size_t bbytes = sizeof(int) * bases.size();
-  std::vector<uint8_t> blob(fbytes + bbytes);
-  std::memcpy(blob.data(), frames.data(), fbytes);
-  std::memcpy(blob.data() + fbytes, bases.data(), bbytes);
-  if (nf > bs.cap) {
-    if (bs.uploaded) cudaEventSynchronize(bs.uploaded);
-    cudaFree(bs.d_frames);
-    cudaFree(bs.d_bases);
-    cudaFreeHost(bs.h_stage);
-    bs.d_frames = nullptr;
-    bs.d_bases = nullptr;
-    bs.h_stage = nullptr;
-    bs.last.clear();
-    const int cap = nf < 4 ? 4 : nf;
-    ORBX_CUDA(cudaMalloc(&bs.d_frames, sizeof(Frame) * cap));
-    ORBX_CUDA(cudaMalloc(&bs.d_bases, sizeof(int) * 3 * (cap + 1)));
-    ORBX_CUDA(cudaMallocHost(&bs.h_stage, sizeof(Frame) * cap + sizeof(int) * 3 * (cap + 1)));
-    if (!bs.d_ticket) ORBX_CUDA(cudaMalloc(&bs.d_ticket, sizeof(unsigned int)));
-    if (!bs.uploaded) ORBX_CUDA(cudaEventCreateWithFlags(&bs.uploaded, cudaEventDisableTiming));
-    bs.cap = cap;
+  const size_t bbytes = (sizeof(int) * bases.size() + 15) / 16 * 16;
+  const size_t jbytes = jobs ? sizeof(MatchJob) * jobs->size() : 0;
+  static_assert(sizeof(Frame) % 8 == 0, "the prefixes and jobs behind the frame table stay aligned");
+  if (tables || nf > kInlineFrames || jobs) {
+    const size_t bytes = fbytes + bbytes + jbytes;
+    std::vector<uint8_t> blob(bytes);
+    std::memcpy(blob.data(), frames.data(), fbytes);
+    std::memcpy(blob.data() + fbytes, bases.data(), sizeof(int) * bases.size());
+    if (jbytes) std::memcpy(blob.data() + fbytes + bbytes, jobs->data(), jbytes);
+    if (bytes > bs.cap) {
+      if (bs.uploaded) cudaEventSynchronize(bs.uploaded);
+      cudaFree(bs.d_tables);
+      cudaFreeHost(bs.h_stage);
+      bs.d_tables = nullptr;
+      bs.h_stage = nullptr;
+      bs.cap = 0;
+      bs.last.clear();
+      ORBX_CUDA(cudaMalloc(&bs.d_tables, bytes));
+      ORBX_CUDA(cudaMallocHost(&bs.h_stage, bytes));
+      if (!bs.uploaded) ORBX_CUDA(cudaEventCreateWithFlags(&bs.uploaded, cudaEventDisableTiming));
+      bs.cap = bytes;
+    }
+    if (bs.last != blob) {
+      ORBX_CUDA(cudaEventSynchronize(bs.uploaded));  // the previous upload has left the staging buffer
+      std::memcpy(bs.h_stage, blob.data(), bytes);
+      bs.last.clear();  // unknown content until the copy is queued
+      ORBX_CUDA(cudaMemcpyAsync(bs.d_tables, bs.h_stage, bytes, cudaMemcpyHostToDevice, c->stream));
+      ORBX_CUDA(cudaEventRecord(bs.uploaded, c->stream));
+      bs.last.swap(blob);
+    }
+    if (d_jobs) *d_jobs = reinterpret_cast<const MatchJob*>(bs.d_tables + fbytes + bbytes);
   }
-  if (bs.last != blob) {
-    ORBX_CUDA(cudaEventSynchronize(bs.uploaded));  // the previous upload has left the staging buffer
-    std::memcpy(bs.h_stage, blob.data(), blob.size());
-    ORBX_CUDA(cudaMemcpyAsync(bs.d_frames, bs.h_stage, fbytes, cudaMemcpyHostToDevice, c->stream));
-    ORBX_CUDA(cudaMemcpyAsync(bs.d_bases, bs.h_stage + fbytes, bbytes, cudaMemcpyHostToDevice, c->stream));
-    ORBX_CUDA(cudaEventRecord(bs.uploaded, c->stream));
-    bs.last.swap(blob);
-  }
+  int* d_bases = bs.d_tables ? reinterpret_cast<int*>(bs.d_tables + fbytes) : nullptr;
   Batch& b = plan->b;
-  b.frames = bs.d_frames;
+  b.frames = reinterpret_cast<Frame*>(bs.d_tables);
   b.n_frames = nf;
-  b.pyr_base = bs.d_bases;
-  b.det_base = bs.d_bases + (nf + 1);
-  b.nms_base = bs.d_bases + 2 * (nf + 1);
+  b.pyr_base = d_bases;
+  b.det_base = d_bases ? d_bases + (nf + 1) : nullptr;
+  b.nms_base = d_bases ? d_bases + 2 * (nf + 1) : nullptr;
   b.nms_ticket = bs.d_ticket;
   b.err = c->d_err;
   b.bounds = c->d_bounds;
@@ -513,6 +542,38 @@ static int launch_frames(orbx_ctx* c, const LaunchPlan& pl, bool compute_desc, c
   ORBX_CUDA(launch_detect(pl.b, pl.det_tiles, s));
   ORBX_CUDA(launch_nms(pl.b, pl.nms_strips, s));
   if (compute_desc) ORBX_CUDA(launch_describe(pl.b, pl.total_max_pts, s, c->describe_bps));
+  return ORBX_OK;
+}
+
+// Issues a launch sequence under the rule of PairGraph: `enqueue` queues it on
+// the context's stream.  Inside a caller's stream capture only a sequence that
+// has run before is recorded.
+template <class Enqueue>
+static int issue_or_replay(orbx_ctx* c, PairGraph& g, std::vector<uint8_t>& key, Enqueue&& enqueue) {
+  const bool same = g.key == key;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  ORBX_CUDA(cudaStreamIsCapturing(c->stream, &cap));
+  if (cap != cudaStreamCaptureStatusNone && !same) return ORBX_ERR_CUDA;
+  if (!same || cap != cudaStreamCaptureStatusNone) {
+    if (!same) g.drop();
+    const int rc = enqueue();
+    if (rc == ORBX_OK) g.key.swap(key);
+    return rc;
+  }
+  if (!g.exec) {
+    ORBX_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+    const int rc = enqueue();
+    const cudaError_t ce = cudaStreamEndCapture(c->stream, &g.graph);
+    if (rc != ORBX_OK || ce != cudaSuccess) {
+      g.drop();
+      (void)cudaGetLastError();
+      return rc != ORBX_OK ? rc : ORBX_ERR_CUDA;
+    }
+    const cudaError_t ie = cudaGraphInstantiate(&g.exec, g.graph, 0);
+    if (ie != cudaSuccess) g.drop();
+    ORBX_CUDA(ie);
+  }
+  ORBX_CUDA(cudaGraphLaunch(g.exec, c->stream));
   return ORBX_OK;
 }
 
@@ -600,8 +661,8 @@ int lower_detect(orbx_ctx* c, const uint8_t* image, uint8_t* octave_images, floa
   if (octave_images)
     ORBX_CUDA(cudaMemcpyAsync(octave_images, ws->pyr_alloc + ws->guard, ws->obytes, cudaMemcpyDeviceToDevice, c->stream));
   if (vmem)
-    ORBX_CUDA(launch_expand_score_map(c->single.d_frames, vmem, reinterpret_cast<int*>(vmem + npx), (long long)npx,
-                                      c->stream));
+    ORBX_CUDA(launch_expand_score_map(ws->occ, ws->vmap, ws->oct8, vmem, reinterpret_cast<int*>(vmem + npx),
+                                      (long long)npx, c->stream));
   return ORBX_OK;
 }
 
@@ -721,14 +782,13 @@ ORBX_API int orbx_destroy(orbx_ctx* c) {
   DeviceGuard g(c->device);
   cudaStreamSynchronize(c->stream);
   for (auto& ws : c->ws) ws_free(ws);
-  for (BatchSlot* bs : {&c->single, &c->pair}) {
-    cudaFree(bs->d_frames);
-    cudaFree(bs->d_bases);
+  for (BatchSlot* bs : {&c->single, &c->pair, &c->pair_b, &c->batch}) {
+    cudaFree(bs->d_tables);
     cudaFree(bs->d_ticket);
     cudaFreeHost(bs->h_stage);
     if (bs->uploaded) cudaEventDestroy(bs->uploaded);
   }
-  if (c->pg.exec) cudaGraphExecDestroy(c->pg.exec);
+  for (PairGraph* pg : {&c->pg, &c->ppg, &c->pho, &c->phs, &c->bg}) pg->drop();
   cudaFree(c->pg.mw.part);
   cudaFree(c->pg.mw.tile_done);
   cudaFree(c->mw.part);
@@ -747,20 +807,10 @@ ORBX_API int orbx_destroy(orbx_ctx* c) {
   cudaFree(c->imma_q);
   cudaFree(c->imma_db);
   for (auto& ws : c->bws) ws_free(ws);
-  cudaFree(c->batch.d_frames);
-  cudaFree(c->batch.d_bases);
-  cudaFree(c->batch.d_ticket);
-  cudaFreeHost(c->batch.h_stage);
-  if (c->batch.uploaded) cudaEventDestroy(c->batch.uploaded);
-  cudaFree(c->d_jobs);
   cudaFree(c->batch_part);
   cudaFree(c->batch_tile_done);
-  if (c->batch_exec) cudaGraphExecDestroy(c->batch_exec);
   persist_free(c->pbatch);
   persist_free(c->ppair);
-  if (c->pho.exec) cudaGraphExecDestroy(c->pho.exec);
-  if (c->phs.exec) cudaGraphExecDestroy(c->phs.exec);
-  if (c->ppg.exec) cudaGraphExecDestroy(c->ppg.exec);
   cudaFree(c->pho.mw.part);
   cudaFree(c->pho.mw.tile_done);
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
@@ -768,11 +818,6 @@ ORBX_API int orbx_destroy(orbx_ctx* c) {
   if (c->ev_join) cudaEventDestroy(c->ev_join);
   cudaFree(c->hmw.part);
   cudaFree(c->hmw.tile_done);
-  cudaFree(c->pair_b.d_frames);
-  cudaFree(c->pair_b.d_bases);
-  cudaFree(c->pair_b.d_ticket);
-  cudaFreeHost(c->pair_b.h_stage);
-  if (c->pair_b.uploaded) cudaEventDestroy(c->pair_b.uploaded);
   if (c->ev_reset) cudaEventDestroy(c->ev_reset);
   cudaFree(c->d_pattern);
   cudaFree(c->d_umax);
@@ -790,11 +835,7 @@ ORBX_API int orbx_set_stream(orbx_ctx* c, void* stream) {
   if (c->own_stream) cudaStreamDestroy(c->stream);
   c->stream = (cudaStream_t)stream;
   c->own_stream = false;
-  if (c->pg.exec) {
-    cudaGraphExecDestroy(c->pg.exec);
-    c->pg.exec = nullptr;
-    c->pg.valid = false;
-  }
+  c->pg.drop();
   return ORBX_OK;
 }
 
@@ -879,14 +920,7 @@ ORBX_API int orbx_init(orbx_ctx* c, const orbx_params* p) {
   ORBX_CUDA(cudaMemcpy(c->d_umax, umax, sizeof(umax), cudaMemcpyHostToDevice));
   if (shape_change)
     for (auto& ws : c->ws) ws_free(ws);
-  for (PairGraph* g : {&c->pg, &c->ppg, &c->pho, &c->phs}) {
-    if (g->exec) {
-      cudaGraphExecDestroy(g->exec);
-      g->exec = nullptr;
-    }
-    g->valid = false;
-  }
-  c->single.last.clear();
+  for (PairGraph* pg : {&c->pg, &c->ppg, &c->pho, &c->phs}) pg->drop();
   c->pair.last.clear();
   c->inited = true;
   return ORBX_OK;
@@ -1015,7 +1049,7 @@ static int persist_prepare(orbx_ctx* c, PersistBufs& pb, const LaunchPlan& pl, c
                            int* grid_out);
 
 // orbx_pair as one persistent launch (orbx_persist.cu) over the pair's two
-// frames: a graph of a counter reset and the launch.
+// frames: a counter reset and the launch.
 static int pair_persistent(orbx_ctx* c, const LaunchPlan& pl, const std::vector<Frame>& frames,
                            const MatchArgs& m) {
   PairGraph& pg = c->ppg;
@@ -1032,31 +1066,11 @@ static int pair_persistent(orbx_ctx* c, const LaunchPlan& pl, const std::vector<
   std::memcpy(key.data(), &a, sizeof(PersistArgs));
   std::memcpy(key.data() + sizeof(PersistArgs), &grid, sizeof(int));
   std::memcpy(key.data() + sizeof(PersistArgs) + sizeof(int), &c->ppair.done_ints, sizeof(size_t));
-  if (!(pg.valid && pg.key == key)) {
-    if (pg.exec) {
-      cudaGraphExecDestroy(pg.exec);
-      pg.exec = nullptr;
-    }
-    pg.valid = false;
-    cudaGraph_t graph = nullptr;
-    ORBX_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t le = cudaMemsetAsync(a.done, 0, sizeof(int) * c->ppair.done_ints, c->stream);
-    if (le == cudaSuccess) le = launch_batch_persistent(a, grid, c->stream);
-    const cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
-    if (le != cudaSuccess) {
-      if (graph) cudaGraphDestroy(graph);
-      (void)cudaGetLastError();
-      return ORBX_ERR_CUDA;
-    }
-    ORBX_CUDA(ce);
-    const cudaError_t ie = cudaGraphInstantiate(&pg.exec, graph, 0);
-    cudaGraphDestroy(graph);
-    ORBX_CUDA(ie);
-    pg.key.swap(key);
-    pg.valid = true;
-  }
-  ORBX_CUDA(cudaGraphLaunch(pg.exec, c->stream));
-  return ORBX_OK;
+  return issue_or_replay(c, pg, key, [&]() -> int {
+    ORBX_CUDA(cudaMemsetAsync(a.done, 0, sizeof(int) * c->ppair.done_ints, c->stream));
+    ORBX_CUDA(launch_batch_persistent(a, grid, c->stream));
+    return ORBX_OK;
+  });
 }
 
 ORBX_API int orbx_pair(orbx_ctx* c, const uint8_t* d_img_a, const uint8_t* d_img_b, int w, int h, int pitch,
@@ -1076,8 +1090,9 @@ ORBX_API int orbx_pair(orbx_ctx* c, const uint8_t* d_img_a, const uint8_t* d_img
   const int shape = (c->pair_form == 1 && mode == ORBX_MATCH_POPC) ? 0 : c->pyr_shape;
   fill_frame(c, c->ws[0], d_img_a, pitch, d_pts_a, d_desc_a, d_n_a, frames[0], -1, shape);
   fill_frame(c, c->ws[1], d_img_b, pitch, d_pts_b, d_desc_b, d_n_b, frames[1], -1, shape);
+  const bool persistent = c->pair_form == 1 && mode == ORBX_MATCH_POPC;
   LaunchPlan pl;
-  if ((rc = upload_batch(c, c->pair, frames, &pl)) != 0) return rc;
+  if ((rc = upload_batch(c, c->pair, frames, &pl, persistent)) != 0) return rc;
   MatchArgs a{};
   a.q = d_desc_a;
   a.db = d_desc_b;
@@ -1087,9 +1102,10 @@ ORBX_API int orbx_pair(orbx_ctx* c, const uint8_t* d_img_a, const uint8_t* d_img
   a.d_ndb = d_n_b;
   a.pts = d_pts_a;
   match_bounds(c, a, c->p.max_pts, c->p.max_pts, c->p.max_pts);
-  if (c->pair_form == 1 && mode == ORBX_MATCH_POPC) return pair_persistent(c, pl, frames, a);
-  // graph key: launch shapes and every pointer baked into the captured launches
-  std::vector<uint8_t> key(sizeof(Batch) + sizeof(MatchArgs) + sizeof(LaunchPlan) + sizeof(int));
+  if (persistent) return pair_persistent(c, pl, frames, a);
+  // key: launch shapes and every pointer baked into the launches
+  const void* ptrs[2] = {c->imma_q, c->imma_db};
+  std::vector<uint8_t> key(sizeof(Batch) + sizeof(MatchArgs) + sizeof(LaunchPlan) + sizeof(int) + sizeof(ptrs));
   {
     uint8_t* k = key.data();
     std::memcpy(k, &pl.b, sizeof(Batch));
@@ -1098,33 +1114,13 @@ ORBX_API int orbx_pair(orbx_ctx* c, const uint8_t* d_img_a, const uint8_t* d_img
     std::memset(&pz.b, 0, sizeof(Batch));
     std::memcpy(k + sizeof(Batch) + sizeof(MatchArgs), &pz, sizeof(LaunchPlan));
     std::memcpy(k + sizeof(Batch) + sizeof(MatchArgs) + sizeof(LaunchPlan), &mode, sizeof(int));
+    std::memcpy(k + sizeof(Batch) + sizeof(MatchArgs) + sizeof(LaunchPlan) + sizeof(int), ptrs, sizeof(ptrs));
   }
-  PairGraph& pg = c->pg;
-  if (!(pg.valid && pg.key == key)) {
-    if (pg.exec) {
-      cudaGraphExecDestroy(pg.exec);
-      pg.exec = nullptr;
-    }
-    pg.valid = false;
-    if ((rc = mw_ensure(pg.mw, c->p.max_pts)) != 0) return rc;
-    cudaGraph_t graph = nullptr;
-    ORBX_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    int lrc = launch_frames(c, pl, true);
-    if (lrc == ORBX_OK) lrc = launch_match(c, pg.mw, a, c->p.max_pts, c->p.max_pts, mode);
-    const cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
-    if (lrc != ORBX_OK) {
-      if (graph) cudaGraphDestroy(graph);
-      return lrc;
-    }
-    ORBX_CUDA(ce);
-    const cudaError_t ie = cudaGraphInstantiate(&pg.exec, graph, 0);
-    cudaGraphDestroy(graph);
-    ORBX_CUDA(ie);
-    pg.key.swap(key);
-    pg.valid = true;
-  }
-  ORBX_CUDA(cudaGraphLaunch(pg.exec, c->stream));
-  return ORBX_OK;
+  if ((rc = mw_ensure(c->pg.mw, c->p.max_pts)) != 0) return rc;
+  return issue_or_replay(c, c->pg, key, [&]() -> int {
+    const int lrc = launch_frames(c, pl, true);
+    return lrc ? lrc : launch_match(c, c->pg.mw, a, c->p.max_pts, c->p.max_pts, mode);
+  });
 }
 
 // cuStreamWriteValue32 through the runtime's driver entry point (no link-time
@@ -1184,7 +1180,7 @@ static int pair_host_overlap(orbx_ctx* c, const uint8_t* h_a, const uint8_t* h_b
   fill_frame(c, c->ws[0], c->io_img[0], pitch, c->io_pts[0], c->io_desc[0], c->io_count, frames[0]);
   fill_frame(c, c->ws[1], c->io_img[1], pitch, c->io_pts[1], c->io_desc[1], c->io_count + 1, frames[1]);
   LaunchPlan pl;
-  if ((rc = upload_batch(c, c->pair, frames, &pl)) != 0) return rc;
+  if ((rc = upload_batch(c, c->pair, frames, &pl, true)) != 0) return rc;
   PairGraph& pg = c->pho;
   if ((rc = mw_ensure(pg.mw, c->p.max_pts)) != 0) return rc;
   std::vector<MatchJob> jobs(1);
@@ -1213,35 +1209,15 @@ static int pair_host_overlap(orbx_ctx* c, const uint8_t* h_a, const uint8_t* h_b
   const int extra[4] = {grid, c->p.max_pts, with_desc ? 1 : 0, (int)c->ppair.done_ints};
   std::memcpy(key.data() + sizeof(PersistArgs), extra, sizeof(extra));
   std::memcpy(key.data() + sizeof(PersistArgs) + sizeof(extra), &map_dev, sizeof(void*));
-  if (!(pg.valid && pg.key == key)) {
-    if (pg.exec) {
-      cudaGraphExecDestroy(pg.exec);
-      pg.exec = nullptr;
-    }
-    pg.valid = false;
-    cudaGraph_t graph = nullptr;
-    ORBX_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    int lrc = launch_batch_persistent(a, grid, c->stream) == cudaSuccess ? ORBX_OK : ORBX_ERR_CUDA;
-    if (lrc == ORBX_OK)
-      lrc = hostio_export_pair(c, c->io_pts[0], c->io_pts[1], c->io_desc[0], c->io_desc[1], c->io_count,
-                               c->p.max_pts, with_desc, res);
-    const cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
-    if (lrc != ORBX_OK) {
-      if (graph) cudaGraphDestroy(graph);
-      (void)cudaGetLastError();
-      return lrc;
-    }
-    ORBX_CUDA(ce);
-    const cudaError_t ie = cudaGraphInstantiate(&pg.exec, graph, 0);
-    cudaGraphDestroy(graph);
-    ORBX_CUDA(ie);
-    pg.key.swap(key);
-    pg.valid = true;
-  }
   // reset the counters and flags, start the launch, then feed it the bands
   ORBX_CUDA(cudaMemsetAsync(a.done, 0, sizeof(int) * c->ppair.done_ints, c->stream));
   ORBX_CUDA(cudaEventRecord(c->ev_reset, c->stream));
-  ORBX_CUDA(cudaGraphLaunch(pg.exec, c->stream));
+  rc = issue_or_replay(c, pg, key, [&]() -> int {
+    ORBX_CUDA(launch_batch_persistent(a, grid, c->stream));
+    return hostio_export_pair(c, c->io_pts[0], c->io_pts[1], c->io_desc[0], c->io_desc[1], c->io_count,
+                              c->p.max_pts, with_desc, res);
+  });
+  if (rc) return rc;
   ORBX_CUDA(cudaStreamWaitEvent(c->copy_stream, c->ev_reset, 0));
   WriteValue32Fn wv = write_value32();
   const uint8_t* src[2] = {h_a, h_b};
@@ -1329,8 +1305,10 @@ static int pair_host_streams(orbx_ctx* c, const uint8_t* h_a, const uint8_t* h_b
     return pair_host_streams_enqueue(c, h_a, h_b, ibytes, pa, pb, m, with_desc, res, ev_uploaded, false);
   const uint8_t* map_dev = nullptr;
   if ((rc = hostio_map(c, c->p.max_pts, res, &map_dev)) != 0) return rc;
+  // key: everything but the host images' addresses, which are parameters of
+  // the graph's two copy nodes
   PairGraph& g = c->phs;
-  const void* ptrs[5] = {h_a, h_b, map_dev, c->hmw.part, ev_uploaded};
+  const void* ptrs[3] = {map_dev, c->hmw.part, ev_uploaded};
   const long long extra[4] = {(long long)ibytes, with_desc ? 1 : 0, c->match_bps, c->describe_bps};
   std::vector<uint8_t> key(2 * sizeof(Batch) + 6 * sizeof(int) + sizeof(MatchArgs) + sizeof(ptrs) + sizeof(extra));
   {
@@ -1348,29 +1326,48 @@ static int pair_host_streams(orbx_ctx* c, const uint8_t* h_a, const uint8_t* h_b
     k += sizeof(ptrs);
     std::memcpy(k, extra, sizeof(extra));
   }
-  if (!(g.valid && g.key == key)) {
-    if (g.exec) {
-      cudaGraphExecDestroy(g.exec);
-      g.exec = nullptr;
+  if (g.exec && g.key == key) {
+    const void* src[2] = {h_a, h_b};
+    for (int i = 0; i < 2; i++) {
+      if (g.copy_src[i] == src[i]) continue;
+      if (cudaGraphExecMemcpyNodeSetParams1D(g.exec, g.copy_node[i], c->io_img[i], src[i], ibytes,
+                                             cudaMemcpyHostToDevice) != cudaSuccess) {
+        (void)cudaGetLastError();
+        g.drop();
+        break;
+      }
+      g.copy_src[i] = src[i];
     }
-    g.valid = false;
-    cudaGraph_t graph = nullptr;
-    ORBX_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    const int lrc = pair_host_streams_enqueue(c, h_a, h_b, ibytes, pa, pb, m, with_desc, res, ev_uploaded, true);
-    const cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
-    if (lrc != ORBX_OK || ce != cudaSuccess) {
-      if (graph) cudaGraphDestroy(graph);
-      (void)cudaGetLastError();
-      return lrc != ORBX_OK ? lrc : ORBX_ERR_CUDA;
-    }
-    const cudaError_t ie = cudaGraphInstantiate(&g.exec, graph, 0);
-    cudaGraphDestroy(graph);
-    ORBX_CUDA(ie);
-    g.key.swap(key);
-    g.valid = true;
   }
-  ORBX_CUDA(cudaGraphLaunch(g.exec, c->stream));
-  return ORBX_OK;
+  const bool had_exec = g.exec != nullptr;
+  rc = issue_or_replay(c, g, key, [&]() -> int {
+    return pair_host_streams_enqueue(c, h_a, h_b, ibytes, pa, pb, m, with_desc, res, ev_uploaded, g.key == key);
+  });
+  if (rc == ORBX_OK && g.exec && !had_exec) {
+    // a new graph: its two copy nodes, by destination
+    size_t n = 0;
+    ORBX_CUDA(cudaGraphGetNodes(g.graph, nullptr, &n));
+    std::vector<cudaGraphNode_t> nodes(n);
+    ORBX_CUDA(cudaGraphGetNodes(g.graph, nodes.data(), &n));
+    g.copy_src[0] = h_a;
+    g.copy_src[1] = h_b;
+    int found = 0;
+    for (cudaGraphNode_t node : nodes) {
+      cudaGraphNodeType type;
+      cudaMemcpy3DParms cp{};
+      if (cudaGraphNodeGetType(node, &type) != cudaSuccess || type != cudaGraphNodeTypeMemcpy ||
+          cudaGraphMemcpyNodeGetParams(node, &cp) != cudaSuccess)
+        continue;
+      for (int i = 0; i < 2; i++)
+        if (cp.dstPtr.ptr == c->io_img[i]) {
+          g.copy_node[i] = node;
+          found |= 1 << i;
+        }
+    }
+    (void)cudaGetLastError();
+    if (found != 3) g.drop();  // already queued; the next call starts over
+  }
+  return rc;
 }
 
 // orbx_pair_host; with `prof`, CUDA events and host clocks between the phases.
@@ -1595,82 +1592,61 @@ ORBX_API int orbx_set_tuning(orbx_ctx* c, const orbx_tuning* t) {
   c->row_deps = t->persist_row_deps;
   c->host_overlap = t->host_overlap;
   c->wait_cycles = (long long)c->wait_us * c->clock_khz / 1000;
-  if (c->batch_exec) {
-    cudaGraphExecDestroy(c->batch_exec);
-    c->batch_exec = nullptr;
-  }
-  c->batch_key.clear();
   // cached graphs baked in the old shapes
-  for (PairGraph* g : {&c->pg, &c->ppg, &c->pho, &c->phs}) {
-    if (g->exec) {
-      cudaGraphExecDestroy(g->exec);
-      g->exec = nullptr;
-    }
-    g->valid = false;
-  }
-  c->single.last.clear();
+  for (PairGraph* pg : {&c->pg, &c->ppg, &c->pho, &c->phs, &c->bg}) pg->drop();
   c->pair.last.clear();
   return ORBX_OK;
 }
 
 static constexpr int kBatchSplitsCap = 16;
 
-// Builds the run table of a persistent launch over `frames` (orbx_persist.cu),
-// uploads the tables to `pb` when their content changed, and fills the launch
-// arguments and grid.  Uploads are synchronous (they happen only when a batch
-// layout is new).
+// Fills the arguments and grid of a persistent launch over `frames`
+// (orbx_persist.cu).  Its item tables depend on the frames' sizes and the
+// launch shapes alone; they are built and uploaded, synchronously, when these
+// are new.  The matching jobs, which hold the callers' buffers, go up through
+// pinned staging when they changed.
 static int persist_prepare(orbx_ctx* c, PersistBufs& pb, const LaunchPlan& pl, const std::vector<Frame>& frames,
                            const std::vector<MatchJob>& jobs, int blocks_per_pair, int group, PersistArgs* out,
                            int* grid_out) {
   const int nf = (int)frames.size();
   const int n_pairs = (int)jobs.size();
-  std::vector<int> pyr_n(nf), det_n(nf), nms_n(nf), desc_n(nf), desc_base(nf + 1, 0);
-  for (int f = 0; f < nf; f++) {
-    const Frame& F = frames[f];
-    pyr_n[f] = F.pyr_tile_base[F.n_oct];
-    det_n[f] = F.det_tiles_x * F.det_tiles_y;
-    nms_n[f] = F.nms_strips;
-    desc_n[f] = std::max(1, std::min(div_up(F.w * F.h, kDescSlicePixels), div_up(F.max_pts, 8)));
-    desc_base[f + 1] = desc_base[f] + desc_n[f];
-  }
-  std::vector<PersistRun> runs;
-  std::vector<int> run_base;
-  std::vector<PersistRows> rows;
-  int n_rows = 0;
-  if (c->row_deps)
-    n_rows = build_persist_runs_rows(frames, desc_n.data(), blocks_per_pair, &runs, &run_base, &rows);
-  else
-    build_persist_runs(nf, group > 0 ? group : nf, pyr_n.data(), det_n.data(), nms_n.data(), desc_n.data(),
-                       blocks_per_pair, &runs, &run_base);
-  // counters: [4 x frames] stage counters, the item counter, [frames] upload flags, row counters
-  const size_t done_ints = 5 * (size_t)nf + 1 + (size_t)n_rows;
-  // one packed item per ticket: a claim decodes its item with one load
-  std::vector<unsigned long long> items((size_t)run_base.back());
-  for (size_t r = 0; r < runs.size(); r++)
-    for (int t = run_base[r]; t < run_base[r + 1]; t++)
-      items[t] = persist_item(runs[r].stage, runs[r].frame, runs[r].first + (t - run_base[r]));
   const int bps_max = persist_blocks_per_sm(c->p.wta_k);
   if (bps_max <= 0) return ORBX_ERR_CUDA;
   const int bps = c->persist_bps > 0 ? std::min(c->persist_bps, bps_max) : bps_max;
   int nsm = 0;
   ORBX_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
   *grid_out = bps * nsm;
-  std::vector<uint8_t> blob(sizeof(unsigned long long) * items.size() + sizeof(int) * (nf + 1) +
-                            sizeof(MatchJob) * n_pairs + sizeof(PersistRows) * rows.size() + sizeof(size_t));
-  {
-    uint8_t* q = blob.data();
-    std::memcpy(q, &done_ints, sizeof(size_t));
-    q += sizeof(size_t);
-    if (!rows.empty()) std::memcpy(q, rows.data(), sizeof(PersistRows) * rows.size());
-    q += sizeof(PersistRows) * rows.size();
-    std::memcpy(q, items.data(), sizeof(unsigned long long) * items.size());
-    q += sizeof(unsigned long long) * items.size();
-    std::memcpy(q, desc_base.data(), sizeof(int) * (nf + 1));
-    q += sizeof(int) * (nf + 1);
-    std::memcpy(q, jobs.data(), sizeof(MatchJob) * n_pairs);
-  }
-  if (pb.last != blob) {
+  std::vector<int> layout = {nf, n_pairs, blocks_per_pair, group, c->row_deps};
+  for (const Frame& F : frames)
+    for (int v : {F.w, F.h, F.n_oct, F.max_pts, F.border, F.nms_rows, F.nms_strips}) layout.push_back(v);
+  if (pb.layout != layout) {
+    std::vector<int> pyr_n(nf), det_n(nf), nms_n(nf), desc_n(nf), desc_base(nf + 1, 0);
+    for (int f = 0; f < nf; f++) {
+      const Frame& F = frames[f];
+      pyr_n[f] = F.pyr_tile_base[F.n_oct];
+      det_n[f] = F.det_tiles_x * F.det_tiles_y;
+      nms_n[f] = F.nms_strips;
+      desc_n[f] = std::max(1, std::min(div_up(F.w * F.h, kDescSlicePixels), div_up(F.max_pts, 8)));
+      desc_base[f + 1] = desc_base[f] + desc_n[f];
+    }
+    std::vector<PersistRun> runs;
+    std::vector<int> run_base;
+    std::vector<PersistRows> rows;
+    int n_rows = 0;
+    if (c->row_deps)
+      n_rows = build_persist_runs_rows(frames, desc_n.data(), blocks_per_pair, &runs, &run_base, &rows);
+    else
+      build_persist_runs(nf, group > 0 ? group : nf, pyr_n.data(), det_n.data(), nms_n.data(), desc_n.data(),
+                         blocks_per_pair, &runs, &run_base);
+    // one packed item per ticket: a claim decodes its item with one load
+    std::vector<unsigned long long> items((size_t)run_base.back());
+    for (size_t r = 0; r < runs.size(); r++)
+      for (int t = run_base[r]; t < run_base[r + 1]; t++)
+        items[t] = persist_item(runs[r].stage, runs[r].frame, runs[r].first + (t - run_base[r]));
+    // counters: [4 x frames] stage counters, the item counter, [frames] upload flags, row counters
+    const size_t done_ints = 5 * (size_t)nf + 1 + (size_t)n_rows;
     ORBX_CUDA(cudaStreamSynchronize(c->stream));
+    pb.layout.clear();
     if (pb.items_cap < items.size()) {
       cudaFree(pb.items);
       pb.items = nullptr;
@@ -1697,76 +1673,71 @@ static int persist_prepare(orbx_ctx* c, PersistBufs& pb, const LaunchPlan& pl, c
     }
     if (!rows.empty())
       ORBX_CUDA(cudaMemcpy(pb.rows, rows.data(), sizeof(PersistRows) * nf, cudaMemcpyHostToDevice));
-    if (pb.jobs_cap < (size_t)n_pairs) {
-      cudaFree(pb.jobs);
-      pb.jobs = nullptr;
-      pb.jobs_cap = 0;
-      ORBX_CUDA(cudaMalloc(&pb.jobs, sizeof(MatchJob) * n_pairs));
-      pb.jobs_cap = n_pairs;
-    }
     ORBX_CUDA(cudaMemcpy(pb.items, items.data(), sizeof(unsigned long long) * items.size(),
                          cudaMemcpyHostToDevice));
     ORBX_CUDA(cudaMemcpy(pb.desc_base, desc_base.data(), sizeof(int) * (nf + 1), cudaMemcpyHostToDevice));
-    ORBX_CUDA(cudaMemcpy(pb.jobs, jobs.data(), sizeof(MatchJob) * n_pairs, cudaMemcpyHostToDevice));
-    pb.last.swap(blob);
+    pb.n_items = items.size();
+    pb.n_rows = n_rows;
+    pb.done_ints = done_ints;
+    pb.layout.swap(layout);
+  }
+  if (pb.jobs_cap < (size_t)n_pairs) {
+    ORBX_CUDA(cudaStreamSynchronize(c->stream));
+    cudaFree(pb.jobs);
+    cudaFreeHost(pb.h_jobs);
+    pb.jobs = nullptr;
+    pb.h_jobs = nullptr;
+    pb.jobs_cap = 0;
+    pb.last_jobs.clear();
+    ORBX_CUDA(cudaMalloc(&pb.jobs, sizeof(MatchJob) * n_pairs));
+    ORBX_CUDA(cudaMallocHost(&pb.h_jobs, sizeof(MatchJob) * n_pairs));
+    if (!pb.jobs_sent) ORBX_CUDA(cudaEventCreateWithFlags(&pb.jobs_sent, cudaEventDisableTiming));
+    pb.jobs_cap = n_pairs;
+  }
+  if (pb.last_jobs.size() != jobs.size() ||
+      std::memcmp(pb.last_jobs.data(), jobs.data(), sizeof(MatchJob) * n_pairs) != 0) {
+    ORBX_CUDA(cudaEventSynchronize(pb.jobs_sent));  // the previous upload has left the staging buffer
+    std::memcpy(pb.h_jobs, jobs.data(), sizeof(MatchJob) * n_pairs);
+    pb.last_jobs.clear();
+    ORBX_CUDA(cudaMemcpyAsync(pb.jobs, pb.h_jobs, sizeof(MatchJob) * n_pairs, cudaMemcpyHostToDevice, c->stream));
+    ORBX_CUDA(cudaEventRecord(pb.jobs_sent, c->stream));
+    pb.last_jobs = jobs;
   }
   PersistArgs& a = *out;
   a = PersistArgs{};
   a.b = pl.b;
   a.items = pb.items;
-  a.run_base_host_total = run_base.back();
+  a.run_base_host_total = (int)pb.n_items;
   a.desc_base = pb.desc_base;
   a.done = pb.done;
   a.item_counter = reinterpret_cast<unsigned int*>(pb.done + 4 * (size_t)nf);
   a.jobs = pb.jobs;
   a.blocks_per_job = blocks_per_pair;
-  if (n_rows > 0) {
+  if (pb.n_rows > 0) {
     a.rows = pb.rows;
     a.rows_done = pb.done + 5 * (size_t)nf + 1;
   }
-  pb.done_ints = done_ints;
   return ORBX_OK;
 }
 
-// The persistent form of orbx_batch_pairs: a graph of one counter reset and
-// one persistent launch.
+// The persistent form of orbx_batch_pairs: one counter reset and one
+// persistent launch.  Of the callers' buffers the launch parameters hold only
+// a batch's inline frames, so other buffers of the same layout replay the graph.
 static int batch_persistent(orbx_ctx* c, const LaunchPlan& pl, const std::vector<Frame>& frames,
-                            const std::vector<MatchJob>& jobs, int blocks_per_pair, std::vector<uint8_t>& key) {
-  const int nf = (int)frames.size();
+                            const std::vector<MatchJob>& jobs, int blocks_per_pair) {
   PersistArgs a;
   int grid = 0;
   int rc = persist_prepare(c, c->pbatch, pl, frames, jobs, blocks_per_pair, c->persist_group, &a, &grid);
   if (rc) return rc;
-  {
-    const int extra[4] = {1, c->persist_group, grid, (int)c->pbatch.done_ints};
-    const size_t k0 = key.size();
-    key.resize(k0 + sizeof(extra) + sizeof(void*));
-    std::memcpy(key.data() + k0, extra, sizeof(extra));
-    std::memcpy(key.data() + k0 + sizeof(extra), &a.done, sizeof(void*));
-  }
-  if (!(c->batch_exec && c->batch_key == key)) {
-    if (c->batch_exec) {
-      cudaGraphExecDestroy(c->batch_exec);
-      c->batch_exec = nullptr;
-    }
-    cudaGraph_t graph = nullptr;
-    ORBX_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t le = cudaMemsetAsync(a.done, 0, sizeof(int) * c->pbatch.done_ints, c->stream);
-    if (le == cudaSuccess) le = launch_batch_persistent(a, grid, c->stream);
-    const cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
-    if (le != cudaSuccess) {
-      if (graph) cudaGraphDestroy(graph);
-      (void)cudaGetLastError();
-      return ORBX_ERR_CUDA;
-    }
-    ORBX_CUDA(ce);
-    const cudaError_t ie = cudaGraphInstantiate(&c->batch_exec, graph, 0);
-    cudaGraphDestroy(graph);
-    ORBX_CUDA(ie);
-    c->batch_key.swap(key);
-  }
-  ORBX_CUDA(cudaGraphLaunch(c->batch_exec, c->stream));
-  return ORBX_OK;
+  const int extra[3] = {1, grid, (int)c->pbatch.done_ints};
+  std::vector<uint8_t> key(sizeof(PersistArgs) + sizeof(extra));
+  std::memcpy(key.data(), &a, sizeof(PersistArgs));
+  std::memcpy(key.data() + sizeof(PersistArgs), extra, sizeof(extra));
+  return issue_or_replay(c, c->bg, key, [&]() -> int {
+    ORBX_CUDA(cudaMemsetAsync(a.done, 0, sizeof(int) * c->pbatch.done_ints, c->stream));
+    ORBX_CUDA(launch_batch_persistent(a, grid, c->stream));
+    return ORBX_OK;
+  });
 }
 
 static int batch_pairs_impl(orbx_ctx* c, int n_pairs, const orbx_image* ia, const orbx_image* ib,
@@ -1798,8 +1769,6 @@ static int batch_pairs_impl(orbx_ctx* c, int n_pairs, const orbx_image* ia, cons
                  (c->batch_form == 1 && !stage_ms) ? 0 : c->pyr_shape);
     }
   }
-  LaunchPlan pl;
-  if ((rc = upload_batch(c, c->batch, frames, &pl)) != 0) return rc;
   // matching jobs, one per pair, with their own slices of the split scratch
   int max_tiles = 1;
   size_t part_words = 0, tile_words = 0;
@@ -1822,11 +1791,6 @@ static int batch_pairs_impl(orbx_ctx* c, int n_pairs, const orbx_image* ia, cons
     ORBX_CUDA(cudaMemset(c->batch_tile_done, 0, tile_words * sizeof(unsigned int)));
     c->batch_part_words = part_words;
     c->batch_tile_words = tile_words;
-    if (c->batch_exec) {
-      cudaGraphExecDestroy(c->batch_exec);
-      c->batch_exec = nullptr;
-    }
-    c->batch_key.clear();
   }
   {
     size_t po = 0, to = 0;
@@ -1852,32 +1816,12 @@ static int batch_pairs_impl(orbx_ctx* c, int n_pairs, const orbx_image* ia, cons
   int blocks_per_pair = c->match_blocks_per_pair;
   if (blocks_per_pair <= 0) blocks_per_pair = std::max(max_tiles, div_up(8 * 148, n_pairs));
   blocks_per_pair = std::max(blocks_per_pair, max_tiles);  // every query tile needs a block
-  // graph key: frames, jobs and launch shapes
-  std::vector<uint8_t> key(sizeof(MatchJob) * n_pairs + c->batch.last.size() + 4 * sizeof(int));
-  {
-    uint8_t* k = key.data();
-    std::memcpy(k, jobs.data(), sizeof(MatchJob) * n_pairs);
-    k += sizeof(MatchJob) * n_pairs;
-    std::memcpy(k, c->batch.last.data(), c->batch.last.size());
-    k += c->batch.last.size();
-    const int shapes[4] = {c->nms_rows, c->describe_bps, blocks_per_pair, mode};
-    std::memcpy(k, shapes, sizeof(shapes));
-  }
-  if (c->batch_form == 1 && !stage_ms) return batch_persistent(c, pl, frames, jobs, blocks_per_pair, key);
+  LaunchPlan pl;
+  const MatchJob* d_jobs = nullptr;
+  if ((rc = upload_batch(c, c->batch, frames, &pl, true, &jobs, &d_jobs)) != 0) return rc;
+  if (c->batch_form == 1 && !stage_ms) return batch_persistent(c, pl, frames, jobs, blocks_per_pair);
   if (stage_ms) {
-    // profiling: the same launches, unrolled, with events between them
-    if (c->jobs_cap < n_pairs) {
-      cudaStreamSynchronize(c->stream);
-      cudaFree(c->d_jobs);
-      c->d_jobs = nullptr;
-      c->jobs_cap = 0;
-      ORBX_CUDA(cudaMalloc(&c->d_jobs, sizeof(MatchJob) * n_pairs));
-      c->jobs_cap = n_pairs;
-    }
-    ORBX_CUDA(cudaMemcpyAsync(c->d_jobs, jobs.data(), sizeof(MatchJob) * n_pairs, cudaMemcpyHostToDevice,
-                              c->stream));
-    ORBX_CUDA(cudaStreamSynchronize(c->stream));
-    c->batch_key.clear();  // the device job table may differ from the captured one now
+    // profiling: the same launches with events between them
     for (auto& e : c->prof_ev)
       if (!e) ORBX_CUDA(cudaEventCreate(&e));
     ORBX_CUDA(cudaEventRecord(c->prof_ev[0], c->stream));
@@ -1889,47 +1833,26 @@ static int batch_pairs_impl(orbx_ctx* c, int n_pairs, const orbx_image* ia, cons
     ORBX_CUDA(cudaEventRecord(c->prof_ev[3], c->stream));
     ORBX_CUDA(launch_describe(pl.b, pl.total_max_pts, c->stream, c->describe_bps));
     ORBX_CUDA(cudaEventRecord(c->prof_ev[4], c->stream));
-    ORBX_CUDA(launch_match_popc_batch(c->d_jobs, n_pairs, blocks_per_pair, c->stream));
+    ORBX_CUDA(launch_match_popc_batch(d_jobs, n_pairs, blocks_per_pair, c->stream));
     ORBX_CUDA(cudaEventRecord(c->prof_ev[5], c->stream));
     ORBX_CUDA(cudaEventSynchronize(c->prof_ev[5]));
     for (int i = 0; i < 5; i++) ORBX_CUDA(cudaEventElapsedTime(&stage_ms[i], c->prof_ev[i], c->prof_ev[i + 1]));
     return ORBX_OK;
   }
-  if (!(c->batch_exec && c->batch_key == key)) {
-    if (c->batch_exec) {
-      cudaGraphExecDestroy(c->batch_exec);
-      c->batch_exec = nullptr;
-    }
-    if (c->jobs_cap < n_pairs) {
-      cudaStreamSynchronize(c->stream);
-      cudaFree(c->d_jobs);
-      c->d_jobs = nullptr;
-      c->jobs_cap = 0;
-      ORBX_CUDA(cudaMalloc(&c->d_jobs, sizeof(MatchJob) * n_pairs));
-      c->jobs_cap = n_pairs;
-    }
-    ORBX_CUDA(cudaMemcpyAsync(c->d_jobs, jobs.data(), sizeof(MatchJob) * n_pairs, cudaMemcpyHostToDevice,
-                              c->stream));
-    ORBX_CUDA(cudaStreamSynchronize(c->stream));
-    cudaGraph_t graph = nullptr;
-    ORBX_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    int lrc = launch_frames(c, pl, true);
-    if (lrc == ORBX_OK)
-      lrc = launch_match_popc_batch(c->d_jobs, n_pairs, blocks_per_pair, c->stream) == cudaSuccess ? ORBX_OK
-                                                                                                     : ORBX_ERR_CUDA;
-    const cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
-    if (lrc != ORBX_OK) {
-      if (graph) cudaGraphDestroy(graph);
-      return lrc;
-    }
-    ORBX_CUDA(ce);
-    const cudaError_t ie = cudaGraphInstantiate(&c->batch_exec, graph, 0);
-    cudaGraphDestroy(graph);
-    ORBX_CUDA(ie);
-    c->batch_key.swap(key);
-  }
-  ORBX_CUDA(cudaGraphLaunch(c->batch_exec, c->stream));
-  return ORBX_OK;
+  // key: the launch parameters (the frame and job tables they point at may
+  // hold other buffers by the next replay)
+  const int extra[8] = {0, pl.pyr_tiles, pl.det_tiles, pl.nms_strips, pl.total_max_pts, c->describe_bps, n_pairs,
+                        blocks_per_pair};
+  std::vector<uint8_t> key(sizeof(Batch) + sizeof(extra) + sizeof(d_jobs));
+  std::memcpy(key.data(), &pl.b, sizeof(Batch));
+  std::memcpy(key.data() + sizeof(Batch), extra, sizeof(extra));
+  std::memcpy(key.data() + sizeof(Batch) + sizeof(extra), &d_jobs, sizeof(d_jobs));
+  return issue_or_replay(c, c->bg, key, [&]() -> int {
+    const int lrc = launch_frames(c, pl, true);
+    if (lrc) return lrc;
+    ORBX_CUDA(launch_match_popc_batch(d_jobs, n_pairs, blocks_per_pair, c->stream));
+    return ORBX_OK;
+  });
 }
 
 ORBX_API int orbx_batch_pairs(orbx_ctx* c, int n_pairs, const orbx_image* ia, const orbx_image* ib,
@@ -2074,7 +1997,7 @@ ORBX_API int orbx_debug_buffers(orbx_ctx* c, uint8_t* h_pyr, uint8_t* h_blur, fl
       cudaFree(dv);
       return ORBX_ERR_NOMEM;
     }
-    cudaError_t e = launch_expand_score_map(c->single.d_frames, dv, dl, (long long)npx, c->stream);
+    cudaError_t e = launch_expand_score_map(ws.occ, ws.vmap, ws.oct8, dv, dl, (long long)npx, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e == cudaSuccess && h_vmap) e = cudaMemcpy(h_vmap, dv, npx * sizeof(float), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && h_layer) e = cudaMemcpy(h_layer, dl, npx * sizeof(int), cudaMemcpyDeviceToHost);

@@ -33,20 +33,20 @@ __global__ void __launch_bounds__(256, 4) k_nms(const __grid_constant__ Batch b)
 
 // Dense reference-layout maps (vmem: f32 scores then i32 octaves,
 // orbd.cu:1576-1577) from the sparse ones, for orbd.h callers and debugging.
-__global__ void k_expand_score_map(const Frame* __restrict__ fr, float* vmap_dense, int* layer_dense,
+__global__ void k_expand_score_map(const uint32_t* __restrict__ occ, const float* __restrict__ vmap,
+                                   const uint8_t* __restrict__ oct8, float* vmap_dense, int* layer_dense,
                                    long long npx) {
-  const Frame& F = fr[0];
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < npx;
        i += (long long)gridDim.x * blockDim.x) {
-    const bool on = (__ldg(F.occ + (i >> 5)) >> (i & 31)) & 1u;
-    vmap_dense[i] = on ? F.vmap[i] : 0.f;
-    layer_dense[i] = on ? (int)F.oct8[i] : 0;
+    const bool on = (__ldg(occ + (i >> 5)) >> (i & 31)) & 1u;
+    vmap_dense[i] = on ? vmap[i] : 0.f;
+    layer_dense[i] = on ? (int)oct8[i] : 0;
   }
 }
 
-cudaError_t launch_expand_score_map(const Frame* d_frame, float* vmap_dense, int* layer_dense, long long npx,
-                                    cudaStream_t s) {
-  k_expand_score_map<<<4 * 148, 256, 0, s>>>(d_frame, vmap_dense, layer_dense, npx);
+cudaError_t launch_expand_score_map(const uint32_t* occ, const float* vmap, const uint8_t* oct8, float* vmap_dense,
+                                    int* layer_dense, long long npx, cudaStream_t s) {
+  k_expand_score_map<<<4 * 148, 256, 0, s>>>(occ, vmap, oct8, vmap_dense, layer_dense, npx);
   return cudaGetLastError();
 }
 

@@ -141,9 +141,9 @@ namespace orbx {
 cudaError_t launch_pyramid_blur(const Batch& b, int total_tiles, cudaStream_t s);
 cudaError_t launch_detect(const Batch& b, int total_tiles, cudaStream_t s);
 cudaError_t launch_nms(const Batch& b, int total_strips, cudaStream_t s);
-// dense reference-layout score and octave maps from the sparse ones (frame 0 of b)
-cudaError_t launch_expand_score_map(const Frame* d_frame, float* vmap_dense, int* layer_dense, long long npx,
-                                    cudaStream_t s);
+// dense reference-layout score and octave maps from the sparse ones
+cudaError_t launch_expand_score_map(const uint32_t* occ, const float* vmap, const uint8_t* oct8, float* vmap_dense,
+                                    int* layer_dense, long long npx, cudaStream_t s);
 cudaError_t launch_describe(const Batch& b, int total_max_pts, cudaStream_t s, int blocks_per_sm = 8);
 
 struct MatchArgs {

@@ -128,7 +128,7 @@ ORBX_API int orbx_match_knn2_static(const uint8_t* d_q, int nq, const uint8_t* d
 
 /* A frame pair end to end: detect + describe A and B in shared launches, then
  * match A -> B (Orbor::detectAndCompute x2 + Orbor::match, main.cpp:233-243).
- * Replayed from a CUDA graph cached per (shape, pointers). */
+ * Calls that repeat the shape and buffers of the call before replay a CUDA graph. */
 ORBX_API int orbx_pair(orbx_ctx* ctx, const uint8_t* d_img_a, const uint8_t* d_img_b, int w, int h, int pitch,
                        orbx_point* d_pts_a, uint8_t* d_desc_a, int* d_n_a, orbx_point* d_pts_b,
                        uint8_t* d_desc_b, int* d_n_b, int mode);
@@ -295,8 +295,9 @@ ORBX_API int orbx_bounds_set_slack(orbx_ctx* ctx, long long bytes);
  * runs in shared launches (one per stage for the whole batch), then every pair
  * is matched A -> B in one launch; or, with tuning batch_form = 1, all of it
  * runs in one persistent launch whose blocks claim (stage, frame, tile) work
- * items from a device queue, waiting per frame on the stage before.  Replayed
- * from a CUDA graph cached per (shapes, pointers, tuning).  Per pair the results are identical to
+ * items from a device queue, waiting per frame on the stage before.  Calls that
+ * repeat the shapes and tuning of the call before replay a CUDA graph, with
+ * other buffers too.  Per pair the results are identical to
  * orbx_pair on that pair with the same cap.  This batches what the reference
  * does one Orbor::detectAndCompute / Orbor::match call at a time
  * (orb.cpp:57-113).  Asynchronous. */
