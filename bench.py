@@ -439,7 +439,7 @@ def run_orbx(args, world, rank, local):
             imma_ms.append(e0.elapsed_time(e1))
     imma_pa, _ = A.to_host()
 
-    # both forms of the device-resident pair: five graph-replayed launches and
+    # both forms of the device-resident pair: five chained launches and
     # one persistent launch with a device work queue
     pair_forms = {}
     keep_t = ctx.get_tuning()
@@ -596,7 +596,7 @@ def run_orbx(args, world, rank, local):
             "scaling": "weak", "vs_baseline": None, "dtype": "u8",
             "data": "synthetic (seeded blobs + polygons + noise, homography-warped partner; cuda-orb_b200/synth.py)",
             "config": pair_config(n, na, nb),
-            "impl_detail": {"matcher": "XOR-popc", "graph": "one CUDA graph per pair (5 kernels)",
+            "impl_detail": {"matcher": "XOR-popc", "launches": "five chained kernels per pair",
                             "matches": matched},
             "e2e": {"value": e2e_total / (e2e_steps * world), "unit": "ms", "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h, "median_ms": statistics.median(e_ms), "steps": e2e_steps,

@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(kDescWarps * 32) k_describe(const __grid_const
   if (!INL && nf <= 8 && (int)threadIdx.x < nf * kFrameLines)
     asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(b.frames + threadIdx.x / kFrameLines) +
                                                   128 * (threadIdx.x % kFrameLines)));
+  chain_wait();
   // exclusive prefix of the per-frame keypoint counts (written by k_nms):
   // thread t scans frames [t*per, (t+1)*per)
   {
@@ -78,22 +79,10 @@ cudaError_t launch_describe(const Batch& b, int total_max_pts, cudaStream_t s, i
   const int cap = 148 * (blocks_per_sm > 0 ? blocks_per_sm : 8);
   if (blocks > cap) blocks = cap;
   const dim3 g(blocks), t(kDescWarps * 32);
-  if (b.n_inline > 0) {
-    if (b.wta_k == 3)
-      k_describe<3, true><<<g, t, 0, s>>>(b);
-    else if (b.wta_k == 4)
-      k_describe<4, true><<<g, t, 0, s>>>(b);
-    else
-      k_describe<2, true><<<g, t, 0, s>>>(b);
-  } else {
-    if (b.wta_k == 3)
-      k_describe<3, false><<<g, t, 0, s>>>(b);
-    else if (b.wta_k == 4)
-      k_describe<4, false><<<g, t, 0, s>>>(b);
-    else
-      k_describe<2, false><<<g, t, 0, s>>>(b);
-  }
-  return cudaGetLastError();
+  const bool inl = b.n_inline > 0;
+  if (b.wta_k == 3) return launch_chained(inl ? k_describe<3, true> : k_describe<3, false>, g, t, s, b);
+  if (b.wta_k == 4) return launch_chained(inl ? k_describe<4, true> : k_describe<4, false>, g, t, s, b);
+  return launch_chained(inl ? k_describe<2, true> : k_describe<2, false>, g, t, s, b);
 }
 
 }  // namespace orbx

@@ -13,12 +13,14 @@ namespace orbx {
 template <int TW, int TH, bool INL>
 __global__ void __launch_bounds__(kPyrThreads, 5) k_pyramid_blur(const __grid_constant__ Batch b) {
   __shared__ PyrSmem<TW, TH> sm;
+  chain_wait();
   pyr_tile<false, TW, TH, INL>(b, blockIdx.x, sm);
 }
 
 template <bool INL>
 __global__ void __launch_bounds__(256, 6) k_detect(const __grid_constant__ Batch b) {
   __shared__ DetSmem sm;
+  chain_wait();
   det_tile<false, INL>(b, blockIdx.x, sm);
 }
 
@@ -26,6 +28,7 @@ template <bool INL>
 __global__ void __launch_bounds__(256, 4) k_nms(const __grid_constant__ Batch b) {
   __shared__ NmsSmem sm;
   __shared__ int s_ticket;
+  chain_wait();
   if (threadIdx.x == 0) s_ticket = (int)atomicAdd(b.nms_ticket, 1u);
   __syncthreads();
   nms_strip<false, INL>(b, s_ticket, sm);
@@ -53,42 +56,27 @@ cudaError_t launch_expand_score_map(const uint32_t* occ, const float* vmap, cons
 cudaError_t launch_pyramid_blur(const Batch& b, int total_tiles, cudaStream_t s) {
   if (total_tiles <= 0) return cudaSuccess;
   const bool inl = b.n_inline > 0;
+  auto run = [&](auto* kernel) { return launch_chained(kernel, total_tiles, kPyrThreads, s, b); };
+#define PYR_SHAPE(i)                                                            \
+  (inl ? run(k_pyramid_blur<kPyrShapeTW[i], kPyrShapeTH[i], true>)              \
+       : run(k_pyramid_blur<kPyrShapeTW[i], kPyrShapeTH[i], false>))
   switch (b.pyr_shape) {
-    case 1:
-      if (inl) k_pyramid_blur<kPyrShapeTW[1], kPyrShapeTH[1], true><<<total_tiles, kPyrThreads, 0, s>>>(b);
-      else k_pyramid_blur<kPyrShapeTW[1], kPyrShapeTH[1], false><<<total_tiles, kPyrThreads, 0, s>>>(b);
-      break;
-    case 2:
-      if (inl) k_pyramid_blur<kPyrShapeTW[2], kPyrShapeTH[2], true><<<total_tiles, kPyrThreads, 0, s>>>(b);
-      else k_pyramid_blur<kPyrShapeTW[2], kPyrShapeTH[2], false><<<total_tiles, kPyrThreads, 0, s>>>(b);
-      break;
-    case 3:
-      if (inl) k_pyramid_blur<kPyrShapeTW[3], kPyrShapeTH[3], true><<<total_tiles, kPyrThreads, 0, s>>>(b);
-      else k_pyramid_blur<kPyrShapeTW[3], kPyrShapeTH[3], false><<<total_tiles, kPyrThreads, 0, s>>>(b);
-      break;
-    default:
-      if (inl) k_pyramid_blur<kPyrShapeTW[0], kPyrShapeTH[0], true><<<total_tiles, kPyrThreads, 0, s>>>(b);
-      else k_pyramid_blur<kPyrShapeTW[0], kPyrShapeTH[0], false><<<total_tiles, kPyrThreads, 0, s>>>(b);
+    case 1: return PYR_SHAPE(1);
+    case 2: return PYR_SHAPE(2);
+    case 3: return PYR_SHAPE(3);
+    default: return PYR_SHAPE(0);
   }
-  return cudaGetLastError();
+#undef PYR_SHAPE
 }
 
 cudaError_t launch_detect(const Batch& b, int total_tiles, cudaStream_t s) {
   if (total_tiles <= 0) return cudaSuccess;
-  if (b.n_inline > 0)
-    k_detect<true><<<total_tiles, 256, 0, s>>>(b);
-  else
-    k_detect<false><<<total_tiles, 256, 0, s>>>(b);
-  return cudaGetLastError();
+  return launch_chained(b.n_inline > 0 ? k_detect<true> : k_detect<false>, total_tiles, 256, s, b);
 }
 
 cudaError_t launch_nms(const Batch& b, int total_strips, cudaStream_t s) {
   if (total_strips <= 0) return cudaSuccess;
-  if (b.n_inline > 0)
-    k_nms<true><<<total_strips, 256, 0, s>>>(b);
-  else
-    k_nms<false><<<total_strips, 256, 0, s>>>(b);
-  return cudaGetLastError();
+  return launch_chained(b.n_inline > 0 ? k_nms<true> : k_nms<false>, total_strips, 256, s, b);
 }
 
 }  // namespace orbx

@@ -107,6 +107,10 @@ __device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned l
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+// Start of a kernel launched by launch_chained: waits until the kernels before
+// it on the stream have finished and their writes are visible.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Index of the frame whose tile range [base[f], base[f+1]) holds t.
 __device__ __forceinline__ int find_frame(const int* base, int n, int t) {
   int lo = 0, hi = n - 1;

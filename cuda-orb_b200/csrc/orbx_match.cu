@@ -15,12 +15,14 @@ namespace orbx {
 __global__ void __launch_bounds__(kMQ) k_match_popc(MatchArgs a, MatchWork w) {
   __shared__ uint4 s_db[kMChunk * 2];
   __shared__ unsigned int s_last;
+  chain_wait();
   match_popc_block<kMQ, false>(a, w, blockIdx.x, gridDim.x, s_db, s_last);
 }
 
 __global__ void __launch_bounds__(kMQ) k_match_popc_batch(const MatchJob* __restrict__ jobs) {
   __shared__ uint4 s_db[kMChunk * 2];
   __shared__ unsigned int s_last;
+  chain_wait();
   const MatchJob& J = jobs[blockIdx.y];
   match_popc_block<kMQ, false>(J.args, J.work, blockIdx.x, gridDim.x, s_db, s_last);
 }
@@ -36,14 +38,12 @@ int match_popc_blocks(int nq_cap, int splits_cap, int blocks_per_sm) {
 
 cudaError_t launch_match_popc(const MatchArgs& a, const MatchWork& w, cudaStream_t s, int blocks_per_sm) {
   if (w.nq_cap <= 0) return cudaSuccess;
-  k_match_popc<<<match_popc_blocks(w.nq_cap, w.splits_cap, blocks_per_sm), kMQ, 0, s>>>(a, w);
-  return cudaGetLastError();
+  return launch_chained(k_match_popc, match_popc_blocks(w.nq_cap, w.splits_cap, blocks_per_sm), kMQ, s, a, w);
 }
 
 cudaError_t launch_match_popc_batch(const MatchJob* d_jobs, int n_jobs, int blocks_per_job, cudaStream_t s) {
   if (n_jobs <= 0 || blocks_per_job <= 0) return cudaSuccess;
-  k_match_popc_batch<<<dim3(blocks_per_job, n_jobs), kMQ, 0, s>>>(d_jobs);
-  return cudaGetLastError();
+  return launch_chained(k_match_popc_batch, dim3(blocks_per_job, n_jobs), kMQ, s, d_jobs);
 }
 
 }  // namespace orbx

@@ -127,8 +127,7 @@ ORBX_API int orbx_match_knn2_static(const uint8_t* d_q, int nq, const uint8_t* d
                                     uint32_t* d_dist2, int32_t* d_idx2, void* cuda_stream);
 
 /* A frame pair end to end: detect + describe A and B in shared launches, then
- * match A -> B (Orbor::detectAndCompute x2 + Orbor::match, main.cpp:233-243).
- * Calls that repeat the shape and buffers of the call before replay a CUDA graph. */
+ * match A -> B (Orbor::detectAndCompute x2 + Orbor::match, main.cpp:233-243). */
 ORBX_API int orbx_pair(orbx_ctx* ctx, const uint8_t* d_img_a, const uint8_t* d_img_b, int w, int h, int pitch,
                        orbx_point* d_pts_a, uint8_t* d_desc_a, int* d_n_a, orbx_point* d_pts_b,
                        uint8_t* d_desc_b, int* d_n_b, int mode);
@@ -240,7 +239,7 @@ typedef struct orbx_tuning {
   int upload_bands;           /* orbx_pair_host: 0 = copy both images, then run the pair; 1..16 = copy them in
                                  this many row bands per image on a second stream while one persistent launch
                                  already processes the bands that have arrived (popcount matching) */
-  int pair_form;              /* orbx_pair: 0 = five graph-replayed launches, 1 = one persistent launch
+  int pair_form;              /* orbx_pair: 0 = five chained launches, 1 = one persistent launch
                                  (popcount matching) */
   int pyr_tile;               /* pyramid + blur tile of the five-launch forms: 0 = 128 x 30, 1 = 64 x 32,
                                  2 = 128 x 16, 3 = 64 x 64 octave pixels (the persistent forms use 128 x 30) */
