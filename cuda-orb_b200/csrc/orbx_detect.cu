@@ -10,11 +10,11 @@ namespace orbx {
 
 // Kernels take the batch as a grid constant so that, for batches whose frame
 // table travels in the launch parameters (INL), the stages read it in place.
-template <int TW, int TH, bool INL>
-__global__ void __launch_bounds__(kPyrThreads, 5) k_pyramid_blur(const __grid_constant__ Batch b) {
-  __shared__ PyrSmem<TW, TH> sm;
+template <int TH, bool INL>
+__global__ void __launch_bounds__(kPyrThreads, 4) k_pyramid_blur(const __grid_constant__ Batch b) {
+  __shared__ PyrSmem<TH> sm;
   chain_wait();
-  pyr_tile<false, TW, TH, INL>(b, blockIdx.x, sm);
+  pyr_tile<false, TH, INL>(b, blockIdx.x, sm);
 }
 
 template <bool INL>
@@ -57,9 +57,7 @@ cudaError_t launch_pyramid_blur(const Batch& b, int total_tiles, cudaStream_t s)
   if (total_tiles <= 0) return cudaSuccess;
   const bool inl = b.n_inline > 0;
   auto run = [&](auto* kernel) { return launch_chained(kernel, total_tiles, kPyrThreads, s, b); };
-#define PYR_SHAPE(i)                                                            \
-  (inl ? run(k_pyramid_blur<kPyrShapeTW[i], kPyrShapeTH[i], true>)              \
-       : run(k_pyramid_blur<kPyrShapeTW[i], kPyrShapeTH[i], false>))
+#define PYR_SHAPE(i) (inl ? run(k_pyramid_blur<kPyrShapeTH[i], true>) : run(k_pyramid_blur<kPyrShapeTH[i], false>))
   switch (b.pyr_shape) {
     case 1: return PYR_SHAPE(1);
     case 2: return PYR_SHAPE(2);

@@ -12,16 +12,13 @@ constexpr int kMaxFramesPerLaunch = 1024;
 constexpr int kInlineFrames = 2;  // frames carried in the launch parameters (a pair)
 constexpr size_t kGuard = 256 * 1024; // zeroed bytes before/after each pyramid
 
-// Pyramid-and-blur tile (octave pixels): the default shape, which the
-// persistent kernel uses; the five-launch kernel also has the other shapes of
-// kPyrShapeTW/TH (tuning pyr_tile), one instantiation each
+// Pyramid-and-blur tile (octave pixels): kPyrTW columns and one of these heights
+// (tuning pyr_tile; 0 picks by size, pyr_shape_for).  The persistent kernel uses
+// the tall one
 constexpr int kPyrThreads = 256;  // threads of every block that runs pyramid tiles
 constexpr int kPyrShapes = 4;
-// 128 x 30 keeps a tile's shared memory (44.1 KB) under the 44.6 KB of five
-// blocks per SM, and a 1080p pair's 1,460 tiles within two waves of them
-constexpr int kPyrShapeTW[kPyrShapes] = {128, 64, 128, 64};
-constexpr int kPyrShapeTH[kPyrShapes] = {30, 32, 16, 64};
-constexpr int kPyrTW = kPyrShapeTW[0];
+constexpr int kPyrShapeTH[kPyrShapes] = {58, 26, 42, 58};
+constexpr int kPyrTW = 128;
 constexpr int kPyrTH = kPyrShapeTH[0];
 // Detect tile (level-0 pixels); 32 keeps octave 4/5 tiles whole
 constexpr int kDetTW = 64;
@@ -86,7 +83,7 @@ struct Frame {
   int max_pts;
   int border;    // max(edge_threshold, 3)
   // tiling
-  int pyr_shape;  // index into kPyrShapeTW/TH of the pyramid tile tables below
+  int pyr_shape;  // index into kPyrShapeTH of the pyramid tile tables below
   int pyr_tiles_x[kMaxOctaves], pyr_tiles_y[kMaxOctaves];
   int pyr_tile_base[kMaxOctaves + 1];  // per-octave prefix within the frame
   int det_tiles_x, det_tiles_y;

@@ -31,7 +31,7 @@
 namespace orbx {
 
 union PersistSmem {
-  PyrSmem<kPyrTW, kPyrTH> pyr;
+  PyrSmem<kPyrTH> pyr;
   DetSmem det;
   NmsSmem nms;
   struct {
@@ -152,9 +152,9 @@ __global__ void __launch_bounds__(kPersistThreads, 4) k_batch_persistent(Persist
         if (p.upload_flags) {
           const int rows = pyr_tile_rows(b.frames[f], local);
           stage_wait(p.upload_flags + f, (rows + p.band_rows - 1) / p.band_rows, b.err, b.wait_cycles);
-          pyr_tile<true>(b, __ldg(b.pyr_base + f) + local, sm.pyr);
+          pyr_tile<true, kPyrTH>(b, __ldg(b.pyr_base + f) + local, sm.pyr);
         } else {
-          pyr_tile<false>(b, __ldg(b.pyr_base + f) + local, sm.pyr);
+          pyr_tile<false, kPyrTH>(b, __ldg(b.pyr_base + f) + local, sm.pyr);
         }
         int* row_ctr = nullptr;
         if (p.rows) {

@@ -57,11 +57,25 @@ __device__ __forceinline__ int find_frame_in(const int* base, int n, int t) {
 // (gDownSampleUnroll4, orbd.cu:514-535; octave 0 is a copy, orbd.cu:1584).
 // The blurred pyramid is the separable 7-tap sigma-2 filter of each octave with
 // reflect-101 borders (gConv2dUnroll, orbd.cu:1273-1338), computed here out of
-// place, so it has no dependence on block scheduling.  One block owns a
-// kPyrTW x kPyrTH octave tile: it stages the tile plus a 3-pixel reflected
-// halo in shared memory, writes the raw tile, and blurs it.  With pyr_src set
-// the octaves are read from an existing pyramid instead (hGassianBlur on a
+// place, so it has no dependence on block scheduling.  With pyr_src set the
+// octaves are read from an existing pyramid instead (hGassianBlur on a
 // caller's buffer, orbd.cu:1732-1773).
+//
+// What bounds it: instruction issue (a pixel needs 14 FP32 operations and 1.9
+// bytes of traffic), and on one frame the latency of a block's two passes.  A
+// block takes kPyrTW columns and TH rows.  First, 8 threads per source row (TH +
+// 6 of them) each read the words of 8 columns of the tile's left half and of 8
+// of its right half straight from global memory, store the raw bytes, and filter
+// the row: the two halves sit in the two halves of packed FP32 registers, so one
+// instruction filters two pixels, and 8 columns share 14 byte-to-float
+// conversions.  Only the filtered rows go through shared memory.  Then each
+// thread takes 4 columns of both halves and 4 consecutive rows, for which it
+// reads 10 filtered rows.  The code that one block runs through is kept short
+// (few unrolled copies, one word-load form per octave): on a frame of one wave
+// of blocks its instruction fetch is part of the time.  For a 1920x1080 pair the
+// form before, which staged bytes and floats of a 128 x 30 tile in shared memory
+// and filtered every row by itself, took 9.09 M warp instructions; this one
+// takes 5.6 M with 58 rows.  24 mixed pairs (147 Mpixel): 558 -> 305 us.
 // ---------------------------------------------------------------------------
 
 // Exact small-integer <-> float conversions on the full-rate pipes: a float
@@ -83,69 +97,104 @@ __device__ __forceinline__ float2 gauss_dot4x2(const float2* k, float2 t0, float
   acc = __ffma2_rn(k[2], t2, acc);
   return __ffma2_rn(k[3], t3, acc);
 }
-// One 4-byte group of staged source columns cx .. cx+3 of a row (reflect-101 at
-// the octave edges).  words: the row is level 0 of a 4-byte aligned image, so
-// interior groups take two aligned words (cx is one past a multiple of 4).
-template <bool PL>
-__device__ __forceinline__ uint32_t pyr_stage_word(const uint8_t* rowp, int cx, int ow, int sh, bool words,
-                                                   BoundsRec* rec, Span src) {
-  if (words && cx >= 1 && cx + 3 < ow) {
-    // bytes cx-1 .. cx+6 lie in [0, pitch_in): cx + 3 < ow <= pitch_in and both words are aligned
-    const uint32_t* wp = reinterpret_cast<const uint32_t*>(rowp + (cx - 1));
-    if (!ORBX_IN(rec, kSitePyrLoad, src, wp, 8)) return 0u;
-    return __byte_perm(ldx<PL>(wp), ldx<PL>(wp + 1), 0x4321);
+
+// Source of one octave's rows.
+struct PyrSrc {
+  const uint8_t* base;
+  long long pitch;  // bytes between octave rows
+  int sh;           // log2 of the bytes between octave pixels
+  int ow;
+  Span span;
+  BoundsRec* rec;
+};
+// How four neighbouring pixels of an octave row load as one word.
+enum : int {
+  kPyrWord = 0,    // octave 0 (or a caller's pyramid): an aligned word
+  kPyrEvery2 = 1,  // octave 1: every second byte of 8 aligned bytes
+  kPyrEvery4 = 2,  // octave 2: every fourth byte of 16 aligned bytes
+  kPyrBytes = 3    // octaves 3, 4 and images whose base or pitch is not aligned: four byte loads
+};
+// Octave columns 4 w .. 4 w + 3 of a row (w inside the octave; columns past its
+// last one hold anything).  An aligned word of a row's last pixel ends inside
+// the row's pitch at octave 0, and at octaves 1 and 2 at worst in the image row
+// below, which exists since octave rows are 2 or 4 image rows apart; byte loads
+// stop at the last pixel.
+template <bool PL, int KIND>
+__device__ __forceinline__ uint32_t pyr_word(const PyrSrc& p, const uint8_t* row, int w) {
+  if constexpr (KIND != kPyrBytes) {
+    const uint8_t* q = row + ((4 << KIND) * w);
+    if (!ORBX_IN(p.rec, kSitePyrLoad, p.span, q, 4 << KIND)) return 0u;
+    if constexpr (KIND == kPyrWord) {
+      return ldx<PL>(reinterpret_cast<const uint32_t*>(q));
+    } else if constexpr (KIND == kPyrEvery2) {
+      const uint2 v = ldx<PL>(reinterpret_cast<const uint2*>(q));
+      return __byte_perm(v.x, v.y, 0x6420);
+    } else {
+      const uint4 v = ldx<PL>(reinterpret_cast<const uint4*>(q));
+      return pack_low_bytes(v.x, v.y, v.z, v.w);
+    }
+  } else {
+    uint32_t v[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint8_t* q = row + (min(4 * w + j, p.ow - 1) << p.sh);
+      v[j] = ORBX_IN(p.rec, kSitePyrLoad, p.span, q, 1) ? ldx<PL>(q) : 0u;
+    }
+    return pack_low_bytes(v[0], v[1], v[2], v[3]);
   }
+}
+
+// The words of columns x - 4 .. x + 11 of a row (x a multiple of 8), columns
+// outside the octave reflected (reflect-101).  The four words are loaded with
+// their indices clamped to the octave; a reflected column that an output needs
+// (at most 3 past an edge) lies in one of them, and with n = ow - x columns left
+// from x on, byte selectors put it in place: column n + e is column n - 2 - e.
+// out[1] takes bytes of words (0, 1), out[2] of (n <= 4 ? 0 : 2, 1), out[3] of
+// (n <= 8 ? 1 : 3, 2), in that order; n >= 12 is the identity.
+__device__ __constant__ uint16_t kPyrSel[13][3] = {
+    {0x0000, 0x0000, 0x0000}, {0x1234, 0x0000, 0x0000}, {0x3454, 0x0002, 0x0000},
+    {0x5654, 0x0034, 0x0000}, {0x7654, 0x0456, 0x0000}, {0x7654, 0x5670, 0x0000},
+    {0x7654, 0x7010, 0x0002}, {0x7654, 0x1210, 0x0034}, {0x7654, 0x3210, 0x0456},
+    {0x7654, 0x3210, 0x5670}, {0x7654, 0x3210, 0x7010}, {0x7654, 0x3210, 0x1210},
+    {0x7654, 0x3210, 0x3210}};
+template <bool PL, int KIND>
+__device__ __forceinline__ void pyr_words_edge(const PyrSrc& p, const uint8_t* row, int x, uint32_t out[4]) {
+  const int n = min(max(p.ow - x, 0), 12);
+  const int w = x >> 2, last = (p.ow - 1) >> 2;
   uint32_t v[4];
 #pragma unroll
-  for (int j = 0; j < 4; j++) {
-    const uint8_t* p = rowp + (reflect101(cx + j, ow) << sh);
-    v[j] = ORBX_IN(rec, kSitePyrLoad, src, p, 1) ? ldx<PL>(p) : 0u;
-  }
-  return pack_low_bytes(v[0], v[1], v[2], v[3]);
+  for (int i = 0; i < 4; i++) v[i] = pyr_word<PL, KIND>(p, row, min(max(w - 1 + i, 0), last));
+  out[0] = x == 0 ? __byte_perm(v[1], 0u, 0x1230) : v[0];  // columns -3, -2, -1 are columns 3, 2, 1
+  out[1] = __byte_perm(v[0], v[1], kPyrSel[n][0]);
+  out[2] = __byte_perm(n <= 4 ? v[0] : v[2], v[1], kPyrSel[n][1]);
+  out[3] = __byte_perm(n <= 8 ? v[1] : v[3], v[2], kPyrSel[n][2]);
 }
-// Row-major walk over items (r, g) with W items per row: item threadIdx.x +
-// k * T for k = 0, 1, .. in a block of T threads, stepped without a division.
-template <int W, int T>
-struct RowWalk {
-  int r, g;
-  __device__ __forceinline__ RowWalk() : r(threadIdx.x / W), g(threadIdx.x % W) {}
-  __device__ __forceinline__ void next() {
-    r += T / W;
-    g += T % W;
-    if (g >= W) {
-      g -= W;
-      r++;
+// The same for a thread's columns of both halves of a tile; inside: the tile's
+// words all lie in the octave.
+template <bool PL, int KIND>
+__device__ __forceinline__ void pyr_words(const PyrSrc& p, const uint8_t* row, int x, bool inside, uint32_t wl[4],
+                                          uint32_t wr[4]) {
+  constexpr int kHalf = kPyrTW / 2;
+  if (inside) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      wl[i] = pyr_word<PL, KIND>(p, row, (x >> 2) - 1 + i);
+      wr[i] = pyr_word<PL, KIND>(p, row, (x >> 2) - 1 + i + kHalf / 4);
     }
+  } else {
+    pyr_words_edge<PL, KIND>(p, row, x, wl);
+    pyr_words_edge<PL, KIND>(p, row, x + kHalf, wr);
   }
-};
+}
 
-// Staged source of a TW x TH tile.  The filters run on column pairs: pair k of a
-// row holds column k of the tile's left half and column k of its right half
-// (each half with its 3-pixel halo on both sides), so one packed instruction
-// filters two output columns.  Pairs are grouped two to a 16-byte slot, and a
-// row's even slots are stored before its odd slots: a thread that works on
-// slots 2g, 2g+1, .. reads slot 2g+m of its row at (m odd) * half + g + m/2,
-// so the lanes of a warp read consecutive 16-byte words for every m.  The raw
-// bytes are staged linearly.
-template <int TW, int TH>
-struct PyrSmem {
-  static constexpr int HW = TW / 2;   // columns per half
-  static constexpr int SW = TW + 8;   // staged bytes per row
-  static constexpr int SW2 = HW + 8;  // staged column pairs per row (3 + HW + 3, padded to 4)
-  static constexpr int SH = TH + 6;
-  __align__(16) float2 src[SH * SW2];
-  __align__(16) uint8_t byte[SH * SW];
-  __align__(16) float2 row[SH * HW];
-};
-
-// Position of pyramid tile t (tile index over the batch) of shape TW x TH.
+// Position of pyramid tile t (tile index over the batch) of TH rows.
 struct PyrTile {
   int f;       // frame
   int o;       // octave
   int lt;      // tile index within the octave
   int x0, y0;  // octave-pixel origin
 };
-template <bool INL, int TW, int TH>
+template <bool INL, int TH>
 __device__ __forceinline__ PyrTile pyr_tile_at(const Batch& b, int t) {
   const int* base = INL ? b.inl_pyr_base : b.pyr_base;
   PyrTile g;
@@ -158,59 +207,50 @@ __device__ __forceinline__ PyrTile pyr_tile_at(const Batch& b, int t) {
   const int tiles_x = F.pyr_tiles_x[o];
   g.o = o;
   g.lt = lt;
-  g.x0 = (lt % tiles_x) * TW;
-  g.y0 = (lt / tiles_x) * TH;
+  const int ty = lt / tiles_x;
+  g.x0 = (lt - ty * tiles_x) * kPyrTW;
+  g.y0 = ty * TH;
   return g;
 }
 
-template <int TW, int TH>
-__host__ __device__ constexpr int pyr_stage_items() {
-  return (PyrSmem<TW, TH>::SH * (PyrSmem<TW, TH>::SW2 / 4) + kPyrThreads - 1) / kPyrThreads;
-}
+// The horizontally filtered rows of a tile.  Column k of the left half and
+// column k of the right half form pair k; two pairs are a 16-byte slot, and
+// slot 4 g + m of a row lies at m * 8 + (g + 4 (m >> 1)) % 8, so that the 8
+// threads that write a row and the 16 that read it touch distinct banks.
+constexpr int kPyrRowSlots = kPyrTW / 4;
+__device__ __forceinline__ int pyr_slot(int g, int m) { return m * 8 + ((g + 4 * (m >> 1)) & 7); }
+template <int TH>
+struct PyrSmem {
+  float4 row[(TH + 6) * kPyrRowSlots];
+};
 
-// Staging loads of tile g: source rows y0-3 .. y0+TH+2; item (r, g) takes
-// columns 4g-3 .. 4g of the left half and of the right half (tile-relative),
-// reflect-101 at the octave edges.  All of a thread's loads are issued before
-// any is used (blocks have kPyrThreads threads).
-template <bool PL, int TW, int TH, bool INL>
-__device__ __forceinline__ void pyr_tile_load(const Batch& b, const PyrTile& g, uint32_t* wa, uint32_t* wb) {
-  using S = PyrSmem<TW, TH>;
-  constexpr int kHW = S::HW, kSH = S::SH, kGroups = S::SW2 / 4;
-  const Frame& F = batch_frame<INL>(b, g.f);
-  const int o = g.o, ow = F.ow[o], oh = F.oh[o], op = F.op[o];
-  const uint8_t* __restrict__ img = F.img;
-  const int pitch_in = F.pitch_in;
-  const uint8_t* __restrict__ psrc = F.pyr_src ? F.pyr_src + F.ooff[o] : nullptr;
-  const bool words0 = (o == 0) && !psrc && ((reinterpret_cast<uintptr_t>(img) | (uintptr_t)pitch_in) & 3u) == 0;
-  const int sh = psrc ? 0 : o;
-  const Span src = psrc ? Span{F.pyr_src, F.ooff[F.n_oct]} : img_span(F);
-  RowWalk<kGroups, kPyrThreads> w;
+// Four columns x .. x + 3 of octave row y as stored: columns past the row carry
+// the caller's padding (the reference copies h * pitch0 bytes, orbd.cu:1584) or
+// zeros.  x is below the octave's pitch.
+template <bool PL>
+__device__ __forceinline__ uint32_t pyr_padded(const PyrSrc& p, bool copy_pad, int x, int y, uint32_t v) {
+  const int n = p.ow - x;
+  if (n >= 4) return v;
+  const uint32_t mask = n <= 0 ? 0u : (1u << (8 * n)) - 1u;
+  uint32_t pad = 0u;
+  if (copy_pad) {
+    const uint8_t* q = p.base + y * p.pitch + x;
 #pragma unroll
-  for (int q = 0; q < pyr_stage_items<TW, TH>(); q++) {
-    wa[q] = wb[q] = 0u;
-    if (w.r < kSH) {
-      const int y = reflect101(g.y0 - 3 + w.r, oh);
-      const uint8_t* rowp = psrc ? psrc + (size_t)y * op : img + (size_t)(y << o) * pitch_in;
-      const int cx = g.x0 - 3 + 4 * w.g;
-      wa[q] = pyr_stage_word<PL>(rowp, cx, ow, sh, words0, b.bounds, src);
-      wb[q] = pyr_stage_word<PL>(rowp, cx + kHW, ow, sh, words0, b.bounds, src);
+    for (int j = 0; j < 4; j++) {
+      const uint32_t v1 = ORBX_IN(p.rec, kSitePyrPadLoad, p.span, q + j, 1) ? ldx<PL>(q + j) : 0u;
+      pad |= v1 << (8 * j);
     }
-    w.next();
   }
+  return (v & mask) | (pad & ~mask);
 }
 
-// The staged words of tile g into shared memory, as float pairs and as bytes,
-// plus the per-frame housekeeping of the frame's first tile.  No barrier.
-template <int TW, int TH, bool INL>
-__device__ __forceinline__ void pyr_tile_stage(const Batch& b, int t, const PyrTile& g, const uint32_t* wa,
-                                               const uint32_t* wb, PyrSmem<TW, TH>& sm) {
-  using S = PyrSmem<TW, TH>;
-  constexpr int kHW = S::HW, kSW = S::SW, kSH = S::SH;
-  constexpr int kRowSlots = S::SW2 / 2;  // 16-byte slots per staged pair row (two planes)
-  constexpr int kGroups = S::SW2 / 4;    // staging items per row = slots per plane of a staged row
-  static_assert(TW % 16 == 0 && S::SW2 % 4 == 0, "pyramid tile width");
-  float4* s_src = reinterpret_cast<float4*>(sm.src);
-  uint8_t* s_byte = sm.byte;
+// One pyramid tile (tile index t over the batch).  PL: the level-0 image is
+// copied in during the same launch (coherent loads instead of the read-only path).
+template <bool PL, int TH, bool INL = false>
+__device__ __forceinline__ void pyr_tile(const Batch& b, int t, PyrSmem<TH>& sm) {
+  static_assert(kPyrTW == 128 && kPyrThreads == 256 && (TH + 6) % 16 == 0, "thread layout of the two passes");
+  constexpr int kHalf = kPyrTW / 2;
+  const PyrTile g = pyr_tile_at<INL, TH>(b, t);
   const Frame& F = batch_frame<INL>(b, g.f);
   if (g.o == 0 && g.lt == 0) {
     for (int i = threadIdx.x; i < F.nms_strips; i += blockDim.x)
@@ -221,160 +261,135 @@ __device__ __forceinline__ void pyr_tile_stage(const Batch& b, int t, const PyrT
     }
   }
   if (t == 0 && threadIdx.x == 0) *b.nms_ticket = 0u;
-  const float2 m23 = pair2(-8388608.0f);
-  RowWalk<kGroups, kPyrThreads> w;
-#pragma unroll
-  for (int q = 0; q < pyr_stage_items<TW, TH>(); q++, w.next()) {
-    const int r = w.r, gg = w.g;
-    if (r >= kSH) break;
-    // pair j = (byte j of wa, byte j of wb) as floats: 2^23 + byte, minus 2^23
-    const float2 p0 = __fadd2_rn(make_float2(byte_bits(wa[q], 0x7540u), byte_bits(wb[q], 0x7540u)), m23);
-    const float2 p1 = __fadd2_rn(make_float2(byte_bits(wa[q], 0x7541u), byte_bits(wb[q], 0x7541u)), m23);
-    const float2 p2 = __fadd2_rn(make_float2(byte_bits(wa[q], 0x7542u), byte_bits(wb[q], 0x7542u)), m23);
-    const float2 p3 = __fadd2_rn(make_float2(byte_bits(wa[q], 0x7543u), byte_bits(wb[q], 0x7543u)), m23);
-    // pairs 4g .. 4g+3 = slots 2g (even plane) and 2g+1 (odd plane) of row r
-    float4* row = s_src + r * kRowSlots + gg;
-    row[0] = make_float4(p0.x, p0.y, p1.x, p1.y);
-    row[kGroups] = make_float4(p2.x, p2.y, p3.x, p3.y);
-    // the halves' halos overlap in the middle: both writes there store the same bytes
-    *reinterpret_cast<uint32_t*>(s_byte + r * kSW + 4 * gg) = wa[q];
-    *reinterpret_cast<uint32_t*>(s_byte + r * kSW + kHW + 4 * gg) = wb[q];
+  const int o = g.o, oh = F.oh[o];
+  PyrSrc src;
+  src.rec = b.bounds;
+  src.ow = F.ow[o];
+  if (F.pyr_src) {
+    src.base = F.pyr_src + F.ooff[o];
+    src.pitch = F.op[o];
+    src.sh = 0;
+    src.span = Span{F.pyr_src, F.ooff[F.n_oct]};
+  } else {
+    src.base = F.img;
+    src.pitch = (long long)F.pitch_in << o;
+    src.sh = o;
+    src.span = img_span(F);
   }
-}
-
-// Blur of the staged tile g and the stores of its raw and blurred bytes:
-// a barrier, the horizontal pass, a barrier, the vertical pass.  PL: the
-// level-0 image was written earlier in the same launch.
-template <bool PL, int TW, int TH, bool INL>
-__device__ __forceinline__ void pyr_tile_filter(const Batch& b, const PyrTile& g, PyrSmem<TW, TH>& sm) {
-  using S = PyrSmem<TW, TH>;
-  constexpr int kHW = S::HW, kSW = S::SW, kSH = S::SH;
-  constexpr int kRowSlots = S::SW2 / 2;
-  constexpr int kOutSlots = kHW / 2;     // 16-byte slots per filtered pair row (two planes)
-  constexpr int kGroups = S::SW2 / 4;
-  float4* s_src = reinterpret_cast<float4*>(sm.src);
-  float4* s_row = reinterpret_cast<float4*>(sm.row);
-  uint8_t* s_byte = sm.byte;
-  const Frame& F = batch_frame<INL>(b, g.f);
-  const int o = g.o, x0 = g.x0, y0 = g.y0;
-  const int ow = F.ow[o], oh = F.oh[o], op = F.op[o];
-  const uint8_t* __restrict__ img = F.img;
-  const int pitch_in = F.pitch_in;
-  const uint8_t* __restrict__ psrc = F.pyr_src ? F.pyr_src + F.ooff[o] : nullptr;
-  __syncthreads();
+  const bool aligned = ((reinterpret_cast<uintptr_t>(src.base) | (uintptr_t)src.pitch) & ((4u << src.sh) - 1u)) == 0;
+  const int kind = src.sh <= 2 && aligned ? src.sh : kPyrBytes;
+  const bool copy_pad = F.pyr_src || (o == 0 && F.pitch_in == F.op[0]);
+  const bool full = g.x0 + kPyrTW <= src.ow;
+  const bool inside = g.x0 > 0 && g.x0 + kPyrTW + 4 <= src.ow;
 
   float2 k[4];
 #pragma unroll
   for (int i = 0; i < 4; i++) k[i] = pair2(b.gauss[i]);
-  // horizontal pass: 4 consecutive output pairs per thread; integer tap sums
-  // are exact in float, so they are summed as floats
-  constexpr int kHG = kHW / 4;  // items per row = slots per plane of a filtered row
-  for (RowWalk<kHG, kPyrThreads> w; w.r < kSH; w.next()) {
-    const int r = w.r, g = w.g;
-    const float4* row = s_src + r * kRowSlots + g;
-    // slots 2g .. 2g+4: even plane g, g+1, g+2 and odd plane g, g+1
-    const float4 e0 = row[0], o0 = row[kGroups], e1 = row[1], o1 = row[kGroups + 1], e2 = row[2];
-    const float2 p[10] = {make_float2(e0.x, e0.y), make_float2(e0.z, e0.w), make_float2(o0.x, o0.y),
-                          make_float2(o0.z, o0.w), make_float2(e1.x, e1.y), make_float2(e1.z, e1.w),
-                          make_float2(o1.x, o1.y), make_float2(o1.z, o1.w), make_float2(e2.x, e2.y),
-                          make_float2(e2.z, e2.w)};
-    float2 q[4];
+  // rows: thread (row, gc) filters columns 8 gc .. 8 gc + 7 of both halves
+  {
+    const float2 m23 = pair2(-8388608.0f);
+    const int gc = threadIdx.x & 7;
+    const int xl = g.x0 + 8 * gc, xr = xl + kHalf;
+#pragma unroll 1
+    for (int r = threadIdx.x >> 3; r < TH + 6; r += 32) {
+      const int yy = g.y0 - 3 + r;
+      if (yy >= oh + 3) break;  // rows below the octave's halo reach no output
+      const uint8_t* row = src.base + reflect101(yy, oh) * src.pitch;
+      uint32_t wl[4], wr[4];  // columns x - 4 .. x + 11
+      int x = xl;
+      asm volatile("" : "+r"(x));  // offsets and selectors formed per row: kept across rows they would spill
+      switch (kind) {
+        case kPyrWord: pyr_words<PL, kPyrWord>(src, row, x, inside, wl, wr); break;
+        case kPyrEvery2: pyr_words<PL, kPyrEvery2>(src, row, x, inside, wl, wr); break;
+        case kPyrEvery4: pyr_words<PL, kPyrEvery4>(src, row, x, inside, wl, wr); break;
+        default: pyr_words<PL, kPyrBytes>(src, row, x, inside, wl, wr);
+      }
+      if (r >= 3 && r < TH + 3 && yy < oh) {
+        uint32_t c[4] = {wl[1], wl[2], wr[1], wr[2]};
+        if (!full) {
 #pragma unroll
-    for (int j = 0; j < 4; j++)
-      q[j] = gauss_dot4x2(k, p[j + 3], __fadd2_rn(p[j + 2], p[j + 4]), __fadd2_rn(p[j + 1], p[j + 5]),
-                          __fadd2_rn(p[j], p[j + 6]));
-    float4* out = s_row + r * kOutSlots + g;
-    out[0] = make_float4(q[0].x, q[0].y, q[1].x, q[1].y);
-    out[kHG] = make_float4(q[2].x, q[2].y, q[3].x, q[3].y);
-  }
-  __syncthreads();
-
-  // vertical pass and stores: 4 consecutive column pairs of one row per thread
-  uint8_t* P = F.pyr + F.ooff[o];
-  uint8_t* B = F.blr + F.ooff[o];
-  const bool copy_pad = (o == 0) && (pitch_in == op);
-  const float2 rne = pair2(12582912.0f);
-  for (RowWalk<kHG, kPyrThreads> w; w.r < TH; w.next()) {
-    const int r = w.r, g = w.g;
-    const int y = y0 + r;
-    if (y >= oh) continue;
-    float2 h[7][4];
-    const float4* col = s_row + r * kOutSlots + g;
-#pragma unroll
-    for (int i = 0; i < 7; i++) {
-      const float4 v0 = col[i * kOutSlots], v1 = col[i * kOutSlots + kHG];
-      h[i][0] = make_float2(v0.x, v0.y);
-      h[i][1] = make_float2(v0.z, v0.w);
-      h[i][2] = make_float2(v1.x, v1.y);
-      h[i][3] = make_float2(v1.z, v1.w);
-    }
-    // rounded to the nearest integer, ties to even, by adding 1.5 * 2^23: the
-    // result's low byte is the blurred pixel (0 <= v <= 255)
-    uint32_t ua[4], ub[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const float2 v = __fadd2_rn(gauss_dot4x2(k, h[3][j], __fadd2_rn(h[2][j], h[4][j]),
-                                               __fadd2_rn(h[1][j], h[5][j]), __fadd2_rn(h[0][j], h[6][j])),
-                                  rne);
-      ua[j] = __float_as_uint(v.x);
-      ub[j] = __float_as_uint(v.y);
-    }
-    const uint8_t* sb = s_byte + (r + 3) * kSW + 4 * g;
-#pragma unroll
-    for (int half = 0; half < 2; half++) {
-      const int x = x0 + half * kHW + 4 * g;
-      if (x >= op) continue;
-      const uint32_t bw = half ? pack_low_bytes(ub[0], ub[1], ub[2], ub[3]) : pack_low_bytes(ua[0], ua[1], ua[2], ua[3]);
-      // raw bytes of the same 4 pixels: staged columns 4g+3 .. 4g+6 of the half
-      const uint32_t* sw = reinterpret_cast<const uint32_t*>(sb + half * kHW);
-      const uint32_t pw = __byte_perm(sw[0], sw[1], 0x6543);
-      const size_t a = (size_t)y * op + x;
-      if (x + 4 <= ow) {
-        if (ORBX_IN(b.bounds, kSitePyrStore, octave_span(F.blr, F, o), B + a, 4))
-          *reinterpret_cast<uint32_t*>(B + a) = bw;
-        if (ORBX_IN(b.bounds, kSitePyrStore, octave_span(F.pyr, F, o), P + a, 4))
-          *reinterpret_cast<uint32_t*>(P + a) = pw;
-      } else {
-        // the group reaches into the row padding: octave 0 carries the caller's
-        // padding bytes (the reference copies h * pitch0 bytes, orbd.cu:1584),
-        // other octaves hold zeros
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          if (x + j < ow) {
-            if (ORBX_IN(b.bounds, kSitePyrStore, octave_span(F.blr, F, o), B + a + j, 1))
-              B[a + j] = (uint8_t)(bw >> (8 * j));
-            if (ORBX_IN(b.bounds, kSitePyrStore, octave_span(F.pyr, F, o), P + a + j, 1))
-              P[a + j] = (uint8_t)(pw >> (8 * j));
-          } else {
-            const uint8_t v =
-                psrc ? (ORBX_IN(b.bounds, kSitePyrPadLoad, (Span{F.pyr_src, F.ooff[F.n_oct]}), psrc + a + j, 1)
-                            ? ldx<PL>(psrc + a + j)
-                            : (uint8_t)0)
-                     : (copy_pad ? (ORBX_IN(b.bounds, kSitePyrPadLoad, img_span(F), img + (size_t)y * pitch_in + x + j, 1)
-                                        ? ldx<PL>(img + (size_t)y * pitch_in + x + j)
-                                        : (uint8_t)0)
-                                 : (uint8_t)0);
-            if (ORBX_IN(b.bounds, kSitePyrStore, octave_span(F.blr, F, o), B + a + j, 1)) B[a + j] = v;
-            if (ORBX_IN(b.bounds, kSitePyrStore, octave_span(F.pyr, F, o), P + a + j, 1)) P[a + j] = v;
-          }
+          for (int i = 0; i < 4; i++)
+            c[i] = pyr_padded<PL>(src, copy_pad, (i < 2 ? xl : xr) + 4 * (i & 1), yy, c[i]);
         }
+        uint8_t* q = F.pyr + F.ooff[o] + (long long)yy * F.op[o] + xl;
+        if (ORBX_IN(b.bounds, kSitePyrStore, octave_span(F.pyr, F, o), q, kHalf + 8)) {
+          *reinterpret_cast<uint2*>(q) = make_uint2(c[0], c[1]);
+          *reinterpret_cast<uint2*>(q + kHalf) = make_uint2(c[2], c[3]);
+        }
+      }
+      // pair j: column x - 3 + j of both halves as floats (2^23 + byte, minus
+      // 2^23); integer tap sums are exact in float, so they are summed as floats
+      float2 p[14];
+#pragma unroll
+      for (int j = 0; j < 14; j++) {
+        const uint32_t sel = 0x7540u + ((j + 1) & 3);
+        p[j] = __fadd2_rn(make_float2(byte_bits(wl[(j + 1) >> 2], sel), byte_bits(wr[(j + 1) >> 2], sel)), m23);
+      }
+      float4* out = sm.row + r * kPyrRowSlots;
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        float2 q[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          const int j = 2 * m + e;
+          q[e] = gauss_dot4x2(k, p[j + 3], __fadd2_rn(p[j + 2], p[j + 4]), __fadd2_rn(p[j + 1], p[j + 5]),
+                              __fadd2_rn(p[j], p[j + 6]));
+        }
+        out[pyr_slot(gc, m)] = make_float4(q[0].x, q[0].y, q[1].x, q[1].y);
       }
     }
   }
-}
+  __syncthreads();
 
-
-// One pyramid tile (tile index t over the batch) of shape TW x TH: it stages
-// the tile plus a 3-pixel reflected halo in shared memory, writes the raw
-// tile, and blurs it.  PL: the level-0 image is copied in during the same
-// launch (coherent loads instead of the read-only path).
-template <bool PL, int TW = kPyrTW, int TH = kPyrTH, bool INL = false>
-__device__ __forceinline__ void pyr_tile(const Batch& b, int t, PyrSmem<TW, TH>& sm) {
-  uint32_t wa[pyr_stage_items<TW, TH>()], wb[pyr_stage_items<TW, TH>()];
-  const PyrTile g = pyr_tile_at<INL, TW, TH>(b, t);
-  pyr_tile_load<PL, TW, TH, INL>(b, g, wa, wb);
-  pyr_tile_stage<TW, TH, INL>(b, t, g, wa, wb, sm);
-  pyr_tile_filter<PL, TW, TH, INL>(b, g, sm);
+  // columns: thread (run, cg) filters rows 4 run .. 4 run + 3 of column pairs
+  // 4 cg .. 4 cg + 3
+  const int cg = threadIdx.x & 15;
+  const int s0 = pyr_slot(cg >> 1, 2 * (cg & 1)), s1 = pyr_slot(cg >> 1, 2 * (cg & 1) + 1);
+  const int xl = g.x0 + 4 * cg, xr = xl + kHalf;
+  // rounded to the nearest integer, ties to even, by adding 1.5 * 2^23: the
+  // result's low byte is the blurred pixel (0 <= v <= 255)
+  const float2 rne = pair2(12582912.0f);
+#pragma unroll 1
+  for (int r0 = 4 * (threadIdx.x >> 4); r0 < TH; r0 += 64) {
+    if (g.y0 + r0 >= oh) break;
+    uint32_t ul[4] = {}, ur[4] = {};  // four blurred columns of each row, per half
+#pragma unroll 1
+    for (int c = 0; c < 2; c++) {  // two column pairs at a time: 40 registers of filtered rows
+      float2 h[10][2];
+#pragma unroll
+      for (int i = 0; i < 10; i++) {
+        const float4 v = sm.row[min(r0 + i, TH + 5) * kPyrRowSlots + (c ? s1 : s0)];
+        h[i][0] = make_float2(v.x, v.y);
+        h[i][1] = make_float2(v.z, v.w);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        float2 v[2];
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+          v[j] = __fadd2_rn(gauss_dot4x2(k, h[i + 3][j], __fadd2_rn(h[i + 2][j], h[i + 4][j]),
+                                         __fadd2_rn(h[i + 1][j], h[i + 5][j]), __fadd2_rn(h[i][j], h[i + 6][j])),
+                            rne);
+        const uint32_t l = __byte_perm(__float_as_uint(v[0].x), __float_as_uint(v[1].x), 0x0040);
+        const uint32_t r = __byte_perm(__float_as_uint(v[0].y), __float_as_uint(v[1].y), 0x0040);
+        ul[i] = __byte_perm(ul[i], l, 0x5432);
+        ur[i] = __byte_perm(ur[i], r, 0x5432);
+      }
+    }
+    uint8_t* q = F.blr + F.ooff[o] + (long long)(g.y0 + r0) * F.op[o] + xl;
+#pragma unroll
+    for (int i = 0; i < 4; i++, q += F.op[o]) {
+      const int y = g.y0 + r0 + i;
+      if (r0 + i >= TH || y >= oh) break;
+      if (!full) {
+        ul[i] = pyr_padded<PL>(src, copy_pad, xl, y, ul[i]);
+        ur[i] = pyr_padded<PL>(src, copy_pad, xr, y, ur[i]);
+      }
+      if (!ORBX_IN(b.bounds, kSitePyrStore, octave_span(F.blr, F, o), q, kHalf + 4)) continue;
+      *reinterpret_cast<uint32_t*>(q) = ul[i];
+      *reinterpret_cast<uint32_t*>(q + kHalf) = ur[i];
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------

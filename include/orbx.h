@@ -241,8 +241,8 @@ typedef struct orbx_tuning {
                                  already processes the bands that have arrived (popcount matching) */
   int pair_form;              /* orbx_pair: 0 = five chained launches, 1 = one persistent launch
                                  (popcount matching) */
-  int pyr_tile;               /* pyramid + blur tile of the five-launch forms: 0 = 128 x 30, 1 = 64 x 32,
-                                 2 = 128 x 16, 3 = 64 x 64 octave pixels (the persistent forms use 128 x 30) */
+  int pyr_tile;               /* pyramid + blur tile of the five-launch forms: 128 columns by 0 = 26 or 58 rows by
+                                 the launch's pixels, 1 = 26, 2 = 42, 3 = 58 octave rows (the persistent forms use 58) */
   int persist_row_deps;       /* persistent launches: 1 = a detect tile row waits only for the pyramid tile rows
                                  it reads (a frame's stages overlap row by row), 0 = for the whole frame */
   int host_overlap;           /* orbx_pair_host with upload_bands = 0: 1 (default) = image B is copied while
