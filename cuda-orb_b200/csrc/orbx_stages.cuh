@@ -406,68 +406,59 @@ __device__ __forceinline__ void pyr_tile(const Batch& b, int t, PyrSmem<TH>& sm)
 // addressing, so reads past an octave edge return the same neighbouring bytes
 // as in the reference, merges the octaves in shared memory, and writes the
 // tile's occupancy bits densely and its scores sparsely (no clearing pass).
+//
+// What bounds it: instruction issue (ALU pipe 56%, issue 60% of active cycles)
+// and, on one frame, the latency of its five phases.  Staging is one 16-byte load
+// per thread for octave 0 and one for the others together; the pre-test compares
+// two centres per instruction in 16-bit lanes; a Harris lane shares the column
+// sums and differences of its three rows between its seven columns.  A
+// 1920x1080 pair takes 10.1 M warp instructions (12.6 M with 4-byte staging,
+// byte-compare pre-test and per-column derivatives), 24 mixed pairs 442 us (541).
 // ---------------------------------------------------------------------------
-constexpr int kHalo = 4;
+constexpr int kHalo = 4;  // rows above and below, and the least columns to the sides
+// The stage of octave o: rows of det_sw(o) bytes, the tile's first column
+// det_left(o) bytes in.  The column halos are as wide as the widest aligned load
+// that divides the tile's start: 16 bytes for octaves 0 to 2, then 8 and 4.
+__host__ __device__ constexpr int det_left(int o) { return o <= 2 ? 16 : o == 3 ? 8 : 4; }
+__host__ __device__ constexpr int det_sw(int o) { return (kDetTW >> o) + 2 * det_left(o); }
+__host__ __device__ constexpr int det_rows(int o) { return (kDetTH >> o) + 2 * kHalo; }
 __host__ __device__ constexpr int det_stage_off(int octave) {
   int s = 0;
-  for (int o = 0; o < octave; o++) s += ((kDetTW >> o) + 2 * kHalo) * ((kDetTH >> o) + 2 * kHalo);
+  for (int o = 0; o < octave; o++) s += (det_sw(o) * det_rows(o) + 15) / 16 * 16;
   return s;
 }
 __host__ __device__ constexpr int det_stage_bytes() { return det_stage_off(kMaxOctaves); }
-
-// dHarrisScore (orbd.cu:651-669) on a shared-memory tile of row stride sw.
-// Integer sums wrap as 32-bit; the final combine is
-// fma(-0.04f, (float)(uint32)(dsxy*dsxy), (float)(int32)(dxx*dyy - dxy*dxy)) * scale^4,
-// which is how the reference build evaluates
-// (dxx*dyy - dxy*dxy - HARRIS_K*(dsxy*dsxy)) * d_scale_sq_sq.
-__device__ __forceinline__ float harris_score(const uint8_t* c, int sw, float scale4) {
-  int dxx = 0, dyy = 0, dxy = 0;
-#pragma unroll 1
-  for (int i = -3; i <= 3; i++) {
-#pragma unroll
-    for (int j = -3; j <= 3; j++) {
-      const uint8_t* q = c + i * sw + j;
-      const int dx = ((int)q[1] - (int)q[-1]) * 2 + ((int)q[-sw + 1] - (int)q[-sw - 1]) +
-                     ((int)q[sw + 1] - (int)q[sw - 1]);
-      const int dy = ((int)q[sw] - (int)q[-sw]) * 2 + ((int)q[sw - 1] - (int)q[-sw - 1]) +
-                     ((int)q[sw + 1] - (int)q[-sw + 1]);
-      dxx += dx * dx;
-      dyy += dy * dy;
-      dxy += dx * dy;
-    }
-  }
-  return harris_combine(dxx, dyy, dxy, scale4);
+// The same for an octave known only at run time: stride, and offset of octave
+// pixel (0, 0) of the tile.
+__device__ __forceinline__ int det_sw_at(int o) {
+  return o <= 2 ? (kDetTW >> o) + 32 : o == 3 ? det_sw(3) : det_sw(4);
 }
-
-// Byte-wise arithmetic on packed words with plain integer operations (the
-// byte-SIMD intrinsics are several instructions each on this architecture).
-constexpr uint32_t kB7 = 0x80808080u, kLo7 = 0x7F7F7F7Fu;
-// bit 7 of each byte set where x < y (unsigned): the 7-bit differences cannot
-// borrow across bytes, and the top bits decide when they differ
-__device__ __forceinline__ uint32_t swar_lt(uint32_t x, uint32_t y) {
-  const uint32_t t = (x | kB7) - (y & kLo7);
-  return ((~x & y) | (~(x ^ y) & ~t)) & kB7;
-}
-// max(v - t, 0) and min(v + t, 255) per byte, t given in every byte
-__device__ __forceinline__ uint32_t swar_sub_sat(uint32_t v, uint32_t t4) {
-  const uint32_t d = ((v | kB7) - (t4 & kLo7)) ^ ((v ^ ~t4) & kB7);
-  return d & ~((swar_lt(v, t4) >> 7) * 0xFFu);
-}
-__device__ __forceinline__ uint32_t swar_add_sat(uint32_t v, uint32_t t4) {
-  const uint32_t s = ((v & kLo7) + (t4 & kLo7)) ^ ((v ^ t4) & kB7);
-  const uint32_t carry = ((v & t4) | ((v | t4) & ~s)) & kB7;
-  return s | ((carry >> 7) * 0xFFu);
+__device__ __forceinline__ int det_origin_at(int o) {
+  constexpr int at[kMaxOctaves] = {det_stage_off(0) + kHalo * det_sw(0) + det_left(0),
+                                   det_stage_off(1) + kHalo * det_sw(1) + det_left(1),
+                                   det_stage_off(2) + kHalo * det_sw(2) + det_left(2),
+                                   det_stage_off(3) + kHalo * det_sw(3) + det_left(3),
+                                   det_stage_off(4) + kHalo * det_sw(4) + det_left(4)};
+  return o == 0 ? at[0] : o == 1 ? at[1] : o == 2 ? at[2] : o == 3 ? at[3] : at[4];
 }
 
 // Necessary condition for FAST-9: every run of 9 ring pixels contains two
 // neighbouring cardinal points (ring positions k and k+4, k = 0, 4, 8, 12), so
 // both of some such pair must be darker than v - t, or both brighter than
 // v + t.  It never changes a result.  Evaluated for four horizontally adjacent
-// centres at once on packed bytes: w points at the aligned word holding them
-// (row stride sw bytes, a multiple of 4); returns bit 7 of each byte whose
-// centre passes.  Saturating v - t and v + t (t <= 255) give the same answers
-// as the signed comparisons p < v - t and p > v + t.
-__device__ __forceinline__ uint32_t fast9_pretest4(const uint8_t* w, int sw, uint32_t t4) {
+// centres at once: w points at the aligned word holding them (row stride sw
+// bytes, a multiple of 4); returns bit 7 of each byte whose centre passes.
+// Some pair (0 or 8, 4 or 12) is darker when max(min(p0, p8), min(p4, p12)) <
+// v - t, and brighter when min(max(p0, p8), max(p4, p12)) > v + t.  Two centres
+// per instruction in 16-bit lanes; k1 is 0x8000 - t - 1 in both lanes, so that
+// bit 15 of each lane is the comparison and no lane borrows from the next.
+__device__ __forceinline__ uint32_t fast9_pretest2(uint32_t v, uint32_t p0, uint32_t p4, uint32_t p8, uint32_t p12,
+                                                   uint32_t k1) {
+  const uint32_t dark = __vmaxu2(__vminu2(p0, p8), __vminu2(p4, p12));
+  const uint32_t bright = __vminu2(__vmaxu2(p0, p8), __vmaxu2(p4, p12));
+  return (v + k1 - dark) | (bright + k1 - v);
+}
+__device__ __forceinline__ uint32_t fast9_pretest4(const uint8_t* w, int sw, uint32_t k1) {
   const uint32_t c = *reinterpret_cast<const uint32_t*>(w);
   const uint32_t cl = *reinterpret_cast<const uint32_t*>(w - 4);
   const uint32_t cr = *reinterpret_cast<const uint32_t*>(w + 4);
@@ -475,14 +466,14 @@ __device__ __forceinline__ uint32_t fast9_pretest4(const uint8_t* w, int sw, uin
   const uint32_t p8 = *reinterpret_cast<const uint32_t*>(w - 3 * sw);   // ring 8: (x, y - 3)
   const uint32_t p4 = __byte_perm(c, cr, 0x6543);                       // ring 4: (x + 3, y)
   const uint32_t p12 = __byte_perm(cl, c, 0x4321);                      // ring 12: (x - 3, y)
-  const uint32_t lo = swar_sub_sat(c, t4), hi = swar_add_sat(c, t4);
-  const uint32_t d0 = swar_lt(p0, lo), d4 = swar_lt(p4, lo), d8 = swar_lt(p8, lo), d12 = swar_lt(p12, lo);
-  const uint32_t b0 = swar_lt(hi, p0), b4 = swar_lt(hi, p4), b8 = swar_lt(hi, p8), b12 = swar_lt(hi, p12);
-  return ((d0 | d8) & (d4 | d12)) | ((b0 | b8) & (b4 | b12));
+  auto lo = [](uint32_t x) { return __byte_perm(x, 0u, 0x4140); };
+  auto hi = [](uint32_t x) { return __byte_perm(x, 0u, 0x4342); };
+  const uint32_t r0 = fast9_pretest2(lo(c), lo(p0), lo(p4), lo(p8), lo(p12), k1);
+  const uint32_t r1 = fast9_pretest2(hi(c), hi(p0), hi(p4), hi(p8), hi(p12), k1);
+  return __byte_perm(r0, r1, 0x7531) & 0x80808080u;
 }
 
-__device__ __forceinline__ float corner_score(const Batch& b, const uint8_t* c, int sw) {
-  if (b.harris) return harris_score(c, sw, b.harris_scale4);
+__device__ __forceinline__ float corner_fast_score(const Batch& b, const uint8_t* c, int sw) {
   const int v = c[0];
   int d[25];
 #pragma unroll
@@ -512,42 +503,47 @@ struct DetSmem {
   int ow[kMaxOctaves], oh[kMaxOctaves];
 };
 
-// Stages octave O of a detect tile with its halo: (32 >> O) + 8 rows of
-// (64 >> O) + 8 bytes starting 4 rows above and 4 bytes left of the tile's
-// octave origin, in the pyramid's linear addressing.
+// Load i of octave O's stage of a detect tile: det_rows(O) rows of det_sw(O)
+// bytes, in the pyramid's linear addressing, 16, 8 or 4 bytes per load (octave
+// offsets and pitches are multiples of 128).
 template <int O, bool P>
-__device__ __forceinline__ void stage_octave(const Frame& F, const uint8_t* pyr, int X0, int Y0, uint8_t* s_stage,
+__device__ __forceinline__ void stage_octave(const Frame& F, const uint8_t* pyr, int X0, int Y0, uint8_t* s_stage, int i,
                                              BoundsRec* rec) {
-  constexpr int sw4 = ((kDetTW >> O) + 2 * kHalo) / 4;
-  constexpr int sh = (kDetTH >> O) + 2 * kHalo;
-  const int op = F.op[O];
-  const uint32_t* src =
-      reinterpret_cast<const uint32_t*>(pyr + F.ooff[O] + (long long)((Y0 >> O) - kHalo) * op + ((X0 >> O) - kHalo));
-  const int op4 = op >> 2;
-  uint32_t* dst = reinterpret_cast<uint32_t*>(s_stage + det_stage_off(O));
-#pragma unroll 4
-  for (int i = threadIdx.x; i < sh * sw4; i += 256) {
-    const int r = i / sw4, w = i - r * sw4;
-    const uint32_t* sp = src + r * op4 + w;
-    dst[i] = ORBX_IN(rec, kSiteDetLoad, guarded_span(pyr, F), sp, 4) ? ldx<P>(sp) : 0u;
-  }
+  constexpr int B = det_left(O);
+  constexpr int per_row = det_sw(O) / B;
+  const int r = i / per_row, c = i - r * per_row;
+  const uint8_t* sp =
+      pyr + F.ooff[O] + (long long)((Y0 >> O) - kHalo + r) * F.op[O] + ((X0 >> O) - det_left(O) + B * c);
+  uint8_t* dp = s_stage + det_stage_off(O) + r * det_sw(O) + B * c;
+  const bool in = ORBX_IN(rec, kSiteDetLoad, guarded_span(pyr, F), sp, B);
+  if constexpr (B == 16)
+    *reinterpret_cast<uint4*>(dp) = in ? ldx<P>(reinterpret_cast<const uint4*>(sp)) : uint4{};
+  else if constexpr (B == 8)
+    *reinterpret_cast<uint2*>(dp) = in ? ldx<P>(reinterpret_cast<const uint2*>(sp)) : uint2{};
+  else
+    *reinterpret_cast<uint32_t*>(dp) = in ? ldx<P>(reinterpret_cast<const uint32_t*>(sp)) : 0u;
 }
+template <int O>
+__host__ __device__ constexpr int det_loads() { return det_rows(O) * (det_sw(O) / det_left(O)); }
 
 // Pre-test of word w (four centres) of octave O of a detect tile: octave O
-// has (32 >> O) rows of (16 >> O) words.  Centres that pass are appended to
-// the tile's candidate list.
+// has (32 >> O) rows of (16 >> O) words.  A warp takes rows r and r + 2 of octave
+// 0, whose words are in distinct banks.  Centres that pass are appended to the
+// tile's candidate list.
 template <int O>
 __device__ __forceinline__ void pretest_word(int w, int X0, int Y0, const uint8_t* s_stage, int ow, int oh,
-                                             uint32_t t4, int* s_n, uint16_t* s_cand) {
+                                             uint32_t k1, int* s_n, uint16_t* s_cand) {
   static_assert(kDetTW == 64 && kDetTH == 32, "word layout assumes 64 x 32 detect tiles");
   constexpr int nwl = 4 - O;  // log2 words per row
-  constexpr int sw = (kDetTW >> O) + 2 * kHalo;
-  constexpr int off = det_stage_off(O);
-  const int ly = w >> nwl, lx = (w & ((1 << nwl) - 1)) << 2;
+  constexpr int sw = det_sw(O);
+  constexpr int origin = det_stage_off(O) + kHalo * sw + det_left(O);
+  int ly = w >> nwl;
+  if constexpr (O == 0) ly = (ly & ~3) | ((ly & 1) << 1) | ((ly >> 1) & 1);
+  const int lx = (w & ((1 << nwl) - 1)) << 2;
   const int x = (X0 >> O) + lx, y = (Y0 >> O) + ly;
   uint32_t m = 0u;
   if (y >= 3 && y < oh - 3 && x < ow - 3) {
-    m = fast9_pretest4(s_stage + off + (ly + kHalo) * sw + (lx + kHalo), sw, t4);
+    m = fast9_pretest4(s_stage + origin + ly * sw + lx, sw, k1);
     if (x < 3 || x + 3 >= ow - 3) {  // border word: keep the centres with 3 <= x + k < ow - 3
       uint32_t vm = 0u;
 #pragma unroll
@@ -556,7 +552,6 @@ __device__ __forceinline__ void pretest_word(int w, int X0, int Y0, const uint8_
       m &= vm;
     }
   }
-  m &= 0x80808080u;
   if (m) {
     int pos = atomicAdd(&s_n[0], __popc(m));
     while (m) {
@@ -598,31 +593,40 @@ __device__ __forceinline__ void det_tile(const Batch& b, int t, DetSmem& sm) {
     s_ow[threadIdx.x] = threadIdx.x < n_oct ? F.ow[threadIdx.x] : 0;
     s_oh[threadIdx.x] = threadIdx.x < n_oct ? F.oh[threadIdx.x] : 0;
   }
-  // Stage every octave's tile with its halo, 4 bytes per load (octave offsets
-  // and pitches are multiples of 128 and (X0 >> o) - 4 is a multiple of 4):
-  // the words of each octave are spread over the whole block.
-  stage_octave<0, P>(F, pyr, X0, Y0, s_stage, b.bounds);
-  if (n_oct > 1) stage_octave<1, P>(F, pyr, X0, Y0, s_stage, b.bounds);
-  if (n_oct > 2) stage_octave<2, P>(F, pyr, X0, Y0, s_stage, b.bounds);
-  if (n_oct > 3) stage_octave<3, P>(F, pyr, X0, Y0, s_stage, b.bounds);
-  if (n_oct > 4) stage_octave<4, P>(F, pyr, X0, Y0, s_stage, b.bounds);
+  // stage every octave's tile with its halo: one load per thread for octave 0,
+  // one for the other octaves together
+  {
+    const int t = threadIdx.x;
+    constexpr int n1 = det_loads<1>(), n2 = n1 + det_loads<2>(), n3 = n2 + det_loads<3>(), n4 = n3 + det_loads<4>();
+    static_assert(det_loads<0>() <= 256 && n4 <= 256, "two staging loads per thread");
+    if (t < det_loads<0>()) stage_octave<0, P>(F, pyr, X0, Y0, s_stage, t, b.bounds);
+    if (t < n1) {
+      if (n_oct > 1) stage_octave<1, P>(F, pyr, X0, Y0, s_stage, t, b.bounds);
+    } else if (t < n2) {
+      if (n_oct > 2) stage_octave<2, P>(F, pyr, X0, Y0, s_stage, t - n1, b.bounds);
+    } else if (t < n3) {
+      if (n_oct > 3) stage_octave<3, P>(F, pyr, X0, Y0, s_stage, t - n2, b.bounds);
+    } else if (t < n4) {
+      if (n_oct > 4) stage_octave<4, P>(F, pyr, X0, Y0, s_stage, t - n3, b.bounds);
+    }
+  }
   __syncthreads();
 
   // 1. cardinal pre-test, four centres per word: the 512 words of octave 0 take
   //    two passes of the block, the 128 + 32 + 8 + 2 words of octaves 1..4 one
   {
-    const uint32_t t4 = (uint32_t)min(max(thr, 0), 255) * 0x01010101u;
+    const uint32_t k1 = (0x7FFFu - (uint32_t)min(max(thr, 0), 255)) * 0x00010001u;
     const int t = threadIdx.x;
-    pretest_word<0>(t, X0, Y0, s_stage, s_ow[0], s_oh[0], t4, s_n, s_cand);
-    pretest_word<0>(t + 256, X0, Y0, s_stage, s_ow[0], s_oh[0], t4, s_n, s_cand);
+    pretest_word<0>(t, X0, Y0, s_stage, s_ow[0], s_oh[0], k1, s_n, s_cand);
+    pretest_word<0>(t + 256, X0, Y0, s_stage, s_ow[0], s_oh[0], k1, s_n, s_cand);
     if (t < 128) {
-      if (n_oct > 1) pretest_word<1>(t, X0, Y0, s_stage, s_ow[1], s_oh[1], t4, s_n, s_cand);
+      if (n_oct > 1) pretest_word<1>(t, X0, Y0, s_stage, s_ow[1], s_oh[1], k1, s_n, s_cand);
     } else if (t < 160) {
-      if (n_oct > 2) pretest_word<2>(t - 128, X0, Y0, s_stage, s_ow[2], s_oh[2], t4, s_n, s_cand);
+      if (n_oct > 2) pretest_word<2>(t - 128, X0, Y0, s_stage, s_ow[2], s_oh[2], k1, s_n, s_cand);
     } else if (t < 168) {
-      if (n_oct > 3) pretest_word<3>(t - 160, X0, Y0, s_stage, s_ow[3], s_oh[3], t4, s_n, s_cand);
+      if (n_oct > 3) pretest_word<3>(t - 160, X0, Y0, s_stage, s_ow[3], s_oh[3], k1, s_n, s_cand);
     } else if (t < 170) {
-      if (n_oct > 4) pretest_word<4>(t - 168, X0, Y0, s_stage, s_ow[4], s_oh[4], t4, s_n, s_cand);
+      if (n_oct > 4) pretest_word<4>(t - 168, X0, Y0, s_stage, s_ow[4], s_oh[4], k1, s_n, s_cand);
     }
   }
   __syncthreads();
@@ -633,8 +637,8 @@ __device__ __forceinline__ void det_tile(const Batch& b, int t, DetSmem& sm) {
     for (int j = threadIdx.x; j < n1; j += blockDim.x) {
       const int e = s_cand[j];
       const int o = e >> 11, ly = (e >> 6) & 31, lx = e & 63;
-      const int sw = (kDetTW >> o) + 2 * kHalo;
-      const uint8_t* c = s_stage + det_stage_off(o) + (ly + kHalo) * sw + (lx + kHalo);
+      const int sw = det_sw_at(o);
+      const uint8_t* c = s_stage + det_origin_at(o) + ly * sw + lx;
       const int v = c[0];
       if (fast9_full(c, sw, v - thr, v + thr)) s_corner[atomicAdd(&s_n[1], 1)] = (uint16_t)e;
     }
@@ -657,18 +661,23 @@ __device__ __forceinline__ void det_tile(const Batch& b, int t, DetSmem& sm) {
         if (j < n2) {
           e = s_corner[j];
           const int o = e >> 11, ly = (e >> 6) & 31, lx = e & 63;
-          const int sw = (kDetTW >> o) + 2 * kHalo;
-          const uint8_t* c = s_stage + det_stage_off(o) + (ly + kHalo) * sw + (lx + kHalo);
+          const int sw = det_sw_at(o);
+          const uint8_t* c = s_stage + det_origin_at(o) + ly * sw + lx;
           if (sub < 7) {  // lane `sub` of the group takes window row sub - 3, its 7 columns unrolled
             const uint8_t* r = c + (sub - 3) * sw;
             const uint8_t* ru = r - sw;
             const uint8_t* rd = r + sw;
+            int s1[9], d1[9];  // column sums (1 2 1) and differences of the three rows, columns -4 .. 4
 #pragma unroll
-            for (int wx = -3; wx <= 3; wx++) {
-              const int dx = ((int)r[wx + 1] - (int)r[wx - 1]) * 2 + ((int)ru[wx + 1] - (int)ru[wx - 1]) +
-                             ((int)rd[wx + 1] - (int)rd[wx - 1]);
-              const int dy = ((int)rd[wx] - (int)ru[wx]) * 2 + ((int)rd[wx - 1] - (int)ru[wx - 1]) +
-                             ((int)rd[wx + 1] - (int)ru[wx + 1]);
+            for (int i = 0; i < 9; i++) {
+              const int u = ru[i - 4], m = r[i - 4], d = rd[i - 4];
+              s1[i] = u + 2 * m + d;
+              d1[i] = d - u;
+            }
+#pragma unroll
+            for (int i = 0; i < 7; i++) {
+              const int dx = s1[i + 2] - s1[i];
+              const int dy = d1[i] + 2 * d1[i + 1] + d1[i + 2];
               dxx += dx * dx;
               dyy += dy * dy;
               dxy += dx * dy;
@@ -694,8 +703,8 @@ __device__ __forceinline__ void det_tile(const Batch& b, int t, DetSmem& sm) {
       for (int j = threadIdx.x; j < n2; j += blockDim.x) {
         const int e = s_corner[j];
         const int o = e >> 11, ly = (e >> 6) & 31, lx = e & 63;
-        const int sw = (kDetTW >> o) + 2 * kHalo;
-        const float score = corner_score(b, s_stage + det_stage_off(o) + (ly + kHalo) * sw + (lx + kHalo), sw);
+        const int sw = det_sw_at(o);
+        const float score = corner_fast_score(b, s_stage + det_origin_at(o) + ly * sw + lx, sw);
         if (score > 0.f) {
           const int m = (ly << o) * kDetTW + (lx << o);
           if (atomicMax(&s_key[m], det_key(score, o)) == 0ull) atomicOr(&s_occ[m >> 5], 1u << (m & 31));
