@@ -70,6 +70,31 @@ __device__ __forceinline__ float fast_score(const int* d, int threshold) {
   return (float)(-b0 - 1);
 }
 
+// Necessary condition for FAST-9: every run of 9 ring pixels contains two
+// neighbouring cardinal points (ring positions k and k+4, k = 0, 4, 8, 12), so
+// both of some such pair must be darker than v - t, or both brighter than
+// v + t.  It never changes a result.  Some pair (0 or 8, 4 or 12) is darker when
+// max(min(p0, p8), min(p4, p12)) < v - t, and brighter when min(max(p0, p8),
+// max(p4, p12)) > v + t.  Two centres per instruction in 16-bit lanes; k1 is
+// 0x8000 - t - 1 in both lanes (0 <= t <= 255), so that bit 15 of each lane is
+// the comparison and no lane borrows from the next.
+__device__ __forceinline__ uint32_t fast9_pretest2(uint32_t v, uint32_t p0, uint32_t p4, uint32_t p8, uint32_t p12,
+                                                   uint32_t k1) {
+  const uint32_t dark = __vmaxu2(__vminu2(p0, p8), __vminu2(p4, p12));
+  const uint32_t bright = __vminu2(__vmaxu2(p0, p8), __vmaxu2(p4, p12));
+  return (v + k1 - dark) | (bright + k1 - v);
+}
+// Four horizontally adjacent centres, c, and the words of their ring positions;
+// bit 7 of each byte whose centre passes.
+__device__ __forceinline__ uint32_t fast9_pretest4(uint32_t c, uint32_t p0, uint32_t p4, uint32_t p8, uint32_t p12,
+                                                   uint32_t k1) {
+  auto lo = [](uint32_t x) { return __byte_perm(x, 0u, 0x4140); };
+  auto hi = [](uint32_t x) { return __byte_perm(x, 0u, 0x4342); };
+  const uint32_t r0 = fast9_pretest2(lo(c), lo(p0), lo(p4), lo(p8), lo(p12), k1);
+  const uint32_t r1 = fast9_pretest2(hi(c), hi(p0), hi(p4), hi(p8), hi(p12), k1);
+  return __byte_perm(r0, r1, 0x7531) & 0x80808080u;
+}
+
 // FAST-9 segment test on a shared-memory tile of row stride sw: a run of 9
 // contiguous ring pixels all darker than v - t or all brighter than v + t (the
 // reference's LUT pre-test and arc loop, orbd.cu:683-740, decide exactly this).

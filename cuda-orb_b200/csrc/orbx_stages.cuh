@@ -442,23 +442,9 @@ __device__ __forceinline__ int det_origin_at(int o) {
   return o == 0 ? at[0] : o == 1 ? at[1] : o == 2 ? at[2] : o == 3 ? at[3] : at[4];
 }
 
-// Necessary condition for FAST-9: every run of 9 ring pixels contains two
-// neighbouring cardinal points (ring positions k and k+4, k = 0, 4, 8, 12), so
-// both of some such pair must be darker than v - t, or both brighter than
-// v + t.  It never changes a result.  Evaluated for four horizontally adjacent
-// centres at once: w points at the aligned word holding them (row stride sw
-// bytes, a multiple of 4); returns bit 7 of each byte whose centre passes.
-// Some pair (0 or 8, 4 or 12) is darker when max(min(p0, p8), min(p4, p12)) <
-// v - t, and brighter when min(max(p0, p8), max(p4, p12)) > v + t.  Two centres
-// per instruction in 16-bit lanes; k1 is 0x8000 - t - 1 in both lanes, so that
-// bit 15 of each lane is the comparison and no lane borrows from the next.
-__device__ __forceinline__ uint32_t fast9_pretest2(uint32_t v, uint32_t p0, uint32_t p4, uint32_t p8, uint32_t p12,
-                                                   uint32_t k1) {
-  const uint32_t dark = __vmaxu2(__vminu2(p0, p8), __vminu2(p4, p12));
-  const uint32_t bright = __vminu2(__vmaxu2(p0, p8), __vmaxu2(p4, p12));
-  return (v + k1 - dark) | (bright + k1 - v);
-}
-__device__ __forceinline__ uint32_t fast9_pretest4(const uint8_t* w, int sw, uint32_t k1) {
+// The pre-test of the four centres in the aligned word at w of a staged tile
+// (row stride sw bytes, a multiple of 4).
+__device__ __forceinline__ uint32_t fast9_pretest_word(const uint8_t* w, int sw, uint32_t k1) {
   const uint32_t c = *reinterpret_cast<const uint32_t*>(w);
   const uint32_t cl = *reinterpret_cast<const uint32_t*>(w - 4);
   const uint32_t cr = *reinterpret_cast<const uint32_t*>(w + 4);
@@ -466,11 +452,7 @@ __device__ __forceinline__ uint32_t fast9_pretest4(const uint8_t* w, int sw, uin
   const uint32_t p8 = *reinterpret_cast<const uint32_t*>(w - 3 * sw);   // ring 8: (x, y - 3)
   const uint32_t p4 = __byte_perm(c, cr, 0x6543);                       // ring 4: (x + 3, y)
   const uint32_t p12 = __byte_perm(cl, c, 0x4321);                      // ring 12: (x - 3, y)
-  auto lo = [](uint32_t x) { return __byte_perm(x, 0u, 0x4140); };
-  auto hi = [](uint32_t x) { return __byte_perm(x, 0u, 0x4342); };
-  const uint32_t r0 = fast9_pretest2(lo(c), lo(p0), lo(p4), lo(p8), lo(p12), k1);
-  const uint32_t r1 = fast9_pretest2(hi(c), hi(p0), hi(p4), hi(p8), hi(p12), k1);
-  return __byte_perm(r0, r1, 0x7531) & 0x80808080u;
+  return fast9_pretest4(c, p0, p4, p8, p12, k1);
 }
 
 __device__ __forceinline__ float corner_fast_score(const Batch& b, const uint8_t* c, int sw) {
@@ -543,7 +525,7 @@ __device__ __forceinline__ void pretest_word(int w, int X0, int Y0, const uint8_
   const int x = (X0 >> O) + lx, y = (Y0 >> O) + ly;
   uint32_t m = 0u;
   if (y >= 3 && y < oh - 3 && x < ow - 3) {
-    m = fast9_pretest4(s_stage + origin + ly * sw + lx, sw, k1);
+    m = fast9_pretest_word(s_stage + origin + ly * sw + lx, sw, k1);
     if (x < 3 || x + 3 >= ow - 3) {  // border word: keep the centres with 3 <= x + k < ow - 3
       uint32_t vm = 0u;
 #pragma unroll
