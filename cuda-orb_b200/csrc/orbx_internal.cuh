@@ -184,7 +184,6 @@ struct MatchWork {          // scratch for split-train merging
   int nq_cap;               // query capacity the grid is sized for
   int splits_cap;           // most train splits per query tile
 };
-int match_popc_blocks(int nq_cap, int splits_cap, int blocks_per_sm = 8);
 
 // int8 tensor-core form (orbx_match_imma.cu)
 struct ImmaLaunch {

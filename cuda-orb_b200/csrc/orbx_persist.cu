@@ -30,6 +30,8 @@
 
 namespace orbx {
 
+constexpr int kPersistThreads = 256;
+
 union PersistSmem {
   PyrSmem<kPyrTH> pyr;
   DetSmem det;
@@ -37,13 +39,9 @@ union PersistSmem {
   struct {
     int umax[32];
   } desc;
-  struct {
-    uint4 db[kMChunk * 2];
-    unsigned int last;
-  } match;
+  MatchSmem<kPersistThreads / kMQ> match;
 };
 
-constexpr int kPersistThreads = 256;
 static_assert(kPersistThreads == kPyrThreads, "pyramid tiles assume kPyrThreads threads per block");
 
 // One thread waits until *ctr >= need (acquire), bounded by wait_cycles.
@@ -214,8 +212,7 @@ __global__ void __launch_bounds__(kPersistThreads, 4) k_batch_persistent(Persist
         stage_wait(done + 3 * nf + fb, __ldg(p.desc_base + fb + 1) - __ldg(p.desc_base + fb), b.err,
                    b.wait_cycles);
         const MatchJob& J = p.jobs[f >> 1];
-        match_popc_block<kPersistThreads, true>(J.args, J.work, local, p.blocks_per_job, sm.match.db,
-                                                sm.match.last);
+        match_popc_block<kPersistThreads / kMQ, true>(J.args, J.work, local, p.blocks_per_job, sm.match);
         break;
       }
     }

@@ -1349,6 +1349,7 @@ __device__ __forceinline__ void describe_keypoint(const Batch& b, const Frame& F
 // k = 2 XOR-popcount matching (orbx_match.cu and the persistent kernel)
 // ---------------------------------------------------------------------------
 constexpr int kMQ = 128;      // queries per block
+constexpr int kMGroups = 4;   // row groups per block of the launched matchers
 constexpr int kMChunk = 512;  // train rows per shared-memory chunk (16 KB)
 constexpr int kIdxBits = kIdxBitsShared;
 constexpr uint32_t kNoKey = kNoKeyShared;
@@ -1358,19 +1359,59 @@ __device__ __forceinline__ void finish_query(const MatchArgs& a, int q, uint32_t
   finish_query_shared(a, q, k1, k2);
 }
 
-// One block's share of a k = 2 search with QPB queries per block (QPB =
-// blockDim.x); bid / nblk replace blockIdx.x / gridDim.x so that a batch launch
-// or a work item of the persistent kernel can run one search each.  P: the
-// descriptors and counts were written earlier in the same launch.
-template <int QPB, bool P>
-__device__ __forceinline__ void match_popc_block(const MatchArgs& a, const MatchWork& w, int bid, int nblk,
-                                                 uint4* s_db, unsigned int& s_last) {
+// Hamming distance of a query (q) and a train row (t0, t1).  Four carry-save
+// adders turn the eight XORed words into one word of ones, one left over, one of
+// twos and one of fours, so four population counts do instead of eight: that
+// unit takes 8 cycles per warp where the ALU takes 2 for each of the adders'
+// eight three-input operations.
+__device__ __forceinline__ uint32_t csa_carry(uint32_t a, uint32_t b, uint32_t c) { return (a & b) | (c & (a | b)); }
+__device__ __forceinline__ uint32_t hamming256(const uint32_t* q, const uint4& t0, const uint4& t1) {
+  const uint32_t x0 = q[0] ^ t0.x, x1 = q[1] ^ t0.y, x2 = q[2] ^ t0.z, x3 = q[3] ^ t0.w;
+  const uint32_t x4 = q[4] ^ t1.x, x5 = q[5] ^ t1.y, x6 = q[6] ^ t1.z, x7 = q[7] ^ t1.w;
+  const uint32_t s1 = x0 ^ x1 ^ x2, c1 = csa_carry(x0, x1, x2);
+  const uint32_t s2 = x3 ^ x4 ^ x5, c2 = csa_carry(x3, x4, x5);
+  const uint32_t s3 = s1 ^ s2 ^ x6, c3 = csa_carry(s1, s2, x6);
+  const uint32_t twos = c1 ^ c2 ^ c3, fours = csa_carry(c1, c2, c3);
+  return __popc(s3) + __popc(x7) + 2 * __popc(twos) + 4 * __popc(fours);
+}
 
+template <int RG>
+struct MatchSmem {
+  uint4 db[kMChunk * 2];
+  uint2 part[(RG - 1) * kMQ];  // the other row groups' best two, per query
+  unsigned int last;
+};
+
+// Merges the row groups' best two of each query; the threads of group 0 get them.
+template <int RG>
+__device__ __forceinline__ void match_merge_groups(MatchSmem<RG>& sm, int rg, int ql, uint32_t& k1, uint32_t& k2) {
+  if (rg) sm.part[(rg - 1) * kMQ + ql] = make_uint2(k1, k2);
+  __syncthreads();
+  if (rg) return;
+#pragma unroll
+  for (int g = 0; g < RG - 1; g++) {
+    const uint2 o = sm.part[g * kMQ + ql];
+    top2_push(k1, k2, o.x);
+    top2_push(k1, k2, o.y);
+  }
+}
+
+// One block's share of a k = 2 search: kMQ queries, one per thread, and RG groups
+// of threads with a share of the train rows each (kMQ * RG threads).  Per query
+// the row groups' and the splits' results are merged as keys, so the outcome does
+// not depend on how the rows are shared out.  bid / nblk replace blockIdx.x /
+// gridDim.x so that a batch launch or a work item of the persistent kernel can run
+// one search each.  P: the descriptors and counts were written earlier in the
+// same launch.
+template <int RG, bool P>
+__device__ __forceinline__ void match_popc_block(const MatchArgs& a, const MatchWork& w, int bid, int nblk,
+                                                 MatchSmem<RG>& sm) {
+  const int ql = threadIdx.x % kMQ, rg = threadIdx.x / kMQ;
   const int nq = min(a.d_nq ? ldx<P>(a.d_nq) : a.nq, w.nq_cap);
   const int ndb = a.d_ndb ? ldx<P>(a.d_ndb) : a.ndb;
   // Spread (query tile, train split) pairs over the launched blocks using the
   // actual counts, which may be far below the capacities the grid was sized for.
-  const int tiles = (nq + QPB - 1) / QPB;
+  const int tiles = (nq + kMQ - 1) / kMQ;
   if (tiles == 0) return;
   int splits = nblk / tiles;
   splits = min(splits, w.splits_cap);
@@ -1379,7 +1420,7 @@ __device__ __forceinline__ void match_popc_block(const MatchArgs& a, const Match
   const int tile = bid / splits;
   const int split = bid - tile * splits;
   if (tile >= tiles) return;
-  const int q = tile * QPB + threadIdx.x;
+  const int q = tile * kMQ + ql;
   const bool active = q < nq;
 
   uint32_t qw[8];
@@ -1394,48 +1435,63 @@ __device__ __forceinline__ void match_popc_block(const MatchArgs& a, const Match
   const int r_beg = (int)((long long)ndb * split / splits);
   const int r_end = (int)((long long)ndb * (split + 1) / splits);
   uint32_t k1 = kNoKey, k2 = kNoKey;
+  uint32_t second = kNoKey >> kIdxBits;  // distance of k2
   const uint4* db4 = reinterpret_cast<const uint4*>(a.db);
   for (int r0 = r_beg; r0 < r_end; r0 += kMChunk) {
     const int rows = min(kMChunk, r_end - r0);
     __syncthreads();
-    for (int i = threadIdx.x; i < rows * 2; i += QPB)
-      s_db[i] = ORBX_IN_ROWS(a.bounds, kSiteMatchDb, r0 + (i >> 1), a.db_cap) ? ldx<P>(db4 + 2 * (size_t)r0 + i)
-                                                                             : uint4{};
+    for (int i = threadIdx.x; i < rows * 2; i += kMQ * RG)
+      sm.db[i] = ORBX_IN_ROWS(a.bounds, kSiteMatchDb, r0 + (i >> 1), a.db_cap) ? ldx<P>(db4 + 2 * (size_t)r0 + i)
+                                                                              : uint4{};
     __syncthreads();
-    for (int j = 0; j < rows; j++) {
-      const uint4 t0 = s_db[2 * j], t1 = s_db[2 * j + 1];
-      const uint32_t d = __popc(qw[0] ^ t0.x) + __popc(qw[1] ^ t0.y) + __popc(qw[2] ^ t0.z) +
-                         __popc(qw[3] ^ t0.w) + __popc(qw[4] ^ t1.x) + __popc(qw[5] ^ t1.y) +
-                         __popc(qw[6] ^ t1.z) + __popc(qw[7] ^ t1.w);
-      top2_push(k1, k2, (d << kIdxBits) | (uint32_t)(r0 + j));
+    const int j_end = rows * (rg + 1) / RG;
+    int j = rows * rg / RG;
+    // four rows at a time: rows come in increasing index order, so only a
+    // distance below the second best can enter the top two
+    for (; j + 4 <= j_end; j += 4) {
+      uint32_t d[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) d[i] = hamming256(qw, sm.db[2 * (j + i)], sm.db[2 * (j + i) + 1]);
+      if (__vimin3_u32(d[0], d[1], min(d[2], d[3])) < second) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) top2_push(k1, k2, (d[i] << kIdxBits) | (uint32_t)(r0 + j + i));
+        second = k2 >> kIdxBits;
+      }
     }
+    for (; j < j_end; j++)
+      top2_push(k1, k2, (hamming256(qw, sm.db[2 * j], sm.db[2 * j + 1]) << kIdxBits) | (uint32_t)(r0 + j));
+    second = k2 >> kIdxBits;
   }
 
+  match_merge_groups<RG>(sm, rg, ql, k1, k2);
   if (splits == 1) {
-    if (active) finish_query(a, q, k1, k2);
+    if (active && rg == 0) finish_query(a, q, k1, k2);
     return;
   }
   // publish this split's partial top-2; the last split to finish the tile merges
-  if (active) {
+  if (active && rg == 0) {
     uint2* part = reinterpret_cast<uint2*>(w.part);
     part[(size_t)split * w.nq_cap + q] = make_uint2(k1, k2);
   }
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) s_last = (atomicAdd(&w.tile_done[tile], 1u) == (unsigned)(splits - 1)) ? 1u : 0u;
+  if (threadIdx.x == 0) sm.last = (atomicAdd(&w.tile_done[tile], 1u) == (unsigned)(splits - 1)) ? 1u : 0u;
   __syncthreads();
-  if (!s_last) return;
+  if (!sm.last) return;
   __threadfence();
   if (threadIdx.x == 0) w.tile_done[tile] = 0u;  // ready for the next launch
-  if (!active) return;
-  const uint2* part = reinterpret_cast<const uint2*>(w.part);
-  uint32_t m1 = kNoKey, m2 = kNoKey;
-  for (int sp = 0; sp < splits; sp++) {
-    const uint2 pk = __ldcg(part + (size_t)sp * w.nq_cap + q);
-    top2_push(m1, m2, pk.x);
-    top2_push(m1, m2, pk.y);
+  const uint2* part = reinterpret_cast<const uint2*>(w.part) + q;
+  k1 = k2 = kNoKey;
+  if (active) {
+#pragma unroll 4
+    for (int sp = rg; sp < splits; sp += RG) {
+      const uint2 pk = __ldcg(part + (size_t)sp * w.nq_cap);
+      top2_push(k1, k2, pk.x);
+      top2_push(k1, k2, pk.y);
+    }
   }
-  finish_query(a, q, m1, m2);
+  match_merge_groups<RG>(sm, rg, ql, k1, k2);
+  if (active && rg == 0) finish_query(a, q, k1, k2);
 }
 
 }  // namespace orbx

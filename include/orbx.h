@@ -230,7 +230,7 @@ typedef struct orbx_frame_out {
 typedef struct orbx_tuning {
   int nms_rows;              /* level-0 rows per NMS strip, 1..16 */
   int describe_blocks_per_sm; /* grid of the orientation + descriptor kernel */
-  int match_blocks_per_sm;    /* grid of the popcount matcher (single pairs) */
+  int match_blocks_per_sm;    /* grid of the popcount matcher (counts on the device), in blocks of 256 threads */
   int match_blocks_per_pair;  /* grid per pair of the batched matcher, 0 = automatic */
   int batch_form;             /* orbx_batch_pairs: 0 = five graph-replayed launches, 1 = one persistent launch */
   int persist_group;          /* persistent form: frames per wave of the work order (even), 0 = all frames */
