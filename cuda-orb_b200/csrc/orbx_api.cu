@@ -593,10 +593,12 @@ static int mw_ensure(MatchWork& mw, int nq_cap) {
   if (mw.part && mw.nq_cap >= nq_cap) return ORBX_OK;
   cudaFree(mw.part);
   cudaFree(mw.tile_done);
+  cudaFree(mw.bound);
   mw = MatchWork();
   const int cap = nq_cap < 128 ? 128 : nq_cap;
   ORBX_CUDA(cudaMalloc(&mw.part, sizeof(uint32_t) * 2 * (size_t)kSplitsCap * cap));
   ORBX_CUDA(cudaMalloc(&mw.tile_done, sizeof(unsigned int) * (size_t)div_up(cap, 128)));
+  ORBX_CUDA(cudaMalloc(&mw.bound, sizeof(uint32_t) * (size_t)cap));
   ORBX_CUDA(cudaMemset(mw.tile_done, 0, sizeof(unsigned int) * (size_t)div_up(cap, 128)));
   mw.nq_cap = cap;
   mw.splits_cap = kSplitsCap;
@@ -801,6 +803,7 @@ ORBX_API int orbx_destroy(orbx_ctx* c) {
   for (PairGraph* pg : {&c->ppg, &c->pho, &c->phs, &c->bg}) pg->drop();
   cudaFree(c->mw.part);
   cudaFree(c->mw.tile_done);
+  cudaFree(c->mw.bound);
   for (int i = 0; i < 2; i++) {
     cudaFree(c->io_img[i]);
     cudaFree(c->io_pts[i]);
@@ -821,11 +824,13 @@ ORBX_API int orbx_destroy(orbx_ctx* c) {
   persist_free(c->ppair);
   cudaFree(c->pho.mw.part);
   cudaFree(c->pho.mw.tile_done);
+  cudaFree(c->pho.mw.bound);
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
   cudaFree(c->hmw.part);
   cudaFree(c->hmw.tile_done);
+  cudaFree(c->hmw.bound);
   if (c->ev_reset) cudaEventDestroy(c->ev_reset);
   cudaFree(c->d_pattern);
   cudaFree(c->d_umax);
@@ -1004,7 +1009,7 @@ static int launch_match(orbx_ctx* c, MatchWork& mw, const MatchArgs& a, int nq_c
   L.db_pm1 = c->imma_db;
   L.nq_cap = nq_cap;
   L.ndb_cap = ndb_cap;
-  L.splits = imma_default_splits(nq_cap);
+  L.splits = imma_default_splits(nq_cap, ndb_cap);
   if (L.splits > mw.splits_cap) L.splits = mw.splits_cap;
   L.err = c->d_err;
   ORBX_CUDA(launch_match_imma(L, c->stream));

@@ -144,10 +144,12 @@ namespace orbx {
 // (griddepcontrol.launch_dependents): waiting blocks would take the places of
 // its own last wave.
 template <class... P, class... A>
-inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, const A&... args) {
+inline cudaError_t launch_chained_smem(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                       const A&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -155,6 +157,10 @@ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, c
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, const A&... args) {
+  return launch_chained_smem(kernel, grid, block, 0, s, args...);
 }
 #endif
 cudaError_t launch_pyramid_blur(const Batch& b, int total_tiles, cudaStream_t s);
@@ -181,6 +187,7 @@ struct MatchArgs {
 struct MatchWork {          // scratch for split-train merging
   uint32_t* part;           // [splits_cap][nq_cap][2] partial top-2 keys
   unsigned int* tile_done;  // [ceil(nq_cap / 128)] arrival counters, self-resetting
+  uint32_t* bound;          // optional [nq_cap], tensor-core form: least second-best key any split has found
   int nq_cap;               // query capacity the grid is sized for
   int splits_cap;           // most train splits per query tile
 };
@@ -201,7 +208,8 @@ struct ImmaLaunch {
 cudaError_t launch_expand_pm1(const uint8_t* bits, int n, const int* d_n, int rows, int8_t* out, cudaStream_t s);
 int imma_rows_q(int n);
 int imma_rows_db(int n);
-int imma_default_splits(int nq_cap);
+constexpr int kImmaMaxSplits = 64;
+int imma_default_splits(int nq_cap, int ndb);
 cudaError_t launch_match_imma(const ImmaLaunch& L, cudaStream_t s);
 
 // Probe rerank of the learned proposal on the int8 tensor cores

@@ -111,14 +111,15 @@ struct ImmaWork {
   MatchWork w{};
   int splits = 1;
 };
-int imma_work_alloc(Arena& a, ImmaWork& iw, int nq_cap, int splits_for, cudaStream_t s, int splits_cap = 0) {
-  iw.splits = imma_default_splits(std::max(1, splits_for));
+int imma_work_alloc(Arena& a, ImmaWork& iw, int nq_cap, int splits_for, int ndb, cudaStream_t s, int splits_cap = 0) {
+  iw.splits = imma_default_splits(std::max(1, splits_for), ndb);
   iw.w.nq_cap = nq_cap;
   iw.w.splits_cap = std::max(iw.splits, splits_cap);
   if (iw.w.splits_cap > 1) {
     const int tiles = (nq_cap + 127) / 128;
     LCHK(a.alloc(&iw.w.part, (size_t)2 * iw.w.splits_cap * nq_cap));
     LCHK(a.alloc(&iw.w.tile_done, (size_t)tiles));
+    LCHK(a.alloc(&iw.w.bound, (size_t)nq_cap));
     LCHK(cudaMemsetAsync(iw.w.tile_done, 0, sizeof(unsigned) * (size_t)tiles, s));
   }
   return ORBX_OK;
@@ -420,7 +421,7 @@ int cluster_kmeans(orbx_learned* L, cudaStream_t s, int* err) {
   k_gather_rows<<<grid1(2ll * C, 256), 256, 0, s>>>(L->db, d_init, C, L->centroids);
   LCHK(cudaMemsetAsync(L->assign, 0xFF, sizeof(int) * (size_t)n, s));
   ImmaWork iw;
-  LRC(imma_work_alloc(t, iw, n, n, s));
+  LRC(imma_work_alloc(t, iw, n, n, C, s));
   const int iters = L->p.kmeans_iters;
   for (int it = 0; it < iters; it++) {
     LRC(imma_knn(s, err, iw, L->db, n, nullptr, L->db_pm1, true, L->centroids, C, cent_pm1, false, dist2, idx2));
@@ -462,7 +463,7 @@ int lists_from_centroids(orbx_learned* L, cudaStream_t s, int* err) {
   LCHK(t.alloc(&changed, 1));
   LCHK(t.alloc(&cent_pm1, (size_t)imma_rows_db(C) * 256));
   ImmaWork iw;
-  LRC(imma_work_alloc(t, iw, n, n, s));
+  LRC(imma_work_alloc(t, iw, n, n, C, s));
   LRC(imma_knn(s, err, iw, L->db, n, nullptr, L->db_pm1, true, L->centroids, C, cent_pm1, false, dist2, idx2));
   LCHK(cudaMemsetAsync(L->assign, 0xFF, sizeof(int) * (size_t)n, s));
   LCHK(cudaMemsetAsync(counts, 0, sizeof(int) * C, s));
@@ -636,7 +637,7 @@ int ensure_search(orbx_learned* L, int nq) {
   // fallback splits sized for about one query in eight; fewer fallback queries
   // split the database scan further, up to 32 ways
   L->fb_work = ImmaWork();
-  LRC(imma_work_alloc(a, L->fb_work, nq, std::max(128, nq / 8), 0, 32));
+  LRC(imma_work_alloc(a, L->fb_work, nq, std::max(128, nq / 8), L->ndb, 0, 32));
   LCHK(cudaDeviceSynchronize());
   L->nq_cap = nq;
   return ORBX_OK;
@@ -737,7 +738,7 @@ ORBX_API int orbx_learned_build(orbx_ctx* ctx, const orbx_learned_params* p, con
                                                                          p->seed ^ 0x73796e74ull, p->flip_lo,
                                                                          p->flip_hi, rows + (size_t)ntrain * 32);
       ImmaWork iw;
-      rc = imma_work_alloc(t, iw, nt, nt, s);
+      rc = imma_work_alloc(t, iw, nt, nt, ndb, s);
       if (rc) break;
       rc = imma_knn(s, err, iw, rows, nt, nullptr, tq, false, L->db, ndb, L->db_pm1, true, dist2, idx2);
       if (rc) break;

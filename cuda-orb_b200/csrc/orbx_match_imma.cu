@@ -2,46 +2,64 @@
 //
 // A 256-bit descriptor b is expanded to 256 int8 values s_k = 2*b_k - 1 (+-1),
 // so for two descriptors dot(s, t) = 256 - 2 * Hamming(s, t), computed exactly
-// by tcgen05.mma kind::i8 with int32 accumulation.  One block owns 128
-// queries (the MMA's M) and walks 256-row database tiles (the MMA's N) with
-// K = 256 = eight K=32 MMA steps per tile:
-//   warp 0     TMA producer: the query tile once, database tiles through a
-//              3-stage shared-memory ring (128-byte swizzle, no multicast);
-//   warp 1     MMA issuer: one elected thread issues the eight MMAs of a tile
+// by tcgen05.mma kind::i8 with int32 accumulation.  One block owns up to 256
+// queries, as two query tiles of 128 (the MMA's M) that stay in shared memory,
+// and walks 256-row database tiles (the MMA's N) with K = 256 = eight K=32 MMA
+// steps per database and query tile:
+//   warp 0     TMA producer: the query tiles once, database tiles through a
+//              2-stage shared-memory ring (128-byte swizzle, no multicast);
+//   warp 1     MMA issuer: one elected thread issues the eight MMAs of a step
 //              into one of two TMEM accumulators (2 x 256 columns) and commits
-//              them to the ring's "empty" and the accumulator's "full" barriers;
-//   warps 2-17 epilogue: each reads its 32 TMEM lanes (queries) over a quarter
-//              of the columns into registers, hands the accumulator straight
-//              back, and keeps a running best / second-best key per query.
+//              them to the ring's "empty" (after a database tile's last step)
+//              and the accumulator's "full" barriers;
+//   warps 2-17 epilogue, two sets of eight: set s takes every second step, i.e.
+//              accumulator s.  A warp reads its 32 TMEM lanes (queries) over half
+//              the columns, 64 at a time, and keeps a running best / second-best
+//              key per query.
+// Steps alternate between the two query tiles of a database tile, so set s holds
+// query tile s; with at most 128 queries there is one query tile, the steps
+// alternate between database tiles, and the sets' results are merged.
 // The block's result per query is the top-2 by (distance, index), the same
 // keys as the XOR-popc kernel (orbx_match.cu), so both forms agree bit for bit.
 // Every barrier wait is bounded by a clock deadline; on expiry the block
 // records kErrImmaTimeout, drains its in-flight copies, frees TMEM and exits.
+//
+// What bounds it: the tensor pipe with its shared-memory reads (660 us for 65536 x
+// 65536 with the epilogue's examination of the values left out) and the epilogue
+// on the ALU.  The maximum test of every chunk adds 25 us; what remains on top, 110
+// us (190 before), are the chunks that pass it.  They are kept few by bounds
+// shared between column halves, sets and database splits, and cheap by looking at
+// their column groups with independent tests and tournaments.  Two query tiles
+// per block read each database tile once for 256 queries.  65536 x 65536: 909 ->
+// 795 us; 16384 x 32768: 211 -> 110 us; 1500 x 262144: 116 -> 96 us.
 #include <cuda.h>
 #include <cudaTypedefs.h>
+
+#include <algorithm>
 
 #include "orbx_device.cuh"
 #include "orbx_internal.cuh"
 
 namespace orbx {
 
-constexpr int kIBM = 128;  // queries per block (MMA M)
+constexpr int kIBM = 128;  // queries per query tile (MMA M)
+constexpr int kIBQ = 2 * kIBM;  // queries per block of k_match_imma
 constexpr int kIBN = 256;  // database rows per tile (MMA N)
 constexpr int kIK = 256;   // bytes per expanded descriptor (MMA K)
-constexpr int kIStages = 3;
-constexpr int kIEpiWarps = 16;  // four per TMEM lane quarter, 64 columns each
+constexpr int kIStages = 2;
+constexpr int kIEpiWarps = 16;  // two sets of two per TMEM lane quarter, 128 columns each
 constexpr int kIThreads = (2 + kIEpiWarps) * 32;
 constexpr uint32_t kIHalfA = kIBM * 128;  // one 128-byte-wide K half of the query tile
 constexpr uint32_t kIHalfB = kIBN * 128;
 constexpr uint32_t kIATile = 2 * kIHalfA;
 constexpr uint32_t kIBTile = 2 * kIHalfB;
 constexpr uint32_t kINumBars = 1 + 2 * kIStages + 4;
-// 1024 bytes of alignment slack, the query tile, the ring, the barriers, TMEM base + abort flag;
-// the end-of-block merge scratch reuses ring stage 0 (free once the last MMA completed)
-constexpr uint32_t kISmemBytes = 1024 + kIATile + kIStages * kIBTile + 8 * kINumBars + 16;
+// 1024 bytes of alignment slack, the query tiles, the ring, the merge scratch
+// (best two per set, column half and row), the barriers, TMEM base + abort flag
+constexpr uint32_t kIMergeBytes = 4 * kIBM * 8;
+constexpr uint32_t kISmemBytes = 1024 + 2 * kIATile + kIStages * kIBTile + kIMergeBytes + 8 * kINumBars + 16;
 // dynamic tiles + the static s_last and per-row bounds (4 x kIBM 16-bit)
 static_assert(kISmemBytes + 16 + 4 * kIBM * 2 <= 232448, "exceeds the 227 KB shared-memory opt-in");
-static_assert(3 * kIBM * sizeof(uint2) <= kIBTile, "merge scratch must fit in one ring stage");
 constexpr uint32_t kITmemCols = 512;
 constexpr long long kIDeadlineCycles = 4000000000ll;  // ~2 s at 2 GHz
 
@@ -124,6 +142,20 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// The same wait for 32 registers being loaded: as its operands they cannot be
+// read before it.
+__device__ __forceinline__ void tmem_wait_ld32(int* v) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                 "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]),
+                 "+r"(v[15]), "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]),
+                 "+r"(v[22]), "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]),
+                 "+r"(v[29])
+               :
+               : "memory");
+  asm volatile("" : "+r"(v[30]), "+r"(v[31])::"memory");
+}
+
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, int* v) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -136,8 +168,9 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, int* v) {
       : "r"(taddr));
 }
 
-// Dot value given to database columns past the end of the set (never selected).
-constexpr int kMaskedDot = -65536;
+// Dot value given to database columns past the end of the set (never selected:
+// below every dot product, -256 .. 256).
+constexpr int kMaskedDot = -400;
 
 // Three-input max of float bit patterns, without flushing denormals.
 __device__ __forceinline__ float fmax3_bits(float a, float b, float c) {
@@ -146,33 +179,10 @@ __device__ __forceinline__ float fmax3_bits(float a, float b, float c) {
   return r;
 }
 
-// Whether any of 32 dot products exceeds thr.  With thr >= 0 the values are
-// reduced as float bit patterns by three-input max: a non-negative int32 is a
-// zero or denormal float and keeps its order, a negative one is a NaN, which
-// max ignores (it cannot exceed a non-negative thr anyway); 16 instructions
-// instead of the 31 of an integer max.  A negative thr takes the integer max.
-__device__ __forceinline__ bool any_exceeds32(const int* v, int thr) {
-  if (thr >= 0) {
-    float m[12];
-#pragma unroll
-    for (int i = 0; i < 10; i++)
-      m[i] = fmax3_bits(__int_as_float(v[3 * i]), __int_as_float(v[3 * i + 1]), __int_as_float(v[3 * i + 2]));
-    m[10] = __int_as_float(v[30]);
-    m[11] = __int_as_float(v[31]);
-    const float r0 = fmax3_bits(m[0], m[1], m[2]), r1 = fmax3_bits(m[3], m[4], m[5]);
-    const float r2 = fmax3_bits(m[6], m[7], m[8]), r3 = fmax3_bits(m[9], m[10], m[11]);
-    const float r = fmax3_bits(r0, r1, fmax3_bits(r2, r3, r3));
-    const int rb = __float_as_int(r);
-    return rb > thr && rb < 0x7F800000;  // all 32 negative: the result is a NaN
-  }
-  int m = v[0];
-#pragma unroll
-  for (int j = 1; j < 32; j++) m = max(m, v[j]);
-  return m > thr;
-}
-
 // Maxima of the column groups 0-8, 9-17, 18-26 and 27-31 of a 32-column chunk,
-// as float bit patterns (the reduction any_exceeds32 uses, for thr >= 0).
+// for comparison with a threshold >= 0: the values are reduced as float bit
+// patterns by three-input max (a non-negative int32 is a zero or denormal float
+// and keeps its order, a negative one is a NaN, which max ignores).
 __device__ __forceinline__ void group_max4(const int* v, float* r) {
   float m[12];
 #pragma unroll
@@ -185,58 +195,100 @@ __device__ __forceinline__ void group_max4(const int* v, float* r) {
   r[2] = fmax3_bits(m[6], m[7], m[8]);
   r[3] = fmax3_bits(m[9], m[10], m[11]);
 }
-// Whether a group maximum from group_max4 exceeds thr >= 0 (a NaN maximum
-// means every value of the group was negative).
-__device__ __forceinline__ bool bits_exceed(float r, int thr) {
-  const int rb = __float_as_int(r);
-  return rb > thr && rb < 0x7F800000;
-}
+// Whether a group maximum from group_max4 exceeds thr >= 0, compared as floats
+// (a NaN maximum means every value of the group was negative).
+__device__ __forceinline__ bool bits_exceed(float r, int thr) { return r > __int_as_float(thr); }
 
-// Global key (distance << 22 | index) of a chunk-local key (dot << 5 | 31 - column).
-__device__ __forceinline__ uint32_t local_to_key(int lk, int g_chunk) {
-  const int dot = lk >> 5;
-  const int col = 31 - (lk & 31);
-  return ((uint32_t)((256 - dot) >> 1) << kIdxBitsShared) | (uint32_t)(g_chunk + col);
-}
-
-// Top two of columns B .. E-1 of a chunk on local keys (dot << 5 | 31 - column),
-// ties keeping the lower column, pushed into (k1, k2).
-template <int B, int E>
-__device__ __forceinline__ void chunk_top2_push(const int* vc, int gc, uint32_t& k1, uint32_t& k2) {
-  int a1 = INT_MIN, a2 = INT_MIN;
+// The best two of columns B .. E-1 of a chunk as local keys u = column - (dot <<
+// SH), least first, so ties keep the lower column: a tournament of minima (its
+// depth, not its 20 operations for nine columns, is what a warp waits for).
+template <int B, int E, int SH>
+__device__ __forceinline__ void chunk_best2(const int* vc, int& u1, int& u2) {
+  constexpr int n = E - B, h = n / 2;
+  int a1[h], a2[h];
 #pragma unroll
-  for (int j = B; j < E; j++) {
-    const int lk = (vc[j] << 5) | (31 - j);
-    a2 = max(a2, min(a1, lk));
-    a1 = max(a1, lk);
+  for (int i = 0; i < h; i++) {
+    const int x = vc[B + 2 * i] * -(1 << SH) + (B + 2 * i), y = vc[B + 2 * i + 1] * -(1 << SH) + (B + 2 * i + 1);
+    a1[i] = min(x, y);
+    a2[i] = max(x, y);
   }
-  if ((a1 >> 5) > kMaskedDot) top2_push_shared(k1, k2, local_to_key(a1, gc));
-  if ((a2 >> 5) > kMaskedDot) top2_push_shared(k1, k2, local_to_key(a2, gc));
+#pragma unroll
+  for (int d = 1; d < h; d *= 2)
+#pragma unroll
+    for (int i = 0; i + d < h; i += 2 * d) {
+      a2[i] = __vimin3_s32(max(a1[i], a1[i + d]), a2[i], a2[i + d]);
+      a1[i] = min(a1[i], a1[i + d]);
+    }
+  u1 = a1[0];
+  u2 = a2[0];
+  if constexpr (n & 1) {
+    const int x = vc[E - 1] * -(1 << SH) + (E - 1);
+    u2 = min(u2, max(u1, x));
+    u1 = min(u1, x);
+  }
+}
+// Those two merged into the running best two keys (distance << 22 | index): base
+// is the key of a zero dot product at the chunk's column 0, and a dot product of
+// one takes 1 << SH off.  Masked columns carry no key.
+template <int B, int E, int SH>
+__device__ __forceinline__ void chunk_top2_push(const int* vc, uint32_t base, uint32_t& k1, uint32_t& k2) {
+  static_assert(kMaskedDot == -400 && SH <= 22, "400 << SH is an int above every other local key (256 << SH)");
+  constexpr int kMaskedU = (int)((uint32_t)(-kMaskedDot - 1) << SH);
+  int u1, u2;
+  chunk_best2<B, E, SH>(vc, u1, u2);
+  const uint32_t p1 = u1 >= kMaskedU ? kNoKeyShared : base + (uint32_t)u1;
+  const uint32_t p2 = u2 >= kMaskedU ? kNoKeyShared : base + (uint32_t)u2;
+  k2 = __vimin3_u32(max(k1, p1), k2, p2);
+  k1 = min(k1, p1);
 }
 
-// Expand 256-bit descriptors to +-1 int8 rows; rows at or past the count are zero.
-__global__ void k_expand_pm1(const uint8_t* __restrict__ bits, int n_host, const int* d_n, int rows,
-                             int8_t* __restrict__ out) {
-  __shared__ unsigned long long lut[256];
+// Sixteen +-1 bytes from 16 bits, through the 256-entry table of 8.
+__device__ __forceinline__ void expand_lut(unsigned long long* lut) {
   for (int i = threadIdx.x; i < 256; i += blockDim.x) {
     unsigned long long v = 0;
     for (int j = 0; j < 8; j++) v |= (unsigned long long)(((i >> j) & 1) ? 0x01u : 0xFFu) << (8 * j);
     lut[i] = v;
   }
+}
+
+// Expands 256-bit descriptors to +-1 int8 rows, rows at or past the count to
+// zeros: the query set, whose rows' shared bounds it also clears, and the
+// database set (either may have no rows) in one launch.  16 bytes per store.
+struct ExpandSet {
+  const uint8_t* bits;
+  int n;
+  const int* d_n;  // optional count on the device
+  int rows;
+  int8_t* out;
+};
+__global__ void __launch_bounds__(256) k_expand_pm1(ExpandSet q, ExpandSet db, uint32_t* bound, int bounds) {
+  __shared__ unsigned long long lut[256];
+  expand_lut(lut);
   __syncthreads();
-  const int n = d_n ? min(*d_n, rows) : min(n_host, rows);
-  const long long total = (long long)rows * 32;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long r = idx >> 5;
-    const unsigned long long v = (r < n) ? lut[bits[idx]] : 0ull;
-    reinterpret_cast<unsigned long long*>(out)[idx] = v;
+  chain_wait();
+  const int nq = q.rows ? (q.d_n ? min(*q.d_n, q.rows) : min(q.n, q.rows)) : 0;
+  const int nd = db.rows ? (db.d_n ? min(*db.d_n, db.rows) : min(db.n, db.rows)) : 0;
+  const long long tq = (long long)q.rows * 16, total = tq + (long long)db.rows * 16;
+  const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  for (long long i = i0; i < bounds; i += step) bound[i] = kNoKeyShared;
+  for (long long i = i0; i < total; i += step) {
+    const bool is_q = i < tq;
+    const ExpandSet& e = is_q ? q : db;
+    const long long k = is_q ? i : i - tq;
+    ulonglong2 v{};
+    if ((k >> 4) < (is_q ? nq : nd)) {
+      const uint8_t* b = e.bits + 2 * k;  // descriptors may start on any byte
+      v = make_ulonglong2(lut[b[0]], lut[b[1]]);
+    }
+    reinterpret_cast<ulonglong2*>(e.out)[k] = v;
   }
 }
 
-// Warp-uniform bounded wait: lane 0 polls, the result is broadcast.
+// Warp-uniform bounded wait: every lane tries once (no broadcast when the phase
+// is over, the common case); after that lane 0 polls and the result is broadcast.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, long long deadline,
                                           volatile int* abort_flag) {
+  if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
   int ok = 0;
   if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, deadline, abort_flag) ? 1 : 0;
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
@@ -249,20 +301,21 @@ __global__ void __launch_bounds__(kIThreads, 1)
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
   uint8_t* sA = smem;
-  uint8_t* sB = sA + kIATile;
-  int* s_merge = reinterpret_cast<int*>(sB);  // used only after the last tile
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sB + kIStages * kIBTile);
+  uint8_t* sB = sA + 2 * kIATile;
+  uint2* s_merge = reinterpret_cast<uint2*>(sB + kIStages * kIBTile);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(s_merge) + kIMergeBytes);
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + kINumBars);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
   __shared__ unsigned int s_last;
-  // each column group's current second-best distance per query row (0xFFFF:
-  // none yet): two keys at or below it exist, so it bounds what the other
-  // column groups keep for that row (1 KB: the dynamic tiles leave 1.9 KB)
+  // current second-best distance per query row of each set and column half
+  // (0xFFFF: none yet): two keys at or below it exist, so it bounds what the
+  // others that scan the same query keep for that row
   __shared__ uint16_t s_d2[4][kIBM];
 
+  chain_wait();
   const int nq = min(a.d_nq ? *a.d_nq : a.nq, w.nq_cap);
   const int ndb = a.d_ndb ? *a.d_ndb : a.ndb;
-  const int qtiles = (nq + kIBM - 1) / kIBM;
+  const int qtiles = (nq + kIBQ - 1) / kIBQ;
   // With the query count on the device, the grid is sized for the capacity;
   // when fewer query tiles are live, their database scans are split further
   // (up to the merge scratch's splits_cap) so that the whole grid works.
@@ -270,10 +323,13 @@ __global__ void __launch_bounds__(kIThreads, 1)
   const int qb = blockIdx.x / splits;
   const int sp = blockIdx.x - qb * splits;
   if (qb >= qtiles) return;  // uniform over the block: before any barrier or TMEM use
+  const int nq_here = min(kIBQ, nq - qb * kIBQ);
+  const bool two = nq_here > kIBM;  // two query tiles
   const int dbtiles = (ndb + kIBN - 1) / kIBN;
   const int t_beg = (int)((long long)dbtiles * sp / splits);
   const int t_end = (int)((long long)dbtiles * (sp + 1) / splits);
   const int ntiles = t_end - t_beg;
+  const int nsteps = two ? 2 * ntiles : ntiles;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -293,7 +349,7 @@ __global__ void __launch_bounds__(kIThreads, 1)
     }
     for (int s = 0; s < 2; s++) {
       mbar_init(BAR_ACCFULL(s), 1);
-      mbar_init(BAR_ACCEMPTY(s), kIEpiWarps);
+      mbar_init(BAR_ACCEMPTY(s), kIEpiWarps / 2);
     }
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -311,20 +367,17 @@ __global__ void __launch_bounds__(kIThreads, 1)
   const uint32_t tmem_base = *s_tmem;
   const long long deadline = clock64() + kIDeadlineCycles;
 
-  // epilogue state (warps 2..17): best and second-best key of this row
-  const int quarter = warp & 3;
-  const int colgrp = (warp >= 2) ? ((warp - 2) >> 2) : 0;
-  uint32_t k1 = kNoKeyShared, k2 = kNoKeyShared;
-
   if (warp == 0) {
     if (lane == 0) {
       // TMA producer
       int issued[kIStages];
       for (int s = 0; s < kIStages; s++) issued[s] = 0;
       bool ok = true;
-      mbar_expect_tx(BAR_A, kIATile);
-      tma_load_2d(smem_u32(sA), &tmQ, 0, qb * kIBM, BAR_A);
-      tma_load_2d(smem_u32(sA + kIHalfA), &tmQ, 128, qb * kIBM, BAR_A);
+      mbar_expect_tx(BAR_A, two ? 2 * kIATile : kIATile);
+      for (int m = 0; m < (two ? 2 : 1); m++) {
+        tma_load_2d(smem_u32(sA + m * kIATile), &tmQ, 0, qb * kIBQ + m * kIBM, BAR_A);
+        tma_load_2d(smem_u32(sA + m * kIATile + kIHalfA), &tmQ, 128, qb * kIBQ + m * kIBM, BAR_A);
+      }
       for (int i = 0; i < ntiles; i++) {
         const int s = i % kIStages;
         const int use = i / kIStages;
@@ -360,13 +413,15 @@ __global__ void __launch_bounds__(kIThreads, 1)
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      // MMA issuer: eight K=32 steps per tile into accumulator (tile & 1)
+      // MMA issuer: eight K=32 MMAs per step into accumulator (step & 1)
       bool ok = mbar_wait(BAR_A, 0, deadline, s_abort);
-      const uint32_t a_lo = smem_u32(sA);
-      for (int i = 0; ok && i < ntiles; i++) {
-        const int s = i % kIStages;
+      const uint32_t a_base = smem_u32(sA);
+      for (int i = 0; ok && i < nsteps; i++) {
+        const int t = two ? i >> 1 : i;
+        const int qt = two ? i & 1 : 0;
+        const int s = t % kIStages;
         const int acc = i & 1;
-        if (!mbar_wait(BAR_BFULL(s), (uint32_t)(i / kIStages) & 1u, deadline, s_abort)) {
+        if (qt == 0 && !mbar_wait(BAR_BFULL(s), (uint32_t)(t / kIStages) & 1u, deadline, s_abort)) {
           ok = false;
           break;
         }
@@ -376,6 +431,7 @@ __global__ void __launch_bounds__(kIThreads, 1)
         }
         tc_fence_after();
         const uint32_t d = tmem_base + (uint32_t)(acc * kIBN);
+        const uint32_t a_lo = a_base + (uint32_t)qt * kIATile;
         const uint32_t b_lo = smem_u32(sB + s * kIBTile);
 #pragma unroll
         for (int k = 0; k < 8; k++) {
@@ -384,7 +440,7 @@ __global__ void __launch_bounds__(kIThreads, 1)
           const uint64_t db = sw128_desc(b_lo + h * kIHalfB) + (uint64_t)(2 * kk);
           umma_i8(d, da, db, kIDesc, k > 0 ? 1u : 0u);
         }
-        umma_commit(BAR_BEMPTY(s));
+        if (!two || qt == 1) umma_commit(BAR_BEMPTY(s));  // the database tile's last step
         umma_commit(BAR_ACCFULL(acc));
       }
       if (!ok) {
@@ -393,83 +449,115 @@ __global__ void __launch_bounds__(kIThreads, 1)
       }
     }
   } else {
-    // epilogue: TMEM lanes 32*(warp&3).. (one query per lane), columns [64*colgrp, +64)
+    // epilogue: steps of this warp's set, TMEM lanes 32 * (warp & 3) .. (one
+    // query per lane), columns [128 * half, + 128)
+    const int set = (warp - 2) >> 3;
+    const int half = ((warp - 2) >> 2) & 1;
+    const int me = 2 * set + half;
+    const int row = (warp & 3) * 32 + lane;
+    const int q = qb * kIBQ + (two ? set * kIBM : 0) + row;
+    uint32_t k1 = kNoKeyShared, k2 = kNoKeyShared;  // best and second-best key of this row
     bool ok = true;
-    for (int i = 0; i < ntiles; i++) {
-      const int acc = i & 1;
-      if (!warp_wait(BAR_ACCFULL(acc), (uint32_t)(i >> 1) & 1u, deadline, s_abort)) {
-        ok = false;
-        break;
+    // second-best bound shared by the blocks that scan this query's other splits
+    uint32_t* gq = (w.bound && splits > 1 && q < nq) ? w.bound + q : nullptr;
+    uint32_t told = kNoKeyShared, asked = kNoKeyShared, heard = kNoKeyShared;  // published, being read, read
+    int thr_gb = kMaskedDot;  // a dot at or below this cannot reach the row's final top two
+    bool warm = false;        // every lane of the warp has a threshold >= 0
+    // (no key yet: far below every dot)
+    auto next_thr = [&]() { return max(thr_gb, 256 - 2 * (int)(k2 >> kIdxBitsShared)); };
+    int thr = kMaskedDot;
+    // columns arrive in increasing index order, so only a strictly larger dot
+    // than the own second best can enter the top two.  Most chunks end at the
+    // maximum test; one that passes looks at the column groups with a value above
+    // the threshold.  These are few (a lane's top two change a few times per scan)
+    // but they were half of the kernel's time when each group was a serial chain
+    // with its own test.
+    auto examine = [&](const int* vc, int gc) {
+      // distance << 22 = (256 - dot) << 21
+      const uint32_t base = (256u << (kIdxBitsShared - 1)) + (uint32_t)gc;
+      if (!warm) {
+        chunk_top2_push<0, 9, kIdxBitsShared - 1>(vc, base, k1, k2);
+        chunk_top2_push<9, 18, kIdxBitsShared - 1>(vc, base, k1, k2);
+        chunk_top2_push<18, 27, kIdxBitsShared - 1>(vc, base, k1, k2);
+        chunk_top2_push<27, 32, kIdxBitsShared - 1>(vc, base, k1, k2);
+        thr = next_thr();
+        warm = __all_sync(0xffffffffu, thr >= 0);
+        return;
       }
+      float gm[4];
+      group_max4(vc, gm);
+      const float cm = fmax3_bits(gm[0], gm[1], fmax3_bits(gm[2], gm[3], gm[3]));
+      if (!__any_sync(0xffffffffu, bits_exceed(cm, thr))) return;
+      const bool h0 = __any_sync(0xffffffffu, bits_exceed(gm[0], thr)),
+                 h1 = __any_sync(0xffffffffu, bits_exceed(gm[1], thr)),
+                 h2 = __any_sync(0xffffffffu, bits_exceed(gm[2], thr)),
+                 h3 = __any_sync(0xffffffffu, bits_exceed(gm[3], thr));
+      if (h0) chunk_top2_push<0, 9, kIdxBitsShared - 1>(vc, base, k1, k2);
+      if (h1) chunk_top2_push<9, 18, kIdxBitsShared - 1>(vc, base, k1, k2);
+      if (h2) chunk_top2_push<18, 27, kIdxBitsShared - 1>(vc, base, k1, k2);
+      if (h3) chunk_top2_push<27, 32, kIdxBitsShared - 1>(vc, base, k1, k2);
+      thr = next_thr();
+    };
+    const uint32_t tcol = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(set * kIBN + half * 128);
+    for (int i = set; i < nsteps; i += 2) {
+      const int n = i >> 1;  // this set's step
+      ok = warp_wait(BAR_ACCFULL(set), (uint32_t)n & 1u, deadline, s_abort);
+      if (!ok) break;
       tc_fence_after();
-      const int g0 = (t_beg + i) * kIBN + colgrp * 64;
-      const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * kIBN + colgrp * 64);
-      int v[64];
-      tmem_ld32(taddr, v);
-      tmem_ld32(taddr + 32u, v + 32);
-      tmem_wait_ld();
-      // the values are in registers: hand the accumulator back to the MMA warp now
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(BAR_ACCEMPTY(acc));
-      if (g0 + 64 > ndb) {
-#pragma unroll
-        for (int j = 0; j < 64; j++)
-          if (g0 + j >= ndb) v[j] = kMaskedDot;
+      const int g0 = (t_beg + (two ? n : i)) * kIBN + half * 128;
+      // bounds from the others of this block that scan the row's query (every
+      // step) and from its other splits (read in the first steps and then every
+      // fourth, used one step later): a column can reach the row's final top two
+      // only at or below their distance (its index may be lower)
+      {
+        heard = min(heard, asked);
+        if (gq && (n < 8 || (n & 3) == 0)) asked = __ldcg(gq);
+        unsigned gbd = heard >> kIdxBitsShared;
+        auto others = [&](int g) { gbd = min(gbd, (unsigned)reinterpret_cast<volatile uint16_t*>(&s_d2[g][0])[row]); };
+        others(me ^ 1);
+        if (!two) {
+          others(me ^ 2);
+          others(me ^ 3);
+        }
+        if (gbd <= 256u) thr_gb = max(thr_gb, 256 - 2 * (int)gbd - 1);
+        thr = max(thr, thr_gb);
       }
-      // the other column groups' second best for this row: a column can reach the
-      // row's final top two only at or below its distance (its index may be lower)
-      const int row = quarter * 32 + lane;
-      unsigned gbd = 0xFFFFu;
-#pragma unroll
-      for (int g = 0; g < 4; g++)
-        if (g != colgrp) gbd = min(gbd, (unsigned)reinterpret_cast<volatile uint16_t*>(&s_d2[g][0])[row]);
-      const int thr_gb = (gbd == 0xFFFFu) ? kMaskedDot : 256 - 2 * (int)gbd - 1;
-      auto next_thr = [&]() {
-        return max(thr_gb, (k2 == kNoKeyShared) ? kMaskedDot : 256 - 2 * (int)(k2 >> kIdxBitsShared));
-      };
-      int thr = next_thr();
-#pragma unroll
+#pragma unroll 1
       for (int c = 0; c < 2; c++) {
-        // columns arrive in increasing index order, so only a strictly larger dot
-        // than the current second best can enter the top two
-        const int* vc = v + 32 * c;
-        const int gc = g0 + 32 * c;
-        if (__any_sync(0xffffffffu, thr < 0)) {  // a lane has no second best yet: the whole chunk (warp-uniform)
-          chunk_top2_push<0, 32>(vc, gc, k1, k2);
-          thr = next_thr();
-          continue;
+        int v0[32], v1[32];
+        tmem_ld32(tcol + 64u * c, v0);
+        tmem_ld32(tcol + 64u * c + 32u, v1);
+        tmem_wait_ld32(v0);
+        tmem_wait_ld32(v1);
+        if (c == 1) {
+          // every column of this half is in registers: hand the accumulator back
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(BAR_ACCEMPTY(set));
         }
-        float gm[4];
-        group_max4(vc, gm);
-        const float cm = fmax3_bits(gm[0], gm[1], fmax3_bits(gm[2], gm[3], gm[3]));
-        if (!__any_sync(0xffffffffu, bits_exceed(cm, thr))) continue;
-        // only the column groups with a value above the threshold, in column
-        // order, the threshold tightening as the top two improve
-        if (__any_sync(0xffffffffu, bits_exceed(gm[0], thr))) {
-          chunk_top2_push<0, 9>(vc, gc, k1, k2);
-          thr = next_thr();
+        const int gc = g0 + 64 * c;
+        if (gc + 64 > ndb) {
+#pragma unroll
+          for (int j = 0; j < 32; j++) {
+            if (gc + j >= ndb) v0[j] = kMaskedDot;
+            if (gc + 32 + j >= ndb) v1[j] = kMaskedDot;
+          }
         }
-        if (__any_sync(0xffffffffu, bits_exceed(gm[1], thr))) {
-          chunk_top2_push<9, 18>(vc, gc, k1, k2);
-          thr = next_thr();
-        }
-        if (__any_sync(0xffffffffu, bits_exceed(gm[2], thr))) {
-          chunk_top2_push<18, 27>(vc, gc, k1, k2);
-          thr = next_thr();
-        }
-        if (__any_sync(0xffffffffu, bits_exceed(gm[3], thr))) {
-          chunk_top2_push<27, 32>(vc, gc, k1, k2);
-          thr = next_thr();
-        }
+        examine(v0, gc);
+        examine(v1, gc + 32);
       }
-      if (k2 != kNoKeyShared) reinterpret_cast<volatile uint16_t*>(&s_d2[colgrp][0])[row] = (uint16_t)(k2 >> kIdxBitsShared);
+      if (k2 < told) {
+        told = k2;
+        reinterpret_cast<volatile uint16_t*>(&s_d2[me][0])[row] = (uint16_t)(k2 >> kIdxBitsShared);
+        // two distinct rows at or below k2: the query's final second best is no worse
+        if (gq) atomicMin(gq, k2);
+      }
     }
     if (!ok) {
       *s_abort = 1;
       if (lane == 0) atomicOr(err, kErrImmaTimeout);
     }
-    if (colgrp > 0) reinterpret_cast<uint2*>(s_merge)[(colgrp - 1) * kIBM + quarter * 32 + lane] = make_uint2(k1, k2);
+    s_merge[me * kIBM + row] = make_uint2(k1, k2);
   }
 #undef BAR_BFULL
 #undef BAR_BEMPTY
@@ -483,24 +571,25 @@ __global__ void __launch_bounds__(kIThreads, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kITmemCols)
                  : "memory");
   }
-  if (warp >= 2 && colgrp == 0) {
-    // merge the four column groups of each row
-    const int row = quarter * 32 + lane;
-    for (int g = 0; g < 3; g++) {
-      const uint2 pk = reinterpret_cast<const uint2*>(s_merge)[g * kIBM + row];
+  // the best two of each query over the block's sets and column halves
+  const int rows = two ? kIBQ : kIBM;
+  for (int r = threadIdx.x; r < rows; r += kIThreads) {
+    const int q = qb * kIBQ + r;
+    if (q >= nq) break;
+    uint32_t k1 = kNoKeyShared, k2 = kNoKeyShared;
+    for (int g = 0; g < (two ? 2 : 4); g++) {
+      const uint2 pk = s_merge[(two ? 2 * (r / kIBM) + g : g) * kIBM + r % kIBM];
       top2_push_shared(k1, k2, pk.x);
       top2_push_shared(k1, k2, pk.y);
     }
-    const int q = qb * kIBM + row;
-    if (q < nq) {
-      if (splits == 1)
-        finish_query_shared(a, q, k1, k2);
-      else
-        reinterpret_cast<uint2*>(w.part)[(size_t)sp * w.nq_cap + q] = make_uint2(k1, k2);
-    }
+    if (splits == 1)
+      finish_query_shared(a, q, k1, k2);
+    else
+      reinterpret_cast<uint2*>(w.part)[(size_t)sp * w.nq_cap + q] = make_uint2(k1, k2);
   }
   if (splits == 1) return;
-  // the last block of this query tile to finish merges the partial top-2 of all splits
+  // the last block of these queries to finish merges the partial top-2 of all
+  // splits: 2 or 4 threads per query
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) s_last = (atomicAdd(&w.tile_done[qb], 1u) == (unsigned)(splits - 1)) ? 1u : 0u;
@@ -508,17 +597,32 @@ __global__ void __launch_bounds__(kIThreads, 1)
   if (!s_last) return;
   __threadfence();
   if (threadIdx.x == 0) w.tile_done[qb] = 0u;
-  if (threadIdx.x >= kIBM) return;
-  const int q = qb * kIBM + threadIdx.x;
-  if (q >= nq) return;
-  const uint2* part = reinterpret_cast<const uint2*>(w.part);
-  uint32_t m1 = kNoKeyShared, m2 = kNoKeyShared;
-  for (int s2 = 0; s2 < splits; s2++) {
-    const uint2 pk = __ldcg(part + (size_t)s2 * w.nq_cap + q);
-    top2_push_shared(m1, m2, pk.x);
-    top2_push_shared(m1, m2, pk.y);
+  const int per = two ? 2 : 4;
+  if (threadIdx.x < rows * per) {
+    const int r = threadIdx.x % rows, g = threadIdx.x / rows;
+    const int q = qb * kIBQ + r;
+    uint32_t m1 = kNoKeyShared, m2 = kNoKeyShared;
+    if (q < nq) {
+      const uint2* part = reinterpret_cast<const uint2*>(w.part) + q;
+#pragma unroll 8
+      for (int s2 = g; s2 < splits; s2 += per) {
+        const uint2 pk = __ldcg(part + (size_t)s2 * w.nq_cap);
+        top2_push_shared(m1, m2, pk.x);
+        top2_push_shared(m1, m2, pk.y);
+      }
+    }
+    s_merge[g * rows + r] = make_uint2(m1, m2);
   }
-  finish_query_shared(a, q, m1, m2);
+  __syncthreads();
+  if (threadIdx.x < rows && qb * kIBQ + (int)threadIdx.x < nq) {
+    uint32_t m1 = kNoKeyShared, m2 = kNoKeyShared;
+    for (int g = 0; g < per; g++) {
+      const uint2 pk = s_merge[g * rows + threadIdx.x];
+      top2_push_shared(m1, m2, pk.x);
+      top2_push_shared(m1, m2, pk.y);
+    }
+    finish_query_shared(a, qb * kIBQ + (int)threadIdx.x, m1, m2);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -902,7 +1006,11 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
         pc = __popc(w0.x) + __popc(w0.y) + __popc(w0.z) + __popc(w0.w) + __popc(w1.x) + __popc(w1.y) +
              __popc(w1.z) + __popc(w1.w);
       }
+      // best two keys of this row over the item, distance << 22 | row within the
+      // cluster: the cluster's list is in increasing database index, so they order
+      // like keys of database indices, into which they are turned at the end
       uint32_t k1 = kNoKeyShared, k2 = kNoKeyShared;
+      const uint32_t bias = (uint32_t)pc << kIdxBitsShared;
       for (int t = 0; t < ri.tiles; t++, g++) {
         const uint32_t acc = g & 1u;
         if (!rr_warp_wait(RR_ACCFULL(acc), (g >> 1) & 1u, s_abort)) {
@@ -917,7 +1025,7 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
         for (int c = 0; c < 2; c++) {
           int v[32];
           tmem_ld32(taddr + 32u * c, v);
-          tmem_wait_ld();
+          tmem_wait_ld32(v);
           if (c == 1) {
             // every column of this group is in registers: hand the accumulator back
             tc_fence_before();
@@ -931,37 +1039,38 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
             for (int j = 0; j < 32; j++)
               if (j >= valid) v[j] = kMaskedDot;
           }
-          // The cluster's list is in increasing database index and the columns
-          // arrive in list order, so only a strictly larger dot' (a strictly
-          // smaller distance) than the current second best's can enter.
-          int thr = (k2 == kNoKeyShared) ? kMaskedDot : pc - (int)(k2 >> kIdxBitsShared);
-          // another item of the same query may already hold a closer second best:
-          // columns farther than it cannot reach the query's top two (equal
-          // distances stay, their index decides)
+          // The columns arrive in list order, so only a strictly larger dot' (a
+          // strictly smaller distance) than the current second best's can enter,
+          // and no column farther than the second best that another item of the
+          // same query holds (equal distances stay, their index decides)
+          int thr = pc - (int)(k2 >> kIdxBitsShared);  // no key yet: below every dot'
           if (gb != kNoKeyShared) thr = max(thr, pc - (int)(gb >> kIdxBitsShared) - 1);
-          if (__any_sync(0xffffffffu, any_exceeds32(v, thr))) {
-            // the chunk's best two on local keys (dot' << 5 | 31 - column): ties keep the lower column
-            int a1 = INT_MIN, a2 = INT_MIN;
-#pragma unroll
-            for (int j = 0; j < 32; j++) {
-              const int lk = (v[j] << 5) | (31 - j);
-              a2 = max(a2, min(a1, lk));
-              a1 = max(a1, lk);
-            }
-            if ((a1 >> 5) > thr) {
-              const int m1 = __ldg(a.pad_members + ri.pbase + col0 + 31 - (a1 & 31));
-              top2_push_shared(k1, k2, ((uint32_t)(pc - (a1 >> 5)) << kIdxBitsShared) | (uint32_t)m1);
-              if ((a2 >> 5) > thr) {
-                const int m2 = __ldg(a.pad_members + ri.pbase + col0 + 31 - (a2 & 31));
-                top2_push_shared(k1, k2, ((uint32_t)(pc - (a2 >> 5)) << kIdxBitsShared) | (uint32_t)m2);
-              }
-            }
+          bool h0 = true, h1 = true, h2 = true, h3 = true;
+          if (__all_sync(0xffffffffu, thr >= 0)) {
+            float gm[4];
+            group_max4(v, gm);
+            const float cm = fmax3_bits(gm[0], gm[1], fmax3_bits(gm[2], gm[3], gm[3]));
+            if (!__any_sync(0xffffffffu, bits_exceed(cm, thr))) continue;
+            h0 = __any_sync(0xffffffffu, bits_exceed(gm[0], thr));
+            h1 = __any_sync(0xffffffffu, bits_exceed(gm[1], thr));
+            h2 = __any_sync(0xffffffffu, bits_exceed(gm[2], thr));
+            h3 = __any_sync(0xffffffffu, bits_exceed(gm[3], thr));
           }
+          const uint32_t base = bias + (uint32_t)col0;
+          if (h0) chunk_top2_push<0, 9, kIdxBitsShared>(v, base, k1, k2);
+          if (h1) chunk_top2_push<9, 18, kIdxBitsShared>(v, base, k1, k2);
+          if (h2) chunk_top2_push<18, 27, kIdxBitsShared>(v, base, k1, k2);
+          if (h3) chunk_top2_push<27, 32, kIdxBitsShared>(v, base, k1, k2);
         }
       }
       if (!ok) break;
       if (slot >= 0) {
-        a.partial[(size_t)slot * kRrGroups + colgrp] = make_uint2(k1, k2);
+        auto member = [&](uint32_t key) {
+          return key == kNoKeyShared
+                     ? key
+                     : (key & ~kIdxMaskShared) | (uint32_t)__ldg(a.pad_members + ri.pbase + (key & kIdxMaskShared));
+        };
+        a.partial[(size_t)slot * kRrGroups + colgrp] = make_uint2(member(k1), member(k2));
         // two distinct rows at or below k2: the query's final second best is no worse
         if (k2 != kNoKeyShared) atomicMin(a.q_bound + (slot >> 3), k2);
       }
@@ -1020,30 +1129,31 @@ static bool make_rows_map(CUtensorMap* m, const void* base, uint64_t rows, uint3
 }
 
 int imma_rows_q(int n) { return (n + kIBM - 1) / kIBM * kIBM; }
+int imma_rows_db(int n) { return (n + kIBN - 1) / kIBN * kIBN; }
 
-// Database splits per query tile so that the grid fills the 148 SMs in whole
-// waves (one 227 KB block per SM): 512 query tiles -> 2 splits -> 1024 blocks.
-int imma_default_splits(int nq_cap) {
-  const int qt = (nq_cap + kIBM - 1) / kIBM;
+// Database splits per 256 queries: of the grids up to 64 splits the one with the
+// least time, whole waves of 148 blocks (one 200 KB block per SM) whose time is
+// their database tiles plus about 10 tiles' worth for starting, finding the first
+// bounds and merging.  65536 x 65536: 256 query tiles x 4 splits; 16384 x 32768:
+// 64 x 2, 122 us against 244 with 64 x 16.
+int imma_default_splits(int nq_cap, int ndb) {
+  const long long qt = (nq_cap + kIBQ - 1) / kIBQ;
+  const int tiles = std::max(1, (ndb + kIBN - 1) / kIBN);
   int best = 1;
-  double best_eff = 0.0;
-  for (int s = 1; s <= 16; s++) {
-    const long long blocks = (long long)qt * s;
-    const long long waves = (blocks + 147) / 148;
-    const double eff = (double)blocks / (double)(waves * 148);
-    if (eff > best_eff + 0.02) {
-      best_eff = eff;
+  double best_cost = 1e300;
+  for (int s = 1; s <= std::min(kImmaMaxSplits, tiles); s++) {
+    const double cost = (double)((qt * s + 147) / 148) * ((double)tiles / s + 10.0);
+    if (cost < best_cost) {
+      best_cost = cost;
       best = s;
     }
   }
   return best;
 }
-int imma_rows_db(int n) { return (n + kIBN - 1) / kIBN * kIBN; }
 
 cudaError_t launch_expand_pm1(const uint8_t* bits, int n, const int* d_n, int rows, int8_t* out, cudaStream_t s) {
-  if (rows <= 0) return cudaSuccess;
-  k_expand_pm1<<<4 * 148, 256, 0, s>>>(bits, n, d_n, rows, out);
-  return cudaGetLastError();
+  return launch_chained(k_expand_pm1, 4 * 148, 256, s, ExpandSet{bits, n, d_n, rows, out}, ExpandSet{},
+                        static_cast<uint32_t*>(nullptr), 0);
 }
 
 cudaError_t launch_match_imma(const ImmaLaunch& L, cudaStream_t s) {
@@ -1057,17 +1167,22 @@ cudaError_t launch_match_imma(const ImmaLaunch& L, cudaStream_t s) {
   const int qrows = imma_rows_q(L.nq_cap);
   const int dbrows = imma_rows_db(L.ndb_cap > 0 ? L.ndb_cap : 1);
   {
-    const int blocks = 4 * 148;
-    if (!L.q_ready) k_expand_pm1<<<blocks, 256, 0, s>>>(L.args.q, L.args.nq, L.args.d_nq, qrows, L.q_pm1);
-    if (L.ndb_cap > 0 && !L.db_ready)
-      k_expand_pm1<<<blocks, 256, 0, s>>>(L.args.db, L.args.ndb, L.args.d_ndb, dbrows, L.db_pm1);
+    ExpandSet q{}, db{};
+    if (!L.q_ready) q = ExpandSet{L.args.q, L.args.nq, L.args.d_nq, qrows, L.q_pm1};
+    if (L.ndb_cap > 0 && !L.db_ready) db = ExpandSet{L.args.db, L.args.ndb, L.args.d_ndb, dbrows, L.db_pm1};
+    const int bounds = L.work.bound ? std::min(L.work.nq_cap, L.nq_cap) : 0;
+    if (q.rows || db.rows || bounds) {
+      const cudaError_t e = launch_chained(k_expand_pm1, 4 * 148, 256, s, q, db, L.work.bound, bounds);
+      if (e != cudaSuccess) return e;
+    }
   }
   CUtensorMap tq, td;
   if (!make_rows_map(&tq, L.q_pm1, (uint64_t)qrows, kIBM)) return cudaErrorInvalidValue;
   if (!make_rows_map(&td, L.db_pm1, (uint64_t)dbrows, kIBN)) return cudaErrorInvalidValue;
-  const int qtiles = qrows / kIBM;
-  k_match_imma<<<qtiles * L.splits, kIThreads, kISmemBytes, s>>>(tq, td, L.args, L.work, L.splits, L.err);
-  return cudaGetLastError();
+  const int qtiles = (L.nq_cap + kIBQ - 1) / kIBQ;
+  const int splits = std::max(1, std::min(L.splits, dbrows / kIBN));
+  return launch_chained_smem(k_match_imma, qtiles * splits, kIThreads, kISmemBytes, s, tq, td, L.args, L.work, splits,
+                             L.err);
 }
 
 cudaError_t launch_rerank_imma(const RerankImmaArgs& a, int max_items, cudaStream_t s) {

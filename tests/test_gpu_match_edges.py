@@ -44,3 +44,28 @@ def test_tile_chunk_and_tie_edges(nq):
         got = A.points[:nq].cpu().numpy()
         assert np.array_equal(got[:, 5], m) and np.array_equal(got[:, 6], d), ndb
     ctx.close()
+
+
+@pytest.mark.parametrize("nq", [1, 127, 128, 129, 255, 256, 257, 600])
+def test_tensor_core_form_equals_popcount_form(nq):
+    """One or two query tiles per block, database rows around the 256-row tiles, few
+    or many splits (which share their bounds), and distances that mostly tie."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    rng = np.random.default_rng(1000 + nq)
+    ctx = orbx.Context(0, orbx.make_params(max_pts=1024))
+    base = rng.integers(0, 256, (40, 32), dtype=np.uint8)
+    base[0], base[1] = 0, 255
+    for ndb in (1, 2, 31, 255, 256, 257, 511, 513, 2048, 9000, 70001):
+        def draw(n):
+            d = base[rng.integers(0, 40, n)]
+            d[:, 5] ^= rng.integers(0, 8, n).astype(np.uint8)
+            return torch.from_numpy(d).cuda()
+        q, db = draw(nq), draw(ndb)
+        torch.cuda.synchronize()
+        want = orbx.knn2(ctx, q, db, orbx.MATCH_POPC)
+        got = orbx.knn2(ctx, q, db, orbx.MATCH_IMMA)
+        ctx.sync()
+        for w, g in zip(want, got):
+            assert torch.equal(w, g), ndb
+    ctx.close()
