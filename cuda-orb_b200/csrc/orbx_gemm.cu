@@ -128,8 +128,44 @@ __device__ __forceinline__ void g_tmem_ld32(uint32_t taddr, float* v) {
 }
 }  // namespace
 
-// Epilogue of 32 columns [n0, n0 + 32) of row m (values in v).
-__device__ __forceinline__ void g_epilogue_chunk(const GemmArgs& g, int split, int m, int n0, float* v, uint32_t* top) {
+// Eight keys into descending order (Batcher's 19 comparators).
+__device__ __forceinline__ void sort8(uint32_t* k) {
+  constexpr int at[19][2] = {{0, 1}, {2, 3}, {4, 5}, {6, 7}, {0, 2}, {1, 3}, {4, 6}, {5, 7}, {1, 2}, {5, 6},
+                             {0, 4}, {1, 5}, {2, 6}, {3, 7}, {2, 4}, {3, 5}, {1, 2}, {3, 4}, {5, 6}};
+#pragma unroll
+  for (int i = 0; i < 19; i++) {
+    const uint32_t hi = max(k[at[i][0]], k[at[i][1]]), lo = min(k[at[i][0]], k[at[i][1]]);
+    k[at[i][0]] = hi;
+    k[at[i][1]] = lo;
+  }
+}
+// The eight largest of two descending lists, into a (descending).
+__device__ __forceinline__ void merge8(uint32_t* a, const uint32_t* b) {
+  uint32_t c[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) c[i] = max(a[i], b[7 - i]);  // a bitonic sequence
+#pragma unroll
+  for (int d = 4; d >= 1; d >>= 1)
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+      if (!(i & d)) {
+        const uint32_t hi = max(c[i], c[i + d]), lo = min(c[i], c[i + d]);
+        c[i] = hi;
+        c[i + d] = lo;
+      }
+#pragma unroll
+  for (int i = 0; i < 8; i++) a[i] = c[i];
+}
+
+// Columns after which a list takes single columns instead of sorting whole
+// chunks: there a column enters some lane's list less than every third time.  A
+// sorted chunk costs 410 instructions, one that enters 24.
+constexpr int kTopSortCols = 512;
+
+// Epilogue of 32 columns [n0, n0 + 32) of row m (values in v); seen: columns the
+// row's top list has taken before.
+__device__ __forceinline__ void g_epilogue_chunk(const GemmArgs& g, int split, int m, int n0, int seen, float* v,
+                                                 uint32_t* top) {
   if (g.bias && g.splits == 1) {
 #pragma unroll
     for (int j = 0; j < 32; j++) v[j] = __fadd_rn(v[j], __ldg(g.bias + n0 + j));
@@ -146,6 +182,18 @@ __device__ __forceinline__ void g_epilogue_chunk(const GemmArgs& g, int split, i
 #pragma unroll
     for (int j = 1; j < 32; j++) mx = fmaxf(mx, v[j]);
     if (!__any_sync(0xffffffffu, top_key(mx, n0) > top[kTopK - 1])) return;  // no column of this chunk can enter
+    if (seen < kTopSortCols) {
+      uint32_t k[32];
+#pragma unroll
+      for (int j = 0; j < 32; j++) k[j] = v[j] == v[j] ? top_key(v[j], n0 + j) : 0u;  // a NaN never enters
+#pragma unroll
+      for (int i = 0; i < 4; i++) sort8(k + 8 * i);
+      merge8(k, k + 8);
+      merge8(k + 16, k + 24);
+      merge8(k, k + 16);
+      merge8(top, k);
+      return;
+    }
     // a key above the 8th needs a logit at least the 8th's (truncated) value
     float f8 = top[kTopK - 1] ? order_bits_float(top[kTopK - 1] & ~((1u << kTopColBits) - 1u)) : -INFINITY;
 #pragma unroll
@@ -263,6 +311,7 @@ __global__ void __launch_bounds__(kGThreads, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *s_tmem;
+  chain_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -376,7 +425,7 @@ __global__ void __launch_bounds__(kGThreads, 1)
             __syncwarp();
             if (lane == 0) g_mbar_arrive(GBAR_ACCEMPTY(acc));
           }
-          g_epilogue_chunk(g, it.split, m, tn * kGBN + half * 128 + c * 32, v, top);
+          g_epilogue_chunk(g, it.split, m, tn * kGBN + half * 128 + c * 32, (row_top ? t * 128 : 0) + c * 32, v, top);
         }
         if (g.mode == kTop8) {
           uint4* dst = reinterpret_cast<uint4*>(g.top_keys + ((size_t)m * (2 * n_tiles) + 2 * tn + half) * kTopK);
@@ -451,8 +500,7 @@ cudaError_t launch_gemm_bf16(const GemmArgs& g, cudaStream_t s) {
     return cudaErrorInvalidValue;
   const int items = g.mode == kTop8Row ? (g.M / kGBM) * gemm_top_parts(g.N / kGBN) : (g.M / kGBM) * (g.N / kGBN) * g.splits;
   const int blocks = items < sms ? items : sms;  // persistent: one block per SM
-  k_gemm_bf16<<<blocks, kGThreads, kGSmemBytes, s>>>(ta, tb, g);
-  return cudaGetLastError();
+  return launch_chained_smem(k_gemm_bf16, blocks, kGThreads, kGSmemBytes, s, ta, tb, g);
 }
 
 }  // namespace orbx

@@ -31,8 +31,12 @@ constexpr uint16_t kBfPlus1 = 0x3F80u, kBfMinus1 = 0xBF80u;
 // out[r][k] = bit k of row r ? +1 : -1 (bit k = byte k / 8, bit k % 8), rows
 // n..rows-1 are zero.  One thread per (row, byte): one 16-byte store.
 __global__ void k_bits_pm1_bf16(const uint8_t* __restrict__ bits, int n, const int* d_n, int rows,
-                                __nv_bfloat16* __restrict__ out) {
+                                __nv_bfloat16* __restrict__ out, SearchReset reset) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  chain_wait();
+  if (t < reset.clusters) reset.counts[t] = 0;
+  if (t < reset.nq) reset.bound[t] = kNoKeyShared;
+  if (t == 0 && reset.fb_count) *reset.fb_count = *reset.rr_counter = 0;
   if (t >= (long long)rows * 32) return;
   const int r = (int)(t >> 5), j = (int)(t & 31);
   const int nv = d_n ? min(*d_n, n) : n;
@@ -396,6 +400,7 @@ __global__ void __launch_bounds__(1024) k_scan_counts(const int* __restrict__ co
   __shared__ int s_sum[1024], s_items[1024];
   const int t = threadIdx.x;
   const int per = (k + 1023) / 1024;
+  chain_wait();
   int local = 0, local_items = 0;
   for (int j = 0; j < per; j++) {
     const int c = t * per + j;
@@ -533,71 +538,91 @@ __global__ void k_labels(const int32_t* __restrict__ idx2, int n, const int* __r
 }
 
 // ---------------------------------------------------------------- search
-// One warp per query: merge the GEMM's top-8 key lists (one per 128 columns,
-// lists * 8 keys) into the query's n_probe best clusters.  margin = logit1 - logit2.  A query
-// whose margin is below margin_thr probes nothing (the exact fallback answers
-// it); otherwise its non-empty probed clusters are counted.  Every partial entry
+// One warp per query: merge the row-wise GEMM's top-8 key lists (2 or 4, so at
+// most one key per lane) into the query's n_probe best clusters.  margin = logit1
+// - logit2, also written to margin_out when given.  A query whose margin is below
+// margin_thr probes nothing (the exact fallback answers it).  Every partial entry
 // (per_slot per probe slot, per_slot <= 4) starts empty.
 __global__ void __launch_bounds__(256) k_select_probes(const uint32_t* __restrict__ keys, int nq, int lists,
                                                        int n_probe, float margin_thr, const int* __restrict__ ivf_offsets,
                                                        int* __restrict__ probes, float* __restrict__ margin,
-                                                       int* __restrict__ probe_counts, uint2* __restrict__ partial,
+                                                       float* __restrict__ margin_out, uint2* __restrict__ partial,
                                                        int per_slot) {
   const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
+  chain_wait();
   if (q >= nq) return;
-  const int nk = lists * kTopK;  // <= 256
-  const int kpl = (nk + 31) >> 5;
-  uint32_t mine[8];
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const int j = lane * kpl + i;
-    mine[i] = (i < kpl && j < nk) ? keys[(size_t)q * nk + j] : 0u;
-  }
-  // the lane's keys in descending order
-#pragma unroll
-  for (int a = 0; a < 7; a++)
-#pragma unroll
-    for (int b = 0; b < 7 - a; b++) {
-      const uint32_t hi = max(mine[b], mine[b + 1]), lo = min(mine[b], mine[b + 1]);
-      mine[b] = hi;
-      mine[b + 1] = lo;
-    }
-  uint32_t best[kTopK];
+  const int nk = lists * kTopK;  // <= 32
+  uint32_t mine = lane < nk ? keys[(size_t)q * nk + lane] : 0u;
+  if (lane < kTopK * per_slot) partial[(size_t)q * kTopK * per_slot + lane] = make_uint2(kNoKeyShared, kNoKeyShared);
+  // the keys are distinct columns: lane i < 8 ends with the i-th largest
+  uint32_t best = 0u, first = 0u, second = 0u;
 #pragma unroll
   for (int i = 0; i < kTopK; i++) {
-    const uint32_t m = __reduce_max_sync(0xffffffffu, mine[0]);
-    best[i] = m;
-    if (mine[0] == m && m != 0u) {
-#pragma unroll
-      for (int k = 0; k < 7; k++) mine[k] = mine[k + 1];
-      mine[7] = 0u;
-    }
+    const uint32_t m = __reduce_max_sync(0xffffffffu, mine);
+    if (i == 0) first = m;
+    if (i == 1) second = m;
+    if (lane == i) best = m;
+    if (mine == m) mine = 0u;
   }
-  const float l1 = order_bits_float(best[0] & ~((1u << kTopColBits) - 1u));
-  const float l2 = order_bits_float(best[1] & ~((1u << kTopColBits) - 1u));
+  const float l1 = order_bits_float(first & ~((1u << kTopColBits) - 1u));
+  const float l2 = order_bits_float(second & ~((1u << kTopColBits) - 1u));
   const float mg = l1 - l2;
   const bool fb = mg < margin_thr;  // answered by the exact fallback: nothing to probe
-  if (lane < kTopK * per_slot) partial[(size_t)q * kTopK * per_slot + lane] = make_uint2(kNoKeyShared, kNoKeyShared);
-  if (lane == 0) margin[q] = mg;
+  if (lane == 0) {
+    margin[q] = mg;
+    if (margin_out) margin_out[q] = mg;
+  }
   if (lane < kTopK) {
-    int c = -1;
-#pragma unroll
-    for (int i = 0; i < kTopK; i++)
-      if (i == lane) c = best[i] ? top_key_col(best[i]) : -1;
+    int c = best ? top_key_col(best) : -1;
     if (lane >= n_probe || fb || c < 0 || ivf_offsets[c + 1] == ivf_offsets[c]) c = -1;
     probes[(size_t)q * kTopK + lane] = c;
-    if (c >= 0) atomicAdd(&probe_counts[c], 1);
   }
 }
 
-// list[cursor[c]++] = q * 8 + slot for every live probe (q, slot) of cluster c
-__global__ void k_fill_probe_lists(const int* __restrict__ probes, int nq, int* __restrict__ cursor,
-                                   int* __restrict__ list) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nq * kTopK) return;
-  const int c = probes[t];
-  if (c >= 0) list[atomicAdd(&cursor[c], 1)] = t;
+// Per-cluster lists of the live probes (q, slot): list[cursor[c]++] = q * 8 +
+// slot.  Popular clusters' counters are what bounds this: atomics of one address
+// follow each other at about 80 ns, and with one per probe the 512 counters of
+// 262144 probes took 43 us to count and 45 us to fill.  A block therefore takes
+// kProbesPerBlock probes, counts them per cluster in shared memory and adds once
+// per cluster and block; filling, that sum is the block's place in the list.
+__global__ void __launch_bounds__(1024) k_count_probes(const int* __restrict__ probes, int n, int clusters,
+                                                       int* __restrict__ counts) {
+  extern __shared__ int s_count[];
+  for (int c = threadIdx.x; c < clusters; c += 1024) s_count[c] = 0;
+  __syncthreads();
+  chain_wait();
+  const int end = min(n, ((int)blockIdx.x + 1) * kProbesPerBlock);
+  for (int t = blockIdx.x * kProbesPerBlock + threadIdx.x; t < end; t += 1024) {
+    const int c = probes[t];
+    if (c >= 0) atomicAdd(&s_count[c], 1);
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < clusters; c += 1024)
+    if (s_count[c]) atomicAdd(&counts[c], s_count[c]);
+}
+__global__ void __launch_bounds__(1024) k_fill_probe_lists(const int* __restrict__ probes, int n, int clusters,
+                                                           int* __restrict__ cursor, int* __restrict__ list) {
+  extern __shared__ int s_count[];
+  constexpr int kPer = kProbesPerBlock / 1024;
+  for (int c = threadIdx.x; c < clusters; c += 1024) s_count[c] = 0;
+  __syncthreads();
+  chain_wait();
+  int cl[kPer], at[kPer];
+#pragma unroll
+  for (int i = 0; i < kPer; i++) {
+    const int t = blockIdx.x * kProbesPerBlock + i * 1024 + threadIdx.x;
+    cl[i] = t < n ? probes[t] : -1;
+  }
+#pragma unroll
+  for (int i = 0; i < kPer; i++) at[i] = cl[i] >= 0 ? atomicAdd(&s_count[cl[i]], 1) : 0;
+  __syncthreads();
+  for (int c = threadIdx.x; c < clusters; c += 1024)
+    if (s_count[c]) s_count[c] = atomicAdd(&cursor[c], s_count[c]);
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kPer; i++)
+    if (cl[i] >= 0) list[s_count[cl[i]] + at[i]] = blockIdx.x * kProbesPerBlock + i * 1024 + threadIdx.x;
 }
 
 constexpr int kRerankChunk = 256;
@@ -662,6 +687,7 @@ __global__ void k_merge_probes(const uint2* __restrict__ partial, int per_slot, 
                                float margin_thr, int max_dist, uint32_t* __restrict__ dist2,
                                int32_t* __restrict__ idx2, int* __restrict__ fb_list, int* __restrict__ fb_count) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  chain_wait();
   if (q >= nq) return;
   uint32_t k1 = kNoKeyShared, k2 = kNoKeyShared;
   const int n = kTopK * per_slot;
@@ -686,6 +712,7 @@ __global__ void k_merge_probes(const uint2* __restrict__ partial, int per_slot, 
 __global__ void k_gather_fallback(const uint8_t* __restrict__ q_desc, const int* __restrict__ fb_list,
                                   const int* __restrict__ fb_count, uint8_t* __restrict__ out) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  chain_wait();
   if ((t >> 1) >= *fb_count) return;
   const int j = t >> 1, h = t & 1;
   reinterpret_cast<uint4*>(out)[2 * (size_t)j + h] =
@@ -694,8 +721,11 @@ __global__ void k_gather_fallback(const uint8_t* __restrict__ q_desc, const int*
 
 __global__ void k_scatter_fallback(const int* __restrict__ fb_list, const int* __restrict__ fb_count,
                                    const uint32_t* __restrict__ fd, const int32_t* __restrict__ fi,
-                                   uint32_t* __restrict__ dist2, int32_t* __restrict__ idx2) {
+                                   uint32_t* __restrict__ dist2, int32_t* __restrict__ idx2,
+                                   int* __restrict__ count_out) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  chain_wait();
+  if (j == 0 && count_out) *count_out = *fb_count;
   if (j >= *fb_count) return;
   const int q = fb_list[j];
   dist2[2 * q] = fd[2 * j];

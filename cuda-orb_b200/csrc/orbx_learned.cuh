@@ -79,7 +79,17 @@ struct AdamStep {
 };
 
 // orbx_learned.cu
-__global__ void k_bits_pm1_bf16(const uint8_t* bits, int n, const int* d_n, int rows, __nv_bfloat16* out);
+// What a search clears before it starts, done by its first kernel.
+struct SearchReset {
+  int clusters;     // counts[clusters]
+  int nq;           // bound[nq], to "no key"
+  int* counts;
+  uint32_t* bound;
+  int* fb_count;
+  int* rr_counter;
+};
+__global__ void k_bits_pm1_bf16(const uint8_t* bits, int n, const int* d_n, int rows, __nv_bfloat16* out,
+                                SearchReset reset);
 __global__ void k_bits_pm1_bf16_t(const uint8_t* bits, int n, int rows, __nv_bfloat16* out);
 __global__ void k_softmax_xent(const float* logits, const int* labels, int S, int n, int rows, int C,
                                float grad_scale, __nv_bfloat16* dL, float* loss, int* correct);
@@ -99,9 +109,11 @@ __global__ void k_count(const int* assign, int n, int* counts);
 __global__ void k_accum_stats(const float* loss, const int* correct, int n, float* acc);
 __global__ void k_labels(const int32_t* idx2, int n, const int* row_sets, int set_width, int S, int* labels);
 __global__ void k_select_probes(const uint32_t* keys, int nq, int lists, int n_probe, float margin_thr,
-                                const int* ivf_offsets, int* probes, float* margin, int* probe_counts,
-                                uint2* partial, int per_slot);
-__global__ void k_fill_probe_lists(const int* probes, int nq, int* cursor, int* list);
+                                const int* ivf_offsets, int* probes, float* margin, float* margin_out, uint2* partial,
+                                int per_slot);
+constexpr int kProbesPerBlock = 8192;  // of k_count_probes and k_fill_probe_lists (1024 threads, clusters ints of shared memory)
+__global__ void k_count_probes(const int* probes, int n, int clusters, int* counts);
+__global__ void k_fill_probe_lists(const int* probes, int n, int clusters, int* cursor, int* list);
 __global__ void k_rerank(const uint8_t* q_desc, const int* list, const int* probe_offsets, const int* item_offsets,
                          int n_clusters, const uint8_t* ivf_desc, const int* ivf_members, const int* ivf_offsets,
                          uint2* partial);
@@ -125,7 +137,7 @@ __global__ void k_stable_scatter(const int32_t* idx, long long total, int per_ro
                                  int* members);
 __global__ void k_gather_fallback(const uint8_t* q_desc, const int* fb_list, const int* fb_count, uint8_t* out);
 __global__ void k_scatter_fallback(const int* fb_list, const int* fb_count, const uint32_t* fd, const int32_t* fi,
-                                   uint32_t* dist2, int32_t* idx2);
+                                   uint32_t* dist2, int32_t* idx2, int* count_out);
 __global__ void k_lsh_probes(const float* proj, int rows_stride, int n, int nbits, int n_probe, const int* ivf_offsets,
                              int* probes, int* probe_counts, int* bucket_out, float* margin, uint2* partial,
                              int per_slot);

@@ -242,7 +242,7 @@ int train_alloc(orbx_learned* L, TrainBufs& T, int B, int S = 1) {
 int forward_backward(orbx_learned* L, TrainBufs& T, const uint8_t* xbits, const int* lbl, int S, cudaStream_t s,
                      int* err) {
   const int B = T.B, C = L->C, Hd = L->Hd;
-  k_bits_pm1_bf16<<<grid1((long long)B * 32, 256), 256, 0, s>>>(xbits, B, nullptr, B, T.X);
+  k_bits_pm1_bf16<<<grid1((long long)B * 32, 256), 256, 0, s>>>(xbits, B, nullptr, B, T.X, SearchReset{});
   k_bits_pm1_bf16_t<<<B / 64, 256, 0, s>>>(xbits, B, B, T.XT);
   LCHK(gemm(s, err, T.X, L->w1b, B, Hd, 256, L->b1, kBiasReluBF16, 1, nullptr, T.H, nullptr, nullptr));
   LCHK(gemm(s, err, T.H, L->w2b, B, C, Hd, L->b2, kStoreF32, 1, T.logits, nullptr, nullptr, nullptr));
@@ -339,11 +339,11 @@ int spill_lists_gemm(orbx_learned* L, int* counts, int* cursor, cudaStream_t s, 
   LCHK(t.alloc(&x, (size_t)chunk * 256));
   LCHK(t.alloc(&keys, (size_t)chunk * (C / 128) * kTopK));
   LCHK(t.alloc(&sel, (size_t)n * S));
-  k_bits_pm1_bf16<<<grid1((long long)C * 32, 256), 256, 0, s>>>(L->centroids, C, nullptr, C, cent);
+  k_bits_pm1_bf16<<<grid1((long long)C * 32, 256), 256, 0, s>>>(L->centroids, C, nullptr, C, cent, SearchReset{});
   for (int off = 0; off < n; off += chunk) {
     const int m = std::min(chunk, n - off);
     const int rows = round_up(m, 128);
-    k_bits_pm1_bf16<<<grid1((long long)rows * 32, 256), 256, 0, s>>>(L->db + (size_t)off * 32, m, nullptr, rows, x);
+    k_bits_pm1_bf16<<<grid1((long long)rows * 32, 256), 256, 0, s>>>(L->db + (size_t)off * 32, m, nullptr, rows, x, SearchReset{});
     LCHK(gemm(s, err, x, cent, rows, C, 256, nullptr, kTop8, 1, nullptr, nullptr, nullptr, keys));
     k_select_topk<<<grid1((long long)m * 32, 256), 256, 0, s>>>(keys, m, C / 128, S, sel + (size_t)off * S);
   }
@@ -496,7 +496,7 @@ int cluster_lsh(orbx_learned* L, cudaStream_t s, int* err, bool make_proj) {
   for (int off = 0; off < n; off += chunk) {
     const int m = std::min(chunk, n - off);
     const int rows = round_up(m, 128);
-    k_bits_pm1_bf16<<<grid1((long long)rows * 32, 256), 256, 0, s>>>(L->db + (size_t)off * 32, m, nullptr, rows, x);
+    k_bits_pm1_bf16<<<grid1((long long)rows * 32, 256), 256, 0, s>>>(L->db + (size_t)off * 32, m, nullptr, rows, x, SearchReset{});
     LCHK(gemm(s, err, x, L->lsh, rows, 256, 256, nullptr, kStoreF32, 1, proj, nullptr, nullptr, nullptr));
     k_lsh_probes<<<grid1(m, 128), 128, 0, s>>>(proj, 256, m, L->p.lsh_bits, 0, nullptr, nullptr, nullptr,
                                                L->assign + off, nullptr, nullptr, 1);
@@ -798,23 +798,29 @@ static int search_impl(orbx_ctx* ctx, orbx_learned* L, const uint8_t* d_q, int n
     if (ev) cudaEventRecord(ev[i], s);
   };
   mark(0);
-  LCHK(cudaMemsetAsync(L->counts, 0, sizeof(int) * C, s));
-  LCHK(cudaMemsetAsync(L->fb_count, 0, sizeof(int), s));
-  k_bits_pm1_bf16<<<grid1((long long)rows * 32, 256), 256, 0, s>>>(d_q, nq, nullptr, rows, L->xq);
+  const int n_slots = nq * kTopK;
+  const unsigned slot_blocks = grid1(n_slots, kProbesPerBlock);
+  const size_t count_smem = sizeof(int) * (size_t)C;
+  // the first kernel also clears the counters; rows * 32 threads cover them all
+  // but the clusters of a very small search
+  SearchReset reset{C, nq, L->counts, L->rr_bound, L->fb_count, L->rr_counter};
+  LCHK(launch_chained(k_bits_pm1_bf16, grid1(std::max((long long)rows * 32, (long long)C), 256), 256, s, d_q, nq,
+                      (const int*)nullptr, rows, L->xq, reset));
   if (mlp) {
     LCHK(gemm(s, err, L->xq, L->w1b, rows, L->Hd, 256, L->b1, kBiasReluBF16, 1, nullptr, L->hq, nullptr, nullptr));
     LCHK(gemm(s, err, L->hq, L->w2b, rows, C, L->Hd, L->b2, kTop8Row, 1, nullptr, nullptr, nullptr, L->keys));
-    k_select_probes<<<grid1((long long)nq * 32, 256), 256, 0, s>>>(L->keys, nq, gemm_top_lists(C), L->p.n_probe, thr,
-                                                                    L->ivf_offsets, L->probes, L->margin, L->counts,
-                                                                    L->partial, per_slot);
+    LCHK(launch_chained(k_select_probes, grid1((long long)nq * 32, 256), 256, s, L->keys, nq, gemm_top_lists(C),
+                        L->p.n_probe, thr, L->ivf_offsets, L->probes, L->margin, d_margin, L->partial, per_slot));
+    LCHK(launch_chained_smem(k_count_probes, slot_blocks, 1024, count_smem, s, L->probes, n_slots, C, L->counts));
   } else {
     LCHK(gemm(s, err, L->xq, L->lsh, rows, 256, 256, nullptr, kStoreF32, 1, L->proj, nullptr, nullptr, nullptr));
     k_lsh_probes<<<grid1(nq, 128), 128, 0, s>>>(L->proj, 256, nq, L->p.lsh_bits, L->p.n_probe, L->ivf_offsets,
                                                 L->probes, L->counts, nullptr, L->margin, L->partial, per_slot);
   }
   mark(1);
-  k_scan_counts<<<1, 1024, 0, s>>>(L->counts, C, L->offsets, L->cursor, kRerankQ, L->items);
-  k_fill_probe_lists<<<grid1((long long)nq * kTopK, 256), 256, 0, s>>>(L->probes, nq, L->cursor, L->list);
+  LCHK(launch_chained(k_scan_counts, 1, 1024, s, L->counts, C, L->offsets, L->cursor, kRerankQ, L->items));
+  LCHK(launch_chained_smem(k_fill_probe_lists, slot_blocks, 1024, count_smem, s, L->probes, n_slots, C, L->cursor,
+                           L->list));
   mark(2);
   const unsigned items_max = grid1((long long)nq * kTopK, kRerankQ) + (unsigned)C;
   if (tensor) {
@@ -832,27 +838,28 @@ static int search_impl(orbx_ctx* ctx, orbx_learned* L, const uint8_t* d_q, int n
     ra.item_counter = L->rr_counter;
     ra.q_bound = L->rr_bound;
     ra.err = err;
-    LCHK(cudaMemsetAsync(L->rr_counter, 0, sizeof(int), s));
-    LCHK(cudaMemsetAsync(L->rr_bound, 0xFF, sizeof(uint32_t) * (size_t)nq, s));
     LCHK(launch_rerank_imma(ra, (int)items_max, s));
   } else {
     k_rerank<<<items_max, kRerankQ, 0, s>>>(d_q, L->list, L->offsets, L->items, C, L->ivf_desc, L->ivf_members,
                                             L->ivf_offsets, L->partial);
   }
   mark(3);
-  k_merge_probes<<<grid1(nq, 256), 256, 0, s>>>(L->partial, per_slot, nq, L->margin, thr, mlp ? L->p.max_distance : 1 << 20,
-                                                 d_dist2, d_idx2, mlp ? L->fb_list : nullptr, L->fb_count);
+  LCHK(launch_chained(k_merge_probes, grid1(nq, 256), 256, s, L->partial, per_slot, nq, L->margin, thr,
+                      mlp ? L->p.max_distance : 1 << 20, d_dist2, d_idx2, mlp ? L->fb_list : nullptr, L->fb_count));
   mark(4);
   LCHK(cudaGetLastError());
   if (mlp) {
-    k_gather_fallback<<<grid1(2ll * nq, 256), 256, 0, s>>>(d_q, L->fb_list, L->fb_count, L->fb_q);
+    LCHK(launch_chained(k_gather_fallback, grid1(2ll * nq, 256), 256, s, d_q, L->fb_list, L->fb_count, L->fb_q));
     LRC(imma_knn(s, err, L->fb_work, L->fb_q, nq, L->fb_count, L->fb_pm1, false, L->db, L->ndb, L->db_pm1, true,
                  L->fb_d, L->fb_i));
-    k_scatter_fallback<<<grid1(nq, 256), 256, 0, s>>>(L->fb_list, L->fb_count, L->fb_d, L->fb_i, d_dist2, d_idx2);
+    LCHK(launch_chained(k_scatter_fallback, grid1(nq, 256), 256, s, L->fb_list, L->fb_count, L->fb_d, L->fb_i, d_dist2,
+                        d_idx2, d_fallback_count));
+  } else {
+    if (d_margin) LCHK(cudaMemcpyAsync(d_margin, L->margin, sizeof(float) * nq, cudaMemcpyDeviceToDevice, s));
+    if (d_fallback_count)
+      LCHK(cudaMemcpyAsync(d_fallback_count, L->fb_count, sizeof(int), cudaMemcpyDeviceToDevice, s));
   }
   mark(5);
-  if (d_margin) LCHK(cudaMemcpyAsync(d_margin, L->margin, sizeof(float) * nq, cudaMemcpyDeviceToDevice, s));
-  if (d_fallback_count) LCHK(cudaMemcpyAsync(d_fallback_count, L->fb_count, sizeof(int), cudaMemcpyDeviceToDevice, s));
   LCHK(cudaGetLastError());
   return ORBX_OK;
 }

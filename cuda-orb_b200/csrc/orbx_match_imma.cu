@@ -763,6 +763,7 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(const_cast<int*>(s_queue) + kRrQueue);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
 
+  chain_wait();
   const int n_items = __ldg(a.item_offsets + a.n_clusters);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -1198,8 +1199,7 @@ cudaError_t launch_rerank_imma(const RerankImmaArgs& a, int max_items, cudaStrea
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return cudaErrorInvalidValue;
   const int blocks = max_items < sms ? max_items : sms;  // persistent: one block per SM
-  k_rerank_imma<<<blocks, kRrThreads, kRrSmemBytes, s>>>(a);
-  return cudaGetLastError();
+  return launch_chained_smem(k_rerank_imma, blocks, kRrThreads, kRrSmemBytes, s, a);
 }
 
 }  // namespace orbx
