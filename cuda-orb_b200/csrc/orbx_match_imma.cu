@@ -228,12 +228,13 @@ __device__ __forceinline__ void chunk_best2(const int* vc, int& u1, int& u2) {
   }
 }
 // Those two merged into the running best two keys (distance << 22 | index): base
-// is the key of a zero dot product at the chunk's column 0, and a dot product of
-// one takes 1 << SH off.  Masked columns carry no key.
-template <int B, int E, int SH>
+// is the key of a zero dot product at the chunk's column 0, and a value of one
+// takes 1 << SH off; the values are dot products times 1 << SCALE.  Masked columns
+// carry no key.
+template <int B, int E, int SH, int SCALE = 0>
 __device__ __forceinline__ void chunk_top2_push(const int* vc, uint32_t base, uint32_t& k1, uint32_t& k2) {
-  static_assert(kMaskedDot == -400 && SH <= 22, "400 << SH is an int above every other local key (256 << SH)");
-  constexpr int kMaskedU = (int)((uint32_t)(-kMaskedDot - 1) << SH);
+  static_assert(kMaskedDot == -400 && SH + SCALE <= 22, "the masked key is an int above every other (256 << 22)");
+  constexpr int kMaskedU = (int)((uint32_t)(-kMaskedDot - 1) << (SH + SCALE));
   int u1, u2;
   chunk_best2<B, E, SH>(vc, u1, u2);
   const uint32_t p1 = u1 >= kMaskedU ? kNoKeyShared : base + (uint32_t)u1;
@@ -641,10 +642,10 @@ __global__ void __launch_bounds__(kIThreads, 1)
 //               accumulators; commits release the expanded stage, the
 //               accumulator and, after an item's last tile, its query tile;
 //   warps 2-9   expanders: at an item's start they gather its slots' queries
-//               as +-1 rows (two threads per row) into one of two query tiles,
-//               then expand each packed tile to 0 / 1 rows into one of two
+//               as signed rows (two threads per row) into one of two query tiles,
+//               then expand each packed tile to masked rows into one of two
 //               database tiles, one row per thread, in the 128-byte swizzled
-//               K-major layout the TMA writes;
+//               K-major layout the TMA writes (rr_db_word);
 //   warps 10-25 epilogue: warp w reads TMEM lanes 32 * (w % 4) and 64 columns,
 //               keeps the top-2 keys (distance << 22 | database index) of each
 //               slot over the item's tiles (distance = popcount(query) - dot')
@@ -653,6 +654,12 @@ __global__ void __launch_bounds__(kIThreads, 1)
 // index order and ties resolve as in the other matchers.  Every wait is bounded (kIDeadlineCycles per
 // wait); on expiry the block records kErrImmaTimeout, drains its copies and
 // exits.
+//
+// What bounds it: the ALU (expansion and the epilogue's tests; the tensor pipe is
+// active 30% of the time).  32768 queries, 8 probes in 512 lists of about 2048
+// rows: 372 us at 11400 warp instructions per 256-row tile, 306 us with the
+// tournament updates, 245 us with the masked expansion (rr_db_word) and the
+// query's shared bound read one tile ahead.
 // ---------------------------------------------------------------------------
 constexpr int kRrExpWarps = 8;
 constexpr int kRrThreads = (2 + kRrExpWarps + kIEpiWarps) * 32;
@@ -698,34 +705,36 @@ __device__ __forceinline__ bool rr_wait(uint32_t bar, uint32_t parity, volatile 
   return mbar_wait(bar, parity, clock64() + kIDeadlineCycles, abort_flag);
 }
 __device__ __forceinline__ bool rr_warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
   int ok = 0;
   if ((threadIdx.x & 31) == 0) ok = rr_wait(bar, parity, abort_flag) ? 1 : 0;
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
-// Four +-1 bytes from four bits: byte j is +1 where bit j of n is set, else -1
-// (the expansion k_expand_pm1 makes).  The multiply spreads bit j to bit 8j
-// without carries (bit positions j + 7i are distinct for j, i < 4).
-__device__ __forceinline__ uint32_t pm1_nibble(uint32_t n) {
-  return 0xFFFFFFFFu ^ (((n * 0x00204081u) & 0x01010101u) * 0xFEu);
+// The order of the 256 products of a dot product is free, and so is how a weight
+// is shared between its factors; both are chosen so that a database row's packed
+// words expand by masking alone.  Output word k (k = 0 .. 7) of a packed word
+// holds its bits k, 8 + k, 16 + k, 24 + k in place, i.e. bytes of 0 or 2^k (bit 7
+// shifted down once: 0 or 64), and the query's bytes are +-2^(6 - k) (+-1 for bit
+// 7): every product is 64 times the query's sign where the row has a one, the
+// accumulator is 64 dot' exactly, and Hamming(q, row) = popcount(q) - dot'.
+// 72 operations per row, against 192 for bytes of 0 and 1 in bit order.
+constexpr int kRrScaleLog = 6;
+__device__ __forceinline__ uint32_t rr_db_word(uint32_t w, int k) {
+  return k < 7 ? w & (0x01010101u << k) : (w >> 1) & 0x40404040u;
 }
-
-// 16-byte chunk cc (K bytes 16 cc .. 16 cc + 15) of a +-1 row from its packed
-// 32-bit word w = words[cc >> 1]: bits 16 (cc & 1) .. + 15.
-__device__ __forceinline__ uint4 pm1_chunk(uint32_t w, int cc) {
-  const uint32_t h = w >> ((cc & 1) * 16);
-  return make_uint4(pm1_nibble(h & 0xFu), pm1_nibble((h >> 4) & 0xFu), pm1_nibble((h >> 8) & 0xFu),
-                    pm1_nibble((h >> 12) & 0xFu));
+__device__ __forceinline__ uint32_t rr_query_word(uint32_t w, int k) {
+  const uint32_t m = k < 7 ? 1u << (6 - k) : 1u, neg = 256u - m;
+  return (neg * 0x01010101u) ^ (((w >> k) & 0x01010101u) * (m ^ neg));
 }
-
-// The same chunk as 0 / 1 bytes (byte j = bit j): a database row in this form
-// gives dot' = sum of the query's +-1 values where the row has a one, and
-// Hamming(q, row) = popcount(q) - dot'.
-__device__ __forceinline__ uint32_t b01_nibble(uint32_t n) { return (n * 0x00204081u) & 0x01010101u; }
-__device__ __forceinline__ uint4 b01_chunk(uint32_t w, int cc) {
-  const uint32_t h = w >> ((cc & 1) * 16);
-  return make_uint4(b01_nibble(h & 0xFu), b01_nibble((h >> 4) & 0xFu), b01_nibble((h >> 8) & 0xFu),
-                    b01_nibble((h >> 12) & 0xFu));
+// 16-byte chunk cc of a row: output words 4 (cc & 1) .. + 3 of packed word w = words[cc >> 1].
+__device__ __forceinline__ uint4 rr_db_chunk(uint32_t w, int cc) {
+  const int k = 4 * (cc & 1);
+  return make_uint4(rr_db_word(w, k), rr_db_word(w, k + 1), rr_db_word(w, k + 2), rr_db_word(w, k + 3));
+}
+__device__ __forceinline__ uint4 rr_query_chunk(uint32_t w, int cc) {
+  const int k = 4 * (cc & 1);
+  return make_uint4(rr_query_word(w, k), rr_query_word(w, k + 1), rr_query_word(w, k + 2), rr_query_word(w, k + 3));
 }
 
 // Swizzled address of chunk cc of row r in a K-major tile of `rows` rows
@@ -946,7 +955,7 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
 #pragma unroll
         for (int j = 0; j < 8; j++) {
           const int cc = 8 * half + j;
-          const uint4 v = (r < ri.rows) ? pm1_chunk(wd[j >> 1], cc) : make_uint4(0u, 0u, 0u, 0u);
+          const uint4 v = (r < ri.rows) ? rr_query_chunk(wd[j >> 1], cc) : make_uint4(0u, 0u, 0u, 0u);
           *reinterpret_cast<uint4*>(sw128_chunk(tile, kIHalfA, r, cc)) = v;
         }
       }
@@ -970,7 +979,7 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
         uint8_t* tile = sX + x * kIBTile;
 #pragma unroll
         for (int cc = 0; cc < 16; cc++)
-          *reinterpret_cast<uint4*>(sw128_chunk(tile, kIHalfB, e, cc)) = b01_chunk(wd[cc >> 1], cc);
+          *reinterpret_cast<uint4*>(sw128_chunk(tile, kIHalfB, e, cc)) = rr_db_chunk(wd[cc >> 1], cc);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(RR_XFULL(x));
@@ -1012,6 +1021,8 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
       // like keys of database indices, into which they are turned at the end
       uint32_t k1 = kNoKeyShared, k2 = kNoKeyShared;
       const uint32_t bias = (uint32_t)pc << kIdxBitsShared;
+      uint32_t asked = slot >= 0 ? __ldcg(a.q_bound + (slot >> 3)) : kNoKeyShared;
+      int thr_gb = kMaskedDot;
       for (int t = 0; t < ri.tiles; t++, g++) {
         const uint32_t acc = g & 1u;
         if (!rr_warp_wait(RR_ACCFULL(acc), (g >> 1) & 1u, s_abort)) {
@@ -1019,8 +1030,10 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
           break;
         }
         tc_fence_after();
-        // the query's bound from its other items so far (any stale value is a valid, looser bound)
-        const uint32_t gb = slot >= 0 ? __ldcg(a.q_bound + (slot >> 3)) : kNoKeyShared;
+        // the query's bound from its other items so far (any stale value is a valid,
+        // looser bound): read while the tile before was examined
+        if (asked != kNoKeyShared) thr_gb = max(thr_gb, pc - (int)(asked >> kIdxBitsShared) - 1);
+        if (slot >= 0) asked = __ldcg(a.q_bound + (slot >> 3));
         const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * (uint32_t)kIBN + colgrp * 64;
 #pragma unroll 1
         for (int c = 0; c < 2; c++) {
@@ -1038,14 +1051,14 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
           if (valid < 32) {
 #pragma unroll
             for (int j = 0; j < 32; j++)
-              if (j >= valid) v[j] = kMaskedDot;
+              if (j >= valid) v[j] = kMaskedDot * (1 << kRrScaleLog);
           }
           // The columns arrive in list order, so only a strictly larger dot' (a
           // strictly smaller distance) than the current second best's can enter,
           // and no column farther than the second best that another item of the
           // same query holds (equal distances stay, their index decides)
-          int thr = pc - (int)(k2 >> kIdxBitsShared);  // no key yet: below every dot'
-          if (gb != kNoKeyShared) thr = max(thr, pc - (int)(gb >> kIdxBitsShared) - 1);
+          // (no key yet: below every dot')
+          const int thr = (1 << kRrScaleLog) * max(pc - (int)(k2 >> kIdxBitsShared), thr_gb);
           bool h0 = true, h1 = true, h2 = true, h3 = true;
           if (__all_sync(0xffffffffu, thr >= 0)) {
             float gm[4];
@@ -1058,10 +1071,10 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
             h3 = __any_sync(0xffffffffu, bits_exceed(gm[3], thr));
           }
           const uint32_t base = bias + (uint32_t)col0;
-          if (h0) chunk_top2_push<0, 9, kIdxBitsShared>(v, base, k1, k2);
-          if (h1) chunk_top2_push<9, 18, kIdxBitsShared>(v, base, k1, k2);
-          if (h2) chunk_top2_push<18, 27, kIdxBitsShared>(v, base, k1, k2);
-          if (h3) chunk_top2_push<27, 32, kIdxBitsShared>(v, base, k1, k2);
+          if (h0) chunk_top2_push<0, 9, kIdxBitsShared - kRrScaleLog, kRrScaleLog>(v, base, k1, k2);
+          if (h1) chunk_top2_push<9, 18, kIdxBitsShared - kRrScaleLog, kRrScaleLog>(v, base, k1, k2);
+          if (h2) chunk_top2_push<18, 27, kIdxBitsShared - kRrScaleLog, kRrScaleLog>(v, base, k1, k2);
+          if (h3) chunk_top2_push<27, 32, kIdxBitsShared - kRrScaleLog, kRrScaleLog>(v, base, k1, k2);
         }
       }
       if (!ok) break;
