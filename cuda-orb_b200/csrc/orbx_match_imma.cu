@@ -974,15 +974,20 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
         const uint4* src = reinterpret_cast<const uint4*>(sP + st * kRrPTile) + 2 * e;
         const uint4 w0 = src[0], w1 = src[1];
         const uint32_t wd[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-        __syncwarp();
-        if (lane == 0) mbar_arrive(RR_PEMPTY(st));
         uint8_t* tile = sX + x * kIBTile;
 #pragma unroll
         for (int cc = 0; cc < 16; cc++)
           *reinterpret_cast<uint4*>(sw128_chunk(tile, kIHalfB, e, cc)) = rr_db_chunk(wd[cc >> 1], cc);
+        // The packed stage is released here, not right after its loads: the stores
+        // and the fence have waited for them, and a copy (async proxy) issued before
+        // they were complete replaced words still to be read (one tile in about
+        // 50000, in one of 25 searches of 32768 queries).
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0) mbar_arrive(RR_XFULL(x));
+        if (lane == 0) {
+          mbar_arrive(RR_XFULL(x));
+          mbar_arrive(RR_PEMPTY(st));
+        }
       }
     }
     if (!ok) {
