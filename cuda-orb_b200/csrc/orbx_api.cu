@@ -131,8 +131,8 @@ struct orbx_ctx {
   BatchSlot single, pair;
   MatchWork mw{};  // matcher scratch of orbx_match, orbx_match_knn2 and orbx_pair
   // int8 tensor-core matcher scratch: +-1 expanded queries / database
-  int8_t* imma_q = nullptr;
-  int8_t* imma_db = nullptr;
+  uint8_t* imma_q = nullptr;
+  uint8_t* imma_db = nullptr;
   size_t imma_q_bytes = 0, imma_db_bytes = 0;
   // orbx_pair_host device buffers
   uint8_t* io_img[2] = {nullptr, nullptr};
@@ -966,8 +966,8 @@ ORBX_API int orbx_detect_and_compute(orbx_ctx* c, const uint8_t* d_image, int w,
 }
 
 static int imma_ensure(orbx_ctx* c, int nq_cap, int ndb_cap) {
-  const size_t qb = (size_t)imma_rows_q(nq_cap < 1 ? 1 : nq_cap) * 256;
-  const size_t db = (size_t)imma_rows_db(ndb_cap < 1 ? 1 : ndb_cap) * 256;
+  const size_t qb = (size_t)imma_rows_q(nq_cap < 1 ? 1 : nq_cap) * kPm1RowBytes;
+  const size_t db = (size_t)imma_rows_db(ndb_cap < 1 ? 1 : ndb_cap) * kPm1RowBytes;
   if (c->imma_q_bytes < qb) {
     cudaFree(c->imma_q);
     c->imma_q = nullptr;

@@ -192,20 +192,21 @@ struct MatchWork {          // scratch for split-train merging
   int splits_cap;           // most train splits per query tile
 };
 
-// int8 tensor-core form (orbx_match_imma.cu)
+// tensor-core form (orbx_match_imma.cu)
+constexpr int kPm1RowBytes = 128;  // an expanded descriptor: 256 4-bit floats, +-1
 struct ImmaLaunch {
   MatchArgs args;     // queries, database, counts, outputs
   MatchWork work;     // split merging (splits_cap >= splits)
-  int8_t* q_pm1;      // [imma_rows_q(nq_cap)][256] scratch
-  int8_t* db_pm1;     // [imma_rows_db(ndb_cap)][256] scratch
+  uint8_t* q_pm1;     // [imma_rows_q(nq_cap)][kPm1RowBytes] scratch
+  uint8_t* db_pm1;    // [imma_rows_db(ndb_cap)][kPm1RowBytes] scratch
   int nq_cap, ndb_cap;
   int splits;         // database splits per query tile
   int* err;
   bool q_ready;       // q_pm1 already holds the expanded queries (rows >= nq zero)
   bool db_ready;      // db_pm1 already holds the expanded database (rows >= ndb zero)
 };
-// bits -> +-1 int8 rows (rows beyond the count are zero); 4 * 148 blocks of 256
-cudaError_t launch_expand_pm1(const uint8_t* bits, int n, const int* d_n, int rows, int8_t* out, cudaStream_t s);
+// bits -> +-1 e2m1 rows (rows beyond the count are zero); 4 * 148 blocks of 256
+cudaError_t launch_expand_pm1(const uint8_t* bits, int n, const int* d_n, int rows, uint8_t* out, cudaStream_t s);
 int imma_rows_q(int n);
 int imma_rows_db(int n);
 constexpr int kImmaMaxSplits = 64;

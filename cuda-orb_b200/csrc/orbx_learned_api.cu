@@ -127,7 +127,7 @@ int imma_work_alloc(Arena& a, ImmaWork& iw, int nq_cap, int splits_for, int ndb,
 
 // Exact k = 2 search with the int8 tensor-core matcher.
 int imma_knn(cudaStream_t s, int* err, const ImmaWork& iw, const uint8_t* q, int nq_cap, const int* d_nq,
-             int8_t* q_pm1, bool q_ready, const uint8_t* db, int ndb, int8_t* db_pm1, bool db_ready, uint32_t* dist2,
+             uint8_t* q_pm1, bool q_ready, const uint8_t* db, int ndb, uint8_t* db_pm1, bool db_ready, uint32_t* dist2,
              int32_t* idx2) {
   ImmaLaunch L{};
   L.args.q = q;
@@ -174,7 +174,7 @@ struct orbx_learned {
   int set_width = 1;
   Arena keep;
   uint8_t* db = nullptr;
-  int8_t* db_pm1 = nullptr;
+  uint8_t* db_pm1 = nullptr;
   uint8_t* centroids = nullptr;
   int* assign = nullptr;
   int* ivf_offsets = nullptr;
@@ -203,7 +203,7 @@ struct orbx_learned {
   uint8_t* fb_q = nullptr;
   uint32_t* fb_d = nullptr;
   int32_t* fb_i = nullptr;
-  int8_t* fb_pm1 = nullptr;
+  uint8_t* fb_pm1 = nullptr;
   ImmaWork fb_work;
   orbx_learned_stats stats{};
 };
@@ -356,7 +356,7 @@ int spill_lists_gemm(orbx_learned* L, int* counts, int* cursor, cudaStream_t s, 
 int alloc_core(orbx_learned* L) {
   const int ndb = L->ndb;
   const size_t per = L->p.proposal == ORBX_PROPOSAL_MLP ? (size_t)std::max(1, L->p.spill) : 1;  // list entries per row
-  if (L->keep.alloc(&L->db, (size_t)ndb * 32) || L->keep.alloc(&L->db_pm1, (size_t)imma_rows_db(ndb) * 256) ||
+  if (L->keep.alloc(&L->db, (size_t)ndb * 32) || L->keep.alloc(&L->db_pm1, (size_t)imma_rows_db(ndb) * kPm1RowBytes) ||
       L->keep.alloc(&L->centroids, (size_t)L->C * 32) || L->keep.alloc(&L->assign, (size_t)ndb) ||
       L->keep.alloc(&L->ivf_offsets, (size_t)L->C + 1) || L->keep.alloc(&L->ivf_members, (size_t)ndb * per) ||
       L->keep.alloc(&L->ivf_desc, (size_t)ndb * per * 32) ||
@@ -409,14 +409,14 @@ int cluster_kmeans(orbx_learned* L, cudaStream_t s, int* err) {
   for (int c = 0; c < C; c++) init[c] = perm[c % n];
   int *d_init, *idx2, *counts, *changed, *cursor;
   uint32_t* dist2;
-  int8_t* cent_pm1;
+  uint8_t* cent_pm1;
   LCHK(t.alloc(&d_init, C));
   LCHK(t.alloc(&idx2, (size_t)2 * n));
   LCHK(t.alloc(&dist2, (size_t)2 * n));
   LCHK(t.alloc(&counts, C));
   LCHK(t.alloc(&cursor, C));
   LCHK(t.alloc(&changed, 1));
-  LCHK(t.alloc(&cent_pm1, (size_t)imma_rows_db(C) * 256));
+  LCHK(t.alloc(&cent_pm1, (size_t)imma_rows_db(C) * kPm1RowBytes));
   LCHK(cudaMemcpyAsync(d_init, init.data(), sizeof(int) * C, cudaMemcpyHostToDevice, s));
   k_gather_rows<<<grid1(2ll * C, 256), 256, 0, s>>>(L->db, d_init, C, L->centroids);
   LCHK(cudaMemsetAsync(L->assign, 0xFF, sizeof(int) * (size_t)n, s));
@@ -455,13 +455,13 @@ int lists_from_centroids(orbx_learned* L, cudaStream_t s, int* err) {
   Arena t;
   int *idx2, *counts, *cursor, *changed;
   uint32_t* dist2;
-  int8_t* cent_pm1;
+  uint8_t* cent_pm1;
   LCHK(t.alloc(&idx2, (size_t)2 * n));
   LCHK(t.alloc(&dist2, (size_t)2 * n));
   LCHK(t.alloc(&counts, C));
   LCHK(t.alloc(&cursor, C));
   LCHK(t.alloc(&changed, 1));
-  LCHK(t.alloc(&cent_pm1, (size_t)imma_rows_db(C) * 256));
+  LCHK(t.alloc(&cent_pm1, (size_t)imma_rows_db(C) * kPm1RowBytes));
   ImmaWork iw;
   LRC(imma_work_alloc(t, iw, n, n, C, s));
   LRC(imma_knn(s, err, iw, L->db, n, nullptr, L->db_pm1, true, L->centroids, C, cent_pm1, false, dist2, idx2));
@@ -633,7 +633,7 @@ int ensure_search(orbx_learned* L, int nq) {
   LCHK(a.alloc(&L->fb_q, (size_t)nq * 32));
   LCHK(a.alloc(&L->fb_d, (size_t)nq * 2));
   LCHK(a.alloc(&L->fb_i, (size_t)nq * 2));
-  LCHK(a.alloc(&L->fb_pm1, (size_t)imma_rows_q(nq) * 256));
+  LCHK(a.alloc(&L->fb_pm1, (size_t)imma_rows_q(nq) * kPm1RowBytes));
   // fallback splits sized for about one query in eight; fewer fallback queries
   // split the database scan further, up to 32 ways
   L->fb_work = ImmaWork();
@@ -719,12 +719,12 @@ ORBX_API int orbx_learned_build(orbx_ctx* ctx, const orbx_learned_params* p, con
       int* labels;
       int32_t* idx2;
       uint32_t* dist2;
-      int8_t* tq;
+      uint8_t* tq;
       uint8_t* rows;
       const int nt = ntrain + p->synth_train;
       const int S = p->label_mode == ORBX_LABEL_LISTED ? L->set_width : 1;
       if (t.alloc(&labels, (size_t)nt * S) || t.alloc(&idx2, 2 * (size_t)nt) || t.alloc(&dist2, 2 * (size_t)nt) ||
-          t.alloc(&tq, (size_t)imma_rows_q(nt) * 256) || t.alloc(&rows, (size_t)nt * 32)) {
+          t.alloc(&tq, (size_t)imma_rows_q(nt) * kPm1RowBytes) || t.alloc(&rows, (size_t)nt * 32)) {
         rc = ORBX_ERR_NOMEM;
         break;
       }

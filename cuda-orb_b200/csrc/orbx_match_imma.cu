@@ -1,17 +1,18 @@
 // Brute-force k = 2 Hamming matching on the 5th-generation tensor cores.
 //
-// A 256-bit descriptor b is expanded to 256 int8 values s_k = 2*b_k - 1 (+-1),
-// so for two descriptors dot(s, t) = 256 - 2 * Hamming(s, t), computed exactly
-// by tcgen05.mma kind::i8 with int32 accumulation.  One block owns up to 256
-// queries, as two query tiles of 128 (the MMA's M) that stay in shared memory,
-// and walks 256-row database tiles (the MMA's N) with K = 256 = eight K=32 MMA
-// steps per database and query tile:
+// A 256-bit descriptor b is expanded to 256 values s_k = 2*b_k - 1 (+-1), so for
+// two descriptors dot(s, t) = 256 - 2 * Hamming(s, t).  The values are 4-bit floats
+// (e2m1, where +-1 is exact) with block scales of 1, multiplied by tcgen05.mma
+// kind::mxf4 into fp32: every partial sum is a whole number of at most 256, so the
+// dot product is exact.  One block owns up to 256 queries, as two query tiles of
+// 128 (the MMA's M) that stay in shared memory, and walks 240-row database tiles
+// (the MMA's N) with K = 256 = four K=64 MMA steps per database and query tile:
 //   warp 0     TMA producer: the query tiles once, database tiles through a
-//              2-stage shared-memory ring (128-byte swizzle, no multicast);
-//   warp 1     MMA issuer: one elected thread issues the eight MMAs of a step
-//              into one of two TMEM accumulators (2 x 256 columns) and commits
-//              them to the ring's "empty" (after a database tile's last step)
-//              and the accumulator's "full" barriers;
+//              4-stage shared-memory ring (128-byte swizzle, no multicast);
+//   warp 1     MMA issuer: one elected thread issues the four MMAs of a step
+//              into one of two TMEM accumulators (240 columns; the scales take
+//              16 of the others) and commits them to the ring's "empty" (after a
+//              database tile's last step) and the accumulator's "full" barriers;
 //   warps 2-17 epilogue, two sets of eight: set s takes every second step, i.e.
 //              accumulator s.  A warp reads its 32 TMEM lanes (queries) over half
 //              the columns, 64 at a time, and keeps a running best / second-best
@@ -24,14 +25,14 @@
 // Every barrier wait is bounded by a clock deadline; on expiry the block
 // records kErrImmaTimeout, drains its in-flight copies, frees TMEM and exits.
 //
-// What bounds it: the tensor pipe with its shared-memory reads (660 us for 65536 x
-// 65536 with the epilogue's examination of the values left out) and the epilogue
-// on the ALU.  The maximum test of every chunk adds 25 us; what remains on top, 110
-// us (190 before), are the chunks that pass it.  They are kept few by bounds
-// shared between column halves, sets and database splits, and cheap by looking at
-// their column groups with independent tests and tournaments.  Two query tiles
-// per block read each database tile once for 256 queries.  65536 x 65536: 909 ->
-// 795 us; 16384 x 32768: 211 -> 110 us; 1500 x 262144: 116 -> 96 us.
+// What bounds it: the epilogue.  With int8 values (kind::i8, half the rate and twice
+// the bytes) 65536 x 65536 took 785 us, of which the tensor pipe needed 660; now the
+// tensor pipe is active 48% of the time and the epilogue's ALU instructions 58%.
+// Most 32-column chunks end at their maximum test; those that pass it are kept few by
+// bounds shared between column halves, sets and database splits, and cheap by
+// looking at their column groups with independent tests and tournaments.  Two query
+// tiles per block read each database tile once for 256 queries.  65536 x 65536: 785
+// -> 666 us; 1500 x 262144: 95 -> 74.5 us.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -44,20 +45,27 @@ namespace orbx {
 
 constexpr int kIBM = 128;  // queries per query tile (MMA M)
 constexpr int kIBQ = 2 * kIBM;  // queries per block of k_match_imma
-constexpr int kIBN = 256;  // database rows per tile (MMA N)
-constexpr int kIK = 256;   // bytes per expanded descriptor (MMA K)
-constexpr int kIStages = 2;
+constexpr int kIBN = 256;  // database rows per tile of k_rerank_imma (MMA N)
+constexpr int kMBN = 240;  // database rows per tile of k_match_imma: two accumulators leave TMEM columns for the scales
+constexpr int kMHalf = kMBN / 2;  // columns of one epilogue warp
+constexpr int kMStages = 4;
 constexpr int kIEpiWarps = 16;  // two sets of two per TMEM lane quarter, 128 columns each
 constexpr int kIThreads = (2 + kIEpiWarps) * 32;
 constexpr uint32_t kIHalfA = kIBM * 128;  // one 128-byte-wide K half of the query tile
 constexpr uint32_t kIHalfB = kIBN * 128;
 constexpr uint32_t kIATile = 2 * kIHalfA;
 constexpr uint32_t kIBTile = 2 * kIHalfB;
-constexpr uint32_t kINumBars = 1 + 2 * kIStages + 4;
+constexpr uint32_t kMATile = kIBM * kPm1RowBytes;  // one 128-byte swizzle row per descriptor
+constexpr uint32_t kMBTile = kMBN * kPm1RowBytes;
+static_assert(kPm1RowBytes == 128 && kMBTile % 1024 == 0, "whole swizzle atoms");
+constexpr uint32_t kMNumBars = 1 + 2 * kMStages + 4;
+// accumulator a starts at TMEM column 256 * a; the scales (all 1) lie between them
+constexpr uint32_t kMAcc = 256;
+constexpr uint32_t kMScaleCol = kMBN, kMScaleCols = 16;
 // 1024 bytes of alignment slack, the query tiles, the ring, the merge scratch
 // (best two per set, column half and row), the barriers, TMEM base + abort flag
 constexpr uint32_t kIMergeBytes = 4 * kIBM * 8;
-constexpr uint32_t kISmemBytes = 1024 + 2 * kIATile + kIStages * kIBTile + kIMergeBytes + 8 * kINumBars + 16;
+constexpr uint32_t kISmemBytes = 1024 + 2 * kMATile + kMStages * kMBTile + kIMergeBytes + 8 * kMNumBars + 16;
 // dynamic tiles + the static s_last and per-row bounds (4 x kIBM 16-bit)
 static_assert(kISmemBytes + 16 + 4 * kIBM * 2 <= 232448, "exceeds the 227 KB shared-memory opt-in");
 constexpr uint32_t kITmemCols = 512;
@@ -66,6 +74,9 @@ constexpr long long kIDeadlineCycles = 4000000000ll;  // ~2 s at 2 GHz
 // instruction descriptor: S32 accumulate, S8 x S8, both K-major, N = 256, M = 128
 constexpr uint32_t kIDesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kIBN >> 3) << 17) |
                             ((uint32_t)(kIBM >> 4) << 24);
+// the same for kind::mxf4: E2M1 x E2M1, UE8M0 scales, both K-major, N = 240, M = 128, K = 64
+constexpr uint32_t kMDesc = (1u << 7) | (1u << 10) | ((uint32_t)(kMBN >> 3) << 17) | (1u << 23) |
+                            ((uint32_t)(kIBM >> 7) << 27);
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -131,6 +142,29 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t d
       "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(tmem_d),
       "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(mask0), "r"(mask1), "r"(mask2), "r"(mask3)
       : "memory");
+}
+
+// One K = 64 step on 4-bit floats with one scale per 32 values (all 1, at sfa and sfb).
+__device__ __forceinline__ void umma_f4(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t sfa,
+                                        uint32_t sfb, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%4], [%5], p;\n\t}" ::"r"(
+          tmem_d),
+      "l"(da), "l"(db), "r"(idesc), "r"(sfa), "r"(sfb), "r"(acc)
+      : "memory");
+}
+
+// Scales of 1 (UE8M0 127) in this warp's 32 lanes of 16 TMEM columns.
+__device__ __forceinline__ void tmem_store_unit_scales(uint32_t taddr) {
+  const uint32_t one = 0x7F7F7F7Fu;
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+      "%1};" ::"r"(taddr),
+      "r"(one)
+      : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
@@ -243,45 +277,126 @@ __device__ __forceinline__ void chunk_top2_push(const int* vc, uint32_t base, ui
   k1 = min(k1, p1);
 }
 
-// Sixteen +-1 bytes from 16 bits, through the 256-entry table of 8.
-__device__ __forceinline__ void expand_lut(unsigned long long* lut) {
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-    unsigned long long v = 0;
-    for (int j = 0; j < 8; j++) v |= (unsigned long long)(((i >> j) & 1) ? 0x01u : 0xFFu) << (8 * j);
-    lut[i] = v;
+// ---- the same on fp32 accumulators (k_match_imma) ----------------------------
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
+        "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]),
+        "=f"(v[16]), "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]),
+        "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_wait_ld32(float* v) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]),
+                 "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]),
+                 "+f"(v[15]), "+f"(v[16]), "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]),
+                 "+f"(v[22]), "+f"(v[23]), "+f"(v[24]), "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]),
+                 "+f"(v[29])
+               :
+               : "memory");
+  asm volatile("" : "+f"(v[30]), "+f"(v[31])::"memory");
+}
+// Value given to columns that hold no database row (below every dot product).
+constexpr float kMaskedDotF = -400.f;
+
+__device__ __forceinline__ float fmax3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float fmin3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+// Maxima of the column groups 0-8, 9-17, 18-26 and 27-31 of a 32-column chunk.
+__device__ __forceinline__ void group_max4(const float* v, float* r) {
+#pragma unroll
+  for (int g = 0; g < 3; g++)
+    r[g] = fmax3(fmax3(v[9 * g], v[9 * g + 1], v[9 * g + 2]), fmax3(v[9 * g + 3], v[9 * g + 4], v[9 * g + 5]),
+                 fmax3(v[9 * g + 6], v[9 * g + 7], v[9 * g + 8]));
+  r[3] = fmax3(fmax3(v[27], v[28], v[29]), v[30], v[31]);
+}
+// The best two of columns B .. E-1 of a chunk, merged into the running best two
+// keys (distance << 22 | index): local keys u = column - 32 * dot, whole numbers
+// below 2^14 and exact in fp32, go through a tournament of minima (its depth, not
+// its 20 operations for nine columns, is what a warp waits for), so ties keep the
+// lower column.  base is the key of a zero dot product at the chunk's column 0, and
+// a value of one takes 1 << SH off.  Masked columns carry no key.
+template <int B, int E, int SH>
+__device__ __forceinline__ void push_best2(const float* vc, uint32_t base, uint32_t& k1, uint32_t& k2) {
+  constexpr int n = E - B, h = n / 2;
+  float a1[h], a2[h];
+#pragma unroll
+  for (int i = 0; i < h; i++) {
+    const float x = fmaf(vc[B + 2 * i], -32.f, (float)(B + 2 * i)),
+                y = fmaf(vc[B + 2 * i + 1], -32.f, (float)(B + 2 * i + 1));
+    a1[i] = fminf(x, y);
+    a2[i] = fmaxf(x, y);
   }
+#pragma unroll
+  for (int d = 1; d < h; d *= 2)
+#pragma unroll
+    for (int i = 0; i + d < h; i += 2 * d) {
+      a2[i] = fmin3(fmaxf(a1[i], a1[i + d]), a2[i], a2[i + d]);
+      a1[i] = fminf(a1[i], a1[i + d]);
+    }
+  float u1 = a1[0], u2 = a2[0];
+  if constexpr (n & 1) {
+    const float x = fmaf(vc[E - 1], -32.f, (float)(E - 1));
+    u2 = fminf(u2, fmaxf(u1, x));
+    u1 = fminf(u1, x);
+  }
+  auto key = [&](float u) {
+    const int i = __float2int_rn(u);
+    return u >= -32.f * kMaskedDotF ? kNoKeyShared : base + ((uint32_t)(i >> 5) << SH) + (uint32_t)(i & 31);
+  };
+  const uint32_t p1 = key(u1), p2 = key(u2);
+  k2 = __vimin3_u32(max(k1, p1), k2, p2);
+  k1 = min(k1, p1);
 }
 
-// Expands 256-bit descriptors to +-1 int8 rows, rows at or past the count to
-// zeros: the query set, whose rows' shared bounds it also clears, and the
-// database set (either may have no rows) in one launch.  16 bytes per store.
+// Expands 256-bit descriptors to rows of 256 e2m1 values (+1: 2, -1: 10), rows at
+// or past the count to zeros: the query set, whose rows' shared bounds it also
+// clears, and the database set (either may have no rows) in one launch.  Four bytes
+// of bits to one 16-byte store; the values of a descriptor come in the order of its
+// bits, least first.
 struct ExpandSet {
   const uint8_t* bits;
   int n;
   const int* d_n;  // optional count on the device
   int rows;
-  int8_t* out;
+  uint8_t* out;
 };
 __global__ void __launch_bounds__(256) k_expand_pm1(ExpandSet q, ExpandSet db, uint32_t* bound, int bounds) {
-  __shared__ unsigned long long lut[256];
-  expand_lut(lut);
+  __shared__ uint32_t lut[256];
+  {
+    uint32_t v = 0;
+    for (int j = 0; j < 8; j++) v |= (((threadIdx.x >> j) & 1u) ? 0x2u : 0xAu) << (4 * j);
+    lut[threadIdx.x] = v;
+  }
   __syncthreads();
   chain_wait();
   const int nq = q.rows ? (q.d_n ? min(*q.d_n, q.rows) : min(q.n, q.rows)) : 0;
   const int nd = db.rows ? (db.d_n ? min(*db.d_n, db.rows) : min(db.n, db.rows)) : 0;
-  const long long tq = (long long)q.rows * 16, total = tq + (long long)db.rows * 16;
+  constexpr int kPer = kPm1RowBytes / 16;  // stores per row
+  const long long tq = (long long)q.rows * kPer, total = tq + (long long)db.rows * kPer;
   const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
   for (long long i = i0; i < bounds; i += step) bound[i] = kNoKeyShared;
   for (long long i = i0; i < total; i += step) {
     const bool is_q = i < tq;
     const ExpandSet& e = is_q ? q : db;
     const long long k = is_q ? i : i - tq;
-    ulonglong2 v{};
-    if ((k >> 4) < (is_q ? nq : nd)) {
-      const uint8_t* b = e.bits + 2 * k;  // descriptors may start on any byte
-      v = make_ulonglong2(lut[b[0]], lut[b[1]]);
+    uint4 v{};
+    if (k / kPer < (is_q ? nq : nd)) {
+      const uint8_t* b = e.bits + 4 * k;  // descriptors may start on any byte
+      v = make_uint4(lut[b[0]], lut[b[1]], lut[b[2]], lut[b[3]]);
     }
-    reinterpret_cast<ulonglong2*>(e.out)[k] = v;
+    reinterpret_cast<uint4*>(e.out)[k] = v;
   }
 }
 
@@ -302,10 +417,10 @@ __global__ void __launch_bounds__(kIThreads, 1)
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
   uint8_t* sA = smem;
-  uint8_t* sB = sA + 2 * kIATile;
-  uint2* s_merge = reinterpret_cast<uint2*>(sB + kIStages * kIBTile);
+  uint8_t* sB = sA + 2 * kMATile;
+  uint2* s_merge = reinterpret_cast<uint2*>(sB + kMStages * kMBTile);
   uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(s_merge) + kIMergeBytes);
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + kINumBars);
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + kMNumBars);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
   __shared__ unsigned int s_last;
   // current second-best distance per query row of each set and column half
@@ -326,7 +441,7 @@ __global__ void __launch_bounds__(kIThreads, 1)
   if (qb >= qtiles) return;  // uniform over the block: before any barrier or TMEM use
   const int nq_here = min(kIBQ, nq - qb * kIBQ);
   const bool two = nq_here > kIBM;  // two query tiles
-  const int dbtiles = (ndb + kIBN - 1) / kIBN;
+  const int dbtiles = (ndb + kMBN - 1) / kMBN;
   const int t_beg = (int)((long long)dbtiles * sp / splits);
   const int t_end = (int)((long long)dbtiles * (sp + 1) / splits);
   const int ntiles = t_end - t_beg;
@@ -337,14 +452,14 @@ __global__ void __launch_bounds__(kIThreads, 1)
   const uint32_t bar0 = smem_u32(bars);
   const uint32_t BAR_A = bar0;
 #define BAR_BFULL(s) (bar0 + 8u * (1 + (s)))
-#define BAR_BEMPTY(s) (bar0 + 8u * (1 + kIStages + (s)))
-#define BAR_ACCFULL(s) (bar0 + 8u * (1 + 2 * kIStages + (s)))
-#define BAR_ACCEMPTY(s) (bar0 + 8u * (3 + 2 * kIStages + (s)))
+#define BAR_BEMPTY(s) (bar0 + 8u * (1 + kMStages + (s)))
+#define BAR_ACCFULL(s) (bar0 + 8u * (1 + 2 * kMStages + (s)))
+#define BAR_ACCEMPTY(s) (bar0 + 8u * (3 + 2 * kMStages + (s)))
 
   for (int i = threadIdx.x; i < 4 * kIBM; i += blockDim.x) (&s_d2[0][0])[i] = 0xFFFFu;
   if (threadIdx.x == 0) {
     mbar_init(BAR_A, 1);
-    for (int s = 0; s < kIStages; s++) {
+    for (int s = 0; s < kMStages; s++) {
       mbar_init(BAR_BFULL(s), 1);
       mbar_init(BAR_BEMPTY(s), 1);
     }
@@ -366,30 +481,33 @@ __global__ void __launch_bounds__(kIThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *s_tmem;
+  // the scales of both operands, before the first MMA: four warps, one per 32 lanes
+  if (warp >= 2 && warp < 6)
+    tmem_store_unit_scales(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kMScaleCol);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
   const long long deadline = clock64() + kIDeadlineCycles;
 
   if (warp == 0) {
     if (lane == 0) {
       // TMA producer
-      int issued[kIStages];
-      for (int s = 0; s < kIStages; s++) issued[s] = 0;
+      int issued[kMStages];
+      for (int s = 0; s < kMStages; s++) issued[s] = 0;
       bool ok = true;
-      mbar_expect_tx(BAR_A, two ? 2 * kIATile : kIATile);
-      for (int m = 0; m < (two ? 2 : 1); m++) {
-        tma_load_2d(smem_u32(sA + m * kIATile), &tmQ, 0, qb * kIBQ + m * kIBM, BAR_A);
-        tma_load_2d(smem_u32(sA + m * kIATile + kIHalfA), &tmQ, 128, qb * kIBQ + m * kIBM, BAR_A);
-      }
+      mbar_expect_tx(BAR_A, two ? 2 * kMATile : kMATile);
+      for (int m = 0; m < (two ? 2 : 1); m++)
+        tma_load_2d(smem_u32(sA + m * kMATile), &tmQ, 0, qb * kIBQ + m * kIBM, BAR_A);
       for (int i = 0; i < ntiles; i++) {
-        const int s = i % kIStages;
-        const int use = i / kIStages;
+        const int s = i % kMStages;
+        const int use = i / kMStages;
         if (use > 0 && !mbar_wait(BAR_BEMPTY(s), (use - 1) & 1, deadline, s_abort)) {
           ok = false;
           break;
         }
-        const int row = (t_beg + i) * kIBN;
-        mbar_expect_tx(BAR_BFULL(s), kIBTile);
-        tma_load_2d(smem_u32(sB + s * kIBTile), &tmD, 0, row, BAR_BFULL(s));
-        tma_load_2d(smem_u32(sB + s * kIBTile + kIHalfB), &tmD, 128, row, BAR_BFULL(s));
+        const int row = (t_beg + i) * kMBN;
+        mbar_expect_tx(BAR_BFULL(s), kMBTile);
+        tma_load_2d(smem_u32(sB + s * kMBTile), &tmD, 0, row, BAR_BFULL(s));
         issued[s]++;
       }
       if (!ok) {
@@ -401,7 +519,7 @@ __global__ void __launch_bounds__(kIThreads, 1)
       long long dl = clock64() + kIDeadlineCycles;
       while (!mbar_try(BAR_A, 0) && clock64() < dl) {
       }
-      for (int s = 0; s < kIStages; s++) {
+      for (int s = 0; s < kMStages; s++) {
         if (issued[s] == 0) continue;
         const uint32_t par = (uint32_t)(issued[s] - 1) & 1u;
         dl = clock64() + kIDeadlineCycles;
@@ -414,15 +532,15 @@ __global__ void __launch_bounds__(kIThreads, 1)
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      // MMA issuer: eight K=32 MMAs per step into accumulator (step & 1)
+      // MMA issuer: four K=64 MMAs per step into accumulator (step & 1)
       bool ok = mbar_wait(BAR_A, 0, deadline, s_abort);
       const uint32_t a_base = smem_u32(sA);
       for (int i = 0; ok && i < nsteps; i++) {
         const int t = two ? i >> 1 : i;
         const int qt = two ? i & 1 : 0;
-        const int s = t % kIStages;
+        const int s = t % kMStages;
         const int acc = i & 1;
-        if (qt == 0 && !mbar_wait(BAR_BFULL(s), (uint32_t)(t / kIStages) & 1u, deadline, s_abort)) {
+        if (qt == 0 && !mbar_wait(BAR_BFULL(s), (uint32_t)(t / kMStages) & 1u, deadline, s_abort)) {
           ok = false;
           break;
         }
@@ -431,16 +549,12 @@ __global__ void __launch_bounds__(kIThreads, 1)
           break;
         }
         tc_fence_after();
-        const uint32_t d = tmem_base + (uint32_t)(acc * kIBN);
-        const uint32_t a_lo = a_base + (uint32_t)qt * kIATile;
-        const uint32_t b_lo = smem_u32(sB + s * kIBTile);
+        const uint32_t d = tmem_base + (uint32_t)acc * kMAcc;
+        const uint32_t sfa = tmem_base + kMScaleCol, sfb = sfa + kMScaleCols / 2;
+        const uint64_t da = sw128_desc(a_base + (uint32_t)qt * kMATile), db = sw128_desc(smem_u32(sB + s * kMBTile));
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-          const int h = k >> 2, kk = k & 3;
-          const uint64_t da = sw128_desc(a_lo + h * kIHalfA) + (uint64_t)(2 * kk);
-          const uint64_t db = sw128_desc(b_lo + h * kIHalfB) + (uint64_t)(2 * kk);
-          umma_i8(d, da, db, kIDesc, k > 0 ? 1u : 0u);
-        }
+        for (int k = 0; k < 4; k++)  // 64 values are 32 bytes of a row: two descriptor units
+          umma_f4(d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), kMDesc, sfa, sfb, k > 0 ? 1u : 0u);
         if (!two || qt == 1) umma_commit(BAR_BEMPTY(s));  // the database tile's last step
         umma_commit(BAR_ACCFULL(acc));
       }
@@ -451,7 +565,7 @@ __global__ void __launch_bounds__(kIThreads, 1)
     }
   } else {
     // epilogue: steps of this warp's set, TMEM lanes 32 * (warp & 3) .. (one
-    // query per lane), columns [128 * half, + 128)
+    // query per lane), columns [120 * half, + 120)
     const int set = (warp - 2) >> 3;
     const int half = ((warp - 2) >> 2) & 1;
     const int me = 2 * set + half;
@@ -462,50 +576,37 @@ __global__ void __launch_bounds__(kIThreads, 1)
     // second-best bound shared by the blocks that scan this query's other splits
     uint32_t* gq = (w.bound && splits > 1 && q < nq) ? w.bound + q : nullptr;
     uint32_t told = kNoKeyShared, asked = kNoKeyShared, heard = kNoKeyShared;  // published, being read, read
-    int thr_gb = kMaskedDot;  // a dot at or below this cannot reach the row's final top two
-    bool warm = false;        // every lane of the warp has a threshold >= 0
+    float thr_gb = kMaskedDotF;  // a dot at or below this cannot reach the row's final top two
     // (no key yet: far below every dot)
-    auto next_thr = [&]() { return max(thr_gb, 256 - 2 * (int)(k2 >> kIdxBitsShared)); };
-    int thr = kMaskedDot;
+    auto next_thr = [&]() { return fmaxf(thr_gb, (float)(256 - 2 * (int)(k2 >> kIdxBitsShared))); };
+    float thr = kMaskedDotF;
     // columns arrive in increasing index order, so only a strictly larger dot
     // than the own second best can enter the top two.  Most chunks end at the
     // maximum test; one that passes looks at the column groups with a value above
     // the threshold.  These are few (a lane's top two change a few times per scan)
     // but they were half of the kernel's time when each group was a serial chain
     // with its own test.
-    auto examine = [&](const int* vc, int gc) {
-      // distance << 22 = (256 - dot) << 21
-      const uint32_t base = (256u << (kIdxBitsShared - 1)) + (uint32_t)gc;
-      if (!warm) {
-        chunk_top2_push<0, 9, kIdxBitsShared - 1>(vc, base, k1, k2);
-        chunk_top2_push<9, 18, kIdxBitsShared - 1>(vc, base, k1, k2);
-        chunk_top2_push<18, 27, kIdxBitsShared - 1>(vc, base, k1, k2);
-        chunk_top2_push<27, 32, kIdxBitsShared - 1>(vc, base, k1, k2);
-        thr = next_thr();
-        warm = __all_sync(0xffffffffu, thr >= 0);
-        return;
-      }
+    auto examine = [&](const float* vc, int gc) {
       float gm[4];
       group_max4(vc, gm);
-      const float cm = fmax3_bits(gm[0], gm[1], fmax3_bits(gm[2], gm[3], gm[3]));
-      if (!__any_sync(0xffffffffu, bits_exceed(cm, thr))) return;
-      const bool h0 = __any_sync(0xffffffffu, bits_exceed(gm[0], thr)),
-                 h1 = __any_sync(0xffffffffu, bits_exceed(gm[1], thr)),
-                 h2 = __any_sync(0xffffffffu, bits_exceed(gm[2], thr)),
-                 h3 = __any_sync(0xffffffffu, bits_exceed(gm[3], thr));
-      if (h0) chunk_top2_push<0, 9, kIdxBitsShared - 1>(vc, base, k1, k2);
-      if (h1) chunk_top2_push<9, 18, kIdxBitsShared - 1>(vc, base, k1, k2);
-      if (h2) chunk_top2_push<18, 27, kIdxBitsShared - 1>(vc, base, k1, k2);
-      if (h3) chunk_top2_push<27, 32, kIdxBitsShared - 1>(vc, base, k1, k2);
+      if (!__any_sync(0xffffffffu, fmax3(gm[0], gm[1], fmaxf(gm[2], gm[3])) > thr)) return;
+      const bool h0 = __any_sync(0xffffffffu, gm[0] > thr), h1 = __any_sync(0xffffffffu, gm[1] > thr),
+                 h2 = __any_sync(0xffffffffu, gm[2] > thr), h3 = __any_sync(0xffffffffu, gm[3] > thr);
+      // distance << 22 = (256 - dot) << 21
+      const uint32_t base = (256u << (kIdxBitsShared - 1)) + (uint32_t)gc;
+      if (h0) push_best2<0, 9, kIdxBitsShared - 1>(vc, base, k1, k2);
+      if (h1) push_best2<9, 18, kIdxBitsShared - 1>(vc, base, k1, k2);
+      if (h2) push_best2<18, 27, kIdxBitsShared - 1>(vc, base, k1, k2);
+      if (h3) push_best2<27, 32, kIdxBitsShared - 1>(vc, base, k1, k2);
       thr = next_thr();
     };
-    const uint32_t tcol = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(set * kIBN + half * 128);
+    const uint32_t tcol = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)set * kMAcc + (uint32_t)(half * kMHalf);
     for (int i = set; i < nsteps; i += 2) {
       const int n = i >> 1;  // this set's step
       ok = warp_wait(BAR_ACCFULL(set), (uint32_t)n & 1u, deadline, s_abort);
       if (!ok) break;
       tc_fence_after();
-      const int g0 = (t_beg + (two ? n : i)) * kIBN + half * 128;
+      const int g0 = (t_beg + (two ? n : i)) * kMBN + half * kMHalf;
       // bounds from the others of this block that scan the row's query (every
       // step) and from its other splits (read in the first steps and then every
       // fourth, used one step later): a column can reach the row's final top two
@@ -520,12 +621,12 @@ __global__ void __launch_bounds__(kIThreads, 1)
           others(me ^ 2);
           others(me ^ 3);
         }
-        if (gbd <= 256u) thr_gb = max(thr_gb, 256 - 2 * (int)gbd - 1);
-        thr = max(thr, thr_gb);
+        if (gbd <= 256u) thr_gb = fmaxf(thr_gb, (float)(256 - 2 * (int)gbd - 1));
+        thr = fmaxf(thr, thr_gb);
       }
 #pragma unroll 1
       for (int c = 0; c < 2; c++) {
-        int v0[32], v1[32];
+        float v0[32], v1[32];
         tmem_ld32(tcol + 64u * c, v0);
         tmem_ld32(tcol + 64u * c + 32u, v1);
         tmem_wait_ld32(v0);
@@ -535,13 +636,16 @@ __global__ void __launch_bounds__(kIThreads, 1)
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(BAR_ACCEMPTY(set));
+          // the last 8 of 2 x 64 columns belong to the other half or to none
+#pragma unroll
+          for (int j = 24; j < 32; j++) v1[j] = kMaskedDotF;
         }
         const int gc = g0 + 64 * c;
         if (gc + 64 > ndb) {
 #pragma unroll
           for (int j = 0; j < 32; j++) {
-            if (gc + j >= ndb) v0[j] = kMaskedDot;
-            if (gc + 32 + j >= ndb) v1[j] = kMaskedDot;
+            if (gc + j >= ndb) v0[j] = kMaskedDotF;
+            if (gc + 32 + j >= ndb) v1[j] = kMaskedDotF;
           }
         }
         examine(v0, gc);
@@ -1135,11 +1239,12 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }
 
 static bool make_rows_map(CUtensorMap* m, const void* base, uint64_t rows, uint32_t box_rows) {
+  // one box is whole rows: 128 bytes, the swizzle's span
   auto enc = tensor_map_encoder();
   if (!enc) return false;
-  cuuint64_t dims[2] = {(cuuint64_t)kIK, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)kIK};
-  cuuint32_t box[2] = {128u, box_rows};
+  cuuint64_t dims[2] = {(cuuint64_t)kPm1RowBytes, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)kPm1RowBytes};
+  cuuint32_t box[2] = {(cuuint32_t)kPm1RowBytes, box_rows};
   cuuint32_t es[2] = {1u, 1u};
   const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, es,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -1148,7 +1253,7 @@ static bool make_rows_map(CUtensorMap* m, const void* base, uint64_t rows, uint3
 }
 
 int imma_rows_q(int n) { return (n + kIBM - 1) / kIBM * kIBM; }
-int imma_rows_db(int n) { return (n + kIBN - 1) / kIBN * kIBN; }
+int imma_rows_db(int n) { return (n + kMBN - 1) / kMBN * kMBN; }
 
 // Database splits per 256 queries: of the grids up to 64 splits the one with the
 // least time, whole waves of 148 blocks (one 200 KB block per SM) whose time is
@@ -1157,7 +1262,7 @@ int imma_rows_db(int n) { return (n + kIBN - 1) / kIBN * kIBN; }
 // 64 x 2, 122 us against 244 with 64 x 16.
 int imma_default_splits(int nq_cap, int ndb) {
   const long long qt = (nq_cap + kIBQ - 1) / kIBQ;
-  const int tiles = std::max(1, (ndb + kIBN - 1) / kIBN);
+  const int tiles = std::max(1, (ndb + kMBN - 1) / kMBN);
   int best = 1;
   double best_cost = 1e300;
   for (int s = 1; s <= std::min(kImmaMaxSplits, tiles); s++) {
@@ -1170,7 +1275,7 @@ int imma_default_splits(int nq_cap, int ndb) {
   return best;
 }
 
-cudaError_t launch_expand_pm1(const uint8_t* bits, int n, const int* d_n, int rows, int8_t* out, cudaStream_t s) {
+cudaError_t launch_expand_pm1(const uint8_t* bits, int n, const int* d_n, int rows, uint8_t* out, cudaStream_t s) {
   return launch_chained(k_expand_pm1, 4 * 148, 256, s, ExpandSet{bits, n, d_n, rows, out}, ExpandSet{},
                         static_cast<uint32_t*>(nullptr), 0);
 }
@@ -1197,9 +1302,9 @@ cudaError_t launch_match_imma(const ImmaLaunch& L, cudaStream_t s) {
   }
   CUtensorMap tq, td;
   if (!make_rows_map(&tq, L.q_pm1, (uint64_t)qrows, kIBM)) return cudaErrorInvalidValue;
-  if (!make_rows_map(&td, L.db_pm1, (uint64_t)dbrows, kIBN)) return cudaErrorInvalidValue;
+  if (!make_rows_map(&td, L.db_pm1, (uint64_t)dbrows, kMBN)) return cudaErrorInvalidValue;
   const int qtiles = (L.nq_cap + kIBQ - 1) / kIBQ;
-  const int splits = std::max(1, std::min(L.splits, dbrows / kIBN));
+  const int splits = std::max(1, std::min(L.splits, dbrows / kMBN));
   return launch_chained_smem(k_match_imma, qtiles * splits, kIThreads, kISmemBytes, s, tq, td, L.args, L.work, splits,
                              L.err);
 }
