@@ -15,7 +15,7 @@
 //              database tile's last step) and the accumulator's "full" barriers;
 //   warps 2-17 epilogue, two sets of eight: set s takes every second step, i.e.
 //              accumulator s.  A warp reads its 32 TMEM lanes (queries) over half
-//              the columns, 64 at a time, and keeps a running best / second-best
+//              the columns, 40 at a time, and keeps a running best / second-best
 //              key per query.
 // Steps alternate between the two query tiles of a database tile, so set s holds
 // query tile s; with at most 128 queries there is one query tile, the steps
@@ -28,7 +28,7 @@
 // What bounds it: the epilogue.  With int8 values (kind::i8, half the rate and twice
 // the bytes) 65536 x 65536 took 785 us, of which the tensor pipe needed 660; now the
 // tensor pipe is active 48% of the time and the epilogue's ALU instructions 58%.
-// Most 32-column chunks end at their maximum test; those that pass it are kept few by
+// Most 40-column chunks end at their maximum test; those that pass it are kept few by
 // bounds shared between column halves, sets and database splits, and cheap by
 // looking at their column groups with independent tests and tournaments.  Two query
 // tiles per block read each database tile once for 256 queries.  65536 x 65536: 785
@@ -47,10 +47,13 @@ constexpr int kIBM = 128;  // queries per query tile (MMA M)
 constexpr int kIBQ = 2 * kIBM;  // queries per block of k_match_imma
 constexpr int kIBN = 256;  // database rows per tile of k_rerank_imma (MMA N)
 constexpr int kMBN = 240;  // database rows per tile of k_match_imma: two accumulators leave TMEM columns for the scales
-constexpr int kMHalf = kMBN / 2;  // columns of one epilogue warp
+constexpr int kMChunk = 40;           // columns an epilogue warp examines at a time
+constexpr int kMParts = 2;            // epilogue warps per set and 32 TMEM lanes
+constexpr int kMChunks = kMBN / (kMChunk * kMParts);  // chunks of one of them per step
+constexpr int kMEpiWarps = 2 * 4 * kMParts;
+constexpr int kMThreads = (2 + kMEpiWarps) * 32;
 constexpr int kMStages = 4;
-constexpr int kIEpiWarps = 16;  // two sets of two per TMEM lane quarter, 128 columns each
-constexpr int kIThreads = (2 + kIEpiWarps) * 32;
+constexpr int kIEpiWarps = 16;  // of k_rerank_imma
 constexpr uint32_t kIHalfA = kIBM * 128;  // one 128-byte-wide K half of the query tile
 constexpr uint32_t kIHalfB = kIBN * 128;
 constexpr uint32_t kIATile = 2 * kIHalfA;
@@ -63,11 +66,11 @@ constexpr uint32_t kMNumBars = 1 + 2 * kMStages + 4;
 constexpr uint32_t kMAcc = 256;
 constexpr uint32_t kMScaleCol = kMBN, kMScaleCols = 16;
 // 1024 bytes of alignment slack, the query tiles, the ring, the merge scratch
-// (best two per set, column half and row), the barriers, TMEM base + abort flag
-constexpr uint32_t kIMergeBytes = 4 * kIBM * 8;
+// (best two per set, column part and row), the barriers, TMEM base + abort flag
+constexpr uint32_t kIMergeBytes = 2 * kMParts * kIBM * 8;
 constexpr uint32_t kISmemBytes = 1024 + 2 * kMATile + kMStages * kMBTile + kIMergeBytes + 8 * kMNumBars + 16;
-// dynamic tiles + the static s_last and per-row bounds (4 x kIBM 16-bit)
-static_assert(kISmemBytes + 16 + 4 * kIBM * 2 <= 232448, "exceeds the 227 KB shared-memory opt-in");
+// dynamic tiles + the static s_last and per-row bounds
+static_assert(kISmemBytes + 16 + 2 * kMParts * kIBM * 4 <= 232448, "exceeds the 227 KB shared-memory opt-in");
 constexpr uint32_t kITmemCols = 512;
 constexpr long long kIDeadlineCycles = 4000000000ll;  // ~2 s at 2 GHz
 
@@ -235,7 +238,7 @@ __device__ __forceinline__ bool bits_exceed(float r, int thr) { return r > __int
 
 // The best two of columns B .. E-1 of a chunk as local keys u = column - (dot <<
 // SH), least first, so ties keep the lower column: a tournament of minima (its
-// depth, not its 20 operations for nine columns, is what a warp waits for).
+// depth, not its 23 operations for ten columns, is what a warp waits for).
 template <int B, int E, int SH>
 __device__ __forceinline__ void chunk_best2(const int* vc, int& u1, int& u2) {
   constexpr int n = E - B, h = n / 2;
@@ -289,16 +292,21 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
         "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
       : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_wait_ld32(float* v) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]),
-                 "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]),
-                 "+f"(v[15]), "+f"(v[16]), "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]),
-                 "+f"(v[22]), "+f"(v[23]), "+f"(v[24]), "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]),
-                 "+f"(v[29])
-               :
-               : "memory");
-  asm volatile("" : "+f"(v[30]), "+f"(v[31])::"memory");
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+               : "r"(taddr));
+}
+// Waits for all loads; the 40 values, as operands, cannot be read before it.
+__device__ __forceinline__ void tmem_wait_ld40(float* v) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 40; i += 8)
+    asm volatile(""
+                 : "+f"(v[i]), "+f"(v[i + 1]), "+f"(v[i + 2]), "+f"(v[i + 3]), "+f"(v[i + 4]), "+f"(v[i + 5]),
+                   "+f"(v[i + 6]), "+f"(v[i + 7])
+                 :
+                 : "memory");
 }
 // Value given to columns that hold no database row (below every dot product).
 constexpr float kMaskedDotF = -400.f;
@@ -313,18 +321,23 @@ __device__ __forceinline__ float fmin3(float a, float b, float c) {
   asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
-// Maxima of the column groups 0-8, 9-17, 18-26 and 27-31 of a 32-column chunk.
+// Conversions of small whole numbers by the add whose rounding leaves them in the low
+// mantissa bits: two operations, where a convert instruction makes the chain wait.
+__device__ __forceinline__ int whole_to_int(float u) { return __float_as_int(u + 12582912.f) - 0x4B400000; }
+__device__ __forceinline__ float int_to_whole(int i) { return __int_as_float(i + 0x4B400000) - 12582912.f; }
+
+// Maxima of the four groups of ten columns of a 40-column chunk.
 __device__ __forceinline__ void group_max4(const float* v, float* r) {
 #pragma unroll
-  for (int g = 0; g < 3; g++)
-    r[g] = fmax3(fmax3(v[9 * g], v[9 * g + 1], v[9 * g + 2]), fmax3(v[9 * g + 3], v[9 * g + 4], v[9 * g + 5]),
-                 fmax3(v[9 * g + 6], v[9 * g + 7], v[9 * g + 8]));
-  r[3] = fmax3(fmax3(v[27], v[28], v[29]), v[30], v[31]);
+  for (int g = 0; g < 4; g++) {
+    const float* w = v + 10 * g;
+    r[g] = fmax3(fmax3(fmax3(w[0], w[1], w[2]), w[3], w[4]), fmax3(w[5], w[6], w[7]), fmaxf(w[8], w[9]));
+  }
 }
 // The best two of columns B .. E-1 of a chunk, merged into the running best two
-// keys (distance << 22 | index): local keys u = column - 32 * dot, whole numbers
-// below 2^14 and exact in fp32, go through a tournament of minima (its depth, not
-// its 20 operations for nine columns, is what a warp waits for), so ties keep the
+// keys (distance << 22 | index): local keys u = column - 64 * dot, whole numbers
+// below 2^15 and exact in fp32, go through a tournament of minima (its depth, not
+// its 23 operations for ten columns, is what a warp waits for), so ties keep the
 // lower column.  base is the key of a zero dot product at the chunk's column 0, and
 // a value of one takes 1 << SH off.  Masked columns carry no key.
 template <int B, int E, int SH>
@@ -333,8 +346,8 @@ __device__ __forceinline__ void push_best2(const float* vc, uint32_t base, uint3
   float a1[h], a2[h];
 #pragma unroll
   for (int i = 0; i < h; i++) {
-    const float x = fmaf(vc[B + 2 * i], -32.f, (float)(B + 2 * i)),
-                y = fmaf(vc[B + 2 * i + 1], -32.f, (float)(B + 2 * i + 1));
+    const float x = fmaf(vc[B + 2 * i], -64.f, (float)(B + 2 * i)),
+                y = fmaf(vc[B + 2 * i + 1], -64.f, (float)(B + 2 * i + 1));
     a1[i] = fminf(x, y);
     a2[i] = fmaxf(x, y);
   }
@@ -347,13 +360,13 @@ __device__ __forceinline__ void push_best2(const float* vc, uint32_t base, uint3
     }
   float u1 = a1[0], u2 = a2[0];
   if constexpr (n & 1) {
-    const float x = fmaf(vc[E - 1], -32.f, (float)(E - 1));
+    const float x = fmaf(vc[E - 1], -64.f, (float)(E - 1));
     u2 = fminf(u2, fmaxf(u1, x));
     u1 = fminf(u1, x);
   }
   auto key = [&](float u) {
-    const int i = __float2int_rn(u);
-    return u >= -32.f * kMaskedDotF ? kNoKeyShared : base + ((uint32_t)(i >> 5) << SH) + (uint32_t)(i & 31);
+    const int i = whole_to_int(u);
+    return u >= -64.f * kMaskedDotF ? kNoKeyShared : base + ((uint32_t)(i >> 6) << SH) + (uint32_t)(i & 63);
   };
   const uint32_t p1 = key(u1), p2 = key(u2);
   k2 = __vimin3_u32(max(k1, p1), k2, p2);
@@ -410,7 +423,7 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, long lo
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
-__global__ void __launch_bounds__(kIThreads, 1)
+__global__ void __launch_bounds__(kMThreads, 1)
     k_match_imma(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmD, MatchArgs a,
                  MatchWork w, int splits, int* err) {
   extern __shared__ uint8_t smem_raw[];
@@ -423,10 +436,10 @@ __global__ void __launch_bounds__(kIThreads, 1)
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + kMNumBars);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
   __shared__ unsigned int s_last;
-  // current second-best distance per query row of each set and column half
-  // (0xFFFF: none yet): two keys at or below it exist, so it bounds what the
-  // others that scan the same query keep for that row
-  __shared__ uint16_t s_d2[4][kIBM];
+  // current second-best key per query row of each set and column part: two keys at
+  // or below it exist, so it bounds what the others that scan the same query keep
+  // for that row
+  __shared__ uint32_t s_k2[2 * kMParts][kIBM];
 
   chain_wait();
   const int nq = min(a.d_nq ? *a.d_nq : a.nq, w.nq_cap);
@@ -456,7 +469,7 @@ __global__ void __launch_bounds__(kIThreads, 1)
 #define BAR_ACCFULL(s) (bar0 + 8u * (1 + 2 * kMStages + (s)))
 #define BAR_ACCEMPTY(s) (bar0 + 8u * (3 + 2 * kMStages + (s)))
 
-  for (int i = threadIdx.x; i < 4 * kIBM; i += blockDim.x) (&s_d2[0][0])[i] = 0xFFFFu;
+  for (int i = threadIdx.x; i < 2 * kMParts * kIBM; i += blockDim.x) (&s_k2[0][0])[i] = kNoKeyShared;
   if (threadIdx.x == 0) {
     mbar_init(BAR_A, 1);
     for (int s = 0; s < kMStages; s++) {
@@ -465,7 +478,7 @@ __global__ void __launch_bounds__(kIThreads, 1)
     }
     for (int s = 0; s < 2; s++) {
       mbar_init(BAR_ACCFULL(s), 1);
-      mbar_init(BAR_ACCEMPTY(s), kIEpiWarps / 2);
+      mbar_init(BAR_ACCEMPTY(s), kMEpiWarps / 2);
     }
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -565,10 +578,10 @@ __global__ void __launch_bounds__(kIThreads, 1)
     }
   } else {
     // epilogue: steps of this warp's set, TMEM lanes 32 * (warp & 3) .. (one
-    // query per lane), columns [120 * half, + 120)
-    const int set = (warp - 2) >> 3;
-    const int half = ((warp - 2) >> 2) & 1;
-    const int me = 2 * set + half;
+    // query per lane), columns [kMChunks * kMChunk * part, + kMChunks * kMChunk)
+    const int set = (warp - 2) / (4 * kMParts);
+    const int part = ((warp - 2) >> 2) % kMParts;
+    const int me = kMParts * set + part;
     const int row = (warp & 3) * 32 + lane;
     const int q = qb * kIBQ + (two ? set * kIBM : 0) + row;
     uint32_t k1 = kNoKeyShared, k2 = kNoKeyShared;  // best and second-best key of this row
@@ -578,7 +591,7 @@ __global__ void __launch_bounds__(kIThreads, 1)
     uint32_t told = kNoKeyShared, asked = kNoKeyShared, heard = kNoKeyShared;  // published, being read, read
     float thr_gb = kMaskedDotF;  // a dot at or below this cannot reach the row's final top two
     // (no key yet: far below every dot)
-    auto next_thr = [&]() { return fmaxf(thr_gb, (float)(256 - 2 * (int)(k2 >> kIdxBitsShared))); };
+    auto next_thr = [&]() { return fmaxf(thr_gb, int_to_whole(256 - 2 * (int)(k2 >> kIdxBitsShared))); };
     float thr = kMaskedDotF;
     // columns arrive in increasing index order, so only a strictly larger dot
     // than the own second best can enter the top two.  Most chunks end at the
@@ -594,66 +607,61 @@ __global__ void __launch_bounds__(kIThreads, 1)
                  h2 = __any_sync(0xffffffffu, gm[2] > thr), h3 = __any_sync(0xffffffffu, gm[3] > thr);
       // distance << 22 = (256 - dot) << 21
       const uint32_t base = (256u << (kIdxBitsShared - 1)) + (uint32_t)gc;
-      if (h0) push_best2<0, 9, kIdxBitsShared - 1>(vc, base, k1, k2);
-      if (h1) push_best2<9, 18, kIdxBitsShared - 1>(vc, base, k1, k2);
-      if (h2) push_best2<18, 27, kIdxBitsShared - 1>(vc, base, k1, k2);
-      if (h3) push_best2<27, 32, kIdxBitsShared - 1>(vc, base, k1, k2);
+      if (h0) push_best2<0, 10, kIdxBitsShared - 1>(vc, base, k1, k2);
+      if (h1) push_best2<10, 20, kIdxBitsShared - 1>(vc, base, k1, k2);
+      if (h2) push_best2<20, 30, kIdxBitsShared - 1>(vc, base, k1, k2);
+      if (h3) push_best2<30, 40, kIdxBitsShared - 1>(vc, base, k1, k2);
       thr = next_thr();
     };
-    const uint32_t tcol = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)set * kMAcc + (uint32_t)(half * kMHalf);
+    const uint32_t tcol = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)set * kMAcc + (uint32_t)(part * kMChunks * kMChunk);
     for (int i = set; i < nsteps; i += 2) {
       const int n = i >> 1;  // this set's step
-      ok = warp_wait(BAR_ACCFULL(set), (uint32_t)n & 1u, deadline, s_abort);
-      if (!ok) break;
-      tc_fence_after();
-      const int g0 = (t_beg + (two ? n : i)) * kMBN + half * kMHalf;
+      const int g0 = (t_beg + (two ? n : i)) * kMBN + part * kMChunks * kMChunk;
       // bounds from the others of this block that scan the row's query (every
-      // step) and from its other splits (read in the first steps and then every
+      // step, while the accumulator is not full yet) and from its other splits (read in the first steps and then every
       // fourth, used one step later): a column can reach the row's final top two
-      // only at or below their distance (its index may be lower)
+      // only below their distance, or at it if its index can be the lower one.  (That
+      // last test matters: columns at the bound's distance are as many as those
+      // below it.)
       {
         heard = min(heard, asked);
         if (gq && (n < 8 || (n & 3) == 0)) asked = __ldcg(gq);
-        unsigned gbd = heard >> kIdxBitsShared;
-        auto others = [&](int g) { gbd = min(gbd, (unsigned)reinterpret_cast<volatile uint16_t*>(&s_d2[g][0])[row]); };
-        others(me ^ 1);
-        if (!two) {
-          others(me ^ 2);
-          others(me ^ 3);
-        }
-        if (gbd <= 256u) thr_gb = fmaxf(thr_gb, (float)(256 - 2 * (int)gbd - 1));
+        uint32_t gb = heard;
+        auto others = [&](int g) { gb = min(gb, reinterpret_cast<volatile uint32_t*>(&s_k2[g][0])[row]); };
+#pragma unroll
+        for (int g = 1; g < kMParts; g++) others(kMParts * set + (part + g) % kMParts);
+        if (!two)
+#pragma unroll
+          for (int g = 0; g < kMParts; g++) others(kMParts * (set ^ 1) + g);
+        thr_gb = fmaxf(thr_gb, int_to_whole(256 - 2 * (int)(gb >> kIdxBitsShared) - ((int)(gb & kIdxMaskShared) >= g0)));
         thr = fmaxf(thr, thr_gb);
       }
+      ok = warp_wait(BAR_ACCFULL(set), (uint32_t)n & 1u, deadline, s_abort);
+      if (!ok) break;
+      tc_fence_after();
 #pragma unroll 1
-      for (int c = 0; c < 2; c++) {
-        float v0[32], v1[32];
-        tmem_ld32(tcol + 64u * c, v0);
-        tmem_ld32(tcol + 64u * c + 32u, v1);
-        tmem_wait_ld32(v0);
-        tmem_wait_ld32(v1);
-        if (c == 1) {
-          // every column of this half is in registers: hand the accumulator back
+      for (int c = 0; c < kMChunks; c++) {
+        float v[kMChunk];
+        tmem_ld32(tcol + (uint32_t)(kMChunk * c), v);
+        tmem_ld8(tcol + (uint32_t)(kMChunk * c) + 32u, v + 32);
+        tmem_wait_ld40(v);
+        if (c == kMChunks - 1) {
+          // every column of this part is in registers: hand the accumulator back
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(BAR_ACCEMPTY(set));
-          // the last 8 of 2 x 64 columns belong to the other half or to none
-#pragma unroll
-          for (int j = 24; j < 32; j++) v1[j] = kMaskedDotF;
         }
-        const int gc = g0 + 64 * c;
-        if (gc + 64 > ndb) {
+        const int gc = g0 + kMChunk * c;
+        if (gc + kMChunk > ndb) {
 #pragma unroll
-          for (int j = 0; j < 32; j++) {
-            if (gc + j >= ndb) v0[j] = kMaskedDotF;
-            if (gc + 32 + j >= ndb) v1[j] = kMaskedDotF;
-          }
+          for (int j = 0; j < kMChunk; j++)
+            if (gc + j >= ndb) v[j] = kMaskedDotF;
         }
-        examine(v0, gc);
-        examine(v1, gc + 32);
+        examine(v, gc);
       }
       if (k2 < told) {
         told = k2;
-        reinterpret_cast<volatile uint16_t*>(&s_d2[me][0])[row] = (uint16_t)(k2 >> kIdxBitsShared);
+        reinterpret_cast<volatile uint32_t*>(&s_k2[me][0])[row] = k2;
         // two distinct rows at or below k2: the query's final second best is no worse
         if (gq) atomicMin(gq, k2);
       }
@@ -676,14 +684,14 @@ __global__ void __launch_bounds__(kIThreads, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kITmemCols)
                  : "memory");
   }
-  // the best two of each query over the block's sets and column halves
+  // the best two of each query over the block's sets and column parts
   const int rows = two ? kIBQ : kIBM;
-  for (int r = threadIdx.x; r < rows; r += kIThreads) {
+  for (int r = threadIdx.x; r < rows; r += kMThreads) {
     const int q = qb * kIBQ + r;
     if (q >= nq) break;
     uint32_t k1 = kNoKeyShared, k2 = kNoKeyShared;
-    for (int g = 0; g < (two ? 2 : 4); g++) {
-      const uint2 pk = s_merge[(two ? 2 * (r / kIBM) + g : g) * kIBM + r % kIBM];
+    for (int g = 0; g < (two ? kMParts : 2 * kMParts); g++) {
+      const uint2 pk = s_merge[(two ? kMParts * (r / kIBM) + g : g) * kIBM + r % kIBM];
       top2_push_shared(k1, k2, pk.x);
       top2_push_shared(k1, k2, pk.y);
     }
@@ -694,7 +702,7 @@ __global__ void __launch_bounds__(kIThreads, 1)
   }
   if (splits == 1) return;
   // the last block of these queries to finish merges the partial top-2 of all
-  // splits: 2 or 4 threads per query
+  // splits: several threads per query
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) s_last = (atomicAdd(&w.tile_done[qb], 1u) == (unsigned)(splits - 1)) ? 1u : 0u;
@@ -702,7 +710,8 @@ __global__ void __launch_bounds__(kIThreads, 1)
   if (!s_last) return;
   __threadfence();
   if (threadIdx.x == 0) w.tile_done[qb] = 0u;
-  const int per = two ? 2 : 4;
+  const int per = two ? kMParts : 2 * kMParts;
+  static_assert(2 * kMParts * kIBM <= kMThreads, "one thread per entry of s_merge");
   if (threadIdx.x < rows * per) {
     const int r = threadIdx.x % rows, g = threadIdx.x / rows;
     const int q = qb * kIBQ + r;
@@ -1305,7 +1314,7 @@ cudaError_t launch_match_imma(const ImmaLaunch& L, cudaStream_t s) {
   if (!make_rows_map(&td, L.db_pm1, (uint64_t)dbrows, kMBN)) return cudaErrorInvalidValue;
   const int qtiles = (L.nq_cap + kIBQ - 1) / kIBQ;
   const int splits = std::max(1, std::min(L.splits, dbrows / kMBN));
-  return launch_chained_smem(k_match_imma, qtiles * splits, kIThreads, kISmemBytes, s, tq, td, L.args, L.work, splits,
+  return launch_chained_smem(k_match_imma, qtiles * splits, kMThreads, kISmemBytes, s, tq, td, L.args, L.work, splits,
                              L.err);
 }
 
