@@ -196,11 +196,11 @@ struct MatchWork {          // scratch for split-train merging
 constexpr int kPm1RowBytes = 128;  // an expanded descriptor: 256 4-bit floats, +-1
 struct ImmaLaunch {
   MatchArgs args;     // queries, database, counts, outputs
-  MatchWork work;     // split merging (splits_cap >= splits)
+  MatchWork work;     // part: [slots][work.nq_cap] best two; tile_done: one per 256 queries
   uint8_t* q_pm1;     // [imma_rows_q(nq_cap)][kPm1RowBytes] scratch
   uint8_t* db_pm1;    // [imma_rows_db(ndb_cap)][kPm1RowBytes] scratch
   int nq_cap, ndb_cap;
-  int splits;         // database splits per query tile
+  int slots;          // slots per query in work.part (imma_slots)
   int* err;
   bool q_ready;       // q_pm1 already holds the expanded queries (rows >= nq zero)
   bool db_ready;      // db_pm1 already holds the expanded database (rows >= ndb zero)
@@ -209,8 +209,8 @@ struct ImmaLaunch {
 cudaError_t launch_expand_pm1(const uint8_t* bits, int n, const int* d_n, int rows, uint8_t* out, cudaStream_t s);
 int imma_rows_q(int n);
 int imma_rows_db(int n);
-constexpr int kImmaMaxSplits = 64;
-int imma_default_splits(int nq_cap, int ndb);
+constexpr int kImmaMaxSlots = 152;  // every SM has a part of one block of queries
+int imma_slots(int nq, int ndb, int max_slots);
 cudaError_t launch_match_imma(const ImmaLaunch& L, cudaStream_t s);
 
 // Probe rerank of the learned proposal on the int8 tensor cores

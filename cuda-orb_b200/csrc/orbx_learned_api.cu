@@ -105,19 +105,18 @@ int pick_splits(int tiles, int kblocks) {
   return s;
 }
 
-// Split-merge scratch of the int8 tensor-core matcher for nq_cap queries,
-// with the database splits chosen for splits_for queries.
+// Merge scratch of the tensor-core matcher for up to nq_cap queries, with the slots
+// that nq_from or more of them need.
 struct ImmaWork {
   MatchWork w{};
-  int splits = 1;
+  int slots = 1;
 };
-int imma_work_alloc(Arena& a, ImmaWork& iw, int nq_cap, int splits_for, int ndb, cudaStream_t s, int splits_cap = 0) {
-  iw.splits = imma_default_splits(std::max(1, splits_for), ndb);
+int imma_work_alloc(Arena& a, ImmaWork& iw, int nq_cap, int nq_from, int ndb, cudaStream_t s) {
+  iw.slots = imma_slots(nq_from, ndb, kImmaMaxSlots);
   iw.w.nq_cap = nq_cap;
-  iw.w.splits_cap = std::max(iw.splits, splits_cap);
-  if (iw.w.splits_cap > 1) {
+  if (iw.slots > 2) {
     const int tiles = (nq_cap + 127) / 128;
-    LCHK(a.alloc(&iw.w.part, (size_t)2 * iw.w.splits_cap * nq_cap));
+    LCHK(a.alloc(&iw.w.part, (size_t)2 * iw.slots * nq_cap));
     LCHK(a.alloc(&iw.w.tile_done, (size_t)tiles));
     LCHK(a.alloc(&iw.w.bound, (size_t)nq_cap));
     LCHK(cudaMemsetAsync(iw.w.tile_done, 0, sizeof(unsigned) * (size_t)tiles, s));
@@ -138,7 +137,7 @@ int imma_knn(cudaStream_t s, int* err, const ImmaWork& iw, const uint8_t* q, int
   L.args.dist2 = dist2;
   L.args.idx2 = idx2;
   L.work = iw.w;
-  L.splits = iw.splits;
+  L.slots = iw.slots;
   L.q_pm1 = q_pm1;
   L.db_pm1 = db_pm1;
   L.nq_cap = nq_cap;
@@ -634,10 +633,9 @@ int ensure_search(orbx_learned* L, int nq) {
   LCHK(a.alloc(&L->fb_d, (size_t)nq * 2));
   LCHK(a.alloc(&L->fb_i, (size_t)nq * 2));
   LCHK(a.alloc(&L->fb_pm1, (size_t)imma_rows_q(nq) * kPm1RowBytes));
-  // fallback splits sized for about one query in eight; fewer fallback queries
-  // split the database scan further, up to 32 ways
+  // the fallback's slots let few queries (512 or more) spread over all SMs
   L->fb_work = ImmaWork();
-  LRC(imma_work_alloc(a, L->fb_work, nq, std::max(128, nq / 8), L->ndb, 0, 32));
+  LRC(imma_work_alloc(a, L->fb_work, nq, std::min(nq, 512), L->ndb, 0));
   LCHK(cudaDeviceSynchronize());
   L->nq_cap = nq;
   return ORBX_OK;

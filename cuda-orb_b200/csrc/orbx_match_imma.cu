@@ -15,7 +15,7 @@
 //              database tile's last step) and the accumulator's "full" barriers;
 //   warps 2-17 epilogue, two sets of eight: set s takes every second step, i.e.
 //              accumulator s.  A warp reads its 32 TMEM lanes (queries) over half
-//              the columns, 40 at a time, and keeps a running best / second-best
+//              the columns, 60 at a time, and keeps a running best / second-best
 //              key per query.
 // Steps alternate between the two query tiles of a database tile, so set s holds
 // query tile s; with at most 128 queries there is one query tile, the steps
@@ -26,28 +26,35 @@
 // records kErrImmaTimeout, drains its in-flight copies, frees TMEM and exits.
 //
 // What bounds it: the epilogue.  With int8 values (kind::i8, half the rate and twice
-// the bytes) 65536 x 65536 took 785 us, of which the tensor pipe needed 660; now the
-// tensor pipe is active 48% of the time and the epilogue's ALU instructions 58%.
-// Most 40-column chunks end at their maximum test; those that pass it are kept few by
-// bounds shared between column halves, sets and database splits, and cheap by
-// looking at their column groups with independent tests and tournaments.  Two query
-// tiles per block read each database tile once for 256 queries.  65536 x 65536: 785
-// -> 666 us; 1500 x 262144: 95 -> 74.5 us.
+// the bytes) 65536 x 65536 took 785 us, 660 of them the tensor pipe's; now the MMAs
+// alone need 336 us, with the loads of their results 357, with the maximum test of
+// every chunk 445.  The rest are the chunks that pass it: a warp that examines one
+// keeps its accumulator, so the others wait for it.  They are kept few by long scans
+// (orbx_match_plan.cuh: 616 -> 532 us) and by bounds shared between column parts, sets
+// and blocks, and cheap by tournaments over column groups.  A chunk is what the
+// registers hold: each costs a round trip to TMEM (40 columns: 563 us).  More, shorter
+// accumulators or more epilogue warps were slower (3 x 160 columns 685 against 646 us,
+// 24 warps 767: each step costs every warp about 700 cycles).  65536 x 65536: 785 ->
+// 532 us; 1500 x 262144: 95 -> 73 us.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <utility>
 
 #include "orbx_device.cuh"
 #include "orbx_internal.cuh"
+#include "orbx_match_plan.cuh"
 
 namespace orbx {
 
 constexpr int kIBM = 128;  // queries per query tile (MMA M)
-constexpr int kIBQ = 2 * kIBM;  // queries per block of k_match_imma
+constexpr int kIBQ = kPlanQueries;  // queries per block of k_match_imma
+static_assert(kIBQ == 2 * kIBM, "two query tiles");
 constexpr int kIBN = 256;  // database rows per tile of k_rerank_imma (MMA N)
-constexpr int kMBN = 240;  // database rows per tile of k_match_imma: two accumulators leave TMEM columns for the scales
-constexpr int kMChunk = 40;           // columns an epilogue warp examines at a time
+constexpr int kMBN = kPlanRows;  // database rows per tile of k_match_imma: two accumulators leave TMEM columns for the scales
+constexpr int kMChunk = 60;           // columns an epilogue warp examines at a time,
+constexpr int kMGroups = 4;           // in so many groups
 constexpr int kMParts = 2;            // epilogue warps per set and 32 TMEM lanes
 constexpr int kMChunks = kMBN / (kMChunk * kMParts);  // chunks of one of them per step
 constexpr int kMEpiWarps = 2 * 4 * kMParts;
@@ -61,14 +68,14 @@ constexpr uint32_t kIBTile = 2 * kIHalfB;
 constexpr uint32_t kMATile = kIBM * kPm1RowBytes;  // one 128-byte swizzle row per descriptor
 constexpr uint32_t kMBTile = kMBN * kPm1RowBytes;
 static_assert(kPm1RowBytes == 128 && kMBTile % 1024 == 0, "whole swizzle atoms");
-constexpr uint32_t kMNumBars = 1 + 2 * kMStages + 4;
+constexpr uint32_t kMNumBars = 2 * 2 + 2 * kMStages + 2 * 2 + 1;  // full and empty: query tiles, ring, accumulators; the epilogue's own
 // accumulator a starts at TMEM column 256 * a; the scales (all 1) lie between them
 constexpr uint32_t kMAcc = 256;
 constexpr uint32_t kMScaleCol = kMBN, kMScaleCols = 16;
-// 1024 bytes of alignment slack, the query tiles, the ring, the merge scratch
+// 1024 bytes of alignment slack, two pairs of query tiles, the ring, the merge scratch
 // (best two per set, column part and row), the barriers, TMEM base + abort flag
 constexpr uint32_t kIMergeBytes = 2 * kMParts * kIBM * 8;
-constexpr uint32_t kISmemBytes = 1024 + 2 * kMATile + kMStages * kMBTile + kIMergeBytes + 8 * kMNumBars + 16;
+constexpr uint32_t kISmemBytes = 1024 + 4 * kMATile + kMStages * kMBTile + kIMergeBytes + 8 * kMNumBars + 16;
 // dynamic tiles + the static s_last and per-row bounds
 static_assert(kISmemBytes + 16 + 2 * kMParts * kIBM * 4 <= 232448, "exceeds the 227 KB shared-memory opt-in");
 constexpr uint32_t kITmemCols = 512;
@@ -297,16 +304,32 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
                : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
                : "r"(taddr));
 }
-// Waits for all loads; the 40 values, as operands, cannot be read before it.
-__device__ __forceinline__ void tmem_wait_ld40(float* v) {
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
+        "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+               : "r"(taddr));
+}
+// N values of the lane's row, loaded and waited for; as operands of the statements
+// after the wait they cannot be read before it.
+template <int N>
+__device__ __forceinline__ void tmem_read(uint32_t taddr, float* v) {
+  static_assert(N % 4 == 0 && N < 64, "loads of 32, 16, 8 and 4");
+  if constexpr (N & 32) tmem_ld32(taddr, v);
+  if constexpr (N & 16) tmem_ld16(taddr + (N & 32), v + (N & 32));
+  if constexpr (N & 8) tmem_ld8(taddr + (N & 48), v + (N & 48));
+  if constexpr (N & 4) tmem_ld4(taddr + (N & 56), v + (N & 56));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < 40; i += 8)
-    asm volatile(""
-                 : "+f"(v[i]), "+f"(v[i + 1]), "+f"(v[i + 2]), "+f"(v[i + 3]), "+f"(v[i + 4]), "+f"(v[i + 5]),
-                   "+f"(v[i + 6]), "+f"(v[i + 7])
-                 :
-                 : "memory");
+  for (int i = 0; i < N; i += 4)
+    asm volatile("" : "+f"(v[i]), "+f"(v[i + 1]), "+f"(v[i + 2]), "+f"(v[i + 3])::"memory");
 }
 // Value given to columns that hold no database row (below every dot product).
 constexpr float kMaskedDotF = -400.f;
@@ -326,13 +349,25 @@ __device__ __forceinline__ float fmin3(float a, float b, float c) {
 __device__ __forceinline__ int whole_to_int(float u) { return __float_as_int(u + 12582912.f) - 0x4B400000; }
 __device__ __forceinline__ float int_to_whole(int i) { return __int_as_float(i + 0x4B400000) - 12582912.f; }
 
-// Maxima of the four groups of ten columns of a 40-column chunk.
-__device__ __forceinline__ void group_max4(const float* v, float* r) {
+// The maximum of N values, by three-input maxima.
+template <int N>
+__device__ __forceinline__ float max_of(const float* v) {
+  float m[N];
 #pragma unroll
-  for (int g = 0; g < 4; g++) {
-    const float* w = v + 10 * g;
-    r[g] = fmax3(fmax3(fmax3(w[0], w[1], w[2]), w[3], w[4]), fmax3(w[5], w[6], w[7]), fmaxf(w[8], w[9]));
+  for (int i = 0; i < N; i++) m[i] = v[i];
+  int n = N;
+#pragma unroll
+  for (int round = 0; round < 4; round++) {
+    int o = 0;
+#pragma unroll
+    for (int i = 0; i < N; i += 3) {
+      if (i + 2 < n) m[o++] = fmax3(m[i], m[i + 1], m[i + 2]);
+      else if (i + 1 < n) m[o++] = fmaxf(m[i], m[i + 1]);
+      else if (i < n) m[o++] = m[i];
+    }
+    n = o;
   }
+  return m[0];
 }
 // The best two of columns B .. E-1 of a chunk, merged into the running best two
 // keys (distance << 22 | index): local keys u = column - 64 * dot, whole numbers
@@ -413,24 +448,132 @@ __global__ void __launch_bounds__(256) k_expand_pm1(ExpandSet q, ExpandSet db, u
   }
 }
 
-// Warp-uniform bounded wait: every lane tries once (no broadcast when the phase
-// is over, the common case); after that lane 0 polls and the result is broadcast.
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, long long deadline,
-                                          volatile int* abort_flag) {
+// A warp's wait: every lane tries once (no broadcast when the phase is over, the
+// common case); after that lane 0 polls and the result is broadcast.
+// Bounded waits of k_match_imma: false when a wait takes longer than
+// kIDeadlineCycles or another role has given up.
+__device__ __forceinline__ bool im_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  if (mbar_try(bar, parity)) return true;
+  return mbar_wait(bar, parity, clock64() + kIDeadlineCycles, abort_flag);
+}
+__device__ __forceinline__ bool im_warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
   int ok = 0;
-  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, deadline, abort_flag) ? 1 : 0;
+  if ((threadIdx.x & 31) == 0) ok = im_wait(bar, parity, abort_flag) ? 1 : 0;
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+
+template <int SIZE, int SH, int... G>
+__device__ __forceinline__ void push_groups(const float* vc, const bool* hit, uint32_t base, uint32_t& k1, uint32_t& k2,
+                                            std::integer_sequence<int, G...>) {
+  ((hit[G] ? push_best2<SIZE * G, SIZE * (G + 1), SH>(vc, base, k1, k2) : (void)0), ...);
+}
+
+__device__ __forceinline__ uint32_t lds_volatile(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts_volatile(uint32_t a, uint32_t v) {
+  asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+// One warp's part of a scan: its 32 queries over its columns of every accumulator of
+// its set.  A function of its own, so that the registers around it are not the loop's.
+struct ScanArgs {
+  uint32_t* gq;       // the lane's query's bound, shared with the blocks that have its other parts, or null
+  uint32_t k2_mine;   // shared memory: this warp's second-best key of the lane's row,
+  uint32_t k2_set;    // that of the other column part,
+  uint32_t k2_other;  // and those of the other set, kIBM apart, or 0 when it has other queries
+  uint32_t tcol, full, empty, phase;
+  int steps, col, stride, ndb;  // first column of the first step, columns from step to step
+  volatile int* abort_flag;
+};
+__device__ __noinline__ bool m_scan(const ScanArgs sa, uint2* best) {
+  static_assert(kMParts == 2, "one other column part");
+  const int lane = threadIdx.x & 31;
+  uint32_t k1 = kNoKeyShared, k2 = kNoKeyShared;  // best and second-best key of this row
+  uint32_t told = kNoKeyShared, asked = kNoKeyShared, heard = kNoKeyShared;  // published, being read, read
+  float thr_gb = kMaskedDotF;  // a dot at or below this cannot reach the row's final top two
+  // (no key yet: far below every dot)
+  auto next_thr = [&]() { return fmaxf(thr_gb, int_to_whole(256 - 2 * (int)(k2 >> kIdxBitsShared))); };
+  float thr = kMaskedDotF;
+  // columns arrive in increasing index order, so only a strictly larger dot
+  // than the own second best can enter the top two.  Most chunks end at the
+  // maximum test; one that passes looks at the column groups with a value above
+  // the threshold.  These are few (a lane's top two change a few times per scan)
+  // but they were half of the kernel's time when each group was a serial chain
+  // with its own test.
+  auto examine = [&](const float* vc, int gc) {
+    constexpr int kSize = kMChunk / kMGroups;
+    float gm[kMGroups];
+#pragma unroll
+    for (int g = 0; g < kMGroups; g++) gm[g] = max_of<kSize>(vc + kSize * g);
+    if (!__any_sync(0xffffffffu, max_of<kMGroups>(gm) > thr)) return;
+    bool hit[kMGroups];
+#pragma unroll
+    for (int g = 0; g < kMGroups; g++) hit[g] = __any_sync(0xffffffffu, gm[g] > thr);
+    // distance << 22 = (256 - dot) << 21
+    const uint32_t base = (256u << (kIdxBitsShared - 1)) + (uint32_t)gc;
+    push_groups<kSize, kIdxBitsShared - 1>(vc, hit, base, k1, k2, std::make_integer_sequence<int, kMGroups>());
+    thr = next_thr();
+  };
+  int c0 = sa.col;  // first column of the step
+  for (int n = 0; n < sa.steps; n++, c0 += sa.stride) {
+    // bounds from the others of this block that scan the row's query (every step,
+    // while the accumulator is not full yet) and from its other parts (read in the
+    // first steps and then every fourth, used one step later): a column can reach the
+    // row's final top two only below their distance, or at it if its index can be the
+    // lower one.
+    {
+      heard = min(heard, asked);
+      if (sa.gq && (n < 8 || (n & 3) == 0)) asked = __ldcg(sa.gq);
+      uint32_t gb = heard;
+      gb = min(gb, lds_volatile(sa.k2_set));
+      if (sa.k2_other)
+        gb = min(gb, min(lds_volatile(sa.k2_other), lds_volatile(sa.k2_other + 4u * kIBM)));
+      thr_gb = fmaxf(thr_gb, int_to_whole(256 - 2 * (int)(gb >> kIdxBitsShared) - ((int)(gb & kIdxMaskShared) >= c0)));
+      thr = fmaxf(thr, thr_gb);
+    }
+    if (!im_warp_wait(sa.full, (sa.phase + (uint32_t)n) & 1u, sa.abort_flag)) return false;
+    tc_fence_after();
+#pragma unroll 1
+    for (int c = 0; c < kMChunks; c++) {
+      float v[kMChunk];
+      tmem_read<kMChunk>(sa.tcol + (uint32_t)(kMChunk * c), v);
+      if (c == kMChunks - 1) {
+        // every column of this part is in registers: hand the accumulator back
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(sa.empty);
+      }
+      const int gc = c0 + kMChunk * c;
+      if (gc + kMChunk > sa.ndb) {
+#pragma unroll
+        for (int j = 0; j < kMChunk; j++)
+          if (gc + j >= sa.ndb) v[j] = kMaskedDotF;
+      }
+      examine(v, gc);
+    }
+    if (k2 < told) {
+      told = k2;
+      sts_volatile(sa.k2_mine, k2);
+      // two distinct rows at or below k2: the query's final second best is no worse
+      if (sa.gq) atomicMin(sa.gq, k2);
+    }
+  }
+  *best = make_uint2(k1, k2);
+  return true;
 }
 
 __global__ void __launch_bounds__(kMThreads, 1)
     k_match_imma(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmD, MatchArgs a,
-                 MatchWork w, int splits, int* err) {
+                 MatchWork w, int slots, int* err) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
   uint8_t* sA = smem;
-  uint8_t* sB = sA + 2 * kMATile;
+  uint8_t* sB = sA + 4 * kMATile;
   uint2* s_merge = reinterpret_cast<uint2*>(sB + kMStages * kMBTile);
   uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(s_merge) + kIMergeBytes);
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + kMNumBars);
@@ -444,39 +587,31 @@ __global__ void __launch_bounds__(kMThreads, 1)
   chain_wait();
   const int nq = min(a.d_nq ? *a.d_nq : a.nq, w.nq_cap);
   const int ndb = a.d_ndb ? *a.d_ndb : a.ndb;
-  const int qtiles = (nq + kIBQ - 1) / kIBQ;
-  // With the query count on the device, the grid is sized for the capacity;
-  // when fewer query tiles are live, their database scans are split further
-  // (up to the merge scratch's splits_cap) so that the whole grid works.
-  if (a.d_nq && w.splits_cap > splits && qtiles > 0) splits = max(splits, min(w.splits_cap, (int)gridDim.x / qtiles));
-  const int qb = blockIdx.x / splits;
-  const int sp = blockIdx.x - qb * splits;
-  if (qb >= qtiles) return;  // uniform over the block: before any barrier or TMEM use
-  const int nq_here = min(kIBQ, nq - qb * kIBQ);
-  const bool two = nq_here > kIBM;  // two query tiles
-  const int dbtiles = (ndb + kMBN - 1) / kMBN;
-  const int t_beg = (int)((long long)dbtiles * sp / splits);
-  const int t_end = (int)((long long)dbtiles * (sp + 1) / splits);
-  const int ntiles = t_end - t_beg;
-  const int nsteps = two ? 2 * ntiles : ntiles;
+  const MPlan plan = m_plan(nq, ndb, slots, (int)gridDim.x);
+  if ((int)blockIdx.x >= plan.grid) return;  // uniform over the block: before any barrier or TMEM use
+  const long long x_beg = m_start(plan, slots, blockIdx.x), x_end = m_start(plan, slots, blockIdx.x + 1);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t bar0 = smem_u32(bars);
-  const uint32_t BAR_A = bar0;
-#define BAR_BFULL(s) (bar0 + 8u * (1 + (s)))
-#define BAR_BEMPTY(s) (bar0 + 8u * (1 + kMStages + (s)))
-#define BAR_ACCFULL(s) (bar0 + 8u * (1 + 2 * kMStages + (s)))
-#define BAR_ACCEMPTY(s) (bar0 + 8u * (3 + 2 * kMStages + (s)))
+#define BAR_AFULL(s) (bar0 + 8u * (s))
+#define BAR_AEMPTY(s) (bar0 + 8u * (2 + (s)))
+#define BAR_BFULL(s) (bar0 + 8u * (4 + (s)))
+#define BAR_BEMPTY(s) (bar0 + 8u * (4 + kMStages + (s)))
+#define BAR_ACCFULL(s) (bar0 + 8u * (4 + 2 * kMStages + (s)))
+#define BAR_ACCEMPTY(s) (bar0 + 8u * (6 + 2 * kMStages + (s)))
+#define BAR_EPI (bar0 + 8u * (8 + 2 * kMStages))
 
   for (int i = threadIdx.x; i < 2 * kMParts * kIBM; i += blockDim.x) (&s_k2[0][0])[i] = kNoKeyShared;
   if (threadIdx.x == 0) {
-    mbar_init(BAR_A, 1);
+    mbar_init(BAR_EPI, kMEpiWarps);
     for (int s = 0; s < kMStages; s++) {
       mbar_init(BAR_BFULL(s), 1);
       mbar_init(BAR_BEMPTY(s), 1);
     }
     for (int s = 0; s < 2; s++) {
+      mbar_init(BAR_AFULL(s), 1);
+      mbar_init(BAR_AEMPTY(s), 1);
       mbar_init(BAR_ACCFULL(s), 1);
       mbar_init(BAR_ACCEMPTY(s), kMEpiWarps / 2);
     }
@@ -500,28 +635,38 @@ __global__ void __launch_bounds__(kMThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const long long deadline = clock64() + kIDeadlineCycles;
 
   if (warp == 0) {
     if (lane == 0) {
       // TMA producer
       int issued[kMStages];
       for (int s = 0; s < kMStages; s++) issued[s] = 0;
+      int parts = 0, tg = 0, a_loads = 0;  // parts, database tiles and query loads so far
       bool ok = true;
-      mbar_expect_tx(BAR_A, two ? 2 * kMATile : kMATile);
-      for (int m = 0; m < (two ? 2 : 1); m++)
-        tma_load_2d(smem_u32(sA + m * kMATile), &tmQ, 0, qb * kIBQ + m * kIBM, BAR_A);
-      for (int i = 0; i < ntiles; i++) {
-        const int s = i % kMStages;
-        const int use = i / kMStages;
-        if (use > 0 && !mbar_wait(BAR_BEMPTY(s), (use - 1) & 1, deadline, s_abort)) {
+      for (long long x = x_beg; ok && x < x_end; parts++) {
+        const MPart r = m_part(plan, x, x_end);
+        x += r.t1 - r.t0;
+        const int ab = parts & 1;
+        if (parts >= 2 && !im_wait(BAR_AEMPTY(ab), (uint32_t)((parts >> 1) - 1) & 1u, s_abort)) {
           ok = false;
           break;
         }
-        const int row = (t_beg + i) * kMBN;
-        mbar_expect_tx(BAR_BFULL(s), kMBTile);
-        tma_load_2d(smem_u32(sB + s * kMBTile), &tmD, 0, row, BAR_BFULL(s));
-        issued[s]++;
+        const bool two = nq - r.qb * kIBQ > kIBM;  // two query tiles
+        a_loads++;
+        mbar_expect_tx(BAR_AFULL(ab), two ? 2 * kMATile : kMATile);
+        for (int m = 0; m < (two ? 2 : 1); m++)
+          tma_load_2d(smem_u32(sA + (2 * ab + m) * kMATile), &tmQ, 0, r.qb * kIBQ + m * kIBM, BAR_AFULL(ab));
+        for (int t = r.t0; t < r.t1; t++, tg++) {
+          const int s = tg % kMStages;
+          const int use = tg / kMStages;
+          if (use > 0 && !im_wait(BAR_BEMPTY(s), (use - 1) & 1, s_abort)) {
+            ok = false;
+            break;
+          }
+          mbar_expect_tx(BAR_BFULL(s), kMBTile);
+          tma_load_2d(smem_u32(sB + s * kMBTile), &tmD, 0, t * kMBN, BAR_BFULL(s));
+          issued[s]++;
+        }
       }
       if (!ok) {
         *s_abort = 1;
@@ -529,8 +674,13 @@ __global__ void __launch_bounds__(kMThreads, 1)
       }
       // Drain before the block may exit: every issued copy has landed and every
       // MMA that read a stage has completed (its commit arrived on "empty").
-      long long dl = clock64() + kIDeadlineCycles;
-      while (!mbar_try(BAR_A, 0) && clock64() < dl) {
+      long long dl;
+      for (int ab = 0; ab < 2; ab++) {
+        const int loads = (a_loads + 1 - ab) >> 1;
+        if (loads == 0) continue;
+        dl = clock64() + kIDeadlineCycles;
+        while (!mbar_try(BAR_AFULL(ab), (uint32_t)(loads - 1) & 1u) && clock64() < dl) {
+        }
       }
       for (int s = 0; s < kMStages; s++) {
         if (issued[s] == 0) continue;
@@ -546,30 +696,37 @@ __global__ void __launch_bounds__(kMThreads, 1)
   } else if (warp == 1) {
     if (lane == 0) {
       // MMA issuer: four K=64 MMAs per step into accumulator (step & 1)
-      bool ok = mbar_wait(BAR_A, 0, deadline, s_abort);
-      const uint32_t a_base = smem_u32(sA);
-      for (int i = 0; ok && i < nsteps; i++) {
-        const int t = two ? i >> 1 : i;
-        const int qt = two ? i & 1 : 0;
-        const int s = t % kMStages;
-        const int acc = i & 1;
-        if (qt == 0 && !mbar_wait(BAR_BFULL(s), (uint32_t)(t / kMStages) & 1u, deadline, s_abort)) {
-          ok = false;
-          break;
-        }
-        if (i >= 2 && !mbar_wait(BAR_ACCEMPTY(acc), (uint32_t)((i - 2) >> 1) & 1u, deadline, s_abort)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t d = tmem_base + (uint32_t)acc * kMAcc;
-        const uint32_t sfa = tmem_base + kMScaleCol, sfb = sfa + kMScaleCols / 2;
-        const uint64_t da = sw128_desc(a_base + (uint32_t)qt * kMATile), db = sw128_desc(smem_u32(sB + s * kMBTile));
+      bool ok = true;
+      int parts = 0, tg = 0, g = 0;  // parts, database tiles and steps so far
+      const uint32_t sfa = tmem_base + kMScaleCol, sfb = sfa + kMScaleCols / 2;
+      for (long long x = x_beg; ok && x < x_end; parts++) {
+        const MPart r = m_part(plan, x, x_end);
+        x += r.t1 - r.t0;
+        const int ab = parts & 1;
+        const int per = nq - r.qb * kIBQ > kIBM ? 2 : 1;
+        const uint64_t da0 = sw128_desc(smem_u32(sA + 2 * ab * kMATile));
+        ok = im_wait(BAR_AFULL(ab), (uint32_t)(parts >> 1) & 1u, s_abort);
+        for (int t = r.t0; ok && t < r.t1; t++, tg++) {
+          const int s = tg % kMStages;
+          ok = im_wait(BAR_BFULL(s), (uint32_t)(tg / kMStages) & 1u, s_abort);
+          const uint64_t db = sw128_desc(smem_u32(sB + s * kMBTile));
+          for (int qt = 0; ok && qt < per; qt++, g++) {
+            const int acc = g & 1;
+            if (g >= 2 && !im_wait(BAR_ACCEMPTY(acc), (uint32_t)((g - 2) >> 1) & 1u, s_abort)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t d = tmem_base + (uint32_t)acc * kMAcc;
+            const uint64_t da = da0 + (uint64_t)(qt * (kMATile >> 4));
 #pragma unroll
-        for (int k = 0; k < 4; k++)  // 64 values are 32 bytes of a row: two descriptor units
-          umma_f4(d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), kMDesc, sfa, sfb, k > 0 ? 1u : 0u);
-        if (!two || qt == 1) umma_commit(BAR_BEMPTY(s));  // the database tile's last step
-        umma_commit(BAR_ACCFULL(acc));
+            for (int k = 0; k < 4; k++)  // 64 values are 32 bytes of a row: two descriptor units
+              umma_f4(d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), kMDesc, sfa, sfb, k > 0 ? 1u : 0u);
+            if (qt == per - 1) umma_commit(BAR_BEMPTY(s));  // the database tile's last step
+            umma_commit(BAR_ACCFULL(acc));
+          }
+        }
+        if (ok) umma_commit(BAR_AEMPTY(ab));
       }
       if (!ok) {
         *s_abort = 1;
@@ -583,99 +740,131 @@ __global__ void __launch_bounds__(kMThreads, 1)
     const int part = ((warp - 2) >> 2) % kMParts;
     const int me = kMParts * set + part;
     const int row = (warp & 3) * 32 + lane;
-    const int q = qb * kIBQ + (two ? set * kIBM : 0) + row;
-    uint32_t k1 = kNoKeyShared, k2 = kNoKeyShared;  // best and second-best key of this row
+    const int e = threadIdx.x - 64;  // of the epilogue's threads
     bool ok = true;
-    // second-best bound shared by the blocks that scan this query's other splits
-    uint32_t* gq = (w.bound && splits > 1 && q < nq) ? w.bound + q : nullptr;
-    uint32_t told = kNoKeyShared, asked = kNoKeyShared, heard = kNoKeyShared;  // published, being read, read
-    float thr_gb = kMaskedDotF;  // a dot at or below this cannot reach the row's final top two
-    // (no key yet: far below every dot)
-    auto next_thr = [&]() { return fmaxf(thr_gb, int_to_whole(256 - 2 * (int)(k2 >> kIdxBitsShared))); };
-    float thr = kMaskedDotF;
-    // columns arrive in increasing index order, so only a strictly larger dot
-    // than the own second best can enter the top two.  Most chunks end at the
-    // maximum test; one that passes looks at the column groups with a value above
-    // the threshold.  These are few (a lane's top two change a few times per scan)
-    // but they were half of the kernel's time when each group was a serial chain
-    // with its own test.
-    auto examine = [&](const float* vc, int gc) {
-      float gm[4];
-      group_max4(vc, gm);
-      if (!__any_sync(0xffffffffu, fmax3(gm[0], gm[1], fmaxf(gm[2], gm[3])) > thr)) return;
-      const bool h0 = __any_sync(0xffffffffu, gm[0] > thr), h1 = __any_sync(0xffffffffu, gm[1] > thr),
-                 h2 = __any_sync(0xffffffffu, gm[2] > thr), h3 = __any_sync(0xffffffffu, gm[3] > thr);
-      // distance << 22 = (256 - dot) << 21
-      const uint32_t base = (256u << (kIdxBitsShared - 1)) + (uint32_t)gc;
-      if (h0) push_best2<0, 10, kIdxBitsShared - 1>(vc, base, k1, k2);
-      if (h1) push_best2<10, 20, kIdxBitsShared - 1>(vc, base, k1, k2);
-      if (h2) push_best2<20, 30, kIdxBitsShared - 1>(vc, base, k1, k2);
-      if (h3) push_best2<30, 40, kIdxBitsShared - 1>(vc, base, k1, k2);
-      thr = next_thr();
+    int g0 = 0;            // steps before this part
+    uint32_t sync_phase = 0;
+    // all epilogue warps: false on a timeout
+    auto epi_sync = [&]() {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(BAR_EPI);
+      const bool done = im_warp_wait(BAR_EPI, sync_phase++ & 1u, s_abort);
+      __syncwarp();
+      return done;
     };
-    const uint32_t tcol = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)set * kMAcc + (uint32_t)(part * kMChunks * kMChunk);
-    for (int i = set; i < nsteps; i += 2) {
-      const int n = i >> 1;  // this set's step
-      const int g0 = (t_beg + (two ? n : i)) * kMBN + part * kMChunks * kMChunk;
-      // bounds from the others of this block that scan the row's query (every
-      // step, while the accumulator is not full yet) and from its other splits (read in the first steps and then every
-      // fourth, used one step later): a column can reach the row's final top two
-      // only below their distance, or at it if its index can be the lower one.  (That
-      // last test matters: columns at the bound's distance are as many as those
-      // below it.)
-      {
-        heard = min(heard, asked);
-        if (gq && (n < 8 || (n & 3) == 0)) asked = __ldcg(gq);
-        uint32_t gb = heard;
-        auto others = [&](int g) { gb = min(gb, reinterpret_cast<volatile uint32_t*>(&s_k2[g][0])[row]); };
-#pragma unroll
-        for (int g = 1; g < kMParts; g++) others(kMParts * set + (part + g) % kMParts);
-        if (!two)
-#pragma unroll
-          for (int g = 0; g < kMParts; g++) others(kMParts * (set ^ 1) + g);
-        thr_gb = fmaxf(thr_gb, int_to_whole(256 - 2 * (int)(gb >> kIdxBitsShared) - ((int)(gb & kIdxMaskShared) >= g0)));
-        thr = fmaxf(thr, thr_gb);
+    long long x = x_beg, uncounted = x_beg;  // pairs before which all parts have been counted in tile_done
+    while (x < x_end) {
+    const MPart r = m_part(plan, x, x_end);
+    x += r.t1 - r.t0;
+    const bool two = nq - r.qb * kIBQ > kIBM;
+    const int nsteps = (two ? 2 : 1) * (r.t1 - r.t0);
+    int n_parts, slot;
+    m_slot(plan, slots, r.qb, r.t0, blockIdx.x, &n_parts, &slot);
+    const int first = set ^ (g0 & 1);  // this set's first step and, of two, its query tile
+    const int q = r.qb * kIBQ + (two ? first * kIBM : 0) + row;
+    // second-best bound shared by the blocks that have the query's other parts
+    ScanArgs sa;
+    sa.gq = (w.bound && n_parts > 1 && q < nq) ? w.bound + q : nullptr;
+    sa.k2_mine = smem_u32(&s_k2[me][row]);
+    sa.k2_set = smem_u32(&s_k2[kMParts * set + (part + 1) % kMParts][row]);
+    sa.k2_other = two ? 0u : smem_u32(&s_k2[kMParts * (set ^ 1)][row]);
+    sa.tcol = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)set * kMAcc + (uint32_t)(part * kMChunks * kMChunk);
+    sa.full = BAR_ACCFULL(set);
+    sa.empty = BAR_ACCEMPTY(set);
+    sa.phase = (uint32_t)((g0 + first) >> 1);
+    sa.steps = (nsteps - first + 1) >> 1;
+    sa.col = (r.t0 + (two ? 0 : first)) * kMBN + part * kMChunks * kMChunk;
+    sa.stride = two ? kMBN : 2 * kMBN;
+    sa.ndb = ndb;
+    sa.abort_flag = s_abort;
+    uint2 best;
+    ok = m_scan(sa, &best);
+    if (!ok) break;
+    g0 += nsteps;
+    // the best two of each query over the block's sets and column parts
+    s_merge[(kMParts * first + part) * kIBM + row] = best;
+    ok = epi_sync();
+    if (!ok) break;
+    s_k2[me][row] = kNoKeyShared;  // for the next part
+    const int rows = two ? kIBQ : kIBM;
+    const bool mine = e < rows && r.qb * kIBQ + e < nq;
+    if (mine) {
+      uint32_t m1 = kNoKeyShared, m2 = kNoKeyShared;
+      for (int g = 0; g < (two ? kMParts : 2 * kMParts); g++) {
+        const uint2 pk = s_merge[(two ? kMParts * (e / kIBM) + g : g) * kIBM + e % kIBM];
+        top2_push_shared(m1, m2, pk.x);
+        top2_push_shared(m1, m2, pk.y);
       }
-      ok = warp_wait(BAR_ACCFULL(set), (uint32_t)n & 1u, deadline, s_abort);
+      if (n_parts == 1)
+        finish_query_shared(a, r.qb * kIBQ + e, m1, m2);
+      else
+        reinterpret_cast<uint2*>(w.part)[(size_t)slot * w.nq_cap + r.qb * kIBQ + e] = make_uint2(m1, m2);
+    }
+    if (n_parts > 1) {
+      // the block that finishes the last part of these queries merges all parts
+      __threadfence();
+      ok = epi_sync();
       if (!ok) break;
-      tc_fence_after();
-#pragma unroll 1
-      for (int c = 0; c < kMChunks; c++) {
-        float v[kMChunk];
-        tmem_ld32(tcol + (uint32_t)(kMChunk * c), v);
-        tmem_ld8(tcol + (uint32_t)(kMChunk * c) + 32u, v + 32);
-        tmem_wait_ld40(v);
-        if (c == kMChunks - 1) {
-          // every column of this part is in registers: hand the accumulator back
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(BAR_ACCEMPTY(set));
+      if (e == 0) s_last = (atomicAdd(&w.tile_done[r.qb], 1u) == (unsigned)(n_parts - 1)) ? 1u : 0u;
+      uncounted = x;
+      ok = epi_sync();
+      if (!ok) break;
+      if (s_last) {
+        __threadfence();
+        if (e == 0) w.tile_done[r.qb] = 0u;
+        const int per = two ? kMParts : 2 * kMParts;
+        if (e < rows * per) {
+          const int qr = r.qb * kIBQ + e % rows;
+          uint32_t m1 = kNoKeyShared, m2 = kNoKeyShared;
+          if (qr < nq) {
+            const uint2* pt = reinterpret_cast<const uint2*>(w.part) + qr;
+#pragma unroll 8
+            for (int s2 = e / rows; s2 < n_parts; s2 += per) {
+              const uint2 pk = __ldcg(pt + (size_t)s2 * w.nq_cap);
+              top2_push_shared(m1, m2, pk.x);
+              top2_push_shared(m1, m2, pk.y);
+            }
+          }
+          s_merge[e] = make_uint2(m1, m2);
         }
-        const int gc = g0 + kMChunk * c;
-        if (gc + kMChunk > ndb) {
-#pragma unroll
-          for (int j = 0; j < kMChunk; j++)
-            if (gc + j >= ndb) v[j] = kMaskedDotF;
+        ok = epi_sync();
+        if (!ok) break;
+        if (mine) {
+          uint32_t m1 = kNoKeyShared, m2 = kNoKeyShared;
+          for (int g = 0; g < per; g++) {
+            const uint2 pk = s_merge[g * rows + e];
+            top2_push_shared(m1, m2, pk.x);
+            top2_push_shared(m1, m2, pk.y);
+          }
+          finish_query_shared(a, r.qb * kIBQ + e, m1, m2);
         }
-        examine(v, gc);
       }
-      if (k2 < told) {
-        told = k2;
-        reinterpret_cast<volatile uint32_t*>(&s_k2[me][0])[row] = k2;
-        // two distinct rows at or below k2: the query's final second best is no worse
-        if (gq) atomicMin(gq, k2);
-      }
+    }
+    uncounted = x;
+    ok = epi_sync();  // s_merge and s_last are free
+    if (!ok) break;
     }
     if (!ok) {
       *s_abort = 1;
       if (lane == 0) atomicOr(err, kErrImmaTimeout);
+      // the counters of the parts not finished return to zero all the same
+      if (e == 0)
+        for (long long y = uncounted; y < x_end;) {
+          const MPart r = m_part(plan, y, x_end);
+          y += r.t1 - r.t0;
+          int n_parts, slot;
+          m_slot(plan, slots, r.qb, r.t0, blockIdx.x, &n_parts, &slot);
+          if (n_parts > 1 && atomicAdd(&w.tile_done[r.qb], 1u) == (unsigned)(n_parts - 1)) w.tile_done[r.qb] = 0u;
+        }
     }
-    s_merge[me * kIBM + row] = make_uint2(k1, k2);
   }
+#undef BAR_AFULL
+#undef BAR_AEMPTY
 #undef BAR_BFULL
 #undef BAR_BEMPTY
 #undef BAR_ACCFULL
 #undef BAR_ACCEMPTY
+#undef BAR_EPI
 
   tc_fence_before();
   __syncthreads();
@@ -683,59 +872,6 @@ __global__ void __launch_bounds__(kMThreads, 1)
   if (warp == 1) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kITmemCols)
                  : "memory");
-  }
-  // the best two of each query over the block's sets and column parts
-  const int rows = two ? kIBQ : kIBM;
-  for (int r = threadIdx.x; r < rows; r += kMThreads) {
-    const int q = qb * kIBQ + r;
-    if (q >= nq) break;
-    uint32_t k1 = kNoKeyShared, k2 = kNoKeyShared;
-    for (int g = 0; g < (two ? kMParts : 2 * kMParts); g++) {
-      const uint2 pk = s_merge[(two ? kMParts * (r / kIBM) + g : g) * kIBM + r % kIBM];
-      top2_push_shared(k1, k2, pk.x);
-      top2_push_shared(k1, k2, pk.y);
-    }
-    if (splits == 1)
-      finish_query_shared(a, q, k1, k2);
-    else
-      reinterpret_cast<uint2*>(w.part)[(size_t)sp * w.nq_cap + q] = make_uint2(k1, k2);
-  }
-  if (splits == 1) return;
-  // the last block of these queries to finish merges the partial top-2 of all
-  // splits: several threads per query
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = (atomicAdd(&w.tile_done[qb], 1u) == (unsigned)(splits - 1)) ? 1u : 0u;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  if (threadIdx.x == 0) w.tile_done[qb] = 0u;
-  const int per = two ? kMParts : 2 * kMParts;
-  static_assert(2 * kMParts * kIBM <= kMThreads, "one thread per entry of s_merge");
-  if (threadIdx.x < rows * per) {
-    const int r = threadIdx.x % rows, g = threadIdx.x / rows;
-    const int q = qb * kIBQ + r;
-    uint32_t m1 = kNoKeyShared, m2 = kNoKeyShared;
-    if (q < nq) {
-      const uint2* part = reinterpret_cast<const uint2*>(w.part) + q;
-#pragma unroll 8
-      for (int s2 = g; s2 < splits; s2 += per) {
-        const uint2 pk = __ldcg(part + (size_t)s2 * w.nq_cap);
-        top2_push_shared(m1, m2, pk.x);
-        top2_push_shared(m1, m2, pk.y);
-      }
-    }
-    s_merge[g * rows + r] = make_uint2(m1, m2);
-  }
-  __syncthreads();
-  if (threadIdx.x < rows && qb * kIBQ + (int)threadIdx.x < nq) {
-    uint32_t m1 = kNoKeyShared, m2 = kNoKeyShared;
-    for (int g = 0; g < per; g++) {
-      const uint2 pk = s_merge[g * rows + threadIdx.x];
-      top2_push_shared(m1, m2, pk.x);
-      top2_push_shared(m1, m2, pk.y);
-    }
-    finish_query_shared(a, qb * kIBQ + (int)threadIdx.x, m1, m2);
   }
 }
 
@@ -1264,24 +1400,11 @@ static bool make_rows_map(CUtensorMap* m, const void* base, uint64_t rows, uint3
 int imma_rows_q(int n) { return (n + kIBM - 1) / kIBM * kIBM; }
 int imma_rows_db(int n) { return (n + kMBN - 1) / kMBN * kMBN; }
 
-// Database splits per 256 queries: of the grids up to 64 splits the one with the
-// least time, whole waves of 148 blocks (one 200 KB block per SM) whose time is
-// their database tiles plus about 10 tiles' worth for starting, finding the first
-// bounds and merging.  65536 x 65536: 256 query tiles x 4 splits; 16384 x 32768:
-// 64 x 2, 122 us against 244 with 64 x 16.
-int imma_default_splits(int nq_cap, int ndb) {
-  const long long qt = (nq_cap + kIBQ - 1) / kIBQ;
-  const int tiles = std::max(1, (ndb + kMBN - 1) / kMBN);
-  int best = 1;
-  double best_cost = 1e300;
-  for (int s = 1; s <= std::min(kImmaMaxSplits, tiles); s++) {
-    const double cost = (double)((qt * s + 147) / 148) * ((double)tiles / s + 10.0);
-    if (cost < best_cost) {
-      best_cost = cost;
-      best = s;
-    }
-  }
-  return best;
+// Slots in which the parts of nq queries' searches fit when every SM has a block
+// (m_plan): up to max_slots.
+int imma_slots(int nq, int ndb, int max_slots) {
+  const MPlan p = m_plan(nq, ndb, 1 << 20, 148);
+  return std::max(1, std::min(max_slots, 148 / std::max(1, p.qtiles) + 1 + 2 * p.panels));
 }
 
 cudaError_t launch_expand_pm1(const uint8_t* bits, int n, const int* d_n, int rows, uint8_t* out, cudaStream_t s) {
@@ -1312,10 +1435,9 @@ cudaError_t launch_match_imma(const ImmaLaunch& L, cudaStream_t s) {
   CUtensorMap tq, td;
   if (!make_rows_map(&tq, L.q_pm1, (uint64_t)qrows, kIBM)) return cudaErrorInvalidValue;
   if (!make_rows_map(&td, L.db_pm1, (uint64_t)dbrows, kMBN)) return cudaErrorInvalidValue;
-  const int qtiles = (L.nq_cap + kIBQ - 1) / kIBQ;
-  const int splits = std::max(1, std::min(L.splits, dbrows / kMBN));
-  return launch_chained_smem(k_match_imma, qtiles * splits, kMThreads, kISmemBytes, s, tq, td, L.args, L.work, splits,
-                             L.err);
+  const int slots = L.work.part && L.work.tile_done ? L.slots : 1;
+  const int grid = m_plan(L.nq_cap, std::max(L.ndb_cap, 0), slots, 148).grid;
+  return launch_chained_smem(k_match_imma, grid, kMThreads, kISmemBytes, s, tq, td, L.args, L.work, slots, L.err);
 }
 
 cudaError_t launch_rerank_imma(const RerankImmaArgs& a, int max_items, cudaStream_t s) {
