@@ -216,7 +216,7 @@ cudaError_t launch_match_imma(const ImmaLaunch& L, cudaStream_t s);
 // Probe rerank of the learned proposal on the int8 tensor cores
 // (orbx_match_imma.cu): per (cluster, up to 128 probing slots), the exact top-2
 // keys of each slot over the cluster's rows, one pair per 64-column group.
-constexpr int kRrGroups = 4;
+constexpr int kRrGroups = 2;
 struct RerankImmaArgs {
   const uint8_t* q_bits;     // [nq][32] queries
   const int* list;           // probing slots grouped by cluster (slot = query * 8 + probe)

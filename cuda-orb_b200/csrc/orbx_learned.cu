@@ -11,6 +11,7 @@
 #include "orbx_device.cuh"
 #include "orbx_internal.cuh"
 #include "orbx_learned.cuh"
+#include "orbx_match_plan.cuh"
 
 namespace orbx {
 
@@ -754,10 +755,10 @@ __global__ void __launch_bounds__(1024) k_probe_pairs(const int* __restrict__ pr
 }
 
 // ---------------------------------------------------------------- padded lists
-// Rows per cluster rounded up to the tensor-core rerank's 256-row tile.
+// Rows per cluster rounded up to the tensor-core rerank's tile.
 __global__ void k_pad_counts(const int* __restrict__ ivf_offsets, int C, int* __restrict__ pad_counts) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < C) pad_counts[c] = (ivf_offsets[c + 1] - ivf_offsets[c] + 255) / 256 * 256;
+  if (c < C) pad_counts[c] = (ivf_offsets[c + 1] - ivf_offsets[c] + kPlanRows - 1) / kPlanRows * kPlanRows;
 }
 
 // Cluster c's padded rows [pad_offsets[c], pad_offsets[c + 1]): its list's

@@ -179,7 +179,7 @@ struct orbx_learned {
   int* ivf_offsets = nullptr;
   int* ivf_members = nullptr;
   uint8_t* ivf_desc = nullptr;
-  // the lists padded per cluster to 256-row tiles (packed rows), for the tensor-core rerank
+  // the lists padded per cluster to whole tiles (packed rows), for the tensor-core rerank
   int pad_rows = 0;
   int* pad_offsets = nullptr;
   int* pad_members = nullptr;

@@ -51,7 +51,6 @@ namespace orbx {
 constexpr int kIBM = 128;  // queries per query tile (MMA M)
 constexpr int kIBQ = kPlanQueries;  // queries per block of k_match_imma
 static_assert(kIBQ == 2 * kIBM, "two query tiles");
-constexpr int kIBN = 256;  // database rows per tile of k_rerank_imma (MMA N)
 constexpr int kMBN = kPlanRows;  // database rows per tile of k_match_imma: two accumulators leave TMEM columns for the scales
 constexpr int kMChunk = 60;           // columns an epilogue warp examines at a time,
 constexpr int kMGroups = 4;           // in so many groups
@@ -60,11 +59,7 @@ constexpr int kMChunks = kMBN / (kMChunk * kMParts);  // chunks of one of them p
 constexpr int kMEpiWarps = 2 * 4 * kMParts;
 constexpr int kMThreads = (2 + kMEpiWarps) * 32;
 constexpr int kMStages = 4;
-constexpr int kIEpiWarps = 16;  // of k_rerank_imma
-constexpr uint32_t kIHalfA = kIBM * 128;  // one 128-byte-wide K half of the query tile
-constexpr uint32_t kIHalfB = kIBN * 128;
-constexpr uint32_t kIATile = 2 * kIHalfA;
-constexpr uint32_t kIBTile = 2 * kIHalfB;
+constexpr int kIEpiWarps = 8;  // of k_rerank_imma
 constexpr uint32_t kMATile = kIBM * kPm1RowBytes;  // one 128-byte swizzle row per descriptor
 constexpr uint32_t kMBTile = kMBN * kPm1RowBytes;
 static_assert(kPm1RowBytes == 128 && kMBTile % 1024 == 0, "whole swizzle atoms");
@@ -81,10 +76,7 @@ static_assert(kISmemBytes + 16 + 2 * kMParts * kIBM * 4 <= 232448, "exceeds the 
 constexpr uint32_t kITmemCols = 512;
 constexpr long long kIDeadlineCycles = 4000000000ll;  // ~2 s at 2 GHz
 
-// instruction descriptor: S32 accumulate, S8 x S8, both K-major, N = 256, M = 128
-constexpr uint32_t kIDesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kIBN >> 3) << 17) |
-                            ((uint32_t)(kIBM >> 4) << 24);
-// the same for kind::mxf4: E2M1 x E2M1, UE8M0 scales, both K-major, N = 240, M = 128, K = 64
+// instruction descriptor for kind::mxf4: E2M1 x E2M1, UE8M0 scales, both K-major, N = 240, M = 128, K = 64
 constexpr uint32_t kMDesc = (1u << 7) | (1u << 10) | ((uint32_t)(kMBN >> 3) << 17) | (1u << 23) |
                             ((uint32_t)(kIBM >> 7) << 27);
 
@@ -144,16 +136,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
-  const uint32_t mask0 = 0, mask1 = 0, mask2 = 0, mask3 = 0;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(tmem_d),
-      "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(mask0), "r"(mask1), "r"(mask2), "r"(mask3)
-      : "memory");
-}
-
 // One K = 64 step on 4-bit floats with one scale per 32 values (all 1, at sfa and sfb).
 __device__ __forceinline__ void umma_f4(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t sfa,
                                         uint32_t sfb, uint32_t acc) {
@@ -184,110 +166,7 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// The same wait for 32 registers being loaded: as its operands they cannot be
-// read before it.
-__device__ __forceinline__ void tmem_wait_ld32(int* v) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
-                 "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]),
-                 "+r"(v[15]), "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]),
-                 "+r"(v[22]), "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]),
-                 "+r"(v[29])
-               :
-               : "memory");
-  asm volatile("" : "+r"(v[30]), "+r"(v[31])::"memory");
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, int* v) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-        "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-        "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr));
-}
-
-// Dot value given to database columns past the end of the set (never selected:
-// below every dot product, -256 .. 256).
-constexpr int kMaskedDot = -400;
-
-// Three-input max of float bit patterns, without flushing denormals.
-__device__ __forceinline__ float fmax3_bits(float a, float b, float c) {
-  float r;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-
-// Maxima of the column groups 0-8, 9-17, 18-26 and 27-31 of a 32-column chunk,
-// for comparison with a threshold >= 0: the values are reduced as float bit
-// patterns by three-input max (a non-negative int32 is a zero or denormal float
-// and keeps its order, a negative one is a NaN, which max ignores).
-__device__ __forceinline__ void group_max4(const int* v, float* r) {
-  float m[12];
-#pragma unroll
-  for (int i = 0; i < 10; i++)
-    m[i] = fmax3_bits(__int_as_float(v[3 * i]), __int_as_float(v[3 * i + 1]), __int_as_float(v[3 * i + 2]));
-  m[10] = __int_as_float(v[30]);
-  m[11] = __int_as_float(v[31]);
-  r[0] = fmax3_bits(m[0], m[1], m[2]);
-  r[1] = fmax3_bits(m[3], m[4], m[5]);
-  r[2] = fmax3_bits(m[6], m[7], m[8]);
-  r[3] = fmax3_bits(m[9], m[10], m[11]);
-}
-// Whether a group maximum from group_max4 exceeds thr >= 0, compared as floats
-// (a NaN maximum means every value of the group was negative).
-__device__ __forceinline__ bool bits_exceed(float r, int thr) { return r > __int_as_float(thr); }
-
-// The best two of columns B .. E-1 of a chunk as local keys u = column - (dot <<
-// SH), least first, so ties keep the lower column: a tournament of minima (its
-// depth, not its 23 operations for ten columns, is what a warp waits for).
-template <int B, int E, int SH>
-__device__ __forceinline__ void chunk_best2(const int* vc, int& u1, int& u2) {
-  constexpr int n = E - B, h = n / 2;
-  int a1[h], a2[h];
-#pragma unroll
-  for (int i = 0; i < h; i++) {
-    const int x = vc[B + 2 * i] * -(1 << SH) + (B + 2 * i), y = vc[B + 2 * i + 1] * -(1 << SH) + (B + 2 * i + 1);
-    a1[i] = min(x, y);
-    a2[i] = max(x, y);
-  }
-#pragma unroll
-  for (int d = 1; d < h; d *= 2)
-#pragma unroll
-    for (int i = 0; i + d < h; i += 2 * d) {
-      a2[i] = __vimin3_s32(max(a1[i], a1[i + d]), a2[i], a2[i + d]);
-      a1[i] = min(a1[i], a1[i + d]);
-    }
-  u1 = a1[0];
-  u2 = a2[0];
-  if constexpr (n & 1) {
-    const int x = vc[E - 1] * -(1 << SH) + (E - 1);
-    u2 = min(u2, max(u1, x));
-    u1 = min(u1, x);
-  }
-}
-// Those two merged into the running best two keys (distance << 22 | index): base
-// is the key of a zero dot product at the chunk's column 0, and a value of one
-// takes 1 << SH off; the values are dot products times 1 << SCALE.  Masked columns
-// carry no key.
-template <int B, int E, int SH, int SCALE = 0>
-__device__ __forceinline__ void chunk_top2_push(const int* vc, uint32_t base, uint32_t& k1, uint32_t& k2) {
-  static_assert(kMaskedDot == -400 && SH + SCALE <= 22, "the masked key is an int above every other (256 << 22)");
-  constexpr int kMaskedU = (int)((uint32_t)(-kMaskedDot - 1) << (SH + SCALE));
-  int u1, u2;
-  chunk_best2<B, E, SH>(vc, u1, u2);
-  const uint32_t p1 = u1 >= kMaskedU ? kNoKeyShared : base + (uint32_t)u1;
-  const uint32_t p2 = u2 >= kMaskedU ? kNoKeyShared : base + (uint32_t)u2;
-  k2 = __vimin3_u32(max(k1, p1), k2, p2);
-  k1 = min(k1, p1);
-}
-
-// ---- the same on fp32 accumulators (k_match_imma) ----------------------------
+// ---- reading and comparing the fp32 accumulators -----------------------------
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -881,47 +760,51 @@ __global__ void __launch_bounds__(kMThreads, 1)
 // A work item is one cluster c with up to 128 of the query slots that probe it
 // (list[probe_offsets[c] ..], grouped by cluster; slot = query * 8 + probe).
 // The cluster's rows are kept packed (32 bytes each, padded per cluster to
-// 256-row tiles) and expanded in shared memory, so HBM carries an eighth of
+// 240-row tiles) and expanded in shared memory, so HBM carries a quarter of
 // the bytes expanded rows would.  The blocks are persistent and claim items
 // from a global counter (items differ widely in size); the producer thread
 // claims them and passes them to the other roles through a small queue:
-//   warp 0      producer: each tile's 8 KB of packed rows by cp.async.bulk
+//   warp 0      producer: each tile's packed rows by cp.async.bulk
 //               into a 4-stage ring;
-//   warp 1      MMA issuer, as in k_match_imma, into two 256-column
+//   warp 1      MMA issuer, as in k_match_imma, into two 240-column
 //               accumulators; commits release the expanded stage, the
 //               accumulator and, after an item's last tile, its query tile;
 //   warps 2-9   expanders: at an item's start they gather its slots' queries
 //               as signed rows (two threads per row) into one of two query tiles,
-//               then expand each packed tile to masked rows into one of two
+//               then expand each packed tile to masked rows into a ring of four
 //               database tiles, one row per thread, in the 128-byte swizzled
-//               K-major layout the TMA writes (rr_db_word);
-//   warps 10-25 epilogue: warp w reads TMEM lanes 32 * (w % 4) and 64 columns,
+//               K-major layout the TMA writes (rr_db_chunk);
+//   warps 10-17 epilogue: warp w reads TMEM lanes 32 * (w % 4) and 120 columns,
 //               keeps the top-2 keys (distance << 22 | database index) of each
 //               slot over the item's tiles (distance = popcount(query) - dot')
-//               and writes them to partial[slot * 4 + column group].
+//               and writes them to partial[slot * 2 + column group].
 // Each cluster's list is in increasing database index, so column order is
 // index order and ties resolve as in the other matchers.  Every wait is bounded (kIDeadlineCycles per
 // wait); on expiry the block records kErrImmaTimeout, drains its copies and
 // exits.
 //
-// What bounds it: the ALU (expansion and the epilogue's tests; the tensor pipe is
-// active 30% of the time).  32768 queries, 8 probes in 512 lists of about 2048
-// rows: 372 us at 11400 warp instructions per 256-row tile, 306 us with the
-// tournament updates, 245 us with the masked expansion (rr_db_word) and the
-// query's shared bound read one tile ahead.
+// What bounds it: the ALU (expansion and the epilogue's tests).  32768 queries, 8
+// probes in 512 lists of about 2048 rows: 372 us with one candidate after another,
+// 306 us with the tournament updates, 245 us with the expansion by masks to int8 and
+// the query's shared bound read one tile ahead, 206 us with 4-bit floats, which halve
+// the expansion's stores, 203 us with 8 epilogue warps that hold 60 columns each
+// instead of 16 with 32 (and half the results to merge: 12.3 -> 8.6 us there).
 // ---------------------------------------------------------------------------
 constexpr int kRrExpWarps = 8;
 constexpr int kRrThreads = (2 + kRrExpWarps + kIEpiWarps) * 32;
 constexpr uint32_t kRrPStages = 4;
-constexpr uint32_t kRrPTile = kIBN * 32;  // packed rows of one tile
+constexpr uint32_t kRrXStages = 4;  // expanded database tiles
+constexpr uint32_t kRrPTile = kMBN * 32;  // packed rows of one tile
 constexpr uint32_t kRrQueue = 8;  // claimed items in flight between the producer and the other roles
-constexpr uint32_t kRrNumBars = 2 + 2 + 2 * kRrPStages + 2 + 2 + 2 + 2 + 2 * kRrQueue;
+constexpr uint32_t kRrNumBars = 2 + 2 + 2 * kRrPStages + 2 * kRrXStages + 2 + 2 + 2 * kRrQueue;
 // the item queue's consumers: the MMA thread, the expander and the epilogue warps
 constexpr uint32_t kRrQueueReaders = 1 + kRrExpWarps + kIEpiWarps;
 constexpr uint32_t kRrSmemBytes =
-    1024 + 2 * kIATile + 2 * kIBTile + kRrPStages * kRrPTile + 8 * kRrNumBars + 4 * kRrQueue + 16;
+    1024 + 2 * kMATile + kRrXStages * kMBTile + kRrPStages * kRrPTile + 8 * kRrNumBars + 4 * kRrQueue + 16;
 static_assert(kRrSmemBytes + 16 <= 232448, "exceeds the 227 KB shared-memory opt-in");
-static_assert(kRrExpWarps * 32 == kIBN && kRrExpWarps * 32 == 2 * kIBM, "one expander thread per row, two per query");
+static_assert(kRrExpWarps * 32 >= kMBN && kRrExpWarps * 32 == 2 * kIBM, "one expander thread per row, two per query");
+constexpr int kRrCols = kMBN / kRrGroups;  // columns of an epilogue warp
+constexpr int kRrChunk = 60;               // examined at a time
 
 struct RrItem {
   int c;      // cluster
@@ -945,7 +828,7 @@ __device__ __forceinline__ RrItem rr_item(const RerankImmaArgs& a, int it) {
   r.rows = min(kIBM, __ldg(a.probe_offsets + lo + 1) - r.e0);
   r.nrow = __ldg(a.ivf_offsets + lo + 1) - __ldg(a.ivf_offsets + lo);
   r.pbase = __ldg(a.pad_offsets + lo);
-  r.tiles = (r.nrow + kIBN - 1) / kIBN;
+  r.tiles = (r.nrow + kMBN - 1) / kMBN;
   return r;
 }
 
@@ -962,34 +845,25 @@ __device__ __forceinline__ bool rr_warp_wait(uint32_t bar, uint32_t parity, vola
 
 // The order of the 256 products of a dot product is free, and so is how a weight
 // is shared between its factors; both are chosen so that a database row's packed
-// words expand by masking alone.  Output word k (k = 0 .. 7) of a packed word
-// holds its bits k, 8 + k, 16 + k, 24 + k in place, i.e. bytes of 0 or 2^k (bit 7
-// shifted down once: 0 or 64), and the query's bytes are +-2^(6 - k) (+-1 for bit
-// 7): every product is 64 times the query's sign where the row has a one, the
-// accumulator is 64 dot' exactly, and Hamming(q, row) = popcount(q) - dot'.
-// 72 operations per row, against 192 for bytes of 0 and 1 in bit order.
-constexpr int kRrScaleLog = 6;
-__device__ __forceinline__ uint32_t rr_db_word(uint32_t w, int k) {
-  return k < 7 ? w & (0x01010101u << k) : (w >> 1) & 0x40404040u;
+// words expand by masking alone.  Output word k (k = 0 .. 3) of a packed word holds
+// its bits k, 4 + k, 8 + k .. in place, i.e. nibbles of 0 or 1 << k: 0.5, 1 or 2 as
+// e2m1 (bit 3, the sign, is shifted down to 0.5).  The query's values are +-2, +-1,
+// +-0.5 and +-2: every product is the query's sign where the row has a one, the
+// accumulator is dot' and Hamming(q, row) = popcount(q) - dot'.  40 operations and
+// eight stores per row.
+__device__ __forceinline__ uint4 rr_db_chunk(uint32_t w) {
+  return make_uint4(w & 0x11111111u, w & 0x22222222u, w & 0x44444444u, (w >> 3) & 0x11111111u);
 }
-__device__ __forceinline__ uint32_t rr_query_word(uint32_t w, int k) {
-  const uint32_t m = k < 7 ? 1u << (6 - k) : 1u, neg = 256u - m;
-  return (neg * 0x01010101u) ^ (((w >> k) & 0x01010101u) * (m ^ neg));
+__device__ __forceinline__ uint32_t rr_query_word(uint32_t w, int k, uint32_t code) {
+  return (code * 0x11111111u) | ((~(w >> k) & 0x11111111u) << 3);
 }
-// 16-byte chunk cc of a row: output words 4 (cc & 1) .. + 3 of packed word w = words[cc >> 1].
-__device__ __forceinline__ uint4 rr_db_chunk(uint32_t w, int cc) {
-  const int k = 4 * (cc & 1);
-  return make_uint4(rr_db_word(w, k), rr_db_word(w, k + 1), rr_db_word(w, k + 2), rr_db_word(w, k + 3));
-}
-__device__ __forceinline__ uint4 rr_query_chunk(uint32_t w, int cc) {
-  const int k = 4 * (cc & 1);
-  return make_uint4(rr_query_word(w, k), rr_query_word(w, k + 1), rr_query_word(w, k + 2), rr_query_word(w, k + 3));
+__device__ __forceinline__ uint4 rr_query_chunk(uint32_t w) {
+  return make_uint4(rr_query_word(w, 0, 4u), rr_query_word(w, 1, 2u), rr_query_word(w, 2, 1u), rr_query_word(w, 3, 4u));
 }
 
-// Swizzled address of chunk cc of row r in a K-major tile of `rows` rows
-// (two 128-byte K halves, each rows x 128 bytes).
-__device__ __forceinline__ uint8_t* sw128_chunk(uint8_t* tile, uint32_t half_bytes, int r, int cc) {
-  return tile + (cc >> 3) * half_bytes + r * 128 + (((cc & 7) ^ (r & 7)) << 4);
+// Swizzled address of 16-byte chunk cc of row r in a K-major tile of 128-byte rows.
+__device__ __forceinline__ uint8_t* sw128_chunk(uint8_t* tile, int r, int cc) {
+  return tile + r * 128 + ((cc ^ (r & 7)) << 4);
 }
 
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -1009,13 +883,40 @@ __device__ __forceinline__ bool rr_next_item(uint32_t qfull, uint32_t qempty, vo
   return true;
 }
 
+// A chunk of N columns, rows col0 .. of the cluster's nrow, against a lane's best two
+// keys (distance = pc - dot').  The columns arrive in list order, so only a strictly
+// larger dot' than the current second best's can enter, and no column farther than
+// the second best that another item of the same query holds (equal distances stay,
+// their index decides).
+template <int N>
+__device__ __forceinline__ void rr_examine(float* v, int col0, int nrow, int pc, float thr_gb, uint32_t& k1,
+                                           uint32_t& k2) {
+  constexpr int kGroups = 4, kSize = N / kGroups;
+  if (nrow - col0 < N) {
+#pragma unroll
+    for (int j = 0; j < N; j++)
+      if (j >= nrow - col0) v[j] = kMaskedDotF;
+  }
+  // (no key yet: below every dot')
+  const float thr = fmaxf(int_to_whole(pc - (int)(k2 >> kIdxBitsShared)), thr_gb);
+  float gm[kGroups];
+#pragma unroll
+  for (int g = 0; g < kGroups; g++) gm[g] = max_of<kSize>(v + kSize * g);
+  if (!__any_sync(0xffffffffu, max_of<kGroups>(gm) > thr)) return;
+  bool hit[kGroups];
+#pragma unroll
+  for (int g = 0; g < kGroups; g++) hit[g] = __any_sync(0xffffffffu, gm[g] > thr);
+  push_groups<kSize, kIdxBitsShared>(v, hit, ((uint32_t)pc << kIdxBitsShared) + (uint32_t)col0, k1, k2,
+                                     std::make_integer_sequence<int, kGroups>());
+}
+
 __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
   uint8_t* sA = smem;               // two query tiles
-  uint8_t* sX = sA + 2 * kIATile;   // two expanded database tiles
-  uint8_t* sP = sX + 2 * kIBTile;   // ring of packed database tiles
+  uint8_t* sX = sA + 2 * kMATile;   // ring of expanded database tiles
+  uint8_t* sP = sX + kRrXStages * kMBTile;   // ring of packed database tiles
   uint64_t* bars = reinterpret_cast<uint64_t*>(sP + kRrPStages * kRrPTile);
   volatile int* s_queue = reinterpret_cast<volatile int*>(bars + kRrNumBars);
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(const_cast<int*>(s_queue) + kRrQueue);
@@ -1031,20 +932,23 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
 #define RR_PFULL(s) (bar0 + 8u * (4 + (s)))
 #define RR_PEMPTY(s) (bar0 + 8u * (4 + kRrPStages + (s)))
 #define RR_XFULL(x) (bar0 + 8u * (4 + 2 * kRrPStages + (x)))
-#define RR_XEMPTY(x) (bar0 + 8u * (6 + 2 * kRrPStages + (x)))
-#define RR_ACCFULL(x) (bar0 + 8u * (8 + 2 * kRrPStages + (x)))
-#define RR_ACCEMPTY(x) (bar0 + 8u * (10 + 2 * kRrPStages + (x)))
-#define RR_QFULL(k) (bar0 + 8u * (12 + 2 * kRrPStages + (k)))
-#define RR_QEMPTY(k) (bar0 + 8u * (12 + 2 * kRrPStages + kRrQueue + (k)))
+#define RR_XEMPTY(x) (bar0 + 8u * (4 + 2 * kRrPStages + kRrXStages + (x)))
+#define RR_REST (4 + 2 * kRrPStages + 2 * kRrXStages)
+#define RR_ACCFULL(x) (bar0 + 8u * (RR_REST + (x)))
+#define RR_ACCEMPTY(x) (bar0 + 8u * (RR_REST + 2 + (x)))
+#define RR_QFULL(k) (bar0 + 8u * (RR_REST + 4 + (k)))
+#define RR_QEMPTY(k) (bar0 + 8u * (RR_REST + 4 + kRrQueue + (k)))
 
   if (threadIdx.x == 0) {
     for (int b = 0; b < 2; b++) {
       mbar_init(RR_AFULL(b), kRrExpWarps);
       mbar_init(RR_AEMPTY(b), 1);
-      mbar_init(RR_XFULL(b), kRrExpWarps);
-      mbar_init(RR_XEMPTY(b), 1);
       mbar_init(RR_ACCFULL(b), 1);
       mbar_init(RR_ACCEMPTY(b), kIEpiWarps);
+    }
+    for (uint32_t x = 0; x < kRrXStages; x++) {
+      mbar_init(RR_XFULL(x), kRrExpWarps);
+      mbar_init(RR_XEMPTY(x), 1);
     }
     for (uint32_t st = 0; st < kRrPStages; st++) {
       mbar_init(RR_PFULL(st), 1);
@@ -1068,6 +972,12 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *s_tmem;
+  // the scales of both operands, before the first MMA: four warps, one per 32 lanes
+  if (warp >= 2 + kRrExpWarps && warp < 6 + kRrExpWarps)
+    tmem_store_unit_scales(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kMScaleCol);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -1097,7 +1007,7 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
             break;
           }
           mbar_expect_tx(RR_PFULL(st), kRrPTile);
-          bulk_load(smem_u32(sP + st * kRrPTile), a.pad_desc + (size_t)(r.pbase + t * kIBN) * 32, kRrPTile,
+          bulk_load(smem_u32(sP + st * kRrPTile), a.pad_desc + (size_t)(r.pbase + t * kMBN) * 32, kRrPTile,
                     RR_PFULL(st));
           issued[st]++;
         }
@@ -1140,26 +1050,23 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
           ok = false;
           break;
         }
-        const uint32_t a_lo = smem_u32(sA + b * kIATile);
+        const uint64_t da = sw128_desc(smem_u32(sA + b * kMATile));
+        const uint32_t sfa = tmem_base + kMScaleCol, sfb = sfa + kMScaleCols / 2;
         for (int t = 0; t < r.tiles; t++, g++) {
-          const uint32_t x = g & 1u;
-          if (!rr_wait(RR_XFULL(x), (g >> 1) & 1u, s_abort) ||
-              (g >= 2 && !rr_wait(RR_ACCEMPTY(x), ((g >> 1) - 1) & 1u, s_abort))) {
+          const uint32_t x = g % kRrXStages, acc = g & 1u;
+          if (!rr_wait(RR_XFULL(x), (g / kRrXStages) & 1u, s_abort) ||
+              (g >= 2 && !rr_wait(RR_ACCEMPTY(acc), ((g >> 1) - 1) & 1u, s_abort))) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t d = tmem_base + x * (uint32_t)kIBN;
-          const uint32_t b_lo = smem_u32(sX + x * kIBTile);
+          const uint32_t d = tmem_base + acc * kMAcc;
+          const uint64_t db = sw128_desc(smem_u32(sX + x * kMBTile));
 #pragma unroll
-          for (int k = 0; k < 8; k++) {
-            const int h = k >> 2, kk = k & 3;
-            const uint64_t da = sw128_desc(a_lo + h * kIHalfA) + (uint64_t)(2 * kk);
-            const uint64_t db = sw128_desc(b_lo + h * kIHalfB) + (uint64_t)(2 * kk);
-            umma_i8(d, da, db, kIDesc, k > 0 ? 1u : 0u);
-          }
+          for (int k = 0; k < 4; k++)
+            umma_f4(d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), kMDesc, sfa, sfb, k > 0 ? 1u : 0u);
           umma_commit(RR_XEMPTY(x));
-          umma_commit(RR_ACCFULL(x));
+          umma_commit(RR_ACCFULL(acc));
         }
         if (!ok) break;
         umma_commit(RR_AEMPTY(b));
@@ -1200,12 +1107,11 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
           w = __ldg(reinterpret_cast<const uint4*>(a.q_bits) + 2 * (size_t)q + half);
         }
         const uint32_t wd[4] = {w.x, w.y, w.z, w.w};
-        uint8_t* tile = sA + b * kIATile;
+        uint8_t* tile = sA + b * kMATile;
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-          const int cc = 8 * half + j;
-          const uint4 v = (r < ri.rows) ? rr_query_chunk(wd[j >> 1], cc) : make_uint4(0u, 0u, 0u, 0u);
-          *reinterpret_cast<uint4*>(sw128_chunk(tile, kIHalfA, r, cc)) = v;
+        for (int j = 0; j < 4; j++) {
+          const uint4 v = (r < ri.rows) ? rr_query_chunk(wd[j]) : make_uint4(0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(sw128_chunk(tile, r, 4 * half + j)) = v;
         }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1214,19 +1120,20 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
       na++;
       // the item's database tiles: row e of each
       for (int t = 0; t < ri.tiles; t++, g++) {
-        const uint32_t st = g % kRrPStages, x = g & 1u;
+        const uint32_t st = g % kRrPStages, x = g % kRrXStages;
         if (!rr_warp_wait(RR_PFULL(st), (g / kRrPStages) & 1u, s_abort) ||
-            (g >= 2 && !rr_warp_wait(RR_XEMPTY(x), ((g >> 1) - 1) & 1u, s_abort))) {
+            (g >= kRrXStages && !rr_warp_wait(RR_XEMPTY(x), (g / kRrXStages - 1) & 1u, s_abort))) {
           ok = false;
           break;
         }
-        const uint4* src = reinterpret_cast<const uint4*>(sP + st * kRrPTile) + 2 * e;
-        const uint4 w0 = src[0], w1 = src[1];
-        const uint32_t wd[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-        uint8_t* tile = sX + x * kIBTile;
+        if (e < kMBN) {
+          const uint4* src = reinterpret_cast<const uint4*>(sP + st * kRrPTile) + 2 * e;
+          const uint4 w0 = src[0], w1 = src[1];
+          const uint32_t wd[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+          uint8_t* tile = sX + x * kMBTile;
 #pragma unroll
-        for (int cc = 0; cc < 16; cc++)
-          *reinterpret_cast<uint4*>(sw128_chunk(tile, kIHalfB, e, cc)) = rr_db_chunk(wd[cc >> 1], cc);
+          for (int cc = 0; cc < 8; cc++) *reinterpret_cast<uint4*>(sw128_chunk(tile, e, cc)) = rr_db_chunk(wd[cc]);
+        }
         // The packed stage is released here, not right after its loads: the stores
         // and the fence have waited for them, and a copy (async proxy) issued before
         // they were complete replaced words still to be read (one tile in about
@@ -1274,9 +1181,8 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
       // cluster: the cluster's list is in increasing database index, so they order
       // like keys of database indices, into which they are turned at the end
       uint32_t k1 = kNoKeyShared, k2 = kNoKeyShared;
-      const uint32_t bias = (uint32_t)pc << kIdxBitsShared;
       uint32_t asked = slot >= 0 ? __ldcg(a.q_bound + (slot >> 3)) : kNoKeyShared;
-      int thr_gb = kMaskedDot;
+      float thr_gb = kMaskedDotF;
       for (int t = 0; t < ri.tiles; t++, g++) {
         const uint32_t acc = g & 1u;
         if (!rr_warp_wait(RR_ACCFULL(acc), (g >> 1) & 1u, s_abort)) {
@@ -1286,50 +1192,21 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
         tc_fence_after();
         // the query's bound from its other items so far (any stale value is a valid,
         // looser bound): read while the tile before was examined
-        if (asked != kNoKeyShared) thr_gb = max(thr_gb, pc - (int)(asked >> kIdxBitsShared) - 1);
+        if (asked != kNoKeyShared) thr_gb = fmaxf(thr_gb, int_to_whole(pc - (int)(asked >> kIdxBitsShared) - 1));
         if (slot >= 0) asked = __ldcg(a.q_bound + (slot >> 3));
-        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * (uint32_t)kIBN + colgrp * 64;
-#pragma unroll 1
-        for (int c = 0; c < 2; c++) {
-          int v[32];
-          tmem_ld32(taddr + 32u * c, v);
-          tmem_wait_ld32(v);
-          if (c == 1) {
-            // every column of this group is in registers: hand the accumulator back
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(RR_ACCEMPTY(acc));
-          }
-          const int col0 = t * kIBN + colgrp * 64 + 32 * c;  // first column's row within the cluster
-          const int valid = ri.nrow - col0;
-          if (valid < 32) {
-#pragma unroll
-            for (int j = 0; j < 32; j++)
-              if (j >= valid) v[j] = kMaskedDot * (1 << kRrScaleLog);
-          }
-          // The columns arrive in list order, so only a strictly larger dot' (a
-          // strictly smaller distance) than the current second best's can enter,
-          // and no column farther than the second best that another item of the
-          // same query holds (equal distances stay, their index decides)
-          // (no key yet: below every dot')
-          const int thr = (1 << kRrScaleLog) * max(pc - (int)(k2 >> kIdxBitsShared), thr_gb);
-          bool h0 = true, h1 = true, h2 = true, h3 = true;
-          if (__all_sync(0xffffffffu, thr >= 0)) {
-            float gm[4];
-            group_max4(v, gm);
-            const float cm = fmax3_bits(gm[0], gm[1], fmax3_bits(gm[2], gm[3], gm[3]));
-            if (!__any_sync(0xffffffffu, bits_exceed(cm, thr))) continue;
-            h0 = __any_sync(0xffffffffu, bits_exceed(gm[0], thr));
-            h1 = __any_sync(0xffffffffu, bits_exceed(gm[1], thr));
-            h2 = __any_sync(0xffffffffu, bits_exceed(gm[2], thr));
-            h3 = __any_sync(0xffffffffu, bits_exceed(gm[3], thr));
-          }
-          const uint32_t base = bias + (uint32_t)col0;
-          if (h0) chunk_top2_push<0, 9, kIdxBitsShared - kRrScaleLog, kRrScaleLog>(v, base, k1, k2);
-          if (h1) chunk_top2_push<9, 18, kIdxBitsShared - kRrScaleLog, kRrScaleLog>(v, base, k1, k2);
-          if (h2) chunk_top2_push<18, 27, kIdxBitsShared - kRrScaleLog, kRrScaleLog>(v, base, k1, k2);
-          if (h3) chunk_top2_push<27, 32, kIdxBitsShared - kRrScaleLog, kRrScaleLog>(v, base, k1, k2);
-        }
+        const uint32_t taddr =
+            tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * kMAcc + (uint32_t)(colgrp * kRrCols);
+        const int col0 = t * kMBN + colgrp * kRrCols;  // first column's row within the cluster
+        static_assert(kRrCols == 2 * kRrChunk, "two chunks");
+        float v[kRrChunk];
+        tmem_read<kRrChunk>(taddr, v);
+        rr_examine<kRrChunk>(v, col0, ri.nrow, pc, thr_gb, k1, k2);
+        tmem_read<kRrChunk>(taddr + (uint32_t)kRrChunk, v);
+        // every column of this group is in registers: hand the accumulator back
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(RR_ACCEMPTY(acc));
+        rr_examine<kRrChunk>(v, col0 + kRrChunk, ri.nrow, pc, thr_gb, k1, k2);
       }
       if (!ok) break;
       if (slot >= 0) {
@@ -1355,6 +1232,7 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
 #undef RR_XFULL
 #undef RR_XEMPTY
 #undef RR_ACCFULL
+#undef RR_REST
 #undef RR_ACCEMPTY
 #undef RR_QFULL
 #undef RR_QEMPTY
