@@ -108,7 +108,9 @@ __device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned l
 }
 
 // Start of a kernel launched by launch_chained: waits until the kernels before
-// it on the stream have finished and their writes are visible.
+// it on the stream have finished and their writes are visible.  What the kernel
+// before may have written is read by coherent loads: it has changed while this kernel
+// was already running, so it is not read-only for it (__ldg, const __restrict__).
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Index of the frame whose tile range [base[f], base[f+1]) holds t.

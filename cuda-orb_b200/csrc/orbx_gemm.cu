@@ -168,7 +168,7 @@ __device__ __forceinline__ void g_epilogue_chunk(const GemmArgs& g, int split, i
                                                  uint32_t* top) {
   if (g.bias && g.splits == 1) {
 #pragma unroll
-    for (int j = 0; j < 32; j++) v[j] = __fadd_rn(v[j], __ldg(g.bias + n0 + j));
+    for (int j = 0; j < 32; j++) v[j] = __fadd_rn(v[j], __ldca(g.bias + n0 + j));
   }
   const size_t off = (size_t)m * g.N + (size_t)n0;
   if (g.mode == kStoreF32) {
@@ -220,7 +220,7 @@ __device__ __forceinline__ void g_epilogue_chunk(const GemmArgs& g, int split, i
     const uint4* aux = reinterpret_cast<const uint4*>(g.aux + off);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      const uint4 w = __ldg(aux + j);
+      const uint4 w = __ldca(aux + j);
       const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
       for (int e = 0; e < 4; e++) {

@@ -31,7 +31,7 @@ constexpr uint16_t kBfPlus1 = 0x3F80u, kBfMinus1 = 0xBF80u;
 // ---------------------------------------------------------------- expansion
 // out[r][k] = bit k of row r ? +1 : -1 (bit k = byte k / 8, bit k % 8), rows
 // n..rows-1 are zero.  One thread per (row, byte): one 16-byte store.
-__global__ void k_bits_pm1_bf16(const uint8_t* __restrict__ bits, int n, const int* d_n, int rows,
+__global__ void k_bits_pm1_bf16(const uint8_t* bits, int n, const int* d_n, int rows,
                                 __nv_bfloat16* __restrict__ out, SearchReset reset) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   chain_wait();
@@ -396,8 +396,8 @@ __global__ void k_assign(const int32_t* __restrict__ idx2, int n, int* __restric
 // offsets[0..k] = exclusive scan of counts[0..k-1]; cursor = copy of offsets;
 // optional items[0..k] = exclusive scan of ceil(counts / per_item).  One block
 // of 1024 threads; k <= 1024 * 8.
-__global__ void __launch_bounds__(1024) k_scan_counts(const int* __restrict__ counts, int k, int* __restrict__ offsets,
-                                                      int* __restrict__ cursor, int per_item, int* __restrict__ items) {
+__global__ void __launch_bounds__(1024) k_scan_counts(const int* counts, int k, int* offsets,
+                                                      int* cursor, int per_item, int* items) {
   __shared__ int s_sum[1024], s_items[1024];
   const int t = threadIdx.x;
   const int per = (k + 1023) / 1024;
@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(256) k_select_probes(const uint32_t* __restric
   chain_wait();
   if (q >= nq) return;
   const int nk = lists * kTopK;  // <= 32
-  uint32_t mine = lane < nk ? keys[(size_t)q * nk + lane] : 0u;
+  uint32_t mine = lane < nk ? __ldca(keys + (size_t)q * nk + lane) : 0u;
   if (lane < kTopK * per_slot) partial[(size_t)q * kTopK * per_slot + lane] = make_uint2(kNoKeyShared, kNoKeyShared);
   // the keys are distinct columns: lane i < 8 ends with the i-th largest
   uint32_t best = 0u, first = 0u, second = 0u;
@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(1024) k_count_probes(const int* __restrict__ p
   chain_wait();
   const int end = min(n, ((int)blockIdx.x + 1) * kProbesPerBlock);
   for (int t = blockIdx.x * kProbesPerBlock + threadIdx.x; t < end; t += 1024) {
-    const int c = probes[t];
+    const int c = __ldca(probes + t);
     if (c >= 0) atomicAdd(&s_count[c], 1);
   }
   __syncthreads();
@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(1024) k_fill_probe_lists(const int* __restrict
 #pragma unroll
   for (int i = 0; i < kPer; i++) {
     const int t = blockIdx.x * kProbesPerBlock + i * 1024 + threadIdx.x;
-    cl[i] = t < n ? probes[t] : -1;
+    cl[i] = t < n ? __ldca(probes + t) : -1;
   }
 #pragma unroll
   for (int i = 0; i < kPer; i++) at[i] = cl[i] >= 0 ? atomicAdd(&s_count[cl[i]], 1) : 0;
@@ -693,7 +693,7 @@ __global__ void k_merge_probes(const uint2* __restrict__ partial, int per_slot, 
   uint32_t k1 = kNoKeyShared, k2 = kNoKeyShared;
   const int n = kTopK * per_slot;
   for (int s = 0; s < n; s++) {
-    const uint2 p = partial[(size_t)q * n + s];
+    const uint2 p = __ldca(partial + (size_t)q * n + s);
     if (p.x != k1 && p.x != k2) top2_push_shared(k1, k2, p.x);
     if (p.y != k1 && p.y != k2) top2_push_shared(k1, k2, p.y);
   }
@@ -710,18 +710,18 @@ __global__ void k_merge_probes(const uint2* __restrict__ partial, int per_slot, 
   finish_query_shared(a, q, k1, k2);
 }
 
-__global__ void k_gather_fallback(const uint8_t* __restrict__ q_desc, const int* __restrict__ fb_list,
-                                  const int* __restrict__ fb_count, uint8_t* __restrict__ out) {
+__global__ void k_gather_fallback(const uint8_t* q_desc, const int* fb_list,
+                                  const int* fb_count, uint8_t* __restrict__ out) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   chain_wait();
-  if ((t >> 1) >= *fb_count) return;
+  if ((t >> 1) >= __ldca(fb_count)) return;
   const int j = t >> 1, h = t & 1;
   reinterpret_cast<uint4*>(out)[2 * (size_t)j + h] =
       reinterpret_cast<const uint4*>(q_desc)[2 * (size_t)fb_list[j] + h];
 }
 
-__global__ void k_scatter_fallback(const int* __restrict__ fb_list, const int* __restrict__ fb_count,
-                                   const uint32_t* __restrict__ fd, const int32_t* __restrict__ fi,
+__global__ void k_scatter_fallback(const int* fb_list, const int* fb_count,
+                                   const uint32_t* fd, const int32_t* fi,
                                    uint32_t* __restrict__ dist2, int32_t* __restrict__ idx2,
                                    int* __restrict__ count_out) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;

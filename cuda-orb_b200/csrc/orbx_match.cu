@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(kMThreads, kMResident) k_match_popc(MatchArgs 
   match_popc_block<kMGroups, false>(a, w, blockIdx.x, gridDim.x, sm);
 }
 
-__global__ void __launch_bounds__(kMThreads, kMResident) k_match_popc_batch(const MatchJob* __restrict__ jobs) {
+__global__ void __launch_bounds__(kMThreads, kMResident) k_match_popc_batch(const MatchJob* jobs) {
   __shared__ MatchSmem<kMGroups> sm;
   chain_wait();
   const MatchJob& J = jobs[blockIdx.y];

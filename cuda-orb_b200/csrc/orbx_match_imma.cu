@@ -812,7 +812,7 @@ struct RrItem {
   int rows;   // slots in this item (1..128)
   int nrow;   // the cluster's database rows
   int pbase;  // first padded row of the cluster
-  int tiles;  // 256-row tiles
+  int tiles;  // 240-row tiles
 };
 
 __device__ __forceinline__ RrItem rr_item(const RerankImmaArgs& a, int it) {
@@ -1103,7 +1103,7 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
         const int r = e >> 1, half = e & 1;
         uint4 w = make_uint4(0u, 0u, 0u, 0u);
         if (r < ri.rows) {
-          const int q = __ldg(a.list + ri.e0 + r) >> 3;
+          const int q = __ldca(a.list + ri.e0 + r) >> 3;
           w = __ldg(reinterpret_cast<const uint4*>(a.q_bits) + 2 * (size_t)q + half);
         }
         const uint32_t wd[4] = {w.x, w.y, w.z, w.w};
@@ -1171,7 +1171,7 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
       // this lane's slot and its query's popcount
       int slot = -1, pc = 0;
       if (row < ri.rows) {
-        slot = __ldg(a.list + ri.e0 + row);
+        slot = __ldca(a.list + ri.e0 + row);
         const uint4* qp = reinterpret_cast<const uint4*>(a.q_bits) + 2 * (size_t)(slot >> 3);
         const uint4 w0 = __ldg(qp), w1 = __ldg(qp + 1);
         pc = __popc(w0.x) + __popc(w0.y) + __popc(w0.z) + __popc(w0.w) + __popc(w1.x) + __popc(w1.y) +

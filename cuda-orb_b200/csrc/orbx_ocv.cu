@@ -117,7 +117,7 @@ __device__ __forceinline__ void ocv_clear(const OcvArgs& a) {
 }
 
 // Level 0 into the level buffer, for images whose rows do not start on 16 bytes.
-__global__ void __launch_bounds__(256) k_ocv_copy0(const __grid_constant__ OcvArgs a, const uint8_t* __restrict__ src,
+__global__ void __launch_bounds__(256) k_ocv_copy0(const __grid_constant__ OcvArgs a, const uint8_t* src,
                                                    int src_pitch) {
   chain_wait();
   ocv_clear(a);
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(256) k_ocv_tiles(const __grid_constant__ OcvAr
     const int x = x0 - 16 + 16 * c, y = reflect101(y0 - 4 + r, h);
     uint4 v{};
     if (x >= 0 && x < V.img_pitch)
-      v = __ldg(reinterpret_cast<const uint4*>(V.img + (long long)y * V.img_pitch + x));
+      v = __ldca(reinterpret_cast<const uint4*>(V.img + (long long)y * V.img_pitch + x));
     *reinterpret_cast<uint4*>(sm.stage + r * kOcvStageSW + 16 * c) = v;
   }
   __syncthreads();

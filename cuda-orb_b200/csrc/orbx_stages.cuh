@@ -9,16 +9,12 @@
 
 namespace orbx {
 
-// Loads of data a stage reads.  Standalone kernels read their inputs through
-// the read-only path; in the persistent kernel a stage reads what an earlier
-// stage wrote in the same launch, after an acquire, so it uses plain
-// (coherent) cached loads instead.
+// Loads of data a stage reads: plain (coherent) cached loads, not the read-only
+// path.  In the persistent kernel an earlier stage wrote it in the same launch, and a
+// chained kernel has started before the kernel that wrote it ended (chain_wait).
 template <bool P, class T>
 __device__ __forceinline__ T ldx(const T* p) {
-  if constexpr (P)
-    return __ldca(p);
-  else
-    return __ldg(p);
+  return __ldca(p);
 }
 
 // The frame table of a launch: from the launch parameters (INL, batches of up
@@ -563,7 +559,7 @@ __device__ __forceinline__ void det_tile(const Batch& b, int t, DetSmem& sm) {
   const int X0 = (lt % F.det_tiles_x) * kDetTW;
   const int Y0 = (lt / F.det_tiles_x) * kDetTH;
   const int n_oct = F.n_oct;
-  const uint8_t* __restrict__ pyr = F.pyr;
+  const uint8_t* pyr = F.pyr;
   const int warp = threadIdx.x >> 5;
   const int thr = b.fast_thr;
 
