@@ -69,3 +69,26 @@ def test_tensor_core_form_equals_popcount_form(nq):
         for w, g in zip(want, got):
             assert torch.equal(w, g), ndb
     ctx.close()
+
+
+@pytest.mark.parametrize("nq", [2100, 2305])
+def test_panels_of_a_large_database(nq):
+    """A database that goes by panels, all queries against one before the next: the
+    last block of queries has one query tile, between blocks with two."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(nq)
+    ndb = 3072 * 240 + 77
+    db = torch.randint(0, 256, (ndb, 32), generator=gen, device="cuda", dtype=torch.uint8)
+    q = torch.randint(0, 256, (nq, 32), generator=gen, device="cuda", dtype=torch.uint8)
+    db[ndb - 1000:] = db[:1000]  # equal distances far apart
+    q[:500] = db[:500]
+    torch.cuda.synchronize()
+    ctx = orbx.Context(0, orbx.make_params(max_pts=1024))
+    want = orbx.knn2(ctx, q, db, orbx.MATCH_POPC)
+    got = orbx.knn2(ctx, q, db, orbx.MATCH_IMMA)
+    ctx.sync()
+    for w, g in zip(want, got):
+        assert torch.equal(w, g)
+    ctx.close()
