@@ -422,7 +422,7 @@ def run_orbx(args, world, rank, local):
     host_pa, host_da = A.to_host()
     host_pb, host_db = B.to_host()
 
-    # the same pair with the int8 tcgen05 matcher (the other exact form)
+    # the same pair with the e2m1 tcgen05 matcher (the other exact form)
     imma_ms = []
     with torch.cuda.stream(stream):
         for _ in range(3):
@@ -557,7 +557,7 @@ def run_orbx(args, world, rank, local):
             ent["bytes"] = work[nm]
             ent["gbs"] = work[nm] / (stage_ms[i] * 1e-3) / 1e9
         else:
-            ent["popc_ops"] = na * nb * 8
+            ent["popc_ops"] = na * nb * 4
         if nm in NCU_WARP_INST:
             # instruction roofline: warp instructions per level-0 pixel of the pair,
             # and the fraction of the SMs' issue slots they fill in the live time
@@ -607,7 +607,7 @@ def run_orbx(args, world, rank, local):
             "gpu_launches": 5 * args.steps,
             "roofline": roofline,
             "kernels": kernels,
-            "pair_int8_tcgen05_matcher": pair_imma,
+            "pair_e2m1_tcgen05_matcher": pair_imma,
             "pair_forms": pair_forms,
             "clocks": clocks,
         }
@@ -631,7 +631,7 @@ def bench_knn2(ctx, stream, dev, peaks):
     out = {}
     with torch.cuda.stream(stream):
         res = {}
-        for name, mode in (("xor_popc", orbx.MATCH_POPC), ("int8_tcgen05", orbx.MATCH_IMMA)):
+        for name, mode in (("xor_popc", orbx.MATCH_POPC), ("e2m1_tcgen05", orbx.MATCH_IMMA)):
             res[name] = orbx.knn2(ctx, q, db, mode)
             ctx.sync()
             ms = []
@@ -643,18 +643,18 @@ def bench_knn2(ctx, stream, dev, peaks):
                 e1.synchronize()
                 ms.append(e0.elapsed_time(e1))
             out[name] = {"ms": statistics.median(ms), "pairs_per_s": pairs / (statistics.median(ms) * 1e-3)}
-        same = bool(torch.equal(res["xor_popc"][0], res["int8_tcgen05"][0]) and
-                    torch.equal(res["xor_popc"][1], res["int8_tcgen05"][1]))
-    popc_peak = SMS * POPC_PER_CLK_PER_SM * peaks.get("sm_max_mhz", 1965.0) * 1e6 / 8
+        same = bool(torch.equal(res["xor_popc"][0], res["e2m1_tcgen05"][0]) and
+                    torch.equal(res["xor_popc"][1], res["e2m1_tcgen05"][1]))
+    popc_peak = SMS * POPC_PER_CLK_PER_SM * peaks.get("sm_max_mhz", 1965.0) * 1e6 / 4
     out["xor_popc"].update({"roofline_pairs_per_s": popc_peak, "frac": out["xor_popc"]["pairs_per_s"] / popc_peak,
-                            "peak_kind": "derived: 148 SMs x 16 popc/clk x max SM clock / 8 popc per pair"})
-    ops = pairs * 512.0  # 256 int8 multiply-adds per pair, 2 ops each
-    t = out["int8_tcgen05"]["ms"] * 1e-3
-    i8_measured = 2.0 * peaks.get("bf16_tflops", 1590.0) * 1e12
-    out["int8_tcgen05"].update({"tops": ops / t / 1e12, "peak_tops_measured_bf16x2": i8_measured / 1e12,
-                                "frac_of_measured": ops / t / i8_measured, "peak_tops_nominal_dense": 4500.0,
-                                "frac_of_nominal": ops / t / 4.5e15,
-                                "note": "int8 dense peak taken as 2x the measured cuBLAS bf16 peak; includes the "
+                            "peak_kind": "derived: 148 SMs x 16 popc/clk x max SM clock / 4 popc per pair"})
+    ops = pairs * 512.0  # 256 multiply-adds per pair, 2 ops each
+    t = out["e2m1_tcgen05"]["ms"] * 1e-3
+    f4_measured = 4.0 * peaks.get("bf16_tflops", 1590.0) * 1e12
+    out["e2m1_tcgen05"].update({"tops": ops / t / 1e12, "peak_tops_measured_bf16x4": f4_measured / 1e12,
+                                "frac_of_measured": ops / t / f4_measured, "peak_tops_nominal_dense": 9000.0,
+                                "frac_of_nominal": ops / t / 9.0e15,
+                                "note": "4-bit float dense peak taken as 4x the measured cuBLAS bf16 peak; includes the "
                                         "+-1 expansion of both 65536 x 32-byte sets"})
     out["bit_exact_popc_vs_tcgen05"] = same
     return out
@@ -765,23 +765,23 @@ def run_match_workload(args, world, rank, local):
     peaks, peak_kind = load_peaks()
     ms1 = total_ms / steps
     if mode == orbx.MATCH_IMMA:
-        # 512 int8 ops per pair (256 multiply-adds); the dense int8 rate is twice bf16
+        # 512 ops per pair (256 multiply-adds); the dense 4-bit float rate is four times bf16
         ach = 65536.0 * 65536.0 * 512 / (ms1 * 1e-3) / 1e12
-        roof = {"kernel": "k_match_imma", "bound": "tensor", "achieved": ach, "peak": 2 * peaks["bf16_tflops"],
-                "unit": "TOP/s (int8)", "frac": ach / (2 * peaks["bf16_tflops"]),
+        roof = {"kernel": "k_match_imma", "bound": "tensor", "achieved": ach, "peak": 4 * peaks["bf16_tflops"],
+                "unit": "TOP/s (4-bit float)", "frac": ach / (4 * peaks["bf16_tflops"]),
                 "traffic": NCU_TRAFFIC.get("k_match_imma"),
-                "peak_kind": f"{peak_kind}: 2 x bf16_tflops (int8 dense rate is twice bf16)"}
+                "peak_kind": f"{peak_kind}: 4 x bf16_tflops (the 4-bit float dense rate is four times bf16)"}
     else:
-        peak_pairs = SMS * POPC_PER_CLK_PER_SM * peaks.get("sm_max_mhz", 1965.0) * 1e6 / 8
+        peak_pairs = SMS * POPC_PER_CLK_PER_SM * peaks.get("sm_max_mhz", 1965.0) * 1e6 / 4
         ach = 65536.0 * 65536.0 / (ms1 * 1e-3)
         roof = {"kernel": "k_match_popc", "bound": "int", "achieved": ach / 1e12, "peak": peak_pairs / 1e12,
                 "unit": "Tpairs/s", "frac": ach / peak_pairs, "traffic": None,
-                "peak_kind": "derived: 148 SMs x 16 popc/clk x max SM clock / 8 popc per pair"}
+                "peak_kind": "derived: 148 SMs x 16 popc/clk x max SM clock / 4 popc per pair"}
     cpu = cpu_baseline_knn2(qh, dbh, budget_s=8.0)
     return {"metric": "Hamming match-pairs/s (exact, k=2, 65536 x 65536)", "value": pairs * steps / (total_ms * 1e-3),
             "unit": "pairs/s", "n_gpus": world, "steps": steps, "warmup": args.warmup,
             "ms_per_step": total_ms / steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "int8" if mode == orbx.MATCH_IMMA else "u32", "data": "synthetic (cuda-orb_b200/synth.py)",
+            "dtype": "e2m1" if mode == orbx.MATCH_IMMA else "u32", "data": "synthetic (cuda-orb_b200/synth.py)",
             "config": {"workload": f"k=2 matching 65536 x 65536, {args.match_mode} form",
                        "l2": "flushed before every step"},
             "roofline": roof, "cpu_baseline": cpu,
@@ -1002,7 +1002,7 @@ def run_learned_workload(args, world, rank, local, with_cpu=True):
     rows, all pipeline descriptors of synthetic 1024 x 1024 images (queries from
     warped copies).  The MLP index is built and trained on the GPU, its fallback
     margin calibrated on held-out queries for recall@1 >= 0.99, then the search
-    is timed against exact int8 tensor-core brute force over the same sets."""
+    is timed against exact tensor-core brute force over the same sets."""
     import torch
 
     import orbx
@@ -1156,8 +1156,8 @@ def run_learned_workload(args, world, rank, local, with_cpu=True):
     pairs = float(nq) * float(ndb)
     cpu = cpu_baseline_knn2(q.cpu().numpy(), db.cpu().numpy()) if with_cpu else None
     phases = dict(zip(["proposal", "probe_lists", "rerank", "merge", "fallback"], prof.tolist()))
-    # Roofline of the dominant phase.  The fallback is exact int8 tensor-core matching
-    # (512 ops per pair, bound: twice the measured bf16 rate); the proposal is the MLP
+    # Roofline of the dominant phase.  The fallback is exact tensor-core matching
+    # (512 ops per pair, bound: four times the measured bf16 rate); the proposal is the MLP
     # (2 * (256 * 512 + 512 * 4096) FLOPs per query, bf16 tensor bound).
     mlp_flop = 2.0 * (256 * 512 + 512 * 4096) * nq
     top = max(("fallback", "proposal", "rerank"), key=lambda k: phases[k])
@@ -1165,17 +1165,17 @@ def run_learned_workload(args, world, rank, local, with_cpu=True):
         ops = float(n_fb) * ndb * 512.0
         achieved = ops / (phases["fallback"] * 1e-3) / 1e12
         roof = {"kernel": "k_match_imma (exact fallback)", "bound": "tensor", "achieved": achieved,
-                "peak": 2.0 * peaks["bf16_tflops"], "unit": "TOP/s (int8)",
-                "frac": achieved / (2.0 * peaks["bf16_tflops"]), "traffic": None,
-                "peak_kind": f"{peak_kind}: 2 x bf16_tflops (int8 dense rate is twice bf16)"}
+                "peak": 4.0 * peaks["bf16_tflops"], "unit": "TOP/s (4-bit float)",
+                "frac": achieved / (4.0 * peaks["bf16_tflops"]), "traffic": None,
+                "peak_kind": f"{peak_kind}: 4 x bf16_tflops (the 4-bit float dense rate is four times bf16)"}
     elif top == "rerank":
         ops = float(probe_pairs) * 512.0
         achieved = ops / (phases["rerank"] * 1e-3) / 1e12
         roof = {"kernel": "k_rerank_imma (probe rerank)", "bound": "tensor", "achieved": achieved,
-                "peak": 2.0 * peaks["bf16_tflops"], "unit": "TOP/s (int8)",
-                "frac": achieved / (2.0 * peaks["bf16_tflops"]), "traffic": None,
-                "peak_kind": f"{peak_kind}: 2 x bf16_tflops (int8 dense rate is twice bf16)",
-                "algorithmic": "512 int8 ops per scanned (query, row) pair"}
+                "peak": 4.0 * peaks["bf16_tflops"], "unit": "TOP/s (4-bit float)",
+                "frac": achieved / (4.0 * peaks["bf16_tflops"]), "traffic": None,
+                "peak_kind": f"{peak_kind}: 4 x bf16_tflops (the 4-bit float dense rate is four times bf16)",
+                "algorithmic": "512 ops per scanned (query, row) pair"}
     else:
         achieved = mlp_flop / (phases["proposal"] * 1e-3) / 1e12
         roof = {"kernel": "k_gemm_bf16 (MLP proposal phase)", "bound": "tensor", "achieved": achieved,
@@ -1191,11 +1191,11 @@ def run_learned_workload(args, world, rank, local, with_cpu=True):
                        "train_rows": train.shape[0], "calibration_rows": cal.shape[0],
                        "n_clusters": 4096, "hidden": 512, "n_probe": 8, "spill": args.learned_spill,
                        "labels": args.learned_labels, "epochs": args.learned_epochs,
-                       "rerank": "int8 tcgen05", "l2": "flushed before every step"},
+                       "rerank": "e2m1 tcgen05", "l2": "flushed before every step"},
             "recall_at_1": recall, "recall_target": LEARNED_RECALL,
             "fallback_rule": {"margin_below": tau_m, "distance_above": tau_d},
             "fallback_fraction": n_fb / nq, "calibration_fallback_fraction": cal_fb,
-            "exact": {"ms": t_exact, "pairs_per_s": pairs / (t_exact * 1e-3), "form": "int8 tcgen05"},
+            "exact": {"ms": t_exact, "pairs_per_s": pairs / (t_exact * 1e-3), "form": "e2m1 tcgen05"},
             "speedup_vs_exact": t_exact / t_learned,
             "operating_points": [dict(c, speedup_vs_exact=t_exact / c["ms"]) for c in curve],
             "ablation": {"recall_mlp_no_fallback": recall_mlp_only,

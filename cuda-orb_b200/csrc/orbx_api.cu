@@ -130,7 +130,7 @@ struct orbx_ctx {
   Workspace ws[2];
   BatchSlot single, pair;
   MatchWork mw{};  // matcher scratch of orbx_match, orbx_match_knn2 and orbx_pair
-  // int8 tensor-core matcher scratch: +-1 expanded queries / database
+  // tensor-core matcher scratch: +-1 expanded queries / database
   uint8_t* imma_q = nullptr;
   uint8_t* imma_db = nullptr;
   size_t imma_q_bytes = 0, imma_db_bytes = 0;

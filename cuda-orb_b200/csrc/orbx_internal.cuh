@@ -185,11 +185,11 @@ struct MatchArgs {
   int unused_;                 // no tail padding: whole-struct bytes key the CUDA graphs
 };
 struct MatchWork {          // scratch for split-train merging
-  uint32_t* part;           // [splits_cap][nq_cap][2] partial top-2 keys
+  uint32_t* part;           // [splits or slots][nq_cap][2] partial top-2 keys
   unsigned int* tile_done;  // [ceil(nq_cap / 128)] arrival counters, self-resetting
   uint32_t* bound;          // optional [nq_cap], tensor-core form: least second-best key any split has found
   int nq_cap;               // query capacity the grid is sized for
-  int splits_cap;           // most train splits per query tile
+  int splits_cap;           // XOR-popc form: most train splits per query tile
 };
 
 // tensor-core form (orbx_match_imma.cu)
@@ -213,9 +213,9 @@ constexpr int kImmaMaxSlots = 152;  // every SM has a part of one block of queri
 int imma_slots(int nq, int ndb, int max_slots);
 cudaError_t launch_match_imma(const ImmaLaunch& L, cudaStream_t s);
 
-// Probe rerank of the learned proposal on the int8 tensor cores
+// Probe rerank of the learned proposal on the tensor cores
 // (orbx_match_imma.cu): per (cluster, up to 128 probing slots), the exact top-2
-// keys of each slot over the cluster's rows, one pair per 64-column group.
+// keys of each slot over the cluster's rows, one pair per 120-column group.
 constexpr int kRrGroups = 2;
 struct RerankImmaArgs {
   const uint8_t* q_bits;     // [nq][32] queries

@@ -3,7 +3,7 @@
 // (orbd.cu:1471-1559, orb.cpp:104-113).
 //
 // Build:  copy + expand the database; Hamming k-majority clustering whose
-//         assignment step is the exact int8 tensor-core k = 2 matcher against
+//         assignment step is the exact tensor-core k = 2 matcher against
 //         the centroids; labels = cluster of each training row's exact nearest
 //         database row; MLP training with the BF16 tcgen05 GEMM (forward and
 //         backward), softmax cross-entropy and Adam, all on the context stream.
@@ -124,7 +124,7 @@ int imma_work_alloc(Arena& a, ImmaWork& iw, int nq_cap, int nq_from, int ndb, cu
   return ORBX_OK;
 }
 
-// Exact k = 2 search with the int8 tensor-core matcher.
+// Exact k = 2 search with the tensor-core matcher.
 int imma_knn(cudaStream_t s, int* err, const ImmaWork& iw, const uint8_t* q, int nq_cap, const int* d_nq,
              uint8_t* q_pm1, bool q_ready, const uint8_t* db, int ndb, uint8_t* db_pm1, bool db_ready, uint32_t* dist2,
              int32_t* idx2) {
@@ -364,7 +364,7 @@ int alloc_core(orbx_learned* L) {
   return ORBX_OK;
 }
 
-// The index's copy of the database and its +-1 layout for the int8 matcher.
+// The index's copy of the database and its +-1 layout for the tensor-core matcher.
 int upload_db(orbx_learned* L, const uint8_t* d_db, cudaStream_t s) {
   LCHK(cudaMemcpyAsync(L->db, d_db, (size_t)L->ndb * 32, cudaMemcpyDeviceToDevice, s));
   LCHK(launch_expand_pm1(L->db, L->ndb, nullptr, imma_rows_db(L->ndb), L->db_pm1, s));
@@ -446,7 +446,7 @@ int cluster_kmeans(orbx_learned* L, cudaStream_t s, int* err) {
 }
 
 // Lists over fixed centroids (a loaded index): every row's exact top-2
-// centroids by the int8 matcher give its cluster and, for spill 1 and 2, its
+// centroids by the tensor-core matcher give its cluster and, for spill 1 and 2, its
 // lists; spill 3 and up go through the GEMM as in clustering.  The same
 // assignment the last clustering iteration makes.
 int lists_from_centroids(orbx_learned* L, cudaStream_t s, int* err) {

@@ -60,7 +60,7 @@ enum {
 
 enum {
   ORBX_MATCH_POPC = 0, /* XOR + popcount over 32-bit words */
-  ORBX_MATCH_IMMA = 1, /* +-1 int8 tcgen05 MMA, Hamming = (256 - dot) / 2 */
+  ORBX_MATCH_IMMA = 1, /* +-1 4-bit float tcgen05 MMA, Hamming = (256 - dot) / 2 */
   ORBX_MATCH_AUTO = 2
 };
 
@@ -357,13 +357,13 @@ typedef struct orbx_learned_params {
   unsigned long long seed;
   int max_distance; /* exact fallback also when the best reranked distance exceeds this (>= 256: off) */
   int spill;        /* MLP: each database row is listed in its `spill` nearest clusters, 1..16
-                       (1, 2: by the int8 matcher; 3..16: by the BF16 GEMM's per-128-centroid
+                       (1, 2: by the tensor-core matcher; 3..16: by the BF16 GEMM's per-128-centroid
                        top 8, exactly the nearest up to 8) */
   int init;         /* ORBX_INIT_CENTROIDS or ORBX_INIT_RANDOM */
   int synth_train;  /* extra training rows: database rows with random bit flips, exactly labelled */
   float flip_lo;    /* per-row bit-flip probability of those rows, uniform in [flip_lo, flip_hi] */
   float flip_hi;
-  int rerank;       /* ORBX_RERANK_TENSOR (int8 tensor cores) or ORBX_RERANK_POPC (XOR-popc) */
+  int rerank;       /* ORBX_RERANK_TENSOR (tensor cores) or ORBX_RERANK_POPC (XOR-popc) */
   int label_mode;   /* training target: ORBX_LABEL_NEAREST or ORBX_LABEL_LISTED */
 } orbx_learned_params;
 /* ORBX_LABEL_NEAREST trains on the cluster of each training row's exact nearest
