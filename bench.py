@@ -47,12 +47,12 @@ SMS = 148
 # on the same 1080p pair, the committed summary of the pair's kernels): the
 # instruction roofline beside the HBM one, since these kernels are issue- and
 # latency-bound.
-NCU_WARP_INST = {"pyramid_blur": 9089420, "detect": 11898158, "nms": 3933009, "describe": 2286742,
-                 "match": 2037180}
+NCU_WARP_INST = {"pyramid_blur": 7086106, "detect": 9440109, "nms": 3932888, "describe": 2291478,
+                 "match": 2978876}
 ISSUE_PER_CLK_PER_SM = 4  # warp instructions issued per clock per SM (one per scheduler)
 
-NCU_TRAFFIC = {"k_pyramid_blur": 4167808, "k_detect": 5666176, "k_nms": 1543552, "k_describe<2>": 5689856,
-               "k_match_popc": 99584, "k_match_imma": 33602560}
+NCU_TRAFFIC = {"k_pyramid_blur": 4179712, "k_detect": 5654016, "k_nms": 1543168, "k_describe<2>": 5689344,
+               "k_match_popc": 97792, "k_match_imma": 17067008}
 
 
 def parse_args(argv=None):
