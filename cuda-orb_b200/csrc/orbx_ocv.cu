@@ -27,6 +27,7 @@
 #include "orbx_device.cuh"
 #include "orbx_fast.cuh"
 #include "orbx_internal.cuh"
+#include "orbx_ocv_stage.cuh"
 
 namespace orbx {
 
@@ -224,15 +225,21 @@ __global__ void __launch_bounds__(256) k_ocv_tiles(const __grid_constant__ OcvAr
   if (t == 0) sm.n_cand = sm.n_key = 0;
   chain_wait();
   // staged rows are reflected at the level's top and bottom; loads past a row's
-  // pitch or before its start are left out (rows start on 16 bytes)
+  // last column or before its start are left out (rows start on 16 bytes)
   static_assert(kOcvStageRows * 6 <= 256, "one staging load per thread");
   if (t < kOcvStageRows * 6) {
     const int r = t / 6, c = t - 6 * r;
     const int x = x0 - 16 + 16 * c, y = reflect101(y0 - 4 + r, h);
-    uint4 v{};
-    if (x >= 0 && x < V.img_pitch)
-      v = __ldca(reinterpret_cast<const uint4*>(V.img + (long long)y * V.img_pitch + x));
-    *reinterpret_cast<uint4*>(sm.stage + r * kOcvStageSW + 16 * c) = v;
+    uint8_t* d = sm.stage + r * kOcvStageSW + 16 * c;
+    const uint8_t* q = V.img + (long long)y * V.img_pitch + x;
+    const int n = ocv_stage_bytes(x, y, w, h);
+    if (n == 16) {
+      *reinterpret_cast<uint4*>(d) = __ldca(reinterpret_cast<const uint4*>(q));
+    } else {
+      *reinterpret_cast<uint4*>(d) = uint4{};
+#pragma unroll 1
+      for (int i = 0; i < n; i++) d[i] = __ldca(q + i);
+    }
   }
   __syncthreads();
   // columns -3 .. -1 and w .. w + 2 reflected (for the blur)
