@@ -44,6 +44,7 @@ struct OcvLevel {
   long long off;       // byte offset of the level in the level buffers
   const uint8_t* img;  // the level's pixels: in the level buffer, or the caller's image
   int img_pitch;
+  int whole;           // columns that are staged by 16-byte loads: past it single pixels
   float fx, fy;        // size of the level below over this one's
   int tile0, tiles_x;  // first tile of the level, tiles per row
   int key0;            // first of the level's key slots over all levels, in blocks of 8
@@ -230,15 +231,15 @@ __global__ void __launch_bounds__(256) k_ocv_tiles(const __grid_constant__ OcvAr
   if (t < kOcvStageRows * 6) {
     const int r = t / 6, c = t - 6 * r;
     const int x = x0 - 16 + 16 * c, y = reflect101(y0 - 4 + r, h);
-    uint8_t* d = sm.stage + r * kOcvStageSW + 16 * c;
     const uint8_t* q = V.img + (long long)y * V.img_pitch + x;
-    const int n = ocv_stage_bytes(x, y, w, h);
-    if (n == 16) {
-      *reinterpret_cast<uint4*>(d) = __ldca(reinterpret_cast<const uint4*>(q));
-    } else {
-      *reinterpret_cast<uint4*>(d) = uint4{};
+    uint8_t* d = sm.stage + r * kOcvStageSW + 16 * c;
+    uint4 v{};
+    const bool whole = x >= 0 && x < V.whole;
+    if (whole) v = __ldca(reinterpret_cast<const uint4*>(q));
+    *reinterpret_cast<uint4*>(d) = v;
+    if (!whole) {
 #pragma unroll 1
-      for (int i = 0; i < n; i++) d[i] = __ldca(q + i);
+      for (int i = 0, n = ocv_stage_bytes(x, y, w, h); i < n; i++) d[i] = __ldca(q + i);
     }
   }
   __syncthreads();
@@ -731,7 +732,7 @@ ORBX_API int orbx_ocv_detect_and_compute(orbx_ctx* ctx, const orbx_ocv_params* p
       }
       if (V.n_keep * (a.harris ? 2 : 1) > kOcvSelCap) return ORBX_ERR_SIZE;
       off += (long long)V.pitch * (V.h + 1);
-      V.img_pitch = V.pitch;
+      V.img_pitch = V.whole = V.pitch;
       if (l > 0) {
         V.fx = (float)a.lv[l - 1].w / (float)V.w;
         V.fy = (float)a.lv[l - 1].h / (float)V.h;
@@ -798,6 +799,7 @@ ORBX_API int orbx_ocv_detect_and_compute(orbx_ctx* ctx, const orbx_ocv_params* p
   if (!copy) {
     a.lv[0].img = d_image;
     a.lv[0].img_pitch = pitch;
+    a.lv[0].whole = w / 16 * 16;
   }
   const dim3 block(64, 4);
   auto grid = [](const OcvLevel& v) { return dim3((v.w + 255) / 256, (v.h + 3) / 4); };
