@@ -112,9 +112,19 @@ __device__ __forceinline__ float ocv_unorder(uint32_t o) {
   return __uint_as_float((o & 0x80000000u) ? (o & 0x7FFFFFFFu) : ~o);
 }
 
+// Blocks of the copy and resize kernels: 64 x 4 threads, 256 columns by 4 rows.  A
+// level may have more rows than a grid's second dimension has blocks; the third
+// carries on.
+constexpr unsigned kOcvGridRows = 65535;
+dim3 ocv_grid(const OcvLevel& V) {
+  const unsigned rows = (V.h + 3) / 4;
+  return dim3((V.w + 255) / 256, std::min(rows, kOcvGridRows), (rows + kOcvGridRows - 1) / kOcvGridRows);
+}
+__device__ __forceinline__ int ocv_row() { return (blockIdx.z * kOcvGridRows + blockIdx.y) * 4 + threadIdx.y; }
+
 // The first launch of a call clears its counters.
 __device__ __forceinline__ void ocv_clear(const OcvArgs& a) {
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.y == 0 && threadIdx.x < 2 * kOcvMaxLevels)
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.y == 0 && threadIdx.x < 2 * kOcvMaxLevels)
     a.ncand[threadIdx.x] = 0;  // ncand, then nsel
 }
 
@@ -124,7 +134,7 @@ __global__ void __launch_bounds__(256) k_ocv_copy0(const __grid_constant__ OcvAr
   chain_wait();
   ocv_clear(a);
   const OcvLevel& V = a.lv[0];
-  const int x = 4 * (blockIdx.x * 64 + threadIdx.x), y = blockIdx.y * 4 + threadIdx.y;
+  const int x = 4 * (blockIdx.x * 64 + threadIdx.x), y = ocv_row();
   if (x >= V.w || y >= V.h) return;
   uint32_t v = 0u;
 #pragma unroll
@@ -139,7 +149,7 @@ __global__ void __launch_bounds__(256) k_ocv_copy0(const __grid_constant__ OcvAr
 __global__ void __launch_bounds__(256) k_ocv_resize(const __grid_constant__ OcvArgs a, int l, int clear) {
   const OcvLevel& D = a.lv[l];
   const OcvLevel& S = a.lv[l - 1];
-  const int xw = 4 * (blockIdx.x * 64 + threadIdx.x), y = blockIdx.y * 4 + threadIdx.y;
+  const int xw = 4 * (blockIdx.x * 64 + threadIdx.x), y = ocv_row();
   const float sy = fmaxf((y + 0.5f) * D.fy - 0.5f, 0.f);
   int y0 = (int)sy;
   const float fy = sy - (float)y0;
@@ -802,13 +812,12 @@ ORBX_API int orbx_ocv_detect_and_compute(orbx_ctx* ctx, const orbx_ocv_params* p
     a.lv[0].whole = w / 16 * 16;
   }
   const dim3 block(64, 4);
-  auto grid = [](const OcvLevel& v) { return dim3((v.w + 255) / 256, (v.h + 3) / 4); };
   if (copy)
-    OCHK(launch_chained(k_ocv_copy0, grid(a.lv[0]), block, s, a, d_image, pitch));
+    OCHK(launch_chained(k_ocv_copy0, ocv_grid(a.lv[0]), block, s, a, d_image, pitch));
   else if (a.L == 1)
     OCHK(cudaMemsetAsync(a.ncand, 0, sizeof(int) * 2 * kOcvMaxLevels, s));
   for (int l = 1; l < a.L; l++)
-    OCHK(launch_chained(k_ocv_resize, grid(a.lv[l]), block, s, a, l, (int)(l == 1 && !copy)));
+    OCHK(launch_chained(k_ocv_resize, ocv_grid(a.lv[l]), block, s, a, l, (int)(l == 1 && !copy)));
   OCHK(launch_chained(k_ocv_tiles, n_tiles, 256, s, a));
   OCHK(launch_chained(k_ocv_select, a.L, 1024, s, a, a.harris ? 2 : 1));
   if (a.harris && n_key_blocks > 0) OCHK(launch_chained(k_ocv_harris, n_key_blocks, 64, s, a));

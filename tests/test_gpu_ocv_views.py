@@ -51,3 +51,21 @@ def test_view_at_the_end_of_its_allocation(ctx, w, h, x0, nlevels):
     want = _run(ctx, copied.data_ptr() + 1, w, h, w + 3, nfeatures=400, nlevels=nlevels)
     assert len(want[0]) > 0
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+def test_more_rows_than_a_grid_dimension(ctx):
+    """An image of more than 4 * 65535 rows, in place and copied: the keypoints of its
+    last rows are those of the same rows alone.  Level 1 is half of level 0, so an even
+    offset keeps its pixels."""
+    w, h, off = 160, 400, 262200
+    tail = torch.zeros((h, w), dtype=torch.uint8, device="cuda")
+    tail[100:] = torch.from_numpy(np.ascontiguousarray(synth.make_image(w, 300, seed=64)[:, :w]))
+    kw = dict(nfeatures=2000, nlevels=2, scale_factor=2.0)
+    want = _run(ctx, tail.data_ptr(), w, h, w, **kw)
+    assert len(want[0]) > 20 and want[0]["octave"].max() == 1
+    for pitch, shift in ((w, 0), (w + 1, 1)):
+        tall = torch.zeros((off + h) * pitch + 1, dtype=torch.uint8, device="cuda")
+        torch.as_strided(tall, (h, w), (pitch, 1), shift + off * pitch).copy_(tail)
+        pts, desc = _run(ctx, tall.data_ptr() + shift, w, off + h, pitch, **kw)
+        pts["y"] -= off
+        assert np.array_equal(pts, want[0]) and np.array_equal(desc, want[1])
