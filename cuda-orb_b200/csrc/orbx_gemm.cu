@@ -22,6 +22,7 @@
 #include "orbx_device.cuh"
 #include "orbx_internal.cuh"
 #include "orbx_learned.cuh"
+#include "orbx_match_plan.cuh"
 
 namespace orbx {
 
@@ -361,6 +362,7 @@ __global__ void __launch_bounds__(kGThreads, 1)
       long long gkb = 0;
       bool ok = true;
       const int my_tiles = my_items * tpi;
+      uint32_t tiles = 0;  // whose accumulator has been committed
       for (int j = 0; ok && j < my_tiles; j++) {
         const int acc = j & 1;
         if (j >= 2 && !g_mbar_wait(GBAR_ACCEMPTY(acc), (uint32_t)(((j >> 1) - 1) & 1), s_abort)) {
@@ -384,11 +386,20 @@ __global__ void __launch_bounds__(kGThreads, 1)
           }
           g_umma_commit(GBAR_EMPTY(s));
         }
-        if (ok) g_umma_commit(GBAR_ACCFULL(acc));
+        if (!ok) break;
+        g_umma_commit(GBAR_ACCFULL(acc));
+        tiles++;
       }
       if (!ok) {
         *s_abort = 1;
         atomicOr(g.err, kErrImmaTimeout);
+      }
+      // the producer drains the ring's "empty" barriers, this thread its other commits
+      for (uint32_t a = 0; a < 2; a++) {
+        const uint32_t uses = m_ring_uses(tiles, 2, a);
+        const long long dl = clock64() + kGDeadlineCycles;
+        while (uses && !g_mbar_try(GBAR_ACCFULL(a), (uses - 1) & 1u) && clock64() < dl) {
+        }
       }
     }
   } else {

@@ -128,6 +128,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long lo
   return true;
 }
 
+// The last of a barrier's `uses` phases, each of one commit, is over (bounded).
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t uses) {
+  if (!uses) return;
+  const long long deadline = clock64() + kIDeadlineCycles;
+  while (!mbar_try(bar, (uses - 1) & 1u) && clock64() < deadline) {
+  }
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
@@ -605,11 +613,17 @@ __global__ void __launch_bounds__(kMThreads, 1)
             umma_commit(BAR_ACCFULL(acc));
           }
         }
-        if (ok) umma_commit(BAR_AEMPTY(ab));
+        if (!ok) break;
+        umma_commit(BAR_AEMPTY(ab));
       }
       if (!ok) {
         *s_abort = 1;
         atomicOr(err, kErrImmaTimeout);
+      }
+      // the producer drains the ring's "empty" barriers, this thread its other commits
+      for (uint32_t i = 0; i < 2; i++) {
+        mbar_drain(BAR_AEMPTY(i), m_ring_uses((uint32_t)parts, 2, i));
+        mbar_drain(BAR_ACCFULL(i), m_ring_uses((uint32_t)g, 2, i));
       }
     }
   } else {
@@ -1076,6 +1090,12 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_rerank_imma(RerankImmaArgs a)
         *s_abort = 1;
         atomicOr(a.err, kErrImmaTimeout);
       }
+      // every commit has arrived (m_ring_uses)
+      for (uint32_t i = 0; i < 2; i++) {
+        mbar_drain(RR_AEMPTY(i), m_ring_uses(na, 2, i));
+        mbar_drain(RR_ACCFULL(i), m_ring_uses(g, 2, i));
+      }
+      for (uint32_t i = 0; i < kRrXStages; i++) mbar_drain(RR_XEMPTY(i), m_ring_uses(g, kRrXStages, i));
     }
   } else if (warp < 2 + kRrExpWarps) {
     // expanders: thread e (0..255)

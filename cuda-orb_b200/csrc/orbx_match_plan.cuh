@@ -85,4 +85,9 @@ __host__ __device__ inline void m_slot(const MPlan& p, int slots, int qb, int t,
   *count = n;
 }
 
+// Of n uses that went round a ring of k entries, those of entry i.  A block does not
+// exit before the last commit to each of its barriers has arrived: the arrival is a
+// write to its shared memory, which may belong to another block by then.
+__host__ __device__ inline unsigned m_ring_uses(unsigned n, unsigned k, unsigned i) { return (n + k - 1 - i) / k; }
+
 }  // namespace orbx
