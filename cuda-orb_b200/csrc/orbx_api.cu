@@ -45,6 +45,7 @@ struct BatchSlot {
   unsigned int* d_ticket = nullptr;
   cudaEvent_t uploaded = nullptr;
   std::vector<uint8_t> last;   // content of the last upload
+  bool captured = false;       // a caller's graph holds these tables
 };
 
 // A launch sequence with the parameters baked into it as `key`.  Capturing and
@@ -84,6 +85,7 @@ struct PersistBufs {
   size_t done_ints = 0;          // counters to clear before each launch
   std::vector<int> layout;       // frame sizes and launch shapes the item tables were built for
   std::vector<MatchJob> last_jobs;  // content of the last upload of jobs
+  bool captured = false;         // a caller's graph holds these tables
 };
 
 static void persist_free(PersistBufs& pb) {
@@ -150,6 +152,9 @@ struct orbx_ctx {
   int describe_bps = 4;  // one wave: 64 registers x 256 threads leave room for 4 blocks per SM
   int match_bps = 8;
   int match_blocks_per_pair = 0;
+  // tables that callers' graphs hold, superseded since: kept until the context is destroyed
+  std::vector<uint8_t*> captured_tables;
+  std::vector<PersistBufs> captured_persist;
   // batched pairs
   std::vector<Workspace> bws;
   BatchSlot batch;
@@ -351,9 +356,13 @@ static void ws_free(Workspace& ws) {
   ws = Workspace();
 }
 
+static bool ws_ready(const orbx_ctx* c, const Workspace& ws, int w, int h, int noct_req = -1) {
+  return ws.pyr_alloc && ws.w == w && ws.h == h && ws.noct_req == (noct_req < 0 ? c->p.noctaves : noct_req);
+}
+
 static int ws_ensure(orbx_ctx* c, Workspace& ws, int w, int h, int noct_req = -1) {
   if (noct_req < 0) noct_req = c->p.noctaves;
-  if (ws.pyr_alloc && ws.w == w && ws.h == h && ws.noct_req == noct_req) return ORBX_OK;
+  if (ws_ready(c, ws, w, h, noct_req)) return ORBX_OK;
   ws_free(ws);
   const int n = compute_layout(w, h, noct_req, ws.oszp);
   if (n < 0) return -n;
@@ -455,6 +464,15 @@ struct LaunchPlan {
   int pyr_tiles = 0, det_tiles = 0, nms_strips = 0, total_max_pts = 0;
 };
 
+// Refuses a call inside a caller's stream capture.  There, copies and clears are
+// recorded instead of done, so nothing that the host afterwards takes as present on
+// the device (tables, cleared workspaces) may be brought there.
+static int refuse_in_capture(orbx_ctx* c) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  ORBX_CUDA(cudaStreamIsCapturing(c->stream, &cap));
+  return cap == cudaStreamCaptureStatusNone ? ORBX_OK : ORBX_ERR_CUDA;
+}
+
 // Fills the launch plan of `frames`.  Their device tables (and the batch's
 // matching jobs behind them) are uploaded when their content changed; frames
 // that travel in the launch parameters need none unless `tables` is set.
@@ -487,20 +505,27 @@ static int upload_batch(orbx_ctx* c, BatchSlot& bs, const std::vector<Frame>& fr
     std::memcpy(blob.data(), frames.data(), fbytes);
     std::memcpy(blob.data() + fbytes, bases.data(), sizeof(int) * bases.size());
     if (jbytes) std::memcpy(blob.data() + fbytes + bbytes, jobs->data(), jbytes);
-    if (bytes > bs.cap) {
-      if (bs.uploaded) cudaEventSynchronize(bs.uploaded);
-      cudaFree(bs.d_tables);
-      cudaFreeHost(bs.h_stage);
-      bs.d_tables = nullptr;
-      bs.h_stage = nullptr;
-      bs.cap = 0;
-      bs.last.clear();
-      ORBX_CUDA(cudaMalloc(&bs.d_tables, bytes));
-      ORBX_CUDA(cudaMallocHost(&bs.h_stage, bytes));
-      if (!bs.uploaded) ORBX_CUDA(cudaEventCreateWithFlags(&bs.uploaded, cudaEventDisableTiming));
-      bs.cap = bytes;
-    }
     if (bs.last != blob) {
+      if (const int rc = refuse_in_capture(c)) return rc;
+      if (bs.captured) {  // these stay as they are for the graph's replays
+        c->captured_tables.push_back(bs.d_tables);
+        bs.d_tables = nullptr;
+        bs.cap = 0;
+        bs.captured = false;
+      }
+      if (bytes > bs.cap) {
+        if (bs.uploaded) cudaEventSynchronize(bs.uploaded);
+        cudaFree(bs.d_tables);
+        cudaFreeHost(bs.h_stage);
+        bs.d_tables = nullptr;
+        bs.h_stage = nullptr;
+        bs.cap = 0;
+        bs.last.clear();
+        ORBX_CUDA(cudaMalloc(&bs.d_tables, bytes));
+        ORBX_CUDA(cudaMallocHost(&bs.h_stage, bytes));
+        if (!bs.uploaded) ORBX_CUDA(cudaEventCreateWithFlags(&bs.uploaded, cudaEventDisableTiming));
+        bs.cap = bytes;
+      }
       ORBX_CUDA(cudaEventSynchronize(bs.uploaded));  // the previous upload has left the staging buffer
       std::memcpy(bs.h_stage, blob.data(), bytes);
       bs.last.clear();  // unknown content until the copy is queued
@@ -557,9 +582,10 @@ static int launch_frames(orbx_ctx* c, const LaunchPlan& pl, bool compute_desc, c
 
 // Issues a launch sequence under the rule of PairGraph: `enqueue` queues it on
 // the context's stream.  Inside a caller's stream capture only a sequence that
-// has run before is recorded.
+// has run before is recorded; *captured tells that it was.
 template <class Enqueue>
-static int issue_or_replay(orbx_ctx* c, PairGraph& g, std::vector<uint8_t>& key, Enqueue&& enqueue) {
+static int issue_or_replay(orbx_ctx* c, PairGraph& g, std::vector<uint8_t>& key, Enqueue&& enqueue,
+                           bool* captured = nullptr) {
   const bool same = g.key == key;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   ORBX_CUDA(cudaStreamIsCapturing(c->stream, &cap));
@@ -568,6 +594,7 @@ static int issue_or_replay(orbx_ctx* c, PairGraph& g, std::vector<uint8_t>& key,
     if (!same) g.drop();
     const int rc = enqueue();
     if (rc == ORBX_OK) g.key.swap(key);
+    if (captured) *captured = cap != cudaStreamCaptureStatusNone;
     return rc;
   }
   if (!g.exec) {
@@ -824,6 +851,8 @@ ORBX_API int orbx_destroy(orbx_ctx* c) {
   cudaFree(c->batch_tile_done);
   persist_free(c->pbatch);
   persist_free(c->ppair);
+  for (uint8_t* t : c->captured_tables) cudaFree(t);
+  for (PersistBufs& pb : c->captured_persist) persist_free(pb);
   cudaFree(c->pho.mw.part);
   cudaFree(c->pho.mw.tile_done);
   cudaFree(c->pho.mw.bound);
@@ -1085,11 +1114,17 @@ static int pair_persistent(orbx_ctx* c, const LaunchPlan& pl, const std::vector<
   std::memcpy(key.data(), &a, sizeof(PersistArgs));
   std::memcpy(key.data() + sizeof(PersistArgs), &grid, sizeof(int));
   std::memcpy(key.data() + sizeof(PersistArgs) + sizeof(int), &c->ppair.done_ints, sizeof(size_t));
-  return issue_or_replay(c, pg, key, [&]() -> int {
-    ORBX_CUDA(cudaMemsetAsync(a.done, 0, sizeof(int) * c->ppair.done_ints, c->stream));
-    ORBX_CUDA(launch_batch_persistent(a, grid, c->stream));
-    return ORBX_OK;
-  });
+  bool captured = false;
+  rc = issue_or_replay(
+      c, pg, key,
+      [&]() -> int {
+        ORBX_CUDA(cudaMemsetAsync(a.done, 0, sizeof(int) * c->ppair.done_ints, c->stream));
+        ORBX_CUDA(launch_batch_persistent(a, grid, c->stream));
+        return ORBX_OK;
+      },
+      &captured);
+  if (captured) c->pair.captured = c->ppair.captured = true;
+  return rc;
 }
 
 ORBX_API int orbx_pair(orbx_ctx* c, const uint8_t* d_img_a, const uint8_t* d_img_b, int w, int h, int pitch,
@@ -1102,14 +1137,19 @@ ORBX_API int orbx_pair(orbx_ctx* c, const uint8_t* d_img_a, const uint8_t* d_img
   // frame pairs hold at most max_pts keypoints each: the popcount form unless asked
   if (mode == ORBX_MATCH_AUTO) mode = ORBX_MATCH_POPC;
   DeviceGuard g(c->device);
+  const bool persistent = c->pair_form == 1 && mode == ORBX_MATCH_POPC;
+  // a call that still has to allocate and clear its workspaces is not captured
+  const MatchWork& mw = persistent ? c->ppg.mw : c->mw;
+  if (!(ws_ready(c, c->ws[0], w, h) && ws_ready(c, c->ws[1], w, h) && mw.part && mw.nq_cap >= c->p.max_pts) &&
+      (rc = refuse_in_capture(c)) != 0)
+    return rc;
   if ((rc = ws_ensure(c, c->ws[0], w, h)) != 0) return rc;
   if ((rc = ws_ensure(c, c->ws[1], w, h)) != 0) return rc;
   if (mode == ORBX_MATCH_IMMA && (rc = imma_ensure(c, c->p.max_pts, c->p.max_pts)) != 0) return rc;
   std::vector<Frame> frames(2);
-  const int shape = (c->pair_form == 1 && mode == ORBX_MATCH_POPC) ? 0 : pyr_shape_for(c, 2ll * w * h);
+  const int shape = persistent ? 0 : pyr_shape_for(c, 2ll * w * h);
   fill_frame(c, c->ws[0], d_img_a, pitch, d_pts_a, d_desc_a, d_n_a, frames[0], -1, shape);
   fill_frame(c, c->ws[1], d_img_b, pitch, d_pts_b, d_desc_b, d_n_b, frames[1], -1, shape);
-  const bool persistent = c->pair_form == 1 && mode == ORBX_MATCH_POPC;
   LaunchPlan pl;
   if ((rc = upload_batch(c, c->pair, frames, &pl, persistent)) != 0) return rc;
   MatchArgs a{};
@@ -1627,6 +1667,16 @@ static int persist_prepare(orbx_ctx* c, PersistBufs& pb, const LaunchPlan& pl, c
   std::vector<int> layout = {nf, n_pairs, blocks_per_pair, group, c->row_deps};
   for (const Frame& F : frames)
     for (int v : {F.w, F.h, F.n_oct, F.max_pts, F.border, F.nms_rows, F.nms_strips}) layout.push_back(v);
+  const bool new_layout = pb.layout != layout;
+  const bool new_jobs = new_layout || pb.last_jobs.size() != jobs.size() ||
+                        std::memcmp(pb.last_jobs.data(), jobs.data(), sizeof(MatchJob) * n_pairs) != 0;
+  if (new_jobs) {
+    if (const int rc = refuse_in_capture(c)) return rc;
+    if (pb.captured) {  // these stay as they are for the graph's replays
+      c->captured_persist.push_back(pb);
+      pb = PersistBufs();
+    }
+  }
   if (pb.layout != layout) {
     std::vector<int> pyr_n(nf), det_n(nf), nms_n(nf), desc_n(nf), desc_base(nf + 1, 0);
     for (int f = 0; f < nf; f++) {
@@ -1737,15 +1787,21 @@ static int batch_persistent(orbx_ctx* c, const LaunchPlan& pl, const std::vector
   int grid = 0;
   int rc = persist_prepare(c, c->pbatch, pl, frames, jobs, blocks_per_pair, c->persist_group, &a, &grid);
   if (rc) return rc;
+  bool captured = false;
   const int extra[3] = {1, grid, (int)c->pbatch.done_ints};
   std::vector<uint8_t> key(sizeof(PersistArgs) + sizeof(extra));
   std::memcpy(key.data(), &a, sizeof(PersistArgs));
   std::memcpy(key.data() + sizeof(PersistArgs), extra, sizeof(extra));
-  return issue_or_replay(c, c->bg, key, [&]() -> int {
-    ORBX_CUDA(cudaMemsetAsync(a.done, 0, sizeof(int) * c->pbatch.done_ints, c->stream));
-    ORBX_CUDA(launch_batch_persistent(a, grid, c->stream));
-    return ORBX_OK;
-  });
+  rc = issue_or_replay(
+      c, c->bg, key,
+      [&]() -> int {
+        ORBX_CUDA(cudaMemsetAsync(a.done, 0, sizeof(int) * c->pbatch.done_ints, c->stream));
+        ORBX_CUDA(launch_batch_persistent(a, grid, c->stream));
+        return ORBX_OK;
+      },
+      &captured);
+  if (captured) c->batch.captured = c->pbatch.captured = true;
+  return rc;
 }
 
 static int batch_pairs_impl(orbx_ctx* c, int n_pairs, const orbx_image* ia, const orbx_image* ib,
@@ -1768,7 +1824,13 @@ static int batch_pairs_impl(orbx_ctx* c, int n_pairs, const orbx_image* ia, cons
   if ((int)c->bws.size() < 2 * n_pairs) c->bws.resize(2 * n_pairs);
   std::vector<Frame> frames(2 * n_pairs);
   long long px = 0;
-  for (int i = 0; i < n_pairs; i++) px += (long long)ia[i].w * ia[i].h + (long long)ib[i].w * ib[i].h;
+  bool ready = true;
+  for (int i = 0; i < n_pairs; i++) {
+    px += (long long)ia[i].w * ia[i].h + (long long)ib[i].w * ib[i].h;
+    ready = ready && ws_ready(c, c->bws[2 * i], ia[i].w, ia[i].h) && ws_ready(c, c->bws[2 * i + 1], ib[i].w, ib[i].h);
+  }
+  // a call that still has to allocate and clear its workspaces is not captured
+  if (!ready && (rc = refuse_in_capture(c)) != 0) return rc;
   for (int i = 0; i < n_pairs; i++) {
     for (int s = 0; s < 2; s++) {
       const orbx_image& im = s ? ib[i] : ia[i];
@@ -1790,6 +1852,7 @@ static int batch_pairs_impl(orbx_ctx* c, int n_pairs, const orbx_image* ia, cons
     tile_words += (size_t)div_up(nq_cap, 128);
   }
   if (c->batch_part_words < part_words || c->batch_tile_words < tile_words) {
+    if ((rc = refuse_in_capture(c)) != 0) return rc;
     cudaStreamSynchronize(c->stream);
     cudaFree(c->batch_part);
     cudaFree(c->batch_tile_done);
@@ -1857,12 +1920,18 @@ static int batch_pairs_impl(orbx_ctx* c, int n_pairs, const orbx_image* ia, cons
   std::memcpy(key.data(), &pl.b, sizeof(Batch));
   std::memcpy(key.data() + sizeof(Batch), extra, sizeof(extra));
   std::memcpy(key.data() + sizeof(Batch) + sizeof(extra), &d_jobs, sizeof(d_jobs));
-  return issue_or_replay(c, c->bg, key, [&]() -> int {
-    const int lrc = launch_frames(c, pl, true);
-    if (lrc) return lrc;
-    ORBX_CUDA(launch_match_popc_batch(d_jobs, n_pairs, blocks_per_pair, c->stream));
-    return ORBX_OK;
-  });
+  bool captured = false;
+  rc = issue_or_replay(
+      c, c->bg, key,
+      [&]() -> int {
+        const int lrc = launch_frames(c, pl, true);
+        if (lrc) return lrc;
+        ORBX_CUDA(launch_match_popc_batch(d_jobs, n_pairs, blocks_per_pair, c->stream));
+        return ORBX_OK;
+      },
+      &captured);
+  if (captured) c->batch.captured = true;
+  return rc;
 }
 
 ORBX_API int orbx_batch_pairs(orbx_ctx* c, int n_pairs, const orbx_image* ia, const orbx_image* ib,

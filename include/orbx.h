@@ -299,7 +299,12 @@ ORBX_API int orbx_bounds_set_slack(orbx_ctx* ctx, long long bytes);
  * other buffers too.  Per pair the results are identical to
  * orbx_pair on that pair with the same cap.  This batches what the reference
  * does one Orbor::detectAndCompute / Orbor::match call at a time
- * (orb.cpp:57-113).  Asynchronous. */
+ * (orb.cpp:57-113).  Asynchronous.
+ * Inside a stream capture a call is accepted when it repeats the call before it
+ * (images, outputs, tuning), whose tables are on the device; otherwise it returns
+ * ORBX_ERR_CUDA and records nothing.  The captured graph keeps its own tables until
+ * the context is destroyed.  It uses the context's workspaces, so it may be replayed
+ * until the context is given a batch of other sizes. */
 ORBX_API int orbx_batch_pairs(orbx_ctx* ctx, int n_pairs, const orbx_image* imgs_a, const orbx_image* imgs_b,
                               const orbx_frame_out* out_a, const orbx_frame_out* out_b, int mode);
 
