@@ -1215,7 +1215,9 @@ static bool memops_ok(orbx_ctx* c) {
 // count to a device flag, while one persistent launch (orbx_persist.cu) is
 // already running: a pyramid tile starts as soon as the rows it reads have
 // arrived, so frame A is processed while frame B is still being copied.  The
-// export kernel follows in the same graph.  Returns the mapped result block.
+// export kernel follows.  Both kernels are loaded before the launch: loading one may
+// have to wait for the device, where the launch waits for bands that are not sent yet.
+// Returns the mapped result block.
 static int pair_host_overlap(orbx_ctx* c, const uint8_t* h_a, const uint8_t* h_b, int w, int h, int pitch,
                              bool with_desc, const uint8_t** res) {
   int rc;
@@ -1256,15 +1258,16 @@ static int pair_host_overlap(orbx_ctx* c, const uint8_t* h_a, const uint8_t* h_b
   const int extra[4] = {grid, c->p.max_pts, with_desc ? 1 : 0, (int)c->ppair.done_ints};
   std::memcpy(key.data() + sizeof(PersistArgs), extra, sizeof(extra));
   std::memcpy(key.data() + sizeof(PersistArgs) + sizeof(extra), &map_dev, sizeof(void*));
-  // reset the counters and flags, start the launch, then feed it the bands
+  if ((rc = hostio_load_export(c)) != 0) return rc;
+  // reset the counters and flags, start the launch, then feed it the bands (also when
+  // the export could not be queued: the launch, if it has started, ends with them)
   ORBX_CUDA(cudaMemsetAsync(a.done, 0, sizeof(int) * c->ppair.done_ints, c->stream));
   ORBX_CUDA(cudaEventRecord(c->ev_reset, c->stream));
-  rc = issue_or_replay(c, pg, key, [&]() -> int {
+  const int issued = issue_or_replay(c, pg, key, [&]() -> int {
     ORBX_CUDA(launch_batch_persistent(a, grid, c->stream));
     return hostio_export_pair(c, c->io_pts[0], c->io_pts[1], c->io_desc[0], c->io_desc[1], c->io_count,
                               c->p.max_pts, with_desc, res);
   });
-  if (rc) return rc;
   ORBX_CUDA(cudaStreamWaitEvent(c->copy_stream, c->ev_reset, 0));
   WriteValue32Fn wv = write_value32();
   const uint8_t* src[2] = {h_a, h_b};
@@ -1278,7 +1281,7 @@ static int pair_host_overlap(orbx_ctx* c, const uint8_t* h_a, const uint8_t* h_b
         return ORBX_ERR_CUDA;
     }
   }
-  return ORBX_OK;
+  return issued;
 }
 
 static bool host_pinned(const void* p) {

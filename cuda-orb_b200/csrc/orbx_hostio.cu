@@ -32,6 +32,7 @@ struct HostIO {
   uint8_t* map = nullptr;      // pinned, mapped: orbx_pair_host results written by the device
   uint8_t* map_dev = nullptr;  // its device address
   size_t map_bytes = 0;
+  bool export_loaded = false;
 };
 
 void hostio_free(HostIO* io) {
@@ -100,6 +101,20 @@ int hostio_map(orbx_ctx* c, int max_pts, const uint8_t** host, const uint8_t** d
   }
   *host = io->map;
   if (dev) *dev = io->map_dev;
+  return ORBX_OK;
+}
+
+// Loads the export kernel on the context's device (kernels load at their first use).
+int hostio_load_export(orbx_ctx* c) {
+  HostIO*& io = ctx_hostio(c);
+  if (!io) io = new HostIO();
+  if (io->export_loaded) return ORBX_OK;
+  cudaFuncAttributes at;
+  if (cudaFuncGetAttributes(&at, k_export_pair) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return ORBX_ERR_CUDA;
+  }
+  io->export_loaded = true;
   return ORBX_OK;
 }
 
