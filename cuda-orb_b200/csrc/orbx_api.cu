@@ -1096,6 +1096,9 @@ static int persist_prepare(orbx_ctx* c, PersistBufs& pb, const LaunchPlan& pl, c
                            const std::vector<MatchJob>& jobs, int blocks_per_pair, int group, PersistArgs* out,
                            int* grid_out);
 
+// Match items of a persistent launch over one pair: every query tile needs one.
+static int pair_match_items(int max_pts) { return std::max(2 * 148, div_up(max_pts, 128)); }
+
 // orbx_pair as one persistent launch (orbx_persist.cu) over the pair's two
 // frames: a counter reset and the launch.
 static int pair_persistent(orbx_ctx* c, const LaunchPlan& pl, const std::vector<Frame>& frames,
@@ -1109,7 +1112,8 @@ static int pair_persistent(orbx_ctx* c, const LaunchPlan& pl, const std::vector<
   jobs[0].work = pg.mw;
   PersistArgs a;
   int grid = 0;
-  if ((rc = persist_prepare(c, c->ppair, pl, frames, jobs, 2 * 148, 0, &a, &grid)) != 0) return rc;
+  if ((rc = persist_prepare(c, c->ppair, pl, frames, jobs, pair_match_items(c->p.max_pts), 0, &a, &grid)) != 0)
+    return rc;
   std::vector<uint8_t> key(sizeof(PersistArgs) + sizeof(int) + sizeof(size_t));
   std::memcpy(key.data(), &a, sizeof(PersistArgs));
   std::memcpy(key.data() + sizeof(PersistArgs), &grid, sizeof(int));
@@ -1243,10 +1247,10 @@ static int pair_host_overlap(orbx_ctx* c, const uint8_t* h_a, const uint8_t* h_b
   jobs[0].args.pts = c->io_pts[0];
   match_bounds(c, jobs[0].args, c->p.max_pts, c->p.max_pts, c->p.max_pts);
   jobs[0].work = pg.mw;
-  const int match_items = 2 * 148;
   PersistArgs a;
   int grid = 0;
-  if ((rc = persist_prepare(c, c->ppair, pl, frames, jobs, match_items, 0, &a, &grid)) != 0) return rc;
+  if ((rc = persist_prepare(c, c->ppair, pl, frames, jobs, pair_match_items(c->p.max_pts), 0, &a, &grid)) != 0)
+    return rc;
   const int bands = c->upload_bands;
   const int band_rows = div_up(h, bands);
   a.upload_flags = a.done + 4 * 2 + 1;

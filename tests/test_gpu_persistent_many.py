@@ -1,0 +1,36 @@
+"""A pair with more keypoints than 296 query tiles of 128 hold: the persistent forms match
+all of them, as the five launches do."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import orbx  # noqa: E402
+
+
+@pytest.mark.parametrize("form", ["pair_form", "upload_bands"])
+def test_every_query_is_matched(form):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    w, h, cap = 2048, 1600, 60000
+    rng = np.random.default_rng(48)
+    a = rng.integers(0, 256, (h, w), dtype=np.uint8)  # noise: a corner every few dozen pixels
+    b = a.copy()
+    b[::7] ^= 3
+    ctx = orbx.Context(0, orbx.make_params(max_pts=cap, noctaves=1, fast_threshold=10))
+
+    def run(bands, pair_form):
+        t = ctx.get_tuning()
+        t.upload_bands, t.host_overlap, t.pair_form = bands, 0, pair_form
+        ctx.set_tuning(t)
+        pa, pb = np.full((cap, 7), -7, np.int32), np.full((cap, 7), -7, np.int32)
+        na, nb = np.zeros(1, np.int32), np.zeros(1, np.int32)
+        ctx.pair_host(a, b, w, h, w, pa, na, pb, nb)
+        return pa, na, pb, nb
+
+    want = run(0, 0)
+    assert want[1][0] > 296 * 128
+    got = run(4, 0) if form == "upload_bands" else run(0, 1)
+    assert all(np.array_equal(g, e) for g, e in zip(got, want))
+    ctx.close()
