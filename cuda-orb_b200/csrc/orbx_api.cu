@@ -15,6 +15,7 @@
 #include "orb_pattern31.h"
 #include "orbx_device.cuh"
 #include "orbx_internal.cuh"
+#include "orbx_match_plan.cuh"
 #include "orbx_persist.cuh"
 
 using namespace orbx;
@@ -615,8 +616,11 @@ static int issue_or_replay(orbx_ctx* c, PairGraph& g, std::vector<uint8_t>& key,
 }
 
 static constexpr int kSplitsCap = 64;
-// Slots of MatchWork::part: the tensor-core form spreads a small query set over all SMs.
-static int part_slots(int nq_cap) { return nq_cap <= 2048 ? kImmaMaxSlots : kSplitsCap; }
+// Best twos in MatchWork::part: the splits of the popcount form or the slots of the
+// tensor-core form.
+static long long part_rows(int nq_cap) {
+  return std::max((long long)kSplitsCap * nq_cap, m_part_rows(nq_cap, (1 << 22) - 1));
+}
 
 static int mw_ensure(MatchWork& mw, int nq_cap) {
   if (mw.part && mw.nq_cap >= nq_cap) return ORBX_OK;
@@ -625,7 +629,7 @@ static int mw_ensure(MatchWork& mw, int nq_cap) {
   cudaFree(mw.bound);
   mw = MatchWork();
   const int cap = nq_cap < 128 ? 128 : nq_cap;
-  ORBX_CUDA(cudaMalloc(&mw.part, sizeof(uint32_t) * 2 * (size_t)part_slots(cap) * cap));
+  ORBX_CUDA(cudaMalloc(&mw.part, sizeof(uint32_t) * 2 * (size_t)part_rows(cap)));
   ORBX_CUDA(cudaMalloc(&mw.tile_done, sizeof(unsigned int) * (size_t)div_up(cap, 128)));
   ORBX_CUDA(cudaMalloc(&mw.bound, sizeof(uint32_t) * (size_t)cap));
   ORBX_CUDA(cudaMemset(mw.tile_done, 0, sizeof(unsigned int) * (size_t)div_up(cap, 128)));
@@ -1044,8 +1048,8 @@ static int launch_match(orbx_ctx* c, MatchWork& mw, const MatchArgs& a, int nq_c
   L.db_pm1 = c->imma_db;
   L.nq_cap = nq_cap;
   L.ndb_cap = ndb_cap;
-  L.slots = imma_slots(nq_cap, ndb_cap, part_slots(mw.nq_cap));
-  if (a.d_nq) L.slots = part_slots(mw.nq_cap);  // fewer queries than the capacity: more parts each
+  L.work.nq_cap = nq_cap;
+  L.part_rows = part_rows(mw.nq_cap);
   L.err = c->d_err;
   ORBX_CUDA(launch_match_imma(L, c->stream));
   return ORBX_OK;

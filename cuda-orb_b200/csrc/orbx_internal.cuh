@@ -185,7 +185,7 @@ struct MatchArgs {
   int unused_;                 // no tail padding: whole-struct bytes key the CUDA graphs
 };
 struct MatchWork {          // scratch for split-train merging
-  uint32_t* part;           // [splits or slots][nq_cap][2] partial top-2 keys
+  uint32_t* part;           // [splits][nq_cap][2] or [slots][queries][2] partial top-2 keys
   unsigned int* tile_done;  // [ceil(nq_cap / 128)] arrival counters, self-resetting
   uint32_t* bound;          // optional [nq_cap], tensor-core form: least second-best key any split has found
   int nq_cap;               // query capacity the grid is sized for
@@ -196,11 +196,11 @@ struct MatchWork {          // scratch for split-train merging
 constexpr int kPm1RowBytes = 128;  // an expanded descriptor: 256 4-bit floats, +-1
 struct ImmaLaunch {
   MatchArgs args;     // queries, database, counts, outputs
-  MatchWork work;     // part: [slots][work.nq_cap] best two; tile_done: one per 256 queries
+  MatchWork work;     // part: [slots][queries] best two; tile_done: one per 256 queries
   uint8_t* q_pm1;     // [imma_rows_q(nq_cap)][kPm1RowBytes] scratch
   uint8_t* db_pm1;    // [imma_rows_db(ndb_cap)][kPm1RowBytes] scratch
   int nq_cap, ndb_cap;
-  int slots;          // slots per query in work.part (imma_slots)
+  long long part_rows;  // best twos that work.part holds (m_part_rows)
   int* err;
   bool q_ready;       // q_pm1 already holds the expanded queries (rows >= nq zero)
   bool db_ready;      // db_pm1 already holds the expanded database (rows >= ndb zero)
@@ -209,8 +209,6 @@ struct ImmaLaunch {
 cudaError_t launch_expand_pm1(const uint8_t* bits, int n, const int* d_n, int rows, uint8_t* out, cudaStream_t s);
 int imma_rows_q(int n);
 int imma_rows_db(int n);
-constexpr int kImmaMaxSlots = 152;  // every SM has a part of one block of queries
-int imma_slots(int nq, int ndb, int max_slots);
 cudaError_t launch_match_imma(const ImmaLaunch& L, cudaStream_t s);
 
 // Probe rerank of the learned proposal on the tensor cores

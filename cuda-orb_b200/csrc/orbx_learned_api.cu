@@ -21,6 +21,7 @@
 
 #include "orbx_internal.cuh"
 #include "orbx_learned.cuh"
+#include "orbx_match_plan.cuh"
 
 using namespace orbx;
 typedef __nv_bfloat16 bf16;
@@ -105,22 +106,19 @@ int pick_splits(int tiles, int kblocks) {
   return s;
 }
 
-// Merge scratch of the tensor-core matcher for up to nq_cap queries, with the slots
-// that nq_from or more of them need.
+// Merge scratch of the tensor-core matcher for up to nq_cap queries, in one allocation.
 struct ImmaWork {
   MatchWork w{};
-  int slots = 1;
+  long long part_rows = 0;
 };
-int imma_work_alloc(Arena& a, ImmaWork& iw, int nq_cap, int nq_from, int ndb, cudaStream_t s) {
-  iw.slots = imma_slots(nq_from, ndb, kImmaMaxSlots);
+int imma_work_alloc(Arena& a, ImmaWork& iw, int nq_cap, int ndb, cudaStream_t s) {
+  iw.part_rows = m_part_rows(nq_cap, ndb);
   iw.w.nq_cap = nq_cap;
-  if (iw.slots > 2) {
-    const int tiles = (nq_cap + 127) / 128;
-    LCHK(a.alloc(&iw.w.part, (size_t)2 * iw.slots * nq_cap));
-    LCHK(a.alloc(&iw.w.tile_done, (size_t)tiles));
-    LCHK(a.alloc(&iw.w.bound, (size_t)nq_cap));
-    LCHK(cudaMemsetAsync(iw.w.tile_done, 0, sizeof(unsigned) * (size_t)tiles, s));
-  }
+  const size_t part = 2 * (size_t)iw.part_rows, tiles = (nq_cap + 127) / 128;
+  LCHK(a.alloc(&iw.w.part, part + tiles + nq_cap));
+  iw.w.tile_done = iw.w.part + part;
+  iw.w.bound = iw.w.tile_done + tiles;
+  LCHK(cudaMemsetAsync(iw.w.tile_done, 0, sizeof(unsigned) * tiles, s));
   return ORBX_OK;
 }
 
@@ -137,7 +135,7 @@ int imma_knn(cudaStream_t s, int* err, const ImmaWork& iw, const uint8_t* q, int
   L.args.dist2 = dist2;
   L.args.idx2 = idx2;
   L.work = iw.w;
-  L.slots = iw.slots;
+  L.part_rows = iw.part_rows;
   L.q_pm1 = q_pm1;
   L.db_pm1 = db_pm1;
   L.nq_cap = nq_cap;
@@ -420,7 +418,7 @@ int cluster_kmeans(orbx_learned* L, cudaStream_t s, int* err) {
   k_gather_rows<<<grid1(2ll * C, 256), 256, 0, s>>>(L->db, d_init, C, L->centroids);
   LCHK(cudaMemsetAsync(L->assign, 0xFF, sizeof(int) * (size_t)n, s));
   ImmaWork iw;
-  LRC(imma_work_alloc(t, iw, n, n, C, s));
+  LRC(imma_work_alloc(t, iw, n, C, s));
   const int iters = L->p.kmeans_iters;
   for (int it = 0; it < iters; it++) {
     LRC(imma_knn(s, err, iw, L->db, n, nullptr, L->db_pm1, true, L->centroids, C, cent_pm1, false, dist2, idx2));
@@ -462,7 +460,7 @@ int lists_from_centroids(orbx_learned* L, cudaStream_t s, int* err) {
   LCHK(t.alloc(&changed, 1));
   LCHK(t.alloc(&cent_pm1, (size_t)imma_rows_db(C) * kPm1RowBytes));
   ImmaWork iw;
-  LRC(imma_work_alloc(t, iw, n, n, C, s));
+  LRC(imma_work_alloc(t, iw, n, C, s));
   LRC(imma_knn(s, err, iw, L->db, n, nullptr, L->db_pm1, true, L->centroids, C, cent_pm1, false, dist2, idx2));
   LCHK(cudaMemsetAsync(L->assign, 0xFF, sizeof(int) * (size_t)n, s));
   LCHK(cudaMemsetAsync(counts, 0, sizeof(int) * C, s));
@@ -633,9 +631,8 @@ int ensure_search(orbx_learned* L, int nq) {
   LCHK(a.alloc(&L->fb_d, (size_t)nq * 2));
   LCHK(a.alloc(&L->fb_i, (size_t)nq * 2));
   LCHK(a.alloc(&L->fb_pm1, (size_t)imma_rows_q(nq) * kPm1RowBytes));
-  // the fallback's slots let few queries (512 or more) spread over all SMs
   L->fb_work = ImmaWork();
-  LRC(imma_work_alloc(a, L->fb_work, nq, std::min(nq, 512), L->ndb, 0));
+  LRC(imma_work_alloc(a, L->fb_work, nq, L->ndb, 0));
   LCHK(cudaDeviceSynchronize());
   L->nq_cap = nq;
   return ORBX_OK;
@@ -736,7 +733,7 @@ ORBX_API int orbx_learned_build(orbx_ctx* ctx, const orbx_learned_params* p, con
                                                                          p->seed ^ 0x73796e74ull, p->flip_lo,
                                                                          p->flip_hi, rows + (size_t)ntrain * 32);
       ImmaWork iw;
-      rc = imma_work_alloc(t, iw, nt, nt, ndb, s);
+      rc = imma_work_alloc(t, iw, nt, ndb, s);
       if (rc) break;
       rc = imma_knn(s, err, iw, rows, nt, nullptr, tq, false, L->db, ndb, L->db_pm1, true, dist2, idx2);
       if (rc) break;

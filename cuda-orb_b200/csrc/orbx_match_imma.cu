@@ -455,7 +455,7 @@ __device__ __noinline__ bool m_scan(const ScanArgs sa, uint2* best) {
 
 __global__ void __launch_bounds__(kMThreads, 1)
     k_match_imma(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmD, MatchArgs a,
-                 MatchWork w, int slots, int* err) {
+                 MatchWork w, long long part_rows, int* err) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
@@ -471,12 +471,25 @@ __global__ void __launch_bounds__(kMThreads, 1)
   // for that row
   __shared__ uint32_t s_k2[2 * kMParts][kIBM];
 
+  // the split lives in shared memory: in registers it cost the scan spills (1500 x
+  // 262144: 78.0 against 72.8 us)
+  __shared__ MPlan plan;
+  __shared__ int slots;
+  __shared__ long long x_beg, x_end;
+
   chain_wait();
   const int nq = min(a.d_nq ? *a.d_nq : a.nq, w.nq_cap);
   const int ndb = a.d_ndb ? *a.d_ndb : a.ndb;
-  const MPlan plan = m_plan(nq, ndb, slots, (int)gridDim.x);
-  if ((int)blockIdx.x >= plan.grid) return;  // uniform over the block: before any barrier or TMEM use
-  const long long x_beg = m_start(plan, slots, blockIdx.x), x_end = m_start(plan, slots, blockIdx.x + 1);
+  if (threadIdx.x == 0) {
+    slots = m_slots(part_rows, nq);
+    plan = m_plan(nq, ndb, slots, (int)gridDim.x);
+    if ((int)blockIdx.x < plan.grid) {
+      x_beg = m_start(plan, slots, blockIdx.x);
+      x_end = m_start(plan, slots, blockIdx.x + 1);
+    }
+  }
+  __syncthreads();
+  if ((int)blockIdx.x >= plan.grid) return;  // uniform over the block: before any other barrier or TMEM use
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -691,7 +704,7 @@ __global__ void __launch_bounds__(kMThreads, 1)
       if (n_parts == 1)
         finish_query_shared(a, r.qb * kIBQ + e, m1, m2);
       else
-        reinterpret_cast<uint2*>(w.part)[(size_t)slot * w.nq_cap + r.qb * kIBQ + e] = make_uint2(m1, m2);
+        reinterpret_cast<uint2*>(w.part)[(size_t)slot * nq + r.qb * kIBQ + e] = make_uint2(m1, m2);
     }
     if (n_parts > 1) {
       // the block that finishes the last part of these queries merges all parts
@@ -713,7 +726,7 @@ __global__ void __launch_bounds__(kMThreads, 1)
             const uint2* pt = reinterpret_cast<const uint2*>(w.part) + qr;
 #pragma unroll 8
             for (int s2 = e / rows; s2 < n_parts; s2 += per) {
-              const uint2 pk = __ldcg(pt + (size_t)s2 * w.nq_cap);
+              const uint2 pk = __ldcg(pt + (size_t)s2 * nq);
               top2_push_shared(m1, m2, pk.x);
               top2_push_shared(m1, m2, pk.y);
             }
@@ -1298,13 +1311,6 @@ static bool make_rows_map(CUtensorMap* m, const void* base, uint64_t rows, uint3
 int imma_rows_q(int n) { return (n + kIBM - 1) / kIBM * kIBM; }
 int imma_rows_db(int n) { return (n + kMBN - 1) / kMBN * kMBN; }
 
-// Slots in which the parts of nq queries' searches fit when every SM has a block
-// (m_plan): up to max_slots.
-int imma_slots(int nq, int ndb, int max_slots) {
-  const MPlan p = m_plan(nq, ndb, 1 << 20, 148);
-  return std::max(1, std::min(max_slots, 148 / std::max(1, p.qtiles) + 1 + 2 * p.panels));
-}
-
 cudaError_t launch_expand_pm1(const uint8_t* bits, int n, const int* d_n, int rows, uint8_t* out, cudaStream_t s) {
   return launch_chained(k_expand_pm1, 4 * 148, 256, s, ExpandSet{bits, n, d_n, rows, out}, ExpandSet{},
                         static_cast<uint32_t*>(nullptr), 0);
@@ -1333,9 +1339,11 @@ cudaError_t launch_match_imma(const ImmaLaunch& L, cudaStream_t s) {
   CUtensorMap tq, td;
   if (!make_rows_map(&tq, L.q_pm1, (uint64_t)qrows, kIBM)) return cudaErrorInvalidValue;
   if (!make_rows_map(&td, L.db_pm1, (uint64_t)dbrows, kMBN)) return cudaErrorInvalidValue;
-  const int slots = L.work.part && L.work.tile_done ? L.slots : 1;
-  const int grid = m_plan(L.nq_cap, std::max(L.ndb_cap, 0), slots, 148).grid;
-  return launch_chained_smem(k_match_imma, grid, kMThreads, kISmemBytes, s, tq, td, L.args, L.work, slots, L.err);
+  const long long part_rows = L.work.part && L.work.tile_done ? L.part_rows : 0;
+  const MPlan plan = m_plan(L.nq_cap, std::max(L.ndb_cap, 0), m_slots(part_rows, L.nq_cap), kPlanGrid);
+  // counts on the device may be smaller than the capacities and spread over more blocks
+  const int grid = L.args.d_nq || L.args.d_ndb ? (int)std::min<long long>(plan.total, kPlanGrid) : plan.grid;
+  return launch_chained_smem(k_match_imma, grid, kMThreads, kISmemBytes, s, tq, td, L.args, L.work, part_rows, L.err);
 }
 
 cudaError_t launch_rerank_imma(const RerankImmaArgs& a, int max_items, cudaStream_t s) {

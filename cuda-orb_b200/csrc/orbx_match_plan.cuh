@@ -85,6 +85,22 @@ __host__ __device__ inline void m_slot(const MPlan& p, int slots, int qb, int t,
   *count = n;
 }
 
+// Merge scratch of searches of up to nq queries in up to ndb rows, in rows of one query's
+// best two.  A search of n queries takes `slots` of them each, by the count it finds on
+// the device, so few queries have as many slots as their parts on all SMs need, whatever
+// the scratch was sized for: 148 / qtiles + 1 + 2 * panels (m_plan) for each of n <= 256 *
+// qtiles.  32768 queries in 131072 rows: 1.1 MB (20 MB as 77 slots for every query).
+constexpr int kPlanGrid = 148;      // blocks of a launch: one per SM
+constexpr int kPlanMaxSlots = 152;  // every SM has a part of one block of queries
+__host__ __device__ inline long long m_part_rows(int nq, int ndb) {
+  const MPlan p = m_plan(nq, ndb, 1 << 20, kPlanGrid);
+  return (long long)kPlanQueries * (kPlanGrid + (long long)p.qtiles * (1 + 2 * p.panels));
+}
+__host__ __device__ inline int m_slots(long long part_rows, int nq) {
+  const long long s = nq > 0 ? part_rows / nq : 0;
+  return s < 1 ? 1 : s > kPlanMaxSlots ? kPlanMaxSlots : (int)s;
+}
+
 // Of n uses that went round a ring of k entries, those of entry i.  A block does not
 // exit before the last commit to each of its barriers has arrived: the arrival is a
 // write to its shared memory, which may belong to another block by then.
