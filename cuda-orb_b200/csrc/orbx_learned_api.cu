@@ -602,37 +602,63 @@ int train_mlp(orbx_learned* L, const uint8_t* d_train, int ntrain, const int* la
   return ORBX_OK;
 }
 
+// Pieces of one allocation, each on 256 bytes: laid out once without a base for the size.
+struct Carve {
+  uint8_t* base = nullptr;
+  size_t bytes = 0;
+  template <class T>
+  void take(T** p, size_t count) {
+    *p = base ? reinterpret_cast<T*>(base + bytes) : nullptr;
+    bytes += (std::max<size_t>(count, 1) * sizeof(T) + 255) / 256 * 256;
+  }
+};
+
+// The search's scratch, one allocation: the first search on an index pays for it
+// (32768 queries, 512 clusters: 0.8 ms, 2.4 ms as 20 allocations).
+void search_layout(orbx_learned* L, int nq, Carve& c) {
+  const int rows = round_up(nq, 128), C = L->C;
+  c.take(&L->xq, (size_t)rows * 256);
+  if (L->p.proposal == ORBX_PROPOSAL_MLP) {
+    c.take(&L->hq, (size_t)rows * L->Hd);
+    c.take(&L->keys, (size_t)rows * (C / 128) * kTopK);
+  } else {
+    c.take(&L->proj, (size_t)rows * 256);
+  }
+  c.take(&L->probes, (size_t)nq * kTopK);
+  c.take(&L->margin, (size_t)nq);
+  c.take(&L->counts, (size_t)C);
+  c.take(&L->offsets, (size_t)C + 1);
+  c.take(&L->cursor, (size_t)C);
+  c.take(&L->items, (size_t)C + 1);
+  c.take(&L->list, (size_t)nq * kTopK);
+  c.take(&L->partial, (size_t)nq * kTopK * kRrGroups);
+  c.take(&L->fb_list, (size_t)nq);
+  c.take(&L->fb_count, 1);
+  c.take(&L->rr_counter, 1);
+  c.take(&L->rr_bound, (size_t)nq);
+  c.take(&L->fb_q, (size_t)nq * 32);
+  c.take(&L->fb_d, (size_t)nq * 2);
+  c.take(&L->fb_i, (size_t)nq * 2);
+  c.take(&L->fb_pm1, (size_t)imma_rows_q(nq) * kPm1RowBytes);
+  ImmaWork& fb = L->fb_work;
+  fb = ImmaWork();
+  fb.part_rows = m_part_rows(nq, L->ndb);
+  fb.w.nq_cap = nq;
+  c.take(&fb.w.part, 2 * (size_t)fb.part_rows);
+  c.take(&fb.w.tile_done, (size_t)(nq + 127) / 128);
+  c.take(&fb.w.bound, (size_t)nq);
+}
+
 int ensure_search(orbx_learned* L, int nq) {
   if (L->nq_cap >= nq) return ORBX_OK;
   L->scratch.release();
   L->nq_cap = 0;
-  const int rows = round_up(nq, 128), C = L->C;
-  Arena& a = L->scratch;
-  LCHK(a.alloc(&L->xq, (size_t)rows * 256));
-  if (L->p.proposal == ORBX_PROPOSAL_MLP) {
-    LCHK(a.alloc(&L->hq, (size_t)rows * L->Hd));
-    LCHK(a.alloc(&L->keys, (size_t)rows * (C / 128) * kTopK));
-  } else {
-    LCHK(a.alloc(&L->proj, (size_t)rows * 256));
-  }
-  LCHK(a.alloc(&L->probes, (size_t)nq * kTopK));
-  LCHK(a.alloc(&L->margin, (size_t)nq));
-  LCHK(a.alloc(&L->counts, (size_t)C));
-  LCHK(a.alloc(&L->offsets, (size_t)C + 1));
-  LCHK(a.alloc(&L->cursor, (size_t)C));
-  LCHK(a.alloc(&L->items, (size_t)C + 1));
-  LCHK(a.alloc(&L->list, (size_t)nq * kTopK));
-  LCHK(a.alloc(&L->partial, (size_t)nq * kTopK * kRrGroups));
-  LCHK(a.alloc(&L->fb_list, (size_t)nq));
-  LCHK(a.alloc(&L->fb_count, 1));
-  LCHK(a.alloc(&L->rr_counter, 1));
-  LCHK(a.alloc(&L->rr_bound, (size_t)nq));
-  LCHK(a.alloc(&L->fb_q, (size_t)nq * 32));
-  LCHK(a.alloc(&L->fb_d, (size_t)nq * 2));
-  LCHK(a.alloc(&L->fb_i, (size_t)nq * 2));
-  LCHK(a.alloc(&L->fb_pm1, (size_t)imma_rows_q(nq) * kPm1RowBytes));
-  L->fb_work = ImmaWork();
-  LRC(imma_work_alloc(a, L->fb_work, nq, L->ndb, 0));
+  Carve size;
+  search_layout(L, nq, size);
+  Carve c;
+  LCHK(L->scratch.alloc(&c.base, size.bytes));
+  search_layout(L, nq, c);
+  LCHK(cudaMemsetAsync(L->fb_work.w.tile_done, 0, sizeof(unsigned) * ((size_t)(nq + 127) / 128), 0));
   LCHK(cudaDeviceSynchronize());
   L->nq_cap = nq;
   return ORBX_OK;
