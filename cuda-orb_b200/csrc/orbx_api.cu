@@ -2010,11 +2010,12 @@ ORBX_API int orbx_autotune_pairs_forms(orbx_ctx* c, int n_pairs, const orbx_imag
   orbx_tuning top5 = keep;  // best of the five-launch form, for the tile-shape pass
   float top5_ms = 1e30f;
   int rc = ORBX_OK;
-  // median of `reps` replays of one candidate (the first call captures its graph)
+  // median of `reps` replays of one candidate (its second call captures its graph)
   auto measure = [&](const orbx_tuning& t, float* out) -> int {
     int r;
     if ((r = orbx_set_tuning(c, &t)) != 0) return r;
-    if ((r = orbx_batch_pairs(c, n_pairs, ia, ib, oa, ob, ORBX_MATCH_POPC)) != 0) return r;
+    for (int k = 0; k < 2; k++)
+      if ((r = orbx_batch_pairs(c, n_pairs, ia, ib, oa, ob, ORBX_MATCH_POPC)) != 0) return r;
     std::vector<float> ms;
     for (int k = 0; k < reps; k++) {
       cudaEventRecord(e0, c->stream);

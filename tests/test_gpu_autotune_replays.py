@@ -1,0 +1,34 @@
+"""The autotuner times replays: with a single repetition its time is that of the calls a
+program then makes, not of the call that captures the graph."""
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import orbx  # noqa: E402
+import synth  # noqa: E402
+
+
+def test_one_repetition_is_a_replay():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    stream = torch.cuda.Stream()
+    ctx = orbx.Context(0, orbx.make_params(max_pts=1000), stream=stream)
+    a, b, _ = synth.make_pair(320, 240, seed=50)
+    pb = orbx.PairBatch([(a, b, 320, 240, 1000)])
+    torch.cuda.synchronize()
+    times = sorted(ctx.autotune_pairs(pb, reps=1)[1] for _ in range(5))
+    for _ in range(3):
+        ctx.batch_pairs(pb)
+    ctx.sync()
+    ms = []
+    for _ in range(21):
+        e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        e0.record(stream)
+        ctx.batch_pairs(pb)
+        e1.record(stream)
+        e1.synchronize()
+        ms.append(e0.elapsed_time(e1))
+    # a call that captures took 68 us here, a replay 41
+    assert times[2] < 1.25 * sorted(ms)[10], (times, sorted(ms))
+    ctx.close()
