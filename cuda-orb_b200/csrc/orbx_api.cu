@@ -412,10 +412,8 @@ static void set_nms_shape(Frame& F, int border, int rows_req) {
 // 640x480 29.7 / 30.8, pair 320x240 36.1 / 37.4, pair 1920x1080 69.0 / 70.5,
 // frame 3839x2157 80.3 / 82.7, batch of 24 pairs (147 Mpixel) 1454 / 1355.
 static constexpr long long kPyrTallPx = 24ll << 20;
-static int pyr_shape_for(const orbx_ctx* c, long long px) {
-  if (c->pyr_shape) return c->pyr_shape;
-  return px < kPyrTallPx ? 1 : 0;
-}
+static int pyr_shape_auto(long long px) { return px < kPyrTallPx ? 1 : 0; }
+static int pyr_shape_for(const orbx_ctx* c, long long px) { return c->pyr_shape ? c->pyr_shape : pyr_shape_auto(px); }
 
 static void fill_frame(const orbx_ctx* c, const Workspace& ws, const uint8_t* img, int pitch_in, orbx_point* pts,
                        uint8_t* desc, int* count, Frame& F, int max_pts = -1, int pyr_shape = 0) {
@@ -2042,10 +2040,13 @@ ORBX_API int orbx_autotune_pairs_forms(orbx_ctx* c, int n_pairs, const orbx_imag
       top5 = t;
     }
   }
-  // second pass: the pyramid tile shapes on the best five-launch candidate
+  // second pass: the other pyramid tile heights on the best five-launch candidate
   if (forms & 1) {
-    for (int shape = 0; shape < kPyrShapes; shape++) {
-      if (shape == top5.pyr_tile) continue;
+    long long px = 0;
+    for (int i = 0; i < n_pairs; i++) px += (long long)ia[i].w * ia[i].h + (long long)ib[i].w * ib[i].h;
+    const int measured = kPyrShapeTH[top5.pyr_tile ? top5.pyr_tile : pyr_shape_auto(px)];
+    for (int shape = 1; shape < kPyrShapes; shape++) {  // 0 stands for one of them
+      if (kPyrShapeTH[shape] == measured) continue;
       orbx_tuning t = top5;
       t.pyr_tile = shape;
       float med = 0.f;

@@ -32,3 +32,20 @@ def test_one_repetition_is_a_replay():
     # a call that captures took 68 us here, a replay 41
     assert times[2] < 1.25 * sorted(ms)[10], (times, sorted(ms))
     ctx.close()
+
+
+def test_the_measured_tile_height_is_not_timed_again():
+    """The automatic height of a small batch is 26 rows (shape 1): trying it under its
+    own number would let noise decide between equals."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    ctx = orbx.Context(0, orbx.make_params(max_pts=1000))
+    a, b, _ = synth.make_pair(320, 240, seed=50)
+    pb = orbx.PairBatch([(a, b, 320, 240, 1000)])
+    torch.cuda.synchronize()
+    for _ in range(8):
+        t, _ = ctx.autotune_pairs_forms(pb, 1, reps=1)
+        assert t.pyr_tile in (0, 2, 3)
+        t.pyr_tile = 0
+        ctx.set_tuning(t)
+    ctx.close()
