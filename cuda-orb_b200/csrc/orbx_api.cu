@@ -832,9 +832,11 @@ ORBX_API int orbx_destroy(orbx_ctx* c) {
     if (bs->uploaded) cudaEventDestroy(bs->uploaded);
   }
   for (PairGraph* pg : {&c->ppg, &c->pho, &c->phs, &c->bg}) pg->drop();
-  cudaFree(c->mw.part);
-  cudaFree(c->mw.tile_done);
-  cudaFree(c->mw.bound);
+  for (MatchWork* mw : {&c->mw, &c->hmw, &c->ppg.mw, &c->pho.mw}) {
+    cudaFree(mw->part);
+    cudaFree(mw->tile_done);
+    cudaFree(mw->bound);
+  }
   for (int i = 0; i < 2; i++) {
     cudaFree(c->io_img[i]);
     cudaFree(c->io_pts[i]);
@@ -855,15 +857,9 @@ ORBX_API int orbx_destroy(orbx_ctx* c) {
   persist_free(c->ppair);
   for (uint8_t* t : c->captured_tables) cudaFree(t);
   for (PersistBufs& pb : c->captured_persist) persist_free(pb);
-  cudaFree(c->pho.mw.part);
-  cudaFree(c->pho.mw.tile_done);
-  cudaFree(c->pho.mw.bound);
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
-  cudaFree(c->hmw.part);
-  cudaFree(c->hmw.tile_done);
-  cudaFree(c->hmw.bound);
   if (c->ev_reset) cudaEventDestroy(c->ev_reset);
   cudaFree(c->d_pattern);
   cudaFree(c->d_umax);
