@@ -1828,6 +1828,7 @@ static int batch_pairs_impl(orbx_ctx* c, int n_pairs, const orbx_image* ia, cons
   DeviceGuard g(c->device);
   if ((int)c->bws.size() < 2 * n_pairs) c->bws.resize(2 * n_pairs);
   std::vector<Frame> frames(2 * n_pairs);
+  const bool persistent = c->batch_form == 1 && !stage_ms;
   long long px = 0;
   bool ready = true;
   for (int i = 0; i < n_pairs; i++) {
@@ -1843,7 +1844,7 @@ static int batch_pairs_impl(orbx_ctx* c, int n_pairs, const orbx_image* ia, cons
       Workspace& ws = c->bws[2 * i + s];
       if ((rc = ws_ensure(c, ws, im.w, im.h)) != 0) return rc;
       fill_frame(c, ws, im.data, im.pitch, o.points, o.desc, o.num_pts, frames[2 * i + s], o.max_pts,
-                 (c->batch_form == 1 && !stage_ms) ? 0 : pyr_shape_for(c, px));
+                 persistent ? 0 : pyr_shape_for(c, px));
     }
   }
   // matching jobs, one per pair, with their own slices of the split scratch
@@ -1896,8 +1897,9 @@ static int batch_pairs_impl(orbx_ctx* c, int n_pairs, const orbx_image* ia, cons
   blocks_per_pair = std::max(blocks_per_pair, max_tiles);  // every query tile needs a block
   LaunchPlan pl;
   const MatchJob* d_jobs = nullptr;
-  if ((rc = upload_batch(c, c->batch, frames, &pl, true, &jobs, &d_jobs)) != 0) return rc;
-  if (c->batch_form == 1 && !stage_ms) return batch_persistent(c, pl, frames, jobs, blocks_per_pair);
+  if ((rc = upload_batch(c, c->batch, frames, &pl, true, persistent ? nullptr : &jobs, &d_jobs)) != 0)
+    return rc;  // the persistent form brings its own job table
+  if (persistent) return batch_persistent(c, pl, frames, jobs, blocks_per_pair);
   if (stage_ms) {
     // profiling: the same launches with events between them
     for (auto& e : c->prof_ev)
