@@ -408,10 +408,13 @@ static void set_nms_shape(Frame& F, int border, int rows_req) {
 
 // Pyramid tile of a launch over frames of `px` level-0 pixels in all.  Tall tiles
 // repeat fewer halo rows (10% against 23% of the row filters) but leave SMs idle
-// in the last wave of their blocks.  26 against 58 rows, us per call: frame
-// 640x480 29.7 / 30.8, pair 320x240 36.1 / 37.4, pair 1920x1080 69.0 / 70.5,
-// frame 3839x2157 80.3 / 82.7, batch of 24 pairs (147 Mpixel) 1454 / 1355.
-static constexpr long long kPyrTallPx = 24ll << 20;
+// in the last wave of their blocks.  From the line on no launch measured is slower
+// with them.  26 against 58 rows, us per call (Mpixel of 2^20): frame 3840x2160 (7.9)
+// 87.8 / 90.3, pair 2560x1440 (7.0) 103.6 / 106.2, pair 3840x2160 (15.8) 192.9 /
+// 192.7, frame 8192x2400 (18.8) 188.0 / 186.0, 3 pairs 2560x1440 (21.1) 268.1 / 257.6,
+// 2 pairs 3840x2160 (31.6) 391.4 / 375.4, 8 of them (126.6) 1445 / 1361.  Batches of
+// small frames gain earlier (12 pairs 640x480, 7.0: 170.6 / 165.6).
+static constexpr long long kPyrTallPx = 16ll << 20;
 static int pyr_shape_auto(long long px) { return px < kPyrTallPx ? 1 : 0; }
 static int pyr_shape_for(const orbx_ctx* c, long long px) { return c->pyr_shape ? c->pyr_shape : pyr_shape_auto(px); }
 
