@@ -234,7 +234,7 @@ typedef struct orbx_tuning {
   int match_blocks_per_pair;  /* grid per pair of the batched matcher, 0 = automatic */
   int batch_form;             /* orbx_batch_pairs: 0 = five graph-replayed launches, 1 = one persistent launch */
   int persist_group;          /* persistent form: frames per wave of the work order (even), 0 = all frames */
-  int persist_blocks_per_sm;  /* persistent form: resident blocks per SM, 0 = the occupancy limit */
+  int persist_blocks_per_sm;  /* persistent form: resident blocks per SM, 0 = as many as fit and have work */
   int wait_timeout_us;        /* bound of every device-side wait, 1 .. 10,000,000 us (default 1,000,000) */
   int upload_bands;           /* orbx_pair_host: 0 = copy both images, then run the pair; 1..16 = copy them in
                                  this many row bands per image on a second stream while one persistent launch

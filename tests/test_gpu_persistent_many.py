@@ -34,3 +34,38 @@ def test_every_query_is_matched(form):
     got = run(4, 0) if form == "upload_bands" else run(0, 1)
     assert all(np.array_equal(g, e) for g, e in zip(got, want))
     ctx.close()
+
+
+@pytest.mark.parametrize("w,h", [(160, 120), (320, 240)])
+def test_small_pairs_take_few_blocks(w, h):
+    """The automatic number of resident blocks is about as fast as the best number, and
+    every number gives the same results."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import synth
+    a, b, _ = synth.make_pair(w, h, seed=3)
+    da, db = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    times, results = [], []
+    for bps in (0, 1, 2, 4):
+        ctx = orbx.Context(0, orbx.make_params(max_pts=5000), stream=stream)
+        t = ctx.get_tuning()
+        t.pair_form, t.persist_blocks_per_sm = 1, bps
+        ctx.set_tuning(t)
+        A, B = orbx.FrameBuffers(5000), orbx.FrameBuffers(5000)
+        ms = []
+        for _ in range(30):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record(stream)
+            for _ in range(8):
+                ctx.pair_ptr(da, db, w, h, a.shape[1], A.points, A.desc, A.count, B.points, B.desc, B.count)
+            e1.record(stream)
+            e1.synchronize()
+            ms.append(e0.elapsed_time(e1))
+        times.append(sorted(ms)[15])
+        results.append(A.to_host() + B.to_host())
+        ctx.close()
+    for r in results[1:]:
+        assert all(np.array_equal(x, y) for x, y in zip(r, results[0]))
+    assert times[0] < 1.2 * min(times[1:]), times
