@@ -34,8 +34,8 @@
 // and blocks, and cheap by tournaments over column groups.  A chunk is what the
 // registers hold: each costs a round trip to TMEM (40 columns: 563 us).  More, shorter
 // accumulators or more epilogue warps were slower (3 x 160 columns 685 against 646 us,
-// 24 warps 767: each step costs every warp about 700 cycles).  65536 x 65536: 785 ->
-// 532 us; 1500 x 262144: 95 -> 73 us.
+// 24 warps 767: each step costs every warp about 700 cycles).  From int8 values to
+// this form: 65536 x 65536 785 -> 532 us, 1500 x 262144 95 -> 73 us.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -455,7 +455,7 @@ __device__ __noinline__ bool m_scan(const ScanArgs sa, uint2* best) {
 
 __global__ void __launch_bounds__(kMThreads, 1)
     k_match_imma(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmD, MatchArgs a,
-                 MatchWork w, long long part_rows, int* err) {
+                 MatchWork w, unsigned part_rows, int* err) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(kMThreads, 1)
   // for that row
   __shared__ uint32_t s_k2[2 * kMParts][kIBM];
 
-  // the split lives in shared memory: in registers it cost the scan spills (1500 x
+  // the split, for the roles: in registers to the end it cost the scan spills (1500 x
   // 262144: 78.0 against 72.8 us)
   __shared__ MPlan plan;
   __shared__ int slots;
@@ -480,16 +480,17 @@ __global__ void __launch_bounds__(kMThreads, 1)
   chain_wait();
   const int nq = min(a.d_nq ? *a.d_nq : a.nq, w.nq_cap);
   const int ndb = a.d_ndb ? *a.d_ndb : a.ndb;
-  if (threadIdx.x == 0) {
-    slots = m_slots(part_rows, nq);
-    plan = m_plan(nq, ndb, slots, (int)gridDim.x);
-    if ((int)blockIdx.x < plan.grid) {
-      x_beg = m_start(plan, slots, blockIdx.x);
-      x_end = m_start(plan, slots, blockIdx.x + 1);
+  {
+    const int sl = m_slots(part_rows, nq);
+    const MPlan p = m_plan(nq, ndb, sl, (int)gridDim.x);
+    if ((int)blockIdx.x >= p.grid) return;  // uniform over the block: before any barrier or TMEM use
+    if (threadIdx.x == 0) {
+      plan = p;
+      slots = sl;
     }
+    if ((threadIdx.x & ~32u) == 0)
+      *(threadIdx.x ? &x_end : &x_beg) = m_start(p, sl, blockIdx.x + (threadIdx.x ? 1 : 0));
   }
-  __syncthreads();
-  if ((int)blockIdx.x >= plan.grid) return;  // uniform over the block: before any other barrier or TMEM use
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -1339,7 +1340,8 @@ cudaError_t launch_match_imma(const ImmaLaunch& L, cudaStream_t s) {
   CUtensorMap tq, td;
   if (!make_rows_map(&tq, L.q_pm1, (uint64_t)qrows, kIBM)) return cudaErrorInvalidValue;
   if (!make_rows_map(&td, L.db_pm1, (uint64_t)dbrows, kMBN)) return cudaErrorInvalidValue;
-  const long long part_rows = L.work.part && L.work.tile_done ? L.part_rows : 0;
+  const unsigned part_rows =
+      L.work.part && L.work.tile_done ? (unsigned)std::min<long long>(L.part_rows, 0xFFFFFFFFll) : 0u;
   const MPlan plan = m_plan(L.nq_cap, std::max(L.ndb_cap, 0), m_slots(part_rows, L.nq_cap), kPlanGrid);
   // counts on the device may be smaller than the capacities and spread over more blocks
   const int grid = L.args.d_nq || L.args.d_ndb ? (int)std::min<long long>(plan.total, kPlanGrid) : plan.grid;

@@ -97,7 +97,8 @@ __host__ __device__ inline long long m_part_rows(int nq, int ndb) {
   return (long long)kPlanQueries * (kPlanGrid + (long long)p.qtiles * (1 + 2 * p.panels));
 }
 __host__ __device__ inline int m_slots(long long part_rows, int nq) {
-  const long long s = nq > 0 ? part_rows / nq : 0;
+  // (the kernel's part_rows has 32 bits, and so has its division)
+  const long long s = nq <= 0 ? 0 : part_rows >> 32 ? part_rows / nq : (long long)((unsigned)part_rows / (unsigned)nq);
   return s < 1 ? 1 : s > kPlanMaxSlots ? kPlanMaxSlots : (int)s;
 }
 
