@@ -51,7 +51,7 @@ struct BatchSlot {
 };
 
 // A launch sequence with the parameters baked into it as `key`.  Capturing and
-// instantiating a graph costs the host 60 to 100 us, more than issuing its
+// instantiating a graph costs the host 30 to 100 us, more than issuing its
 // launches (about 3 us each), and pays only when the same buffers come again:
 // a call whose key is not the previous call's is issued launch by launch, the
 // next call with the same key captures the graph, and later ones replay it.
@@ -1019,12 +1019,14 @@ static int imma_ensure(orbx_ctx* c, int nq_cap, int ndb_cap) {
   return ORBX_OK;
 }
 
-// AUTO picks the tensor-core form once the pair count pays for its expansion pass
-// and fixed cost.  At 2^24 pairs it takes 16.5 to 27 us (128 x 131072 to 65536 x 256)
-// against 28 to 58 for the popcount form, at 2^23 14 to 19 against 17 to 32, at 2^22 14
-// to 16 against 11 to 19.  The line is above the crossing because what is compared may
-// be capacities, with fewer rows counted on the device, and because the form's scratch
-// is allocated at the first call that takes it.
+// AUTO picks the tensor-core form from the pair count at which every shape measured is
+// faster with it than with the popcount form (us, 128 x 131072 / 512 x 32768 / 2048 x
+// 8192 / 8192 x 2048 / 32768 x 512): 27.6 / 20.8 / 17.3 / 20.0 / 22.7 against 58.2 /
+// 32.5 / 28.9 / 30.9 / 29.2 at 2^24 pairs.  At 2^23 32768 x 256 still loses (19.8
+// against 16.3), the others take 14.6 to 19.7 against 17.6 to 32.5; at 2^22 only 128
+// queries gain.  For orbx_match what is compared are the capacities: at a cap of 10000
+// it takes the tensor-core form however few rows are counted (1100 x 1100: 14.4 against
+// 8.6; 4000 x 4000: 18.1 against 30.3).
 static int resolve_mode(int mode, long long nq, long long ndb) {
   if (mode == ORBX_MATCH_AUTO) return (nq * ndb >= (1ll << 24) && nq >= 128) ? ORBX_MATCH_IMMA : ORBX_MATCH_POPC;
   return mode;
@@ -1329,9 +1331,10 @@ static int pair_host_streams_enqueue(orbx_ctx* c, const uint8_t* h_a, const uint
 // processed on the context's stream while image B is copied, then processed,
 // on the copy stream; matching and the export follow on the context's stream
 // once both are done.  The same five kernels per frame as orbx_pair.  When
-// both images are in pinned memory the sequence is captured once into a CUDA
-// graph (keyed on the images' addresses and every launch parameter) and
-// replayed, which removes the gaps between ten separately issued launches.
+// both images are in pinned memory, a call whose launch parameters are the previous
+// call's captures the sequence into a CUDA graph, and later ones replay it, which
+// removes the gaps between ten separately issued launches.  The images' addresses are
+// not among those parameters: they are set in the graph's two copy nodes.
 static int pair_host_streams(orbx_ctx* c, const uint8_t* h_a, const uint8_t* h_b, int w, int h, int pitch,
                              bool with_desc, const uint8_t** res, cudaEvent_t ev_uploaded = nullptr) {
   int rc;
@@ -1490,7 +1493,7 @@ static int pair_host_impl(orbx_ctx* c, const uint8_t* h_img_a, const uint8_t* h_
       return rc;
     }
     if (prof) {
-      // the uploads end on the copy stream; kernels and export are one graph
+      // the uploads end on the copy stream; kernels and export follow each other
       ORBX_CUDA(cudaEventRecord(prof->ev[1], c->copy_stream));
       ORBX_CUDA(cudaEventRecord(prof->ev[2], c->stream));
       ORBX_CUDA(cudaEventRecord(prof->ev[3], c->stream));

@@ -222,7 +222,7 @@ struct RerankImmaArgs {
   const int* item_offsets;   // [C + 1] exclusive scan of ceil(slots / 128)
   int n_clusters;
   const int* ivf_offsets;    // [C + 1] list offsets: the cluster's row count
-  const int* pad_offsets;    // [C + 1] the cluster's first padded row (multiples of 256)
+  const int* pad_offsets;    // [C + 1] the cluster's first padded row (multiples of 240)
   const int* pad_members;    // [pad_rows] database index of each padded row, -1 in the padding
   const uint8_t* pad_desc;   // [pad_rows][32] packed rows of the padded lists (padding zero), 16-byte aligned
   uint2* partial;            // [slots][kRrGroups] top-2 keys

@@ -71,7 +71,8 @@ __device__ __forceinline__ int find_frame_in(const int* base, int n, int t) {
 // of blocks its instruction fetch is part of the time.  For a 1920x1080 pair the
 // form before, which staged bytes and floats of a 128 x 30 tile in shared memory
 // and filtered every row by itself, took 9.09 M warp instructions; this one
-// takes 5.6 M with 58 rows.  24 mixed pairs (147 Mpixel): 558 -> 305 us.
+// takes 7.09 M with the pair's 26-row tiles (5.6 M with 58 rows).  24 mixed pairs
+// (147 Mpixel, 58 rows): 558 -> 305 us.
 // ---------------------------------------------------------------------------
 
 // Exact small-integer <-> float conversions on the full-rate pipes: a float
@@ -403,12 +404,12 @@ __device__ __forceinline__ void pyr_tile(const Batch& b, int t, PyrSmem<TH>& sm)
 // as in the reference, merges the octaves in shared memory, and writes the
 // tile's occupancy bits densely and its scores sparsely (no clearing pass).
 //
-// What bounds it: instruction issue (ALU pipe 56%, issue 60% of active cycles)
+// What bounds it: instruction issue (ALU pipe 50%, issue 60% of active cycles)
 // and, on one frame, the latency of its five phases.  Staging is one 16-byte load
 // per thread for octave 0 and one for the others together; the pre-test compares
 // two centres per instruction in 16-bit lanes; a Harris lane shares the column
 // sums and differences of its three rows between its seven columns.  A
-// 1920x1080 pair takes 10.1 M warp instructions (12.6 M with 4-byte staging,
+// 1920x1080 pair takes 9.44 M warp instructions (11.9 M with 4-byte staging,
 // byte-compare pre-test and per-column derivatives), 24 mixed pairs 442 us (541).
 // ---------------------------------------------------------------------------
 constexpr int kHalo = 4;  // rows above and below, and the least columns to the sides

@@ -203,7 +203,7 @@ ORBX_API int orbx_ocv_detect_and_compute(orbx_ctx* ctx, const orbx_ocv_params* p
                                          int pitch, orbx_ocv_keypoint* d_keypoints, uint8_t* d_desc, int* d_n,
                                          int cap);
 
-/* Profiling variant of orbx_pair: the same launches without the graph, with a
+/* Profiling variant of orbx_pair: the five launches, with a
  * CUDA event between consecutive kernels; writes the milliseconds of the
  * pyramid/blur, detect, NMS, describe and match kernels to stage_ms[0..4].
  * Synchronises the stream. */
@@ -232,7 +232,8 @@ typedef struct orbx_tuning {
   int describe_blocks_per_sm; /* grid of the orientation + descriptor kernel */
   int match_blocks_per_sm;    /* grid of the popcount matcher (counts on the device), in blocks of 256 threads */
   int match_blocks_per_pair;  /* grid per pair of the batched matcher, 0 = automatic */
-  int batch_form;             /* orbx_batch_pairs: 0 = five graph-replayed launches, 1 = one persistent launch */
+  int batch_form;             /* orbx_batch_pairs: 0 = five launches, 1 = one persistent launch (either
+                                 replayed from a graph when calls repeat their shapes) */
   int persist_group;          /* persistent form: frames per wave of the work order (even), 0 = all frames */
   int persist_blocks_per_sm;  /* persistent form: resident blocks per SM, 0 = as many as fit and have work */
   int wait_timeout_us;        /* bound of every device-side wait, 1 .. 10,000,000 us (default 1,000,000) */
