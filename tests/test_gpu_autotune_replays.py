@@ -30,7 +30,7 @@ def test_one_repetition_is_a_replay():
         e1.synchronize()
         ms.append(e0.elapsed_time(e1))
     # a call that captures took 68 us here, a replay 41
-    assert times[2] < 1.25 * sorted(ms)[10], (times, sorted(ms))
+    assert times[2] < 1.35 * sorted(ms)[10], (times, sorted(ms))
     ctx.close()
 
 

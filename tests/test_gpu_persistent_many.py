@@ -68,4 +68,4 @@ def test_small_pairs_take_few_blocks(w, h):
         ctx.close()
     for r in results[1:]:
         assert all(np.array_equal(x, y) for x, y in zip(r, results[0]))
-    assert times[0] < 1.2 * min(times[1:]), times
+    assert times[0] < 1.3 * min(times[1:]), times  # 1.4 at 320x240 with every block resident, 1.0 as it is
